@@ -392,7 +392,7 @@ bool run_gemm(const GemmReq& q) {
     return false;
   }
   const bool row = is_row(q.order), ta = !is_nt(q.ta), tb = !is_nt(q.tb);
-  GemmArgs g{};
+  XGemmArgs<double> g{};
   g.M = q.M;
   g.N = q.N;
   g.K = (q.alpha == 0.0) ? 0 : q.K;   // dbdgemm.ccog:78-80
@@ -405,8 +405,9 @@ bool run_gemm(const GemmReq& q) {
     g.sbk = tb ? q.ldb : 1;  g.sbj = tb ? 1 : q.ldb;
     g.sci = 1;               g.scj = q.ldc;
   }
-  g.alpha = q.alpha;
-  g.beta = q.beta;
+  g.ar = q.alpha;
+  g.alpha_one = q.alpha == 1.0;
+  g.br = q.beta;
   g.mode = q.mode;
   if (q.mode == kOutBinned && g.K == 0) return true;   // binnedBLAS_dbdgemm touches nothing
   if (!o) {
@@ -442,8 +443,10 @@ bool run_gemm(const GemmReq& q) {
   if (!ok) return false;
   g.C = q.mode == kOutValue ? dC : nullptr;
   g.Cbin = q.mode == kOutBinned ? dC : nullptr;
+  GemmPlan plan;
+  if (!gemm_decompose(o->gemm_plan, w, g.M, g.N, g.K, &plan)) return false;
   count_launch();
-  if (!cuda_ok(o->gemm(g, s, nullptr, nullptr), "gemm launch")) return false;
+  if (!cuda_ok(o->gemm(g, plan, s), "gemm launch")) return false;
   if (c_host) {
     if (!cuda_ok(cudaMemcpyAsync(q.C, dC, c_bytes, cudaMemcpyDeviceToHost, s), "copy C") ||
         !cuda_ok(cudaStreamSynchronize(s), "cudaStreamSynchronize"))

@@ -329,8 +329,10 @@ bool run_xgemm(const XGemmReq<E, CX>& q) {
   if (!ok) return false;
   g.C = q.mode == kOutValue ? dC : nullptr;
   g.Cbin = q.mode == kOutBinned ? dC : nullptr;
+  GemmPlan plan;
+  if (!gemm_decompose(o->gemm_plan, w, g.M, g.N, g.K, &plan)) return false;
   count_launch();
-  if (!cuda_ok(o->gemm(g, s), "gemm launch")) return false;
+  if (!cuda_ok(o->gemm(g, plan, s), "gemm launch")) return false;
   if (c_host) {
     if (!cuda_ok(cudaMemcpyAsync(q.C, dC, c_bytes, cudaMemcpyDeviceToHost, s), "copy C") ||
         !cuda_ok(cudaStreamSynchronize(s), "cudaStreamSynchronize"))

@@ -20,7 +20,7 @@
 #include <vector>
 
 #include "rb_blas1_impl.cuh"
-#include "rb_blas23_impl.cuh"
+#include "rb_gemm_tile.cuh"
 #include "rb_host.h"
 #include "../../include/reproblas_b200.h"
 
@@ -56,7 +56,7 @@ struct Args {
   double* states;         // [nseg * 2F] or null
   double* records;        // chunk records
   unsigned* tickets;      // [nseg]
-  const GemmArgs* gemms;
+  const XGemmArgs<double>* gemms;
   unsigned* counters;     // [0] next item, [1] CTAs finished
 };
 
@@ -185,10 +185,11 @@ __device__ __forceinline__ void cta_chunk(const Args& a, const Item& it, double*
 }
 
 template <int F, int TM, int TN>
-__global__ void __launch_bounds__(256) batched_kernel(Args a) {
+__global__ void __launch_bounds__(256, 2) batched_kernel(Args a) {
   __shared__ int s_item;
   __shared__ double smem[32 * (2 * F + 2)];
-  using Cfg = GemmCfg<F, TM, TN>;
+  extern __shared__ __align__(16) unsigned char tile_smem[];
+  using Tile = gt::Tile<double, false, F, TM, TN>;
 #pragma unroll 1
   for (;;) {
     if (threadIdx.x == 0) s_item = (int)atomicAdd(a.counters, 1u);
@@ -197,7 +198,13 @@ __global__ void __launch_bounds__(256) batched_kernel(Args a) {
     if (id >= a.nitems) break;
     const Item it = a.items[id];
     if (it.type == kItemTile) {
-      gemm_tile<F, TM, TN>(a.gemms[it.a], (long long)it.b * Cfg::BM, (long long)it.c * Cfg::BN);
+      const XGemmArgs<double> g = a.gemms[it.a];
+      const long long m0 = (long long)it.b * Tile::BM, n0 = (long long)it.c * Tile::BN;
+      Tile t;
+      t.attach(tile_smem);
+      t.zero(g, m0, n0);
+      t.reduce(g, m0, n0, 0, g.K > 0 ? (g.K + Tile::BK - 1) / Tile::BK : 1);
+      t.finish(g, m0, n0, nullptr, 0, 0, 0, [](long long) { return 0ll; });
     } else if (it.type == kItemSmall) {
       const int w = threadIdx.x >> 5;
       if (w < it.b) warp_segment<F>(a, a.small[it.a + w]);
@@ -233,15 +240,27 @@ __host__ __device__ constexpr int tile_tn(int t) {
   return t == 2 ? 4 : (t == 0 || t == 4 ? 1 : 2);
 }
 
+// dynamic shared memory of the kernel of a tile shape: the dgemm tile's stages and carries
+template <int F>
+size_t batched_smem(int tile) {
+  switch (tile) {
+    case 0: return gt::Geo<double, false, F, 1, 1>::SMEM;
+    case 1: return gt::Geo<double, false, F, 2, 2>::SMEM;
+    case 3: return gt::Geo<double, false, F, 1, 2>::SMEM;
+    case 4: return gt::Geo<double, false, F, 2, 1>::SMEM;
+    default: return gt::Geo<double, false, F, 2, 4>::SMEM;
+  }
+}
+
 template <int F>
 cudaError_t launch_batched(int tile, dim3 grid, const Args& a, cudaStream_t s) {
   switch (tile) {
-    case 0: batched_kernel<F, 1, 1><<<grid, 256, 0, s>>>(a); break;
-    case 1: batched_kernel<F, 2, 2><<<grid, 256, 0, s>>>(a); break;
-    case 3: batched_kernel<F, 1, 2><<<grid, 256, 0, s>>>(a); break;
-    case 4: batched_kernel<F, 2, 1><<<grid, 256, 0, s>>>(a); break;
+    case 0: batched_kernel<F, 1, 1><<<grid, 256, batched_smem<F>(tile), s>>>(a); break;
+    case 1: batched_kernel<F, 2, 2><<<grid, 256, batched_smem<F>(tile), s>>>(a); break;
+    case 3: batched_kernel<F, 1, 2><<<grid, 256, batched_smem<F>(tile), s>>>(a); break;
+    case 4: batched_kernel<F, 2, 1><<<grid, 256, batched_smem<F>(tile), s>>>(a); break;
     default:
-      if constexpr (F <= 3) batched_kernel<F, 2, 4><<<grid, 256, 0, s>>>(a);
+      if constexpr (F <= 3) batched_kernel<F, 2, 4><<<grid, 256, batched_smem<F>(tile), s>>>(a);
       else return cudaErrorInvalidValue;
       break;
   }
@@ -276,7 +295,7 @@ struct rb_batch_plan {
   const double* Y = nullptr;
   double* results = nullptr;
   double* states = nullptr;
-  std::vector<rb::GemmArgs> gemms;
+  std::vector<rb::XGemmArgs<double>> gemms;
   std::vector<std::pair<double*, size_t>> c_extents;   // device C regions (pointer, bytes)
   // configuration
   int tile = 1;
@@ -290,7 +309,7 @@ struct rb_batch_plan {
   int* d_small = nullptr;
   double* d_records = nullptr;
   unsigned* d_tickets = nullptr;
-  rb::GemmArgs* d_gemms = nullptr;
+  rb::XGemmArgs<double>* d_gemms = nullptr;
   unsigned* d_counters = nullptr;
   int grid = 1;
   bool built = false;
@@ -368,7 +387,7 @@ bool build_config(rb_batch_plan* p) {
   }
   const int bm = tile_bm(p->tile), bn = tile_bn(p->tile);
   for (size_t g = 0; g < p->gemms.size(); g++) {
-    const GemmArgs& ga = p->gemms[g];
+    const XGemmArgs<double>& ga = p->gemms[g];
     for (long long i = 0; i < (ga.M + bm - 1) / bm; i++)
       for (long long j = 0; j < (ga.N + bn - 1) / bn; j++) {
         Item it{};
@@ -421,7 +440,11 @@ bool build_config(rb_batch_plan* p) {
   int occ = 1;
   const void* k = p->fold == 2 ? bt::batched_ptr<2>(p->tile)
                                : (p->fold == 3 ? bt::batched_ptr<3>(p->tile) : bt::batched_ptr<4>(p->tile));
-  if (!k || cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k, 256, 0) != cudaSuccess) {
+  const size_t smem = p->fold == 2 ? bt::batched_smem<2>(p->tile)
+                                   : (p->fold == 3 ? bt::batched_smem<3>(p->tile) : bt::batched_smem<4>(p->tile));
+  if (!k ||
+      cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess ||
+      cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k, 256, smem) != cudaSuccess) {
     cudaGetLastError();
     occ = 1;
   }
@@ -526,7 +549,7 @@ rb_batch_plan* rb_batch_plan_create(const int fold, const int nseg, const long l
     }
     const bool row = d.order == 'r' || d.order == 'R';
     const bool ta = !(d.transa == 'n' || d.transa == 'N'), tb = !(d.transb == 'n' || d.transb == 'N');
-    GemmArgs g{};
+    XGemmArgs<double> g{};
     g.M = d.m; g.N = d.n; g.K = d.alpha == 0.0 ? 0 : d.k;
     if (row) {
       g.sai = ta ? 1 : d.lda; g.sak = ta ? d.lda : 1;
@@ -537,13 +560,13 @@ rb_batch_plan* rb_batch_plan_create(const int fold, const int nseg, const long l
       g.sbk = tb ? d.ldb : 1; g.sbj = tb ? 1 : d.ldb;
       g.sci = 1; g.scj = d.ldc;
     }
-    g.A = d.A; g.B = d.B; g.alpha = d.alpha; g.beta = d.beta; g.mode = kOutValue; g.C = d.C;
+    g.A = d.A; g.B = d.B; g.ar = d.alpha; g.alpha_one = d.alpha == 1.0; g.br = d.beta; g.mode = kOutValue; g.C = d.C;
     p->gemms.push_back(g);
     const size_t ext = ((size_t)(g.M - 1) * g.sci + (size_t)(g.N - 1) * g.scj + 1) * sizeof(double);
     p->c_extents.push_back({d.C, ext});
   }
-  if (cudaMalloc(&p->d_gemms, std::max<size_t>(16, p->gemms.size() * sizeof(GemmArgs))) != cudaSuccess ||
-      (p->gemms.size() && cudaMemcpy(p->d_gemms, p->gemms.data(), p->gemms.size() * sizeof(GemmArgs),
+  if (cudaMalloc(&p->d_gemms, std::max<size_t>(16, p->gemms.size() * sizeof(XGemmArgs<double>))) != cudaSuccess ||
+      (p->gemms.size() && cudaMemcpy(p->d_gemms, p->gemms.data(), p->gemms.size() * sizeof(XGemmArgs<double>),
                                      cudaMemcpyHostToDevice) != cudaSuccess) ||
       cudaMalloc(&p->d_tickets, std::max<size_t>(16, p->segs.size() * sizeof(unsigned))) != cudaSuccess ||
       cudaMemset(p->d_tickets, 0, std::max<size_t>(16, p->segs.size() * sizeof(unsigned))) != cudaSuccess ||

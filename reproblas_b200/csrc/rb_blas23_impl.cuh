@@ -1,4 +1,5 @@
-// rb_blas23_impl.cuh -- binned dgemv and plain binned dgemm on sm_100a.
+// rb_blas23_impl.cuh -- binned dgemv on sm_100a, and the table of the FP64 gemv / gemm
+// kernels of a fold (the gemm tile is in rb_gemm_tile.cuh).
 //
 // Every output entry is one binned dot product, so the state of each entry depends only on
 // the multiset of its products (plus the beta*y / beta*C initial value), exactly as in the
@@ -12,6 +13,7 @@
 // products (the host passes an empty reduction).
 #pragma once
 #include "rb_binned.cuh"
+#include "rb_gemm_tile.cuh"
 #include "rb_kernels.cuh"
 #include "rb_ptx.cuh"
 
@@ -337,278 +339,10 @@ __global__ void __launch_bounds__(256, F <= 3 ? 3 : 2) gemv_cols_kernel(GemvArgs
   else gemv_cols_body<F, 1>(g, sm);
 }
 
-// ---------------------------------------------------------------------------------------
-// Plain binned dgemm. CTA tile BM x BN of C entries, TM x TN entries per thread, each with
-// its own fold-F accumulator in registers; K in tiles of BK through shared memory, with
-// fl(alpha*A) formed when the A tile is stored. Operands use general strides
-//   op(A)_ik = A[i*sai + k*sak], op(B)_kj = B[k*sbk + j*sbj], C_ij = C[i*sci + j*scj]
-// which cover both orders and both transposes.
-// ---------------------------------------------------------------------------------------
-template <int F, int TM, int TN>
-struct GemmCfg {
-  static constexpr int TX = 16, TY = 16;            // 256 threads
-  static constexpr int BM = TY * TM, BN = TX * TN;
-  static constexpr int BK = 32;
-};
-
-// Reductions longer than this use the per-K-tile magnitude bound in gemm_tile (shorter ones,
-// e.g. the batched form's small instances, gain less than the bound's pass costs).
-constexpr long long kBoundMinK = 256;
-
-// Upper bound of every magnitude whose 32-bit key (BT<double>::key: high word, sign cleared)
-// is at most k: the largest double with that high word.
-__device__ __forceinline__ double key_ceiling(unsigned k) {
-  return __longlong_as_double((long long)(((unsigned long long)k << 32) | 0xffffffffull));
-}
-
-// Shared-memory row of TN (1, 2 or 4) adjacent doubles, 16-byte aligned when TN > 1.
-template <int TN>
-__device__ __forceinline__ void lds_row(const double* p, double (&v)[TN]) {
-  if constexpr (TN == 1) {
-    v[0] = p[0];
-  } else {
-#pragma unroll
-    for (int t = 0; t < TN; t += 2) {
-      const double2 w = *(const double2*)(p + t);
-      v[t] = w.x;
-      v[t + 1] = w.y;
-    }
-  }
-}
-
-// One BM x BN tile of C at (m0, n0), computed by the 256 threads of the calling CTA (the
-// caller must keep the whole CTA in step: the tile uses __syncthreads). Thread (tx, ty) owns
-// the TM x TN entries at rows ty*TM.. and columns tx*TN.. of the tile, so that its operands
-// sit next to each other in the shared tiles and load as 16-byte vectors.
-//
-// Per K tile the CTA records the largest-magnitude key of every row of op(A) and column of
-// op(B) in it (a warp-wide max per row / column). When, for every entry of a thread, the
-// product of the two magnitude bounds stays below the entry's cap and the tile's deposits fit
-// the endurance, no product of the tile can need an index raise, a renormalisation or a
-// non-finite branch: the tile's products are deposited without per-product checks, exactly
-// as the per-step fast path (tileN) would deposit them. Otherwise the tile takes the
-// per-step path. Both give the same state.
-// PIPE: whole K tiles of pair-loading operands are prefetched into registers (the plain
-// dgemm kernel; the batched kernel's tiles keep the registers for occupancy).
-template <int F, int TM, int TN, bool PIPE = false>
-__device__ __forceinline__ void gemm_tile(const GemmArgs& g, long long m0, long long n0) {
-  using Cfg = GemmCfg<F, TM, TN>;
-  using B = BT<double>;
-  constexpr int BM = Cfg::BM, BN = Cfg::BN, BK = Cfg::BK;
-  constexpr int LDA = BM + 2, LDB = BN + 2;   // even strides: rows stay 16-byte aligned
-  __shared__ __align__(16) double As[BK][LDA];
-  __shared__ __align__(16) double Bs[BK][LDB];
-  __shared__ unsigned rowkey[BM], colkey[BN];
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int tx = tid % Cfg::TX, ty = tid / Cfg::TX;
-  const int ra = ty * TM, cb = tx * TN;   // this thread's first row / column in the tile
-
-  Acc<double, F> acc[TM * TN];   // entry (i, j) at i * TN + j
-#pragma unroll
-  for (int e = 0; e < TM * TN; e++) acc[e].zero();
-
-  const bool a_k_fast = g.sak == 1;   // which stride is unit decides the load order
-  const bool b_j_fast = g.sbj == 1;
-  // whole tiles with a unit stride, an even leading dimension and a 16-byte aligned base
-  // load 16-byte pairs
-  const bool a_pairs = a_k_fast && (g.sai & 1) == 0 && ((uintptr_t)g.A & 15) == 0 && m0 + BM <= g.M;
-  const bool b_pairs = b_j_fast && (g.sbk & 1) == 0 && ((uintptr_t)g.B & 15) == 0 && n0 + BN <= g.N;
-  // When every K tile is whole and both operands load pairs, the next K tile's pairs are
-  // loaded into registers while the current one is deposited.
-  constexpr int APV = BM * BK / 2 / 256, BPV = BK * BN / 2 / 256;   // pairs per thread
-  static_assert(APV * 512 == BM * BK && BPV * 512 == BK * BN, "pair split");
-  const bool pipe = PIPE && a_pairs && b_pairs && g.K % BK == 0;
-  double2 pa[APV], pb[BPV];
-  auto fetch = [&](long long k0) {
-#pragma unroll
-    for (int u = 0; u < APV; u++) {
-      const int e = tid + 256 * u, i = e / (BK / 2), k = 2 * (e % (BK / 2));
-      pa[u] = __ldg((const double2*)(g.A + (m0 + i) * g.sai + k0 + k));
-    }
-#pragma unroll
-    for (int u = 0; u < BPV; u++) {
-      const int e = tid + 256 * u, k = e / (BN / 2), j = 2 * (e % (BN / 2));
-      pb[u] = __ldg((const double2*)(g.B + (k0 + k) * g.sbk + n0 + j));
-    }
-  };
-  if (pipe) fetch(0);
-
-#pragma unroll 1
-  for (long long k0 = 0; k0 < g.K; k0 += BK) {
-    const bool k_whole = k0 + BK <= g.K;
-    if (pipe) {
-#pragma unroll
-      for (int u = 0; u < APV; u++) {
-        const int e = tid + 256 * u, i = e / (BK / 2), k = 2 * (e % (BK / 2));
-        double v0 = pa[u].x, v1 = pa[u].y;
-        if (g.alpha != 1.0) {
-          v0 = __dmul_rn(v0, g.alpha);
-          v1 = __dmul_rn(v1, g.alpha);
-        }
-        As[k][i] = v0;
-        As[k + 1][i] = v1;
-      }
-#pragma unroll
-      for (int u = 0; u < BPV; u++) {
-        const int e = tid + 256 * u, k = e / (BN / 2), j = 2 * (e % (BN / 2));
-        *(double2*)&Bs[k][j] = pb[u];
-      }
-      if (k0 + BK < g.K) fetch(k0 + BK);
-    } else if (a_pairs && k_whole) {
-#pragma unroll 1
-      for (int e = tid; e < BM * BK / 2; e += 256) {
-        const int i = e / (BK / 2), k = 2 * (e % (BK / 2));
-        const double2 v = __ldg((const double2*)(g.A + (m0 + i) * g.sai + k0 + k));
-        double v0 = v.x, v1 = v.y;
-        if (g.alpha != 1.0) {
-          v0 = __dmul_rn(v0, g.alpha);
-          v1 = __dmul_rn(v1, g.alpha);
-        }
-        As[k][i] = v0;
-        As[k + 1][i] = v1;
-      }
-    } else {
-#pragma unroll 1
-      for (int e = tid; e < BM * BK; e += 256) {
-        int i, k;
-        if (a_k_fast) { k = e % BK; i = e / BK; } else { i = e % BM; k = e / BM; }
-        const long long gi = m0 + i, gk = k0 + k;
-        double v = 0.0;
-        if (gi < g.M && gk < g.K) {
-          v = __ldg(g.A + gi * g.sai + gk * g.sak);
-          if (g.alpha != 1.0) v = __dmul_rn(v, g.alpha);
-        }
-        As[k][i] = v;
-      }
-    }
-    // B tile: BK x BN
-    if (pipe) {
-      // stored above
-    } else if (b_pairs && k_whole) {
-#pragma unroll 1
-      for (int e = tid; e < BK * BN / 2; e += 256) {
-        const int k = e / (BN / 2), j = 2 * (e % (BN / 2));
-        *(double2*)&Bs[k][j] = __ldg((const double2*)(g.B + (k0 + k) * g.sbk + n0 + j));
-      }
-    } else {
-#pragma unroll 1
-      for (int e = tid; e < BK * BN; e += 256) {
-        int k, j;
-        if (b_j_fast) { j = e % BN; k = e / BN; } else { k = e % BK; j = e / BK; }
-        const long long gk = k0 + k, gj = n0 + j;
-        double v = 0.0;
-        if (gk < g.K && gj < g.N) v = __ldg(g.B + gk * g.sbk + gj * g.sbj);
-        Bs[k][j] = v;
-      }
-    }
-    __syncthreads();
-    const int kmax = (g.K - k0) < BK ? (int)(g.K - k0) : BK;
-    const int kend = (kmax + 3) & ~3;   // whole steps of 4; past K both tiles hold zeros
-    // Long reductions (the bound pays for its pass and barrier): largest key of each row of
-    // the A tile and each column of the B tile (lane = k), then the entries' bounds. g.K is
-    // the same for the whole CTA.
-    bool fast = false;
-    if (g.K > kBoundMinK) {
-#pragma unroll 1
-      for (int r = warp; r < BM + BN; r += 8) {
-        const double v = r < BM ? As[lane][r] : Bs[lane][r - BM];
-        const unsigned m = __reduce_max_sync(0xffffffffu, B::key(v));
-        if (lane == 0) {
-          if (r < BM) rowkey[r] = m;
-          else colkey[r - BM] = m;
-        }
-      }
-      __syncthreads();
-      fast = true;
-#pragma unroll
-      for (int i = 0; i < TM; i++) {
-        const double au = key_ceiling(rowkey[ra + i]);
-#pragma unroll
-        for (int j = 0; j < TN; j++) {
-          const unsigned bound = B::key(__dmul_rn(au, key_ceiling(colkey[cb + j])));
-          fast = fast && acc[i * TN + j].fast(bound, kend);
-        }
-      }
-    }
-    if (fast) {
-#pragma unroll
-      for (int e = 0; e < TM * TN; e++) acc[e].deposits += kend;
-#pragma unroll 1
-      for (int kk = 0; kk < kend; kk += 4) {
-#pragma unroll
-        for (int q = 0; q < 4; q++) {
-          double av[TM], bv[TN];
-          lds_row<TM>(&As[kk + q][ra], av);
-          lds_row<TN>(&Bs[kk + q][cb], bv);
-#pragma unroll
-          for (int i = 0; i < TM; i++)
-#pragma unroll
-            for (int j = 0; j < TN; j++) acc[i * TN + j].deposit(__dmul_rn(av[i], bv[j]));
-        }
-      }
-    } else {
-      // per-step path: the key max of every entry's 4 products; when all entries are on
-      // their fast path the deposit chains are interleaved (tileN)
-#pragma unroll 1
-      for (int kk = 0; kk < kend; kk += 4) {
-        double p[TM * TN][4];
-#pragma unroll
-        for (int q = 0; q < 4; q++) {
-          double av[TM], bv[TN];
-          lds_row<TM>(&As[kk + q][ra], av);
-          lds_row<TN>(&Bs[kk + q][cb], bv);
-#pragma unroll
-          for (int i = 0; i < TM; i++)
-#pragma unroll
-            for (int j = 0; j < TN; j++) p[i * TN + j][q] = __dmul_rn(av[i], bv[j]);
-        }
-        tileN<double, F, 4, TM * TN>(acc, p);
-      }
-    }
-    __syncthreads();
-  }
-
-#pragma unroll
-  for (int i = 0; i < TM; i++)
-#pragma unroll
-    for (int j = 0; j < TN; j++) {
-      const long long gi = m0 + ra + i, gj = n0 + cb + j;
-      if (gi < g.M && gj < g.N) {
-        acc[i * TN + j].renorm();
-        const long long off = gi * g.sci + gj * g.scj;
-        finish_entry<F>(acc[i * TN + j], g.mode, g.C + off, g.beta, g.Cbin + off * 2 * F);
-      }
-    }
-}
-
-template <int F, int TM, int TN>
-__global__ void __launch_bounds__(256, 2) gemm_kernel(GemmArgs g) {
-  using Cfg = GemmCfg<F, TM, TN>;
-  gemm_tile<F, TM, TN, true>(g, (long long)blockIdx.y * Cfg::BM, (long long)blockIdx.x * Cfg::BN);
-}
-
 template <int F>
 cudaError_t launch_gemv(const GemvArgs& g, bool rows, dim3 grid, cudaStream_t s) {
   if (rows) gemv_rows_kernel<F><<<grid, 256, 0, s>>>(g);
   else gemv_cols_kernel<F><<<grid, 256, 0, s>>>(g);
-  return cudaGetLastError();
-}
-
-template <int F>
-cudaError_t launch_gemm(const GemmArgs& g, cudaStream_t s, int* bm, int* bn) {
-  if constexpr (F <= 4) {
-    using Cfg = GemmCfg<F, 2, 2>;
-    dim3 grid((unsigned)((g.N + Cfg::BN - 1) / Cfg::BN), (unsigned)((g.M + Cfg::BM - 1) / Cfg::BM));
-    if (bm) *bm = Cfg::BM;
-    if (bn) *bn = Cfg::BN;
-    gemm_kernel<F, 2, 2><<<grid, 256, 0, s>>>(g);
-  } else {
-    using Cfg = GemmCfg<F, 1, 1>;
-    dim3 grid((unsigned)((g.N + Cfg::BN - 1) / Cfg::BN), (unsigned)((g.M + Cfg::BM - 1) / Cfg::BM));
-    if (bm) *bm = Cfg::BM;
-    if (bn) *bn = Cfg::BN;
-    gemm_kernel<F, 1, 1><<<grid, 256, 0, s>>>(g);
-  }
   return cudaGetLastError();
 }
 
@@ -622,7 +356,8 @@ template <int F>
 Blas23FoldOps make_blas23_ops() {
   Blas23FoldOps o;
   o.gemv = launch_gemv<F>;
-  o.gemm = launch_gemm<F>;
+  o.gemm_plan = gt::plan_gemm<double, false, F>;
+  o.gemm = gt::launch_gemm<double, false, F>;
   // the TMA-fed gemv kernels fit their registers (17 warps per SM) up to fold 3
   if constexpr (F <= 3) {
     o.gemv_stream = gs::launch_gemv_stream<F>;

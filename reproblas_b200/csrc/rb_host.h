@@ -80,6 +80,10 @@ struct Workspace {
   void* hresult() { return (void*)(hsmall + 2112); }
   void* hresult_dev() { return (void*)(hsmall_dev + 2112); }   // hresult() as kernels address it
 
+  // partial states of gemm tiles cut between CTAs (grow on demand; see gemm_decompose)
+  unsigned char* parts = nullptr;
+  size_t parts_bytes = 0;
+
   bool ensure_ring(size_t chunk);
   bool ensure_big(size_t bytes);
   bool ensure_tickets(size_t n);
@@ -89,6 +93,13 @@ struct Workspace {
 // Locked workspace of the calling thread's current device and stream, or nullptr (error
 // set); with create = false, nullptr when no call has made one yet.
 Workspace* acquire_workspace(std::unique_lock<std::mutex>* lock, bool create = true);
+
+// Decomposition of an M x N x K gemm on workspace w's stream through a fold's planner: cut tiles
+// when that pays and the scratch for their partial states can be had, else whole tiles (no
+// scratch). A captured launch keeps to whole tiles, so that a graph never holds the address
+// of scratch that a later call may replace.
+bool gemm_decompose(cudaError_t (*plan)(long long, long long, long long, int, bool, GemmPlan*),
+                    Workspace* w, long long M, long long N, long long K, GemmPlan* p);
 
 // cudaMalloc, or a reported cudaErrorMemoryAllocation while the allocation-failure test hook
 // (rb_debug_fail_allocations) has failures left.

@@ -109,19 +109,6 @@ struct GemvArgs {
   unsigned* tickets;          // cols kernel: one per column block, zero on entry
 };
 
-struct GemmArgs {
-  long long M, N, K;
-  const double* A;
-  long long sai, sak;         // op(A)_ik = A[i*sai + k*sak]
-  const double* B;
-  long long sbk, sbj;         // op(B)_kj = B[k*sbk + j*sbj]
-  double alpha, beta;
-  int mode;
-  double* C;                  // kOutValue
-  double* Cbin;               // kOutBinned
-  long long sci, scj;         // C_ij at offset i*sci + j*scj (values or states)
-};
-
 // TMA-fed dgemv (rb_gemv_stream.cuh): A is R x C row-major behind a 2-D tensor map.
 struct GemvStreamArgs {
   long long R, C;        // A is R x C (row-major view)
@@ -148,9 +135,47 @@ struct GemvStreamArgs {
 // kernels (stop_after < 0 and wait_polls 0 when unset).
 void pipeline_fault(long long* stop_after, long long* wait_polls);
 
+// One gemm of any element type. E is the real element type; complex operands are interleaved
+// (re, im) pairs and every stride counts whole (complex) elements.
+template <typename E>
+struct XGemmArgs {
+  long long M, N, K;
+  const E* A;
+  long long sai, sak;         // op(A)_ik = A[i*sai + k*sak]
+  const E* B;
+  long long sbk, sbj;         // op(B)_kj = B[k*sbk + j*sbj]
+  E ar, ai, br, bi;
+  int alpha_one;
+  int conja, conjb;           // conjugate op(A) / op(B) (complex ConjTrans)
+  int mode;
+  E* C;                       // kOutValue
+  E* Cbin;                    // kOutBinned
+  long long sci, scj;         // C_ij at offset i*sci + j*scj (values or states)
+};
+
+// Decomposition of one gemm (rb_gemm_tile.cuh). Work is counted in units: one K block of one
+// C tile. The units, tile-major, are split evenly over `grid` CTAs; a tile cut between CTAs
+// leaves one partial state per CTA in `scratch` and is finished by the last of them to
+// arrive (`tickets`, one per tile, zero on entry and on exit).
+struct GemmPlan {
+  long long units;            // tiles * nkb
+  long long nkb;              // K blocks per tile
+  long long ntn;              // tiles along N
+  long long tiles;
+  int grid;
+  int cut;                    // some tile is cut: scratch and tickets are needed
+  int shape;                  // kernel variant (tile shape)
+  size_t scratch_bytes;
+  void* scratch;
+  unsigned* tickets;
+};
+
 struct Blas23FoldOps {
   cudaError_t (*gemv)(const GemvArgs& g, bool rows, dim3 grid, cudaStream_t s);
-  cudaError_t (*gemm)(const GemmArgs& g, cudaStream_t s, int* bm, int* bn);
+  // decomposition of an M x N x K product (whole_tiles: no tile is cut between CTAs)
+  cudaError_t (*gemm_plan)(long long M, long long N, long long K, int sms, bool whole_tiles,
+                           GemmPlan* p);
+  cudaError_t (*gemm)(const XGemmArgs<double>& g, const GemmPlan& p, cudaStream_t s);
   // TMA-fed dgemv (nullptr for folds it does not cover)
   cudaError_t (*gemv_stream)(const GemvStreamArgs& g, const CUtensorMap& tm, const CUtensorMap& tmx,
                              bool rows, int grid, cudaStream_t s);
@@ -186,25 +211,12 @@ struct XGemvArgs {
 };
 
 template <typename E>
-struct XGemmArgs {
-  long long M, N, K;
-  const E* A;
-  long long sai, sak;         // op(A)_ik = A[i*sai + k*sak]
-  const E* B;
-  long long sbk, sbj;         // op(B)_kj = B[k*sbk + j*sbj]
-  E ar, ai, br, bi;
-  int alpha_one;
-  int conja, conjb;           // conjugate op(A) / op(B) (complex ConjTrans)
-  int mode;
-  E* C;                       // kOutValue
-  E* Cbin;                    // kOutBinned
-  long long sci, scj;         // C_ij at offset i*sci + j*scj (values or states)
-};
-
-template <typename E>
 struct XOps {
   cudaError_t (*gemv)(const XGemvArgs<E>& g, bool rows, dim3 grid, cudaStream_t s);
-  cudaError_t (*gemm)(const XGemmArgs<E>& g, cudaStream_t s);
+  // decomposition of an M x N x K product (whole_tiles: no tile is cut between CTAs)
+  cudaError_t (*gemm_plan)(long long M, long long N, long long K, int sms, bool whole_tiles,
+                           GemmPlan* p);
+  cudaError_t (*gemm)(const XGemmArgs<E>& g, const GemmPlan& p, cudaStream_t s);
   // bx_i = fl(alpha * x_i) for i < n, contiguous (the rows kernel's vector input)
   cudaError_t (*scale_x)(const E* x, long long n, long long incx, E ar, E ai, int alpha_one,
                          E* bx, int grid, cudaStream_t s);

@@ -119,6 +119,7 @@ void Workspace::release() {
   if (hsmall) { cudaFreeHost(hsmall); hsmall = nullptr; }
   if (big) { cudaFree(big); big = nullptr; big_bytes = 0; }
   if (tickets) { cudaFree(tickets); tickets = nullptr; ntickets = 0; }
+  if (parts) { cudaFree(parts); parts = nullptr; parts_bytes = 0; }
   if (copy_stream) { cudaStreamDestroy(copy_stream); copy_stream = nullptr; }
 }
 
@@ -169,6 +170,41 @@ bool Workspace::ensure_tickets(size_t n) {
   }
   if (!cuda_ok(cudaMemset(tickets, 0, want * sizeof(unsigned)), "cudaMemset")) return false;
   ntickets = want;
+  return true;
+}
+
+bool gemm_decompose(cudaError_t (*plan)(long long, long long, long long, int, bool, GemmPlan*),
+                    Workspace* w, long long M, long long N, long long K, GemmPlan* p) {
+  DeviceInfo di;
+  if (!device_info(&di)) return false;
+  if (!cuda_ok(plan(M, N, K, di.sms, false, p), "gemm kernel attributes")) return false;
+  if (!p->cut) return true;
+  cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
+  bool have = cudaStreamIsCapturing(w->stream, &st) == cudaSuccess && st == cudaStreamCaptureStatusNone;
+  if (!have) cudaGetLastError();
+  if (have && p->scratch_bytes > w->parts_bytes) {
+    // drain the stream first: kernels in flight may still use the old buffer
+    if (!cuda_ok(cudaStreamSynchronize(w->stream), "cudaStreamSynchronize")) return false;
+    if (w->parts) { cudaFree(w->parts); w->parts = nullptr; w->parts_bytes = 0; }
+    if (dev_malloc((void**)&w->parts, p->scratch_bytes) == cudaSuccess) {
+      w->parts_bytes = p->scratch_bytes;
+    } else {
+      cudaGetLastError();
+      w->parts = nullptr;
+      have = false;
+    }
+  }
+  if (have && (size_t)p->tiles > w->ntickets) {
+    // a failed ticket allocation is no error here: whole tiles need none
+    have = w->ensure_tickets((size_t)p->tiles);
+    if (!have) {
+      cudaGetLastError();
+      rb_clear_error();
+    }
+  }
+  if (!have) return cuda_ok(plan(M, N, K, di.sms, true, p), "gemm kernel attributes");
+  p->scratch = w->parts;
+  p->tickets = w->tickets;
   return true;
 }
 

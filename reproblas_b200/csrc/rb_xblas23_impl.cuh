@@ -19,181 +19,11 @@
 #pragma once
 #include <atomic>
 
-#include "rb_binned.cuh"
-#include "rb_kernels.cuh"
+#include "rb_entry.cuh"
+#include "rb_gemm_tile.cuh"
 
 namespace rb {
 namespace xb {
-
-template <typename E, bool CX> struct Val { E r, i; };
-
-// Element `idx` of a real or complex (interleaved pair) array.
-template <typename E, bool CX>
-__device__ __forceinline__ Val<E, CX> ldv(const E* p, long long idx) {
-  Val<E, CX> v;
-  if constexpr (CX) {
-    v.r = __ldg(p + 2 * idx);
-    v.i = __ldg(p + 2 * idx + 1);
-  } else {
-    v.r = __ldg(p + idx);
-    v.i = E(0);
-  }
-  return v;
-}
-
-// fl(v * alpha) as the reference forms it.
-template <typename E, bool CX>
-__device__ __forceinline__ Val<E, CX> scale(Val<E, CX> v, E ar, E ai) {
-  using B = BT<E>;
-  Val<E, CX> o;
-  if constexpr (CX) {
-    o.r = B::sub(B::mul(v.r, ar), B::mul(v.i, ai));
-    o.i = B::add(B::mul(v.r, ai), B::mul(v.i, ar));
-  } else {
-    o.r = B::mul(v.r, ar);
-    o.i = E(0);
-  }
-  return o;
-}
-
-// The values one product a*b deposits: D = 1 (real) or 2 per component, at column q*D of
-// v[component].
-template <typename E, bool CX, int KD>
-__device__ __forceinline__ void products(Val<E, CX> a, Val<E, CX> b, E (&v)[CX ? 2 : 1][KD],
-                                         int q) {
-  using B = BT<E>;
-  if constexpr (CX) {
-    v[0][2 * q] = B::mul(a.r, b.r);
-    v[0][2 * q + 1] = -B::mul(a.i, b.i);
-    v[1][2 * q] = B::mul(a.r, b.i);
-    v[1][2 * q + 1] = B::mul(a.i, b.r);
-  } else {
-    v[0][q] = B::mul(a.r, b.r);
-  }
-}
-
-// binned -> value conversion of one component (ddmconv / ssmconv).
-template <typename E, int F>
-__device__ __forceinline__ E convx(const E* p, const E* c, int inc) {
-  if constexpr (sizeof(E) == 8) return conv<F>(p, c, inc);
-  else return sconv<F>(p, c, inc);
-}
-
-// Finish one output entry from the renormalised state of its products, a[0..NC-1]:
-// kOutValue deposits beta*y into it (nothing when beta == 0, y itself when beta == 1;
-// rzgemv.c:47-59 starts from binned(beta*y) -- the same multiset, so the same state) and
-// writes the converted value to yout; yin holds y (read by the caller, possibly early).
-// kOutBinned merges into the caller's state (reference layout: NC-interleaved primaries,
-// then carries).
-template <typename E, bool CX, int F>
-__device__ __forceinline__ void finish_from(Acc<E, F>* a, int mode, const E* yin, E* yout, E br,
-                                            E bi, E* yb) {
-  constexpr int NC = CX ? 2 : 1;
-  using B = BT<E>;
-  if (mode == kOutValue) {
-    const bool bzero = br == E(0) && (!CX || bi == E(0));
-    const bool bone = br == E(1) && (!CX || bi == E(0));
-    E init[NC];
-    if constexpr (CX) {
-      const E yr = yin[0], yi = yin[1];
-      if (bone) {
-        init[0] = yr;
-        init[1] = yi;
-      } else {
-        init[0] = B::sub(B::mul(yr, br), B::mul(yi, bi));
-        init[1] = B::add(B::mul(yr, bi), B::mul(yi, br));
-      }
-    } else {
-      init[0] = bone ? yin[0] : B::mul(yin[0], br);
-    }
-#pragma unroll
-    for (int c = 0; c < NC; c++) {
-      if (!bzero) {
-        E v[1] = {init[c]};
-        a[c].template tile<1>(v, 1);
-      }
-      a[c].renorm();
-      E p[F], q[F];
-      a[c].store(p, q, 1);
-      yout[c] = convx<E, F>(p, q, 1);
-    }
-  } else {
-#pragma unroll
-    for (int c = 0; c < NC; c++) {
-      Acc<E, F> prev;
-      prev.load(yb + c, yb + NC * F + c, NC);
-      prev.merge(a[c]);
-      prev.renorm();
-      prev.store(yb + c, yb + NC * F + c, NC);
-    }
-  }
-}
-
-template <typename E, bool CX, int F>
-__device__ __forceinline__ void finish(Acc<E, F>* a, int mode, E* yv, E br, E bi, E* yb) {
-  constexpr int NC = CX ? 2 : 1;
-  E yin[NC];
-#pragma unroll
-  for (int c = 0; c < NC; c++) yin[c] = E(0);
-  if (mode == kOutValue) {
-#pragma unroll
-    for (int c = 0; c < NC; c++) yin[c] = yv[c];
-  }
-  finish_from<E, CX, F>(a, mode, yin, yv, br, bi, yb);
-}
-
-template <typename E>
-__device__ __forceinline__ E flags_to(unsigned f) {
-  if constexpr (sizeof(E) == 8) return __longlong_as_double((long long)f);
-  else return __uint_as_float(f);
-}
-template <typename E>
-__device__ __forceinline__ unsigned flags_from(E v) {
-  if constexpr (sizeof(E) == 8) return (unsigned)__double_as_longlong(v);
-  else return __float_as_uint(v);
-}
-
-// Record of one accumulator: F primaries, F carries, the flags word; element q of the record
-// at rec[q * stride].
-template <typename E, int F>
-__device__ __forceinline__ void put_rec(const Acc<E, F>& a, E* rec, long long stride) {
-#pragma unroll
-  for (int i = 0; i < F; i++) {
-    rec[i * stride] = a.pri[i];
-    rec[(F + i) * stride] = a.car[i];
-  }
-  rec[2 * F * stride] = flags_to<E>(a.flags);
-}
-// GLOBAL: the record was written by another CTA (read through L2); else shared memory.
-template <typename E, int F, bool GLOBAL>
-__device__ __forceinline__ void merge_rec(Acc<E, F>& a, const E* rec, long long stride) {
-  Acc<E, F> o;
-  o.zero();
-#pragma unroll
-  for (int i = 0; i < F; i++) {
-    o.pri[i] = GLOBAL ? __ldcg(rec + i * stride) : rec[i * stride];
-    o.car[i] = GLOBAL ? __ldcg(rec + (F + i) * stride) : rec[(F + i) * stride];
-  }
-  o.flags = flags_from<E>(GLOBAL ? __ldcg(rec + 2 * F * stride) : rec[2 * F * stride]);
-  o.set_idx_from_pri();
-  a.merge(o);
-}
-
-// 16-byte read-only load of 16 / sizeof(E) reals (the address is 16-byte aligned).
-template <typename E>
-__device__ __forceinline__ void ld16(const E* p, E (&v)[16 / sizeof(E)]) {
-  if constexpr (sizeof(E) == 8) {
-    const double2 t = __ldg((const double2*)p);
-    v[0] = t.x;
-    v[1] = t.y;
-  } else {
-    const float4 t = __ldg((const float4*)p);
-    v[0] = t.x;
-    v[1] = t.y;
-    v[2] = t.z;
-    v[3] = t.w;
-  }
-}
 
 // Deposit one tile into the NC accumulators of an entry: complex entries interleave their
 // real and imaginary chains (tile2); every one of the KD values counts toward the endurance.
@@ -642,163 +472,6 @@ __global__ void __launch_bounds__(256, F <= 3 ? ColsCfg<E, CX>::MIN_CTAS : 2) xg
   if (threadIdx.x == 0) g.tickets[blockIdx.x] = 0u;
 }
 
-// ---------------------------------------------------------------------------------------
-// gemm. CTA tile BM x BN of C entries, TM x TN entries per thread, each with NC fold-F
-// accumulators in registers; K in tiles of BK through shared memory. op(A) is conjugated
-// (conja) and multiplied by alpha when its tile is stored; op(B) is conjugated (conjb).
-// Operands use general strides (in elements):
-//   op(A)_ik = A[i*sai + k*sak], op(B)_kj = B[k*sbk + j*sbj], C_ij = C[i*sci + j*scj].
-// ---------------------------------------------------------------------------------------
-template <typename E, bool CX, int TM, int TN>
-struct XGemmCfg {
-  static constexpr int TX = 16, TY = 16;   // 256 threads
-  static constexpr int BM = TY * TM, BN = TX * TN;
-  static constexpr int BK = CX ? 16 : 32;
-};
-
-template <typename E, bool CX, int F, int TM, int TN>
-__global__ void __launch_bounds__(256) xgemm_kernel(XGemmArgs<E> g) {
-  using Cfg = XGemmCfg<E, CX, TM, TN>;
-  constexpr int NC = CX ? 2 : 1, D = CX ? 2 : 1;
-  constexpr int BM = Cfg::BM, BN = Cfg::BN, BK = Cfg::BK;
-  constexpr int NA = TM * TN * NC;   // accumulators per thread
-  __shared__ E As[NC][BK][BM + 1];
-  __shared__ E Bs[NC][BK][BN + 1];
-  const int tid = threadIdx.x;
-  const int tx = tid % Cfg::TX, ty = tid / Cfg::TX;
-  const long long m0 = (long long)blockIdx.y * BM, n0 = (long long)blockIdx.x * BN;
-
-  Acc<E, F> acc[NA];   // entry (i, j), component q at (i * TN + j) * NC + q
-#pragma unroll
-  for (int e = 0; e < NA; e++) acc[e].zero();
-
-  const bool a_k_fast = g.sak == 1;
-  const bool b_j_fast = g.sbj == 1;
-  // whole tiles of unit-stride operands whose rows start 16-byte aligned load 16-byte
-  // vectors of VE elements
-  constexpr int PER = 16 / (int)sizeof(E), VE = PER / NC;
-  const bool a_vec = a_k_fast && ((g.sai * NC * (long long)sizeof(E)) & 15) == 0 &&
-                     ((uintptr_t)g.A & 15) == 0 && m0 + BM <= g.M;
-  const bool b_vec = b_j_fast && ((g.sbk * NC * (long long)sizeof(E)) & 15) == 0 &&
-                     ((uintptr_t)g.B & 15) == 0 && n0 + BN <= g.N;
-
-#pragma unroll 1
-  for (long long k0 = 0; k0 < g.K; k0 += BK) {
-    const bool k_whole = k0 + BK <= g.K;
-    if (a_vec && k_whole) {
-#pragma unroll 1
-      for (int e = tid; e < BM * BK / VE; e += 256) {
-        const int i = e / (BK / VE), k = (e % (BK / VE)) * VE;
-        E raw[PER];
-        ld16<E>(g.A + ((m0 + i) * g.sai + k0 + k) * NC, raw);
-#pragma unroll
-        for (int w = 0; w < VE; w++) {
-          Val<E, CX> v;
-          v.r = raw[w * NC];
-          v.i = CX ? raw[w * NC + NC - 1] : E(0);
-          if (CX && g.conja) v.i = -v.i;
-          if (!g.alpha_one) v = scale<E, CX>(v, g.ar, g.ai);
-          As[0][k + w][i] = v.r;
-          if constexpr (CX) As[NC - 1][k + w][i] = v.i;
-        }
-      }
-    } else {
-#pragma unroll 1
-      for (int e = tid; e < BM * BK; e += 256) {
-        int i, k;
-        if (a_k_fast) { k = e % BK; i = e / BK; } else { i = e % BM; k = e / BM; }
-        const long long gi = m0 + i, gk = k0 + k;
-        Val<E, CX> v{E(0), E(0)};
-        if (gi < g.M && gk < g.K) {
-          v = ldv<E, CX>(g.A, gi * g.sai + gk * g.sak);
-          if (CX && g.conja) v.i = -v.i;
-          if (!g.alpha_one) v = scale<E, CX>(v, g.ar, g.ai);
-        }
-        As[0][k][i] = v.r;
-        if constexpr (CX) As[NC - 1][k][i] = v.i;
-      }
-    }
-    if (b_vec && k_whole) {
-#pragma unroll 1
-      for (int e = tid; e < BK * BN / VE; e += 256) {
-        const int k = e / (BN / VE), j = (e % (BN / VE)) * VE;
-        E raw[PER];
-        ld16<E>(g.B + ((k0 + k) * g.sbk + n0 + j) * NC, raw);
-#pragma unroll
-        for (int w = 0; w < VE; w++) {
-          Bs[0][k][j + w] = raw[w * NC];
-          if constexpr (CX) Bs[NC - 1][k][j + w] = g.conjb ? -raw[w * NC + NC - 1] : raw[w * NC + NC - 1];
-        }
-      }
-    } else {
-#pragma unroll 1
-      for (int e = tid; e < BK * BN; e += 256) {
-        int k, j;
-        if (b_j_fast) { j = e % BN; k = e / BN; } else { k = e % BK; j = e / BK; }
-        const long long gk = k0 + k, gj = n0 + j;
-        Val<E, CX> v{E(0), E(0)};
-        if (gk < g.K && gj < g.N) {
-          v = ldv<E, CX>(g.B, gk * g.sbk + gj * g.sbj);
-          if (CX && g.conjb) v.i = -v.i;
-        }
-        Bs[0][k][j] = v.r;
-        if constexpr (CX) Bs[NC - 1][k][j] = v.i;
-      }
-    }
-    __syncthreads();
-    const int kmax = (g.K - k0) < BK ? (int)(g.K - k0) : BK;
-    // past K both tiles hold zeros, whose products deposit nothing
-#pragma unroll 1
-    for (int kk = 0; kk < BK; kk += 4) {
-      if (kk >= kmax) break;
-      Val<E, CX> av[TM][4], bv[TN][4];
-#pragma unroll
-      for (int q = 0; q < 4; q++) {
-#pragma unroll
-        for (int i = 0; i < TM; i++) {
-          av[i][q].r = As[0][kk + q][ty + i * Cfg::TY];
-          av[i][q].i = CX ? As[NC - 1][kk + q][ty + i * Cfg::TY] : E(0);
-        }
-#pragma unroll
-        for (int j = 0; j < TN; j++) {
-          bv[j][q].r = Bs[0][kk + q][tx + j * Cfg::TX];
-          bv[j][q].i = CX ? Bs[NC - 1][kk + q][tx + j * Cfg::TX] : E(0);
-        }
-      }
-      E p[NA][4 * D];
-#pragma unroll
-      for (int i = 0; i < TM; i++)
-#pragma unroll
-        for (int j = 0; j < TN; j++)
-#pragma unroll
-          for (int q = 0; q < 4; q++) {
-            E v[NC][4 * D];
-            products<E, CX, 4 * D>(av[i][q], bv[j][q], v, q);
-#pragma unroll
-            for (int c = 0; c < NC; c++)
-#pragma unroll
-              for (int d = 0; d < D; d++) p[(i * TN + j) * NC + c][q * D + d] = v[c][q * D + d];
-          }
-      tileN<E, F, 4 * D, NA>(acc, p);
-    }
-    __syncthreads();
-  }
-
-#pragma unroll
-  for (int i = 0; i < TM; i++)
-#pragma unroll
-    for (int j = 0; j < TN; j++) {
-      const long long gi = m0 + ty + i * Cfg::TY, gj = n0 + tx + j * Cfg::TX;
-      if (gi < g.M && gj < g.N) {
-        Acc<E, F>* e = acc + (i * TN + j) * NC;
-#pragma unroll
-        for (int q = 0; q < NC; q++) e[q].renorm();
-        const long long off = gi * g.sci + gj * g.scj;
-        finish<E, CX, F>(e, g.mode, g.C + off * NC, g.br, g.bi, g.Cbin + off * 2 * F * NC);
-      }
-    }
-}
-
 template <typename E, bool CX, int F>
 cudaError_t launch_xgemv(const XGemvArgs<E>& g, bool rows, dim3 grid, cudaStream_t s) {
   if (rows) {
@@ -833,27 +506,10 @@ cudaError_t launch_xscale(const E* x, long long n, long long incx, E ar, E ai, i
   return cudaGetLastError();
 }
 
-// Register budget: real folds up to 4 and complex folds up to 3 take 2x2 / 1x2 entries per
-// thread; larger folds one entry.
-template <typename E, bool CX, int F>
-struct XGemmShape {
-  static constexpr bool big = CX ? F <= 3 : F <= 4;
-  static constexpr int TM = big && !CX ? 2 : 1;
-  static constexpr int TN = big ? 2 : 1;
-};
-
-template <typename E, bool CX, int F>
-cudaError_t launch_xgemm(const XGemmArgs<E>& g, cudaStream_t s) {
-  using Sh = XGemmShape<E, CX, F>;
-  using Cfg = XGemmCfg<E, CX, Sh::TM, Sh::TN>;
-  dim3 grid((unsigned)((g.N + Cfg::BN - 1) / Cfg::BN), (unsigned)((g.M + Cfg::BM - 1) / Cfg::BM));
-  xgemm_kernel<E, CX, F, Sh::TM, Sh::TN><<<grid, 256, 0, s>>>(g);
-  return cudaGetLastError();
-}
-
 template <typename E, bool CX, int F>
 constexpr XOps<E> make_xops() {
-  return XOps<E>{launch_xgemv<E, CX, F>, launch_xgemm<E, CX, F>, launch_xscale<E, CX>};
+  return XOps<E>{launch_xgemv<E, CX, F>, gt::plan_gemm<E, CX, F>, gt::launch_gemm<E, CX, F>,
+                 launch_xscale<E, CX>};
 }
 
 }  // namespace xb
