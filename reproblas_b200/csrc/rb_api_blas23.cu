@@ -1,113 +1,202 @@
-// rb_api_blas23.cu -- C ABI for the binned dgemv / dgemm (reproBLAS_* / binnedBLAS_* names).
+// rb_api_blas23.cu -- C ABI for the binned gemv / gemm of every element type:
+// reproBLAS_r[dszc]gemv, r[dszc]gemm, [dszc]gemv, [dszc]gemm and binnedBLAS_dbdgemv, sbsgemv,
+// zbzgemv, cbcgemv, dbdgemm, sbsgemm, zbzgemm, cbcgemm (include/reproBLAS.h:61-93, 130-161;
+// include/binnedBLAS.h:99-133).
 //
-// Both orders and transposes are mapped onto the kernels' canonical forms the way the
-// reference does it: column-major is row-major with the transpose flipped
-// (src/binnedBLAS/dbdgemv.ccog:146-158); dgemm uses general operand strides. Host operands
-// are copied to a device workspace first; outputs are copied back before returning.
+// Orders and transposes map onto the kernels' forms the way the reference does it:
+// column-major is row-major with the transpose flipped (dbdgemv.ccog:146-158,
+// zbzgemv.ccog:184-196), gemm takes general operand strides. TransA / TransB: 'n'/'N' no transpose, 't'/'T' transpose, anything else the
+// conjugate transpose (the reference's default branches; for real elements every non-'n'
+// form is the transpose). Complex alpha and beta are read from host memory as two adjacent
+// reals, like the reference does. Host operands are copied to a device workspace first;
+// outputs are copied back before returning.
+//
+// One deliberate difference: the reference's column-major conjugate-transpose zbzgemv /
+// cbcgemv cut each column's dot into blocks of MIN(X_BLOCK, N - j) elements while j runs
+// over the M rows (zbzgemv.ccog:214-218, cbcgemv.ccog:214-218), which equals the mathematical
+// A^H x only when M == N. Here every entry is the full A^H x.
 #include <cstring>
-#include <map>
 #include <string>
-#include <utility>
 
+#include "rb_gemv_stream.cuh"
 #include "rb_host.h"
 #include "../../include/reproblas_b200.h"
 
 namespace rb {
 namespace {
 
-const Blas23FoldOps* ops23(int fold) {
-  switch (fold) {
-    case 2: return &blas23_fold2;
-    case 3: return &blas23_fold3;
-    case 4: return &blas23_fold4;
-    case 5: return &blas23_fold5;
-    case 6: return &blas23_fold6;
-    case 7: return &blas23_fold7;
-    case 8: return &blas23_fold8;
-    default: return nullptr;
+bool xrow(char o) { return o == 'r' || o == 'R'; }
+bool xnt(char t) { return t == 'n' || t == 'N'; }
+bool xplain_t(char t) { return t == 't' || t == 'T'; }
+
+// The fixed-fold kernels (folds 2..8); nullptr above them, where the run-time fold path runs.
+template <typename E, bool CX>
+const XOps<E>* xops_for(int fold) {
+  if (fold < 2 || fold > kMaxFold) return nullptr;
+  if constexpr (sizeof(E) == 8) {
+    static const XOps<double>* const d[] = {&xops_d_f2, &xops_d_f3, &xops_d_f4, &xops_d_f5,
+                                            &xops_d_f6, &xops_d_f7, &xops_d_f8};
+    static const XOps<double>* const z[] = {&xops_z_f2, &xops_z_f3, &xops_z_f4, &xops_z_f5,
+                                            &xops_z_f6, &xops_z_f7, &xops_z_f8};
+    return (CX ? z : d)[fold - 2];
+  } else {
+    static const XOps<float>* const s[] = {&xops_s_f2, &xops_s_f3, &xops_s_f4, &xops_s_f5,
+                                           &xops_s_f6, &xops_s_f7, &xops_s_f8};
+    static const XOps<float>* const c[] = {&xops_c_f2, &xops_c_f3, &xops_c_f4, &xops_c_f5,
+                                           &xops_c_f6, &xops_c_f7, &xops_c_f8};
+    return (CX ? c : s)[fold - 2];
   }
 }
 
-bool is_row(char o) { return o == 'r' || o == 'R'; }
-bool is_nt(char t) { return t == 'n' || t == 'N'; }
+// alpha / beta: real scalars, or the two reals a complex pointer addresses
+template <typename E, bool CX>
+struct Scalar {
+  E r, i;
+};
+template <typename E, bool CX>
+Scalar<E, CX> read_scalar(E v) { return {v, E(0)}; }
+template <typename E, bool CX>
+Scalar<E, CX> read_scalar(const void* p) {
+  const E* q = (const E*)p;
+  return {q[0], q[1]};
+}
 
-struct GemvReq {
+template <typename E, bool CX>
+struct XGemvReq {
   int fold;
   char order, trans;
   int M, N;
-  double alpha;
-  const double* A;
+  Scalar<E, CX> alpha;
+  const void* A;
   int lda;
-  const double* X;
+  const void* X;
   int incX;
-  double beta;
-  double* Y;        // values (kOutValue) or binned states (kOutBinned)
+  Scalar<E, CX> beta;
+  void* Y;          // values (kOutValue) or binned states (kOutBinned)
   int incY;
   int mode;
 };
 
-// fl(alpha * x_i) into a contiguous buffer zero-padded to npad entries, for the TMA-fed
-// kernels when x is strided or misaligned; the product is the one dbdgemv forms before its
-// dots.
-__global__ void scale_x_kernel(const double* x, long long n, long long incx, double alpha,
-                               double* bx, long long npad) {
-  const long long step = (long long)gridDim.x * blockDim.x;
-  for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < npad; i += step) {
-    double v = 0.0;
-    if (i < n) {
-      v = x[i * incx];
-      if (alpha != 1.0) v = __dmul_rn(v, alpha);
+unsigned gemv_slot(bool rows, int G, int es, int phases) {
+  return rows ? gs::slot_bytes<true>(G, es, phases) : gs::slot_bytes<false>(G, es, phases);
+}
+
+// Tensor maps of the stored Rs x Cs matrix, one per phase of its rows, in 8-byte words (the
+// copies move bits, whatever the element type): phase h starts at the 16-byte boundary at or
+// before row h and its rows span the elements' bytes from there.
+bool gemv_maps(GemvMaps* maps, const void* A, size_t es, long long Rs, long long Cs, long long lda,
+               int phases, bool rows, int G) {
+  auto enc = tensor_map_encoder();
+  if (!enc) {
+    set_error(RB_ERR_CUDA, "gemv: cuTensorMapEncodeTiled is unavailable");
+    return false;
+  }
+  // box: a stage's rows of one phase, slots of the width the kernel expects (slot_bytes); rows
+  // kernel, one phase: 128 bytes of a group's rows, swizzled
+  const bool swz = rows && phases == 1;
+  const cuuint32_t slot = swz ? 128u : gemv_slot(rows, G, (int)es, phases);
+  const cuuint32_t stage_rows = rows ? 512u / G : (cuuint32_t)(128 / es) * G;
+  for (int h = 0; h < phases && h < Rs; h++) {
+    const uintptr_t row = (uintptr_t)A + (size_t)h * lda * es;
+    const size_t shift = row % 16;
+    cuuint64_t dims[2] = {(cuuint64_t)((shift + (size_t)Cs * es + 7) / 8),
+                          (cuuint64_t)((Rs - h + phases - 1) / phases)};
+    cuuint64_t strides[1] = {(cuuint64_t)phases * lda * es};
+    cuuint32_t box[2] = {slot / 8, stage_rows / phases};
+    cuuint32_t estr[2] = {1u, 1u};
+    const CUresult r = enc(&maps->m[h], CU_TENSOR_MAP_DATA_TYPE_FLOAT64, 2, (void*)(row - shift), dims,
+                           strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                           swz ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_NONE,
+                           CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    if (r != CUDA_SUCCESS) {
+      set_error(RB_ERR_CUDA, "gemv: cuTensorMapEncodeTiled failed (" + std::to_string((int)r) + ")");
+      return false;
     }
-    bx[i] = v;
   }
+  // fewer rows than phases: the other phases hold no row (their boxes are loaded all the same,
+  // into slots that nothing reads)
+  for (int h = (int)Rs; h < phases; h++) maps->m[h] = maps->m[0];
+  return true;
 }
 
-// CTAs per SM of the TMA-fed kernels, per (device, fold); the first query also opts the
-// kernels in to their shared memory on that device. Returns -1 on a CUDA error (recorded),
-// 0 when a kernel does not fit on an SM, 1 otherwise.
-int stream_occupancy(const Blas23FoldOps* o, int device, int fold, int* rows_per_sm,
-                      int* cols_per_sm) {
-  static std::mutex mu;
-  static std::map<std::pair<int, int>, std::pair<int, int>> cache;
-  std::lock_guard<std::mutex> g(mu);
-  auto key = std::make_pair(device, fold);
-  auto it = cache.find(key);
-  if (it == cache.end()) {
-    int r = 0, c = 0;
-    if (!cuda_ok(o->gemv_stream_prepare(&r, &c), "gemv stream kernel attributes")) return -1;
-    it = cache.emplace(key, std::make_pair(r, c)).first;
+template <typename E, bool CX>
+bool run_xgemv(const XGemvReq<E, CX>& q) {
+  constexpr int NC = CX ? 2 : 1;
+  if (q.M == 0 || q.N == 0) return true;   // r[szc]gemv.c: early return
+  const int maxf = sizeof(E) == 8 ? kMaxFoldD : kMaxFoldS;
+  if (q.fold < 2 || q.fold > maxf) {
+    set_error(RB_ERR_INVALID_ARG, "fold must be in [2, " + std::to_string(maxf) + "]");
+    return false;
   }
-  *rows_per_sm = it->second.first;
-  *cols_per_sm = it->second.second;
-  return (*rows_per_sm > 0 && *cols_per_sm > 0) ? 1 : 0;
-}
-
-// dgemv through the TMA-fed kernels (rb_gemv_stream.cuh). The caller checked: alpha != 0,
-// lda even, A 16-byte aligned (or on the host), dimensions below 2^31.
-bool run_gemv_stream(const GemvReq& q, const Blas23FoldOps* o, Workspace* w, const DeviceInfo& di,
-                     bool nt, long long Rs, long long Cs, int rows_per_sm, int cols_per_sm) {
-  cudaStream_t s = w->stream;
+  const XOps<E>* o = xops_for<E, CX>(q.fold);
+  if (q.M < 0 || q.N < 0 || q.lda < 1 || q.incX < 0 || q.incY < 1) {
+    set_error(RB_ERR_INVALID_ARG, "gemv: negative size, lda < 1, incX < 0 or incY < 1");
+    return false;
+  }
+  // row-major view of the stored matrix: Rs rows x Cs columns
+  bool nt = xnt(q.trans);
+  const bool conj = CX && !nt && !xplain_t(q.trans);
+  long long Rs = q.M, Cs = q.N;
+  if (!xrow(q.order)) { Rs = q.N; Cs = q.M; nt = !nt; }
+  if (q.lda < Cs) { set_error(RB_ERR_INVALID_ARG, "gemv: lda smaller than the row length"); return false; }
   const long long nout = nt ? Rs : Cs, nred = nt ? Cs : Rs;
-  const long long REC = 2 * q.fold + 1;
-  GemvStreamArgs g{};
-  g.R = Rs;
-  g.C = Cs;
-  // G thread groups per output (2, 4 or 8): units are bands of P = 512/G rows (stages of
-  // 16G columns) or blocks of P columns (stages of 16G rows), split evenly over one CTA per
-  // resident slot (every CTA gets at least one stage). Take the smallest G for which the
-  // last CTA of a cut unit merges at most about 4 parts per thread.
-  const long long gmax = (long long)di.sms * (nt ? rows_per_sm : cols_per_sm);
+  const bool alpha_zero = q.alpha.r == E(0) && q.alpha.i == E(0);
+  const long long nred_eff = alpha_zero ? 0 : nred;            // [szc]b[szc]gemv: alpha == 0
+  if (q.mode == kOutBinned && nred_eff == 0) return true;       // binned form touches nothing
+  if (!o) {
+    // folds above the register-resident kernels: one thread per entry (rb_foldn.cu)
+    EntryReq<E> e{};
+    e.fold = q.fold;
+    e.mode = q.mode;
+    e.M = nout; e.N = 1; e.K = nred_eff;
+    e.A = q.A; e.sai = nt ? q.lda : 1; e.sak = nt ? 1 : q.lda;
+    e.B = q.X; e.sbk = q.incX; e.sbj = 0;
+    e.ar = q.alpha.r; e.ai = q.alpha.i; e.br = q.beta.r; e.bi = q.beta.i;
+    e.alpha_on_b = true;
+    e.conja = conj;
+    e.C = q.Y; e.sci = q.incY; e.scj = 0;
+    return run_entries_n<E, CX>(e);
+  }
+
+  std::unique_lock<std::mutex> lock;
+  Workspace* w = acquire_workspace(&lock);
+  if (!w) return false;
+  cudaStream_t s = w->stream;
+  DeviceInfo di;
+  if (!device_info(&di)) return false;
+
+  const size_t es = sizeof(E) * NC;
+  const size_t per_state = (size_t)2 * q.fold * es;
+  const size_t a_bytes = nred_eff > 0 ? ((size_t)(Rs - 1) * q.lda + Cs) * es : 0;
+  const size_t x_bytes = span(nred_eff, q.incX, es);
+  const size_t y_bytes = q.mode == kOutValue ? span(nout, q.incY, es)
+                                             : ((size_t)(nout - 1) * q.incY + 1) * per_state;
+  // Decomposition (rb_gemv_stream.cuh): G thread groups per output; units are bands or blocks
+  // of P = 512/G outputs, stages cover 128/es*G elements of the reduction, and the stages of
+  // all units are split evenly over one CTA per SM (every CTA gets at least one). Take the
+  // smallest G for which the last CTA of a cut unit merges at most about 4 parts per thread.
+  const long long pe = 128 / (long long)es;
   long long nunits = 0, nb = 0, T = 0, grid = 0, parts = 0;
   auto shape = [&](int G) {
     const long long P = 512 / G;
     nunits = (nout + P - 1) / P;
-    nb = (nred + 16 * G - 1) / (16 * G);   // stages of 16G columns (rows) / 16G rows (cols)
+    nb = nred_eff > 0 ? (nred_eff + pe * G - 1) / (pe * G) : 1;
     T = nunits * nb;
-    grid = T < gmax ? T : gmax;
+    grid = T < di.sms ? T : di.sms;
     // a unit meets at most ceil((nb-1) / min_range) + 1 CTA ranges, min_range = floor(T/grid)
     parts = nb / (T / grid) + 2;
   };
+  // phases the rows are taken in: the fewest whose pitch is a multiple of 16 bytes, at least
+  // two when A itself is misaligned (host operands are copied to aligned device memory)
+  const bool a_dev = a_bytes && on_device(q.A);
+  const uintptr_t a_mis = a_dev ? (uintptr_t)q.A % 16 : 0;
+  int phases = 1;
+  while (((size_t)phases * q.lda * es) % 16 != 0) phases *= 2;
+  if (phases == 1 && a_mis != 0) phases = 2;
+  // columns: a box is at most 256 words of 8 bytes wide, and a thread's rows are of one phase
   int G = 2;
+  if (!nt)
+    while (gemv_slot(false, G, (int)es, phases) > 2048 || G < phases) G *= 2;
   for (;;) {
     shape(G);
     if ((parts + G - 1) / G <= 4 || G == 8) break;
@@ -126,81 +215,53 @@ bool run_gemv_stream(const GemvReq& q, const Blas23FoldOps* o, Workspace* w, con
       shape(G);
     }
   }
-  g.groups = G;
-  g.kslots = nb / (T / grid) + 2;
-  const long long ntickets = nunits;
-  const size_t part_bytes = (size_t)nout * g.kslots * REC * 8;
-  if (!w->ensure_tickets((size_t)ntickets)) return false;
-
-  const size_t per_out = q.mode == kOutValue ? 8 : (size_t)2 * q.fold * 8;
-  const size_t a_bytes = ((size_t)(Rs - 1) * q.lda + Cs) * 8;
-  const size_t x_bytes = span(nred, q.incX, 8);
-  const size_t y_bytes = q.mode == kOutValue ? span(nout, q.incY, 8)
-                                             : ((size_t)(nout - 1) * q.incY + 1) * per_out;
-  const bool a_host = !on_device(q.A), x_host = !on_device(q.X), y_host = !on_device(q.Y);
-  // x is read in place when unit-stride and 16-byte aligned (host copies are aligned);
-  // otherwise fl(alpha*x) is gathered into bx by a small kernel first
-  const bool x_direct = q.incX == 1 && (x_host || ((uintptr_t)q.X % 16) == 0);
-  const size_t need = part_bytes + (x_direct ? 0 : (size_t)nred * 8) + (a_host ? a_bytes : 0) +
-                      (x_host ? x_bytes : 0) + (y_host ? y_bytes : 0) + 6 * 256;
+  const long long kslots = nb / (T / grid) + 2;
+  const size_t part_bytes = (size_t)nout * kslots * NC * (2 * q.fold + 1) * sizeof(E);
+  if (!w->ensure_tickets((size_t)nunits * 16)) return false;   // one per unit and consumer warp
+  const bool a_host = a_bytes && !a_dev, x_host = x_bytes && !on_device(q.X);
+  const bool y_host = !on_device(q.Y);
+  const size_t need = part_bytes + (a_host ? a_bytes : 0) + (x_host ? x_bytes : 0) +
+                      (y_host ? y_bytes : 0) + 4 * 256;
   if (!w->ensure_big(need)) return false;
   Bump b{w->big};
   bool ok = true;
-  const double* dA = (const double*)to_device(q.A, a_bytes, &b, s, &ok);
-  const double* dX = (const double*)to_device(q.X, x_bytes, &b, s, &ok);
-  double* dY = (double*)to_device(q.Y, y_bytes, &b, s, &ok);
-  double* bx = x_direct ? nullptr : (double*)b.take((size_t)nred * 8);
-  double* part = (double*)b.take(part_bytes);
+  const E* dA = (const E*)to_device(q.A, a_bytes, &b, s, &ok);
+  const E* dX = (const E*)to_device(q.X, x_bytes, &b, s, &ok);
+  E* dY = (E*)to_device(q.Y, y_bytes, &b, s, &ok);
+  E* part = (E*)b.take(part_bytes);
   if (!ok) return false;
 
-  auto enc = tensor_map_encoder();
-  if (!enc) {
-    set_error(RB_ERR_CUDA, "gemv: cuTensorMapEncodeTiled is unavailable");
-    return false;
-  }
-  CUtensorMap tm, tmx;
-  cuuint64_t dims[2] = {(cuuint64_t)Cs, (cuuint64_t)Rs};
-  cuuint64_t strides[1] = {(cuuint64_t)q.lda * 8};
-  // rows kernel: boxes of 16 columns x P rows, 128-byte swizzle; cols kernel: P x 16G
-  const cuuint32_t P = 512u / (cuuint32_t)G;
-  cuuint32_t box[2] = {nt ? 16u : P, nt ? P : 16u * (cuuint32_t)G};
-  cuuint32_t estr[2] = {1u, 1u};
-  CUresult r = enc(&tm, CU_TENSOR_MAP_DATA_TYPE_FLOAT64, 2, (void*)dA, dims, strides, box, estr,
-                   CU_TENSOR_MAP_INTERLEAVE_NONE,
-                   nt ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_NONE,
-                   CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-  // x (or bx): boxes of one stage's 16G entries (a rank-1 map reads no stride)
-  cuuint64_t xdims[1] = {(cuuint64_t)nred};
-  cuuint32_t xbox[1] = {16u * (cuuint32_t)G};
-  if (r == CUDA_SUCCESS)
-    r = enc(&tmx, CU_TENSOR_MAP_DATA_TYPE_FLOAT64, 1, (void*)(x_direct ? dX : bx), xdims, strides,
-            xbox, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
-            CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-  if (r != CUDA_SUCCESS) {
-    set_error(RB_ERR_CUDA, "gemv: cuTensorMapEncodeTiled failed (" + std::to_string((int)r) + ")");
-    return false;
-  }
-
-  g.alpha = q.alpha;
-  g.scale_x = x_direct && q.alpha != 1.0;
-  g.beta = q.beta;
+  XGemvArgs<E> g{};
+  g.R = nt ? nout : nred_eff;
+  g.C = nt ? nred_eff : nout;
+  g.A = dA;
+  g.lda = q.lda;
+  g.x = dX;
+  g.incx = q.incX;
+  g.ar = q.alpha.r;
+  g.ai = q.alpha.i;
+  g.br = q.beta.r;
+  g.bi = q.beta.i;
+  g.alpha_one = q.alpha.r == E(1) && q.alpha.i == E(0);
+  g.conj = conj ? 1 : 0;
   g.mode = q.mode;
   g.y = q.mode == kOutValue ? dY : nullptr;
   g.ybin = q.mode == kOutBinned ? dY : nullptr;
   g.incy = q.incY;
+  g.nb = (int)nb;
+  g.q = (int)(T / grid);
+  g.rem = (int)(T % grid);
   g.scratch = part;
+  g.kslots = kslots;
   g.tickets = w->tickets;
   g.status = w->dstatus();
+  g.groups = G;
+  g.phases = phases;
   pipeline_fault(&g.stop_after, &g.wait_polls);
-  if (!x_direct) {
-    count_launch();
-    long long sgrid = (nred + 255) / 256;
-    if (sgrid > (long long)di.sms * 4) sgrid = (long long)di.sms * 4;
-    scale_x_kernel<<<(unsigned)sgrid, 256, 0, s>>>(dX, nred, q.incX, q.alpha, bx, nred);
-    if (!cuda_ok(cudaGetLastError(), "gemv scale launch")) return false;
-  }
+  GemvMaps maps{};
+  if (nred_eff > 0 && !gemv_maps(&maps, dA, (size_t)es, Rs, Cs, q.lda, phases, nt, G)) return false;
   count_launch();
-  if (!cuda_ok(o->gemv_stream(g, tm, tmx, nt, (int)grid, s), "gemv launch")) return false;
+  if (!cuda_ok(o->gemv(g, maps, nt, (int)grid, s), "gemv launch")) return false;
   if (y_host) {
     int* hs = w->hstatus();
     if (!cuda_ok(cudaMemcpyAsync(q.Y, dY, y_bytes, cudaMemcpyDeviceToHost, s), "copy y") ||
@@ -208,7 +269,7 @@ bool run_gemv_stream(const GemvReq& q, const Blas23FoldOps* o, Workspace* w, con
         !cuda_ok(cudaStreamSynchronize(s), "cudaStreamSynchronize"))
       return false;
     if (*hs != 0) {
-      cudaMemsetAsync(w->dstatus(), 0, 4, s);
+      w->reset_after_abort();
       set_error(RB_ERR_CUDA, "gemv: a pipeline wait timed out (affected entries are NaN)");
       return false;
     }
@@ -216,186 +277,42 @@ bool run_gemv_stream(const GemvReq& q, const Blas23FoldOps* o, Workspace* w, con
   return true;
 }
 
-bool run_gemv(const GemvReq& q) {
-  if (q.M == 0 || q.N == 0) return true;   // rdgemv.c:43-45
-  if (q.fold < 2 || q.fold > kMaxFoldD) {
-    set_error(RB_ERR_INVALID_ARG, "fold must be in [2, 52]");
-    return false;
-  }
-  const Blas23FoldOps* o = q.fold <= kMaxFold ? ops23(q.fold) : nullptr;
-  if (q.M < 0 || q.N < 0 || q.lda < 1 || q.incX < 0 || q.incY < 1) {
-    set_error(RB_ERR_INVALID_ARG, "gemv: negative size, lda < 1, incX < 0 or incY < 1");
-    return false;
-  }
-  // row-major view of the stored matrix: Rs rows x Cs columns
-  bool nt = is_nt(q.trans);
-  long long Rs = q.M, Cs = q.N;
-  if (!is_row(q.order)) { Rs = q.N; Cs = q.M; nt = !nt; }
-  if (q.lda < Cs) { set_error(RB_ERR_INVALID_ARG, "gemv: lda smaller than the row length"); return false; }
-  const long long nout = nt ? Rs : Cs, nred = nt ? Cs : Rs;
-  const long long nred_eff = q.alpha == 0.0 ? 0 : nred;   // dbdgemv.ccog:70-72
-  if (q.mode == kOutBinned && nred_eff == 0) return true;  // binnedBLAS_dbdgemv touches nothing
-  if (!o) {
-    // folds above the register-resident kernels: one thread per entry (rb_foldn.cu)
-    EntryReq<double> e{};
-    e.fold = q.fold;
-    e.mode = q.mode;
-    e.M = nout; e.N = 1; e.K = nred_eff;
-    e.A = q.A; e.sai = nt ? q.lda : 1; e.sak = nt ? 1 : q.lda;
-    e.B = q.X; e.sbk = q.incX; e.sbj = 0;
-    e.ar = q.alpha; e.br = q.beta;
-    e.alpha_on_b = true;
-    e.C = q.Y; e.sci = q.incY; e.scj = 0;
-    return run_entries_n<double, false>(e);
-  }
-
-  std::unique_lock<std::mutex> lock;
-  Workspace* w = acquire_workspace(&lock);
-  if (!w) return false;
-  cudaStream_t s = w->stream;
-
-  const size_t per_out = q.mode == kOutValue ? 8 : (size_t)2 * q.fold * 8;
-  const size_t a_bytes = nred_eff > 0 ? ((size_t)(Rs - 1) * q.lda + Cs) * 8 : 0;
-  const size_t x_bytes = span(nred_eff, q.incX, 8);
-  const size_t y_bytes = q.mode == kOutValue ? span(nout, q.incY, 8)
-                                             : ((size_t)(nout - 1) * q.incY + 1) * per_out;
-  // column kernel partials
-  int col_blocks = 0, nchunks = 1;
-  size_t part_bytes = 0;
-  DeviceInfo di;
-  if (!device_info(&di)) return false;
-  // 16-byte loads when rows (and x for the row kernel) are 16-byte aligned
-  const bool a_al = (q.lda % 2) == 0;
-  const bool vec = nt ? (a_al && q.incX == 1) : (a_al && (nout % 2) == 0);
-  // TMA-fed kernels: row pitch a multiple of 16 bytes, A 16-byte aligned (host operands are
-  // copied to aligned device memory), tensor coordinates within int, and rows long enough /
-  // outputs numerous enough to fill the ring's boxes
-  const bool a_ptr_al = !on_device(q.A) || ((uintptr_t)q.A % 16) == 0;
-  if (o->gemv_stream && nred_eff > 0 && a_al && a_ptr_al && Rs < (1ll << 31) && Cs < (1ll << 31) &&
-      (nt ? nred_eff >= 512 : nout >= 128)) {
-    int rps = 0, cps = 0;
-    const int occ = stream_occupancy(o, di.device, q.fold, &rps, &cps);
-    if (occ < 0) return false;
-    if (occ > 0) return run_gemv_stream(q, o, w, di, nt, Rs, Cs, rps, cps);
-  }
-  int groups = 1;
-  if (!nt) {
-    // Column kernel shape: G row groups per CTA, T = 256/G threads per group, W columns per
-    // thread. Cost model in units of one row per thread: the streaming part (waves of CTAs
-    // times rows per thread, plus the in-CTA tree merge) and the serial merge of the chunk
-    // partials in the last CTA of each column block (about 4 units per merge).
-    const long long W = vec ? 2 : 1;
-    const long long slots = (long long)di.sms * 3;
-    long long best = -1;
-    for (int G = 1; G <= 8; G *= 2) {
-      const long long cols = (256 / G) * W;
-      const long long cb = (nout + cols - 1) / cols;
-      const long long maxch = (nred_eff + 8 * G - 1) / (8 * G);   // >= 8 rows per group
-      const long long lg = G == 1 ? 0 : G == 2 ? 1 : G == 4 ? 2 : 3;
-      // chunks: fill the slots exactly once (floor) or just over (ceil)
-      for (long long ch : {slots / cb, (slots + cb - 1) / cb}) {
-        if (ch > maxch) ch = maxch;
-        if (ch < 1) ch = 1;
-        const long long rpt = ((nred_eff + ch - 1) / ch + G - 1) / G;
-        const long long waves = (cb * ch + slots - 1) / slots;
-        const long long cost = waves * (rpt + 8 * lg) + 4 * ((ch + G - 1) / G + 2 * lg);
-        if (best < 0 || cost < best) {
-          best = cost;
-          groups = G;
-          col_blocks = (int)cb;
-          nchunks = (int)ch;
-        }
-      }
-    }
-    part_bytes = (size_t)nchunks * nout * (2 * q.fold + 1) * 8;
-    if (!w->ensure_tickets((size_t)col_blocks)) return false;
-  }
-  const bool a_host = a_bytes && !on_device(q.A), x_host = x_bytes && !on_device(q.X);
-  const bool y_host = !on_device(q.Y);
-  size_t need = part_bytes + (a_host ? a_bytes : 0) + (x_host ? x_bytes : 0) +
-                (y_host ? y_bytes : 0) + 4 * 256;
-  if (!w->ensure_big(need)) return false;
-  Bump b{w->big};
-  bool ok = true;
-  const double* dA = (const double*)to_device(q.A, a_bytes, &b, s, &ok);
-  const double* dX = (const double*)to_device(q.X, x_bytes, &b, s, &ok);
-  double* dY = (double*)to_device(q.Y, y_bytes, &b, s, &ok);
-  double* part = part_bytes ? (double*)b.take(part_bytes) : nullptr;
-  if (!ok) return false;
-
-  GemvArgs g{};
-  g.vec = vec && ((uintptr_t)dA % 16) == 0 && (!nt || ((uintptr_t)dX % 16) == 0);
-  g.A = dA;
-  g.lda = q.lda;
-  g.x = dX;
-  g.incx = q.incX;
-  g.alpha = q.alpha;
-  g.beta = q.beta;
-  g.mode = q.mode;
-  g.y = q.mode == kOutValue ? dY : nullptr;
-  g.ybin = q.mode == kOutBinned ? dY : nullptr;
-  g.incy = q.incY;
-  count_launch();
-  cudaError_t e;
-  if (nt) {
-    g.R = nout;
-    g.C = nred_eff;
-    long long target_warps = (long long)di.sms * 16;   // a warp per row is enough in flight
-    int S = 1;
-    while (S < 8 && nout * S < target_warps) S *= 2;
-    g.split = S;
-    const int rows_per_cta = 8 / S;
-    dim3 grid((unsigned)((nout + rows_per_cta - 1) / rows_per_cta));
-    e = o->gemv(g, true, grid, s);
-  } else {
-    g.C = nout;
-    g.R = nred_eff;
-    g.split = groups;
-    g.scratch = part;
-    g.tickets = w->tickets;
-    dim3 grid((unsigned)col_blocks, (unsigned)nchunks);
-    e = o->gemv(g, false, grid, s);
-  }
-  if (!cuda_ok(e, "gemv launch")) return false;
-  if (y_host) {
-    if (!cuda_ok(cudaMemcpyAsync(q.Y, dY, y_bytes, cudaMemcpyDeviceToHost, s), "copy y") ||
-        !cuda_ok(cudaStreamSynchronize(s), "cudaStreamSynchronize"))
-      return false;
-  }
-  return true;
-}
-
-struct GemmReq {
+template <typename E, bool CX>
+struct XGemmReq {
   int fold;
   char order, ta, tb;
   int M, N, K;
-  double alpha;
-  const double* A;
+  Scalar<E, CX> alpha;
+  const void* A;
   int lda;
-  const double* B;
+  const void* B;
   int ldb;
-  double beta;
-  double* C;       // values or binned states
+  Scalar<E, CX> beta;
+  void* C;          // values or binned states
   int ldc;
   int mode;
 };
 
-bool run_gemm(const GemmReq& q) {
-  if (q.M == 0 || q.N == 0) return true;   // rdgemm.c:50-52
-  if (q.fold < 2 || q.fold > kMaxFoldD) {
-    set_error(RB_ERR_INVALID_ARG, "fold must be in [2, 52]");
+template <typename E, bool CX>
+bool run_xgemm(const XGemmReq<E, CX>& q) {
+  constexpr int NC = CX ? 2 : 1;
+  if (q.M == 0 || q.N == 0) return true;   // r[szc]gemm.c: early return
+  const int maxf = sizeof(E) == 8 ? kMaxFoldD : kMaxFoldS;
+  if (q.fold < 2 || q.fold > maxf) {
+    set_error(RB_ERR_INVALID_ARG, "fold must be in [2, " + std::to_string(maxf) + "]");
     return false;
   }
-  const Blas23FoldOps* o = q.fold <= kMaxFold ? ops23(q.fold) : nullptr;
+  const XOps<E>* o = xops_for<E, CX>(q.fold);
   if (q.M < 0 || q.N < 0 || q.K < 0 || q.lda < 1 || q.ldb < 1 || q.ldc < 1) {
     set_error(RB_ERR_INVALID_ARG, "gemm: negative size or leading dimension < 1");
     return false;
   }
-  const bool row = is_row(q.order), ta = !is_nt(q.ta), tb = !is_nt(q.tb);
-  XGemmArgs<double> g{};
+  const bool row = xrow(q.order), ta = !xnt(q.ta), tb = !xnt(q.tb);
+  XGemmArgs<E> g{};
   g.M = q.M;
   g.N = q.N;
-  g.K = (q.alpha == 0.0) ? 0 : q.K;   // dbdgemm.ccog:78-80
+  const bool alpha_zero = q.alpha.r == E(0) && q.alpha.i == E(0);
+  g.K = alpha_zero ? 0 : q.K;   // [szc]b[szc]gemm: alpha == 0 deposits nothing
   if (row) {
     g.sai = ta ? 1 : q.lda;  g.sak = ta ? q.lda : 1;
     g.sbk = tb ? 1 : q.ldb;  g.sbj = tb ? q.ldb : 1;
@@ -405,41 +322,48 @@ bool run_gemm(const GemmReq& q) {
     g.sbk = tb ? q.ldb : 1;  g.sbj = tb ? 1 : q.ldb;
     g.sci = 1;               g.scj = q.ldc;
   }
-  g.ar = q.alpha;
-  g.alpha_one = q.alpha == 1.0;
-  g.br = q.beta;
+  g.ar = q.alpha.r;
+  g.ai = q.alpha.i;
+  g.br = q.beta.r;
+  g.bi = q.beta.i;
+  g.alpha_one = q.alpha.r == E(1) && q.alpha.i == E(0);
+  g.conja = (CX && ta && !xplain_t(q.ta)) ? 1 : 0;
+  g.conjb = (CX && tb && !xplain_t(q.tb)) ? 1 : 0;
   g.mode = q.mode;
-  if (q.mode == kOutBinned && g.K == 0) return true;   // binnedBLAS_dbdgemm touches nothing
+  if (q.mode == kOutBinned && g.K == 0) return true;   // binned form touches nothing
   if (!o) {
     // folds above the register-resident kernels: one thread per entry (rb_foldn.cu)
-    EntryReq<double> e{};
+    EntryReq<E> e{};
     e.fold = q.fold;
     e.mode = q.mode;
     e.M = g.M; e.N = g.N; e.K = g.K;
     e.A = q.A; e.sai = g.sai; e.sak = g.sak;
     e.B = q.B; e.sbk = g.sbk; e.sbj = g.sbj;
-    e.ar = q.alpha; e.br = q.beta;
+    e.ar = g.ar; e.ai = g.ai; e.br = g.br; e.bi = g.bi;
+    e.conja = g.conja != 0;
+    e.conjb = g.conjb != 0;
     e.C = q.C; e.sci = g.sci; e.scj = g.scj;
-    return run_entries_n<double, false>(e);
+    return run_entries_n<E, CX>(e);
   }
 
   std::unique_lock<std::mutex> lock;
   Workspace* w = acquire_workspace(&lock);
   if (!w) return false;
   cudaStream_t s = w->stream;
-  const size_t per = q.mode == kOutValue ? 8 : (size_t)2 * q.fold * 8;
-  const size_t a_bytes = g.K ? ((size_t)(g.M - 1) * g.sai + (size_t)(g.K - 1) * g.sak + 1) * 8 : 0;
-  const size_t b_bytes = g.K ? ((size_t)(g.K - 1) * g.sbk + (size_t)(g.N - 1) * g.sbj + 1) * 8 : 0;
+  const size_t es = sizeof(E) * NC;
+  const size_t per = q.mode == kOutValue ? es : (size_t)2 * q.fold * es;
+  const size_t a_bytes = g.K ? ((size_t)(g.M - 1) * g.sai + (size_t)(g.K - 1) * g.sak + 1) * es : 0;
+  const size_t b_bytes = g.K ? ((size_t)(g.K - 1) * g.sbk + (size_t)(g.N - 1) * g.sbj + 1) * es : 0;
   const size_t c_bytes = ((size_t)(g.M - 1) * g.sci + (size_t)(g.N - 1) * g.scj + 1) * per;
   const bool a_host = a_bytes && !on_device(q.A), b_host = b_bytes && !on_device(q.B);
   const bool c_host = !on_device(q.C);
-  size_t need = (a_host ? a_bytes : 0) + (b_host ? b_bytes : 0) + (c_host ? c_bytes : 0) + 3 * 256;
+  const size_t need = (a_host ? a_bytes : 0) + (b_host ? b_bytes : 0) + (c_host ? c_bytes : 0) + 3 * 256;
   if (need > 3 * 256 && !w->ensure_big(need)) return false;
   Bump bm{w->big};
   bool ok = true;
-  g.A = (const double*)to_device(q.A, a_bytes, &bm, s, &ok);
-  g.B = (const double*)to_device(q.B, b_bytes, &bm, s, &ok);
-  double* dC = (double*)to_device(q.C, c_bytes, &bm, s, &ok);
+  g.A = (const E*)to_device(q.A, a_bytes, &bm, s, &ok);
+  g.B = (const E*)to_device(q.B, b_bytes, &bm, s, &ok);
+  E* dC = (E*)to_device(q.C, c_bytes, &bm, s, &ok);
   if (!ok) return false;
   g.C = q.mode == kOutValue ? dC : nullptr;
   g.Cbin = q.mode == kOutBinned ? dC : nullptr;
@@ -455,17 +379,42 @@ bool run_gemm(const GemmReq& q) {
   return true;
 }
 
+template <typename E, bool CX, typename S>
+void gemv_entry(int fold, char Order, char TransA, int M, int N, S alpha, const void* A, int lda,
+                const void* X, int incX, S beta, void* Y, int incY, int mode) {
+  XGemvReq<E, CX> q{fold, Order, TransA, M, N, read_scalar<E, CX>(alpha), A, lda, X, incX,
+                    read_scalar<E, CX>(beta), Y, incY, mode};
+  run_xgemv<E, CX>(q);
+}
+
+template <typename E, bool CX, typename S>
+void gemm_entry(int fold, char Order, char TransA, char TransB, int M, int N, int K, S alpha,
+                const void* A, int lda, const void* B, int ldb, S beta, void* C, int ldc,
+                int mode) {
+  XGemmReq<E, CX> q{fold, Order, TransA, TransB, M, N, K, read_scalar<E, CX>(alpha), A, lda, B,
+                    ldb, read_scalar<E, CX>(beta), C, ldc, mode};
+  run_xgemm<E, CX>(q);
+}
+
+// beta of the binned forms: 1 (merge into the caller's states; unused in that mode)
+template <typename E, bool CX>
+const void* one_scalar() {
+  static const E one[2] = {E(1), E(0)};
+  return one;
+}
+
 }  // namespace
 }  // namespace rb
 
 extern "C" {
 
+// ---- FP64 real -------------------------------------------------------------------------------
 void reproBLAS_rdgemv(const int fold, const char Order, const char TransA, const int M,
                       const int N, const double alpha, const double* A, const int lda,
                       const double* X, const int incX, const double beta, double* Y,
                       const int incY) {
-  rb::GemvReq q{fold, Order, TransA, M, N, alpha, A, lda, X, incX, beta, Y, incY, rb::kOutValue};
-  rb::run_gemv(q);
+  rb::gemv_entry<double, false, double>(fold, Order, TransA, M, N, alpha, A, lda, X, incX, beta, Y,
+                                        incY, rb::kOutValue);
 }
 void reproBLAS_dgemv(const char Order, const char TransA, const int M, const int N,
                      const double alpha, const double* A, const int lda, const double* X,
@@ -475,16 +424,15 @@ void reproBLAS_dgemv(const char Order, const char TransA, const int M, const int
 void binnedBLAS_dbdgemv(const int fold, const char Order, const char TransA, const int M,
                         const int N, const double alpha, const double* A, const int lda,
                         const double* X, const int incX, double_binned* Y, const int incY) {
-  rb::GemvReq q{fold, Order, TransA, M, N, alpha, A, lda, X, incX, 1.0, Y, incY, rb::kOutBinned};
-  rb::run_gemv(q);
+  rb::gemv_entry<double, false, double>(fold, Order, TransA, M, N, alpha, A, lda, X, incX, 1.0, Y,
+                                        incY, rb::kOutBinned);
 }
 void reproBLAS_rdgemm(const int fold, const char Order, const char TransA, const char TransB,
                       const int M, const int N, const int K, const double alpha, const double* A,
                       const int lda, const double* B, const int ldb, const double beta,
                       double* C, const int ldc) {
-  rb::GemmReq q{fold, Order, TransA, TransB, M, N, K, alpha, A, lda, B, ldb, beta, C, ldc,
-                rb::kOutValue};
-  rb::run_gemm(q);
+  rb::gemm_entry<double, false, double>(fold, Order, TransA, TransB, M, N, K, alpha, A, lda, B, ldb,
+                                        beta, C, ldc, rb::kOutValue);
 }
 void reproBLAS_dgemm(const char Order, const char TransA, const char TransB, const int M,
                      const int N, const int K, const double alpha, const double* A,
@@ -496,9 +444,128 @@ void binnedBLAS_dbdgemm(const int fold, const char Order, const char TransA, con
                         const int M, const int N, const int K, const double alpha,
                         const double* A, const int lda, const double* B, const int ldb,
                         double_binned* C, const int ldc) {
-  rb::GemmReq q{fold, Order, TransA, TransB, M, N, K, alpha, A, lda, B, ldb, 1.0, C, ldc,
-                rb::kOutBinned};
-  rb::run_gemm(q);
+  rb::gemm_entry<double, false, double>(fold, Order, TransA, TransB, M, N, K, alpha, A, lda, B, ldb,
+                                        1.0, C, ldc, rb::kOutBinned);
+}
+
+// ---- FP32 real -------------------------------------------------------------------------------
+void reproBLAS_rsgemv(const int fold, const char Order, const char TransA, const int M,
+                      const int N, const float alpha, const float* A, const int lda,
+                      const float* X, const int incX, const float beta, float* Y,
+                      const int incY) {
+  rb::gemv_entry<float, false, float>(fold, Order, TransA, M, N, alpha, A, lda, X, incX, beta, Y,
+                                      incY, rb::kOutValue);
+}
+void reproBLAS_sgemv(const char Order, const char TransA, const int M, const int N,
+                     const float alpha, const float* A, const int lda, const float* X,
+                     const int incX, const float beta, float* Y, const int incY) {
+  reproBLAS_rsgemv(3, Order, TransA, M, N, alpha, A, lda, X, incX, beta, Y, incY);
+}
+void binnedBLAS_sbsgemv(const int fold, const char Order, const char TransA, const int M,
+                        const int N, const float alpha, const float* A, const int lda,
+                        const float* X, const int incX, float_binned* Y, const int incY) {
+  rb::gemv_entry<float, false, float>(fold, Order, TransA, M, N, alpha, A, lda, X, incX, 1.0f, Y,
+                                      incY, rb::kOutBinned);
+}
+void reproBLAS_rsgemm(const int fold, const char Order, const char TransA, const char TransB,
+                      const int M, const int N, const int K, const float alpha, const float* A,
+                      const int lda, const float* B, const int ldb, const float beta, float* C,
+                      const int ldc) {
+  rb::gemm_entry<float, false, float>(fold, Order, TransA, TransB, M, N, K, alpha, A, lda, B, ldb,
+                                      beta, C, ldc, rb::kOutValue);
+}
+void reproBLAS_sgemm(const char Order, const char TransA, const char TransB, const int M,
+                     const int N, const int K, const float alpha, const float* A, const int lda,
+                     const float* B, const int ldb, const float beta, float* C, const int ldc) {
+  reproBLAS_rsgemm(3, Order, TransA, TransB, M, N, K, alpha, A, lda, B, ldb, beta, C, ldc);
+}
+void binnedBLAS_sbsgemm(const int fold, const char Order, const char TransA, const char TransB,
+                        const int M, const int N, const int K, const float alpha, const float* A,
+                        const int lda, const float* B, const int ldb, float_binned* C,
+                        const int ldc) {
+  rb::gemm_entry<float, false, float>(fold, Order, TransA, TransB, M, N, K, alpha, A, lda, B, ldb,
+                                      1.0f, C, ldc, rb::kOutBinned);
+}
+
+// ---- FP64 complex ------------------------------------------------------------------------------
+void reproBLAS_rzgemv(const int fold, const char Order, const char TransA, const int M,
+                      const int N, const void* alpha, const void* A, const int lda,
+                      const void* X, const int incX, const void* beta, void* Y, const int incY) {
+  rb::gemv_entry<double, true, const void*>(fold, Order, TransA, M, N, alpha, A, lda, X, incX,
+                                            beta, Y, incY, rb::kOutValue);
+}
+void reproBLAS_zgemv(const char Order, const char TransA, const int M, const int N,
+                     const void* alpha, const void* A, const int lda, const void* X,
+                     const int incX, const void* beta, void* Y, const int incY) {
+  reproBLAS_rzgemv(3, Order, TransA, M, N, alpha, A, lda, X, incX, beta, Y, incY);
+}
+void binnedBLAS_zbzgemv(const int fold, const char Order, const char TransA, const int M,
+                        const int N, const void* alpha, const void* A, const int lda,
+                        const void* X, const int incX, double_complex_binned* Y,
+                        const int incY) {
+  rb::gemv_entry<double, true, const void*>(fold, Order, TransA, M, N, alpha, A, lda, X, incX,
+                                            rb::one_scalar<double, true>(), Y, incY,
+                                            rb::kOutBinned);
+}
+void reproBLAS_rzgemm(const int fold, const char Order, const char TransA, const char TransB,
+                      const int M, const int N, const int K, const void* alpha, const void* A,
+                      const int lda, const void* B, const int ldb, const void* beta, void* C,
+                      const int ldc) {
+  rb::gemm_entry<double, true, const void*>(fold, Order, TransA, TransB, M, N, K, alpha, A, lda,
+                                            B, ldb, beta, C, ldc, rb::kOutValue);
+}
+void reproBLAS_zgemm(const char Order, const char TransA, const char TransB, const int M,
+                     const int N, const int K, const void* alpha, const void* A, const int lda,
+                     const void* B, const int ldb, const void* beta, void* C, const int ldc) {
+  reproBLAS_rzgemm(3, Order, TransA, TransB, M, N, K, alpha, A, lda, B, ldb, beta, C, ldc);
+}
+void binnedBLAS_zbzgemm(const int fold, const char Order, const char TransA, const char TransB,
+                        const int M, const int N, const int K, const void* alpha, const void* A,
+                        const int lda, const void* B, const int ldb, double_complex_binned* C,
+                        const int ldc) {
+  rb::gemm_entry<double, true, const void*>(fold, Order, TransA, TransB, M, N, K, alpha, A, lda,
+                                            B, ldb, rb::one_scalar<double, true>(), C, ldc,
+                                            rb::kOutBinned);
+}
+
+// ---- FP32 complex ------------------------------------------------------------------------------
+void reproBLAS_rcgemv(const int fold, const char Order, const char TransA, const int M,
+                      const int N, const void* alpha, const void* A, const int lda,
+                      const void* X, const int incX, const void* beta, void* Y, const int incY) {
+  rb::gemv_entry<float, true, const void*>(fold, Order, TransA, M, N, alpha, A, lda, X, incX,
+                                           beta, Y, incY, rb::kOutValue);
+}
+void reproBLAS_cgemv(const char Order, const char TransA, const int M, const int N,
+                     const void* alpha, const void* A, const int lda, const void* X,
+                     const int incX, const void* beta, void* Y, const int incY) {
+  reproBLAS_rcgemv(3, Order, TransA, M, N, alpha, A, lda, X, incX, beta, Y, incY);
+}
+void binnedBLAS_cbcgemv(const int fold, const char Order, const char TransA, const int M,
+                        const int N, const void* alpha, const void* A, const int lda,
+                        const void* X, const int incX, float_complex_binned* Y, const int incY) {
+  rb::gemv_entry<float, true, const void*>(fold, Order, TransA, M, N, alpha, A, lda, X, incX,
+                                           rb::one_scalar<float, true>(), Y, incY,
+                                           rb::kOutBinned);
+}
+void reproBLAS_rcgemm(const int fold, const char Order, const char TransA, const char TransB,
+                      const int M, const int N, const int K, const void* alpha, const void* A,
+                      const int lda, const void* B, const int ldb, const void* beta, void* C,
+                      const int ldc) {
+  rb::gemm_entry<float, true, const void*>(fold, Order, TransA, TransB, M, N, K, alpha, A, lda,
+                                           B, ldb, beta, C, ldc, rb::kOutValue);
+}
+void reproBLAS_cgemm(const char Order, const char TransA, const char TransB, const int M,
+                     const int N, const int K, const void* alpha, const void* A, const int lda,
+                     const void* B, const int ldb, const void* beta, void* C, const int ldc) {
+  reproBLAS_rcgemm(3, Order, TransA, TransB, M, N, K, alpha, A, lda, B, ldb, beta, C, ldc);
+}
+void binnedBLAS_cbcgemm(const int fold, const char Order, const char TransA, const char TransB,
+                        const int M, const int N, const int K, const void* alpha, const void* A,
+                        const int lda, const void* B, const int ldb, float_complex_binned* C,
+                        const int ldc) {
+  rb::gemm_entry<float, true, const void*>(fold, Order, TransA, TransB, M, N, K, alpha, A, lda,
+                                           B, ldb, rb::one_scalar<float, true>(), C, ldc,
+                                           rb::kOutBinned);
 }
 
 }  // extern "C"

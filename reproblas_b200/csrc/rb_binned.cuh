@@ -453,54 +453,177 @@ __device__ __forceinline__ void tileN(Acc<T, F> (&a)[N], const T (&v)[N][K]) {
   for (int n = 0; n < N; n++) a[n].template tile<K>(v[n], K);
 }
 
-// Merge the renormalised accumulators a[n] of the 32 lanes of a warp, for N accumulators at
-// once; every lane ends with the merged states (a butterfly). The lanes first move to the
-// warp's coarsest index (dmdupdate: the alignment merge() performs per pair, done once) and
-// an empty accumulator becomes the zero state at that index (its primaries the bins, its
-// carries 0: merging it changes nothing). Every pair merge is then merge()'s equal-index
-// branch, the same arithmetic and renormalisation, on the primaries and carries alone, and
-// the N chains are interleaved. The non-finite classes are OR-ed once.
+// ---- merges of renormalised states in integers ------------------------------------------
+// A renormalised primary is bin + m * ulp with 0 <= m < 2^kQ (its two leading mantissa bits are
+// the bin's), and a carry counts units of 2^kQ ulps, so bin i of a state is the integer
+// m + car * 2^kQ and merging states of one index (dmdmadd) is integer addition: the m's and the
+// carries add separately, in any order, and one step at the end moves the overflow of the m's
+// into the carry, which gives dmdmadd's renormalised result. Unlike dmdmadd pair by pair this
+// has no renormalisation and no FP64 chain per pair. Carries are below 2^31 / 32 in every
+// state a kernel forms itself (a call deposits at most 2^32 values per state, and 2^kQ ulps
+// take 2^11 of the largest deposits, 2^9 in FP32).
+template <typename T> struct Fix;
+template <> struct Fix<double> {
+  using M = unsigned long long;
+  static constexpr int kQ = 50;
+};
+template <> struct Fix<float> {
+  using M = unsigned int;
+  static constexpr int kQ = 21;
+};
+template <typename T>
+__device__ __forceinline__ typename Fix<T>::M fix_of(T pri) {
+  return BT<T>::bits(pri) & (((typename Fix<T>::M)1 << Fix<T>::kQ) - 1);
+}
+// the primary of bin `bin` with (m mod 2^kQ); the rest of m goes to *carry
+template <typename T, typename C>
+__device__ __forceinline__ T fix_back(T bin, typename Fix<T>::M m, C* carry) {
+  constexpr int Q = Fix<T>::kQ;
+  *carry += (C)(int)(m >> Q);
+  return BT<T>::from(BT<T>::bits(bin) | (m & (((typename Fix<T>::M)1 << Q) - 1)));
+}
+
+// Running sum of renormalised states held by one thread (at most 2^11 of them).
+template <typename T, int F>
+struct SumAcc {
+  using B = BT<T>;
+  typename Fix<T>::M m[F];
+  T car[F];
+  int idx;
+  unsigned flags;
+  __device__ __forceinline__ void zero() {
+    idx = kEmpty;
+    flags = 0;
+  }
+  __device__ __forceinline__ void set(const Acc<T, F>& a) {
+    idx = a.idx;
+#pragma unroll
+    for (int i = 0; i < F; i++) {
+      m[i] = fix_of<T>(a.pri[i]);
+      car[i] = a.car[i];
+    }
+  }
+  __device__ __forceinline__ void get(Acc<T, F>& a) const {
+    a.zero();
+    a.flags = flags;
+    if (idx == kEmpty) return;
+#pragma unroll
+    for (int i = 0; i < F; i++) {
+      a.car[i] = car[i];
+      a.pri[i] = fix_back<T>(B::bin(idx + i), m[i], &a.car[i]);
+    }
+    a.set_idx(idx);
+  }
+  __device__ __forceinline__ void add(const Acc<T, F>& o) {
+    flags |= o.flags;
+    if (o.idx == kEmpty) return;
+    if (idx == kEmpty) {
+      set(o);
+    } else if (idx == o.idx) {
+#pragma unroll
+      for (int i = 0; i < F; i++) {
+        m[i] += fix_of<T>(o.pri[i]);
+        car[i] = B::add(car[i], o.car[i]);
+      }
+    } else {
+      Acc<T, F> t;
+      get(t);
+      t.merge(o);
+      set(t);
+    }
+  }
+};
+
+// Sum over the lanes of a warp of an integer below 2^kQ (REDUX adds 32-bit words: an FP64
+// mantissa goes as two 25-bit halves, whose sums over 32 lanes stay below 2^30).
+__device__ __forceinline__ unsigned long long warp_sum_fix(unsigned long long m) {
+  const unsigned lo = __reduce_add_sync(0xffffffffu, (unsigned)m & 0x1ffffffu);
+  const unsigned hi = __reduce_add_sync(0xffffffffu, (unsigned)(m >> 25));
+  return ((unsigned long long)hi << 25) + lo;
+}
+__device__ __forceinline__ unsigned warp_sum_fix(unsigned m) { return __reduce_add_sync(0xffffffffu, m); }
+
+// Move accumulator a (renormalised) to index `ni`, at most its own; an empty one becomes the zero
+// state there (its primaries the bins, its carries 0: merging it changes nothing).
+template <typename T, int F>
+__device__ __forceinline__ void align_to(Acc<T, F>& a, int ni) {
+  if (a.idx == kEmpty) {
+#pragma unroll
+    for (int i = 0; i < F; i++) { a.pri[i] = BT<T>::bin(ni + i); a.car[i] = T(0); }
+    a.set_idx(ni);
+  } else if (a.idx > ni) {
+    a.raise_to(ni);
+  }
+}
+
+// Merge the renormalised accumulators a[n] of the 32 lanes of a warp, for N accumulators;
+// every lane ends with the merged states, renormalised. The lanes first move to the warp's
+// coarsest index (dmdupdate: the alignment merge() performs per pair, done once), then the
+// bins are summed as integers. The non-finite classes are OR-ed.
 template <typename T, int F, int N>
 __device__ __forceinline__ void warp_merge_all(Acc<T, F> (&a)[N]) {
   using B = BT<T>;
-  int m[N];
-  T bins[N][F];
 #pragma unroll
   for (int n = 0; n < N; n++) {
     a[n].flags = __reduce_or_sync(0xffffffffu, a[n].flags);
-    m[n] = __reduce_min_sync(0xffffffffu, a[n].idx);   // kEmpty is above every index
-    if (m[n] != kEmpty) {
-      if (a[n].idx == kEmpty) {
+    const int ni = __reduce_min_sync(0xffffffffu, a[n].idx);   // kEmpty is above every index
+    if (ni == kEmpty) continue;                                // warp-uniform
+    align_to(a[n], ni);
 #pragma unroll
-        for (int i = 0; i < F; i++) { a[n].pri[i] = B::bin(m[n] + i); a[n].car[i] = T(0); }
-        a[n].set_idx(m[n]);
-      } else if (a[n].idx > m[n]) {
-        a[n].raise_to(m[n]);
-      }
+    for (int i = 0; i < F; i++) {
+      int c = __reduce_add_sync(0xffffffffu, (int)a[n].car[i]);
+      a[n].pri[i] = fix_back<T>(B::bin(ni + i), warp_sum_fix(fix_of<T>(a[n].pri[i])), &c);
+      a[n].car[i] = (T)c;
     }
-#pragma unroll
-    for (int i = 0; i < F; i++) bins[n][i] = B::bin(m[n] + i);
-  }
-#pragma unroll
-  for (int s = 16; s; s >>= 1) {
-#pragma unroll
-    for (int n = 0; n < N; n++) {
-      if (m[n] == kEmpty) continue;   // warp-uniform
-#pragma unroll
-      for (int i = 0; i < F; i++) {
-        const T p = __shfl_xor_sync(0xffffffffu, a[n].pri[i], s);
-        const T c = __shfl_xor_sync(0xffffffffu, a[n].car[i], s);
-        a[n].pri[i] = B::add(a[n].pri[i], B::sub(p, bins[n][i]));
-        a[n].car[i] = B::add(a[n].car[i], c);
-      }
-      a[n].renorm();
-    }
+    a[n].deposits = 0;
   }
 }
 
 template <typename T, int F>
 __device__ __forceinline__ void warp_merge_all(Acc<T, F>& a) {
   warp_merge_all<T, F, 1>(*reinterpret_cast<Acc<T, F>(*)[1]>(&a));
+}
+
+// The same over the lanes that differ only in the lane bits from `first` (a power of two) up:
+// with first = 8, lanes l, l + 8, l + 16 and l + 24; each of them ends with the merged states.
+template <typename T, int F, int N>
+__device__ __forceinline__ void lanes_merge(Acc<T, F> (&a)[N], int first) {
+  using B = BT<T>;
+#pragma unroll
+  for (int n = 0; n < N; n++) {
+    int ni = a[n].idx;
+#pragma unroll 1
+    for (int s = first; s < 32; s <<= 1) {
+      const int o = __shfl_xor_sync(0xffffffffu, ni, s);
+      ni = o < ni ? o : ni;
+      a[n].flags |= __shfl_xor_sync(0xffffffffu, a[n].flags, s);
+    }
+    const bool some = ni != kEmpty;
+    if (some) align_to(a[n], ni);
+    typename Fix<T>::M m[F];
+    int c[F];
+#pragma unroll
+    for (int i = 0; i < F; i++) {
+      m[i] = fix_of<T>(a[n].pri[i]);
+      c[i] = (int)a[n].car[i];
+    }
+#pragma unroll 1
+    for (int s = first; s < 32; s <<= 1) {
+#pragma unroll
+      for (int i = 0; i < F; i++) {
+        m[i] += __shfl_xor_sync(0xffffffffu, m[i], s);
+        c[i] += __shfl_xor_sync(0xffffffffu, c[i], s);
+      }
+    }
+    if (some) {
+#pragma unroll
+      for (int i = 0; i < F; i++) {
+        a[n].pri[i] = fix_back<T>(B::bin(ni + i), m[i], &c[i]);
+        a[n].car[i] = (T)c[i];
+      }
+    }
+    a[n].deposits = 0;
+  }
 }
 
 // binned_ddmconv (src/binned/ddmconv.c:23-81): fixed-order conversion to double with
@@ -554,9 +677,32 @@ __device__ inline double conv_n(const int F, const double* pri, const double* ca
   return Y;
 }
 
+// The same for a fixed fold, from registers: the common case (no scaling) unrolled, the others
+// through conv_n on a copy in local memory.
+template <int F>
+__device__ __noinline__ double conv_scaled(const double* pri, const double* car) {
+  return conv_n(F, pri, car, 1);
+}
 template <int F>
 __device__ __forceinline__ double conv(const double* pri, const double* car, int inc) {
-  return conv_n(F, pri, car, inc);
+  using B = BT<double>;
+  const double p0 = pri[0];
+  if ((B::bits(p0) & B::kAbsMask) >= 0x7ff0000000000000ull) return p0;
+  if (p0 == 0.0) return 0.0;
+  const int X = B::mindex(p0);
+  if (X <= 3) {
+    double p[F], c[F];
+#pragma unroll
+    for (int i = 0; i < F; i++) { p[i] = pri[i * inc]; c[i] = car[i * inc]; }
+    return conv_scaled<F>(p, c);
+  }
+  double Y = __dadd_rn(0.0, __dmul_rn(car[0], B::bin6(X)));
+#pragma unroll
+  for (int i = 1; i < F; i++) {
+    Y = __dadd_rn(Y, __dmul_rn(car[i * inc], B::bin6(X + i)));
+    Y = __dadd_rn(Y, __dsub_rn(pri[(i - 1) * inc], B::bin(X + i - 1)));
+  }
+  return __dadd_rn(Y, __dsub_rn(pri[(F - 1) * inc], B::bin(X + F - 1)));
 }
 
 // binned_ssmconv (src/binned/ssmconv.c:22-57): accumulated in double, rounded to float.
@@ -585,9 +731,32 @@ __device__ inline float sconv_n(const int F, const float* pri, const float* car,
   return __double2float_rn(Y);
 }
 
+// The same for a fixed fold, from registers (see conv).
+template <int F>
+__device__ __noinline__ float sconv_scaled(const float* pri, const float* car) {
+  return sconv_n(F, pri, car, 1);
+}
 template <int F>
 __device__ __forceinline__ float sconv(const float* pri, const float* car, int inc) {
-  return sconv_n(F, pri, car, inc);
+  using B = BT<float>;
+  const float p0 = pri[0];
+  if ((B::bits(p0) & B::kAbsMask) >= 0x7f800000u) return p0;
+  if (p0 == 0.0f) return 0.0f;
+  const int X = B::mindex(p0);
+  if (X == 0) {
+    float p[F], c[F];
+#pragma unroll
+    for (int i = 0; i < F; i++) { p[i] = pri[i * inc]; c[i] = car[i * inc]; }
+    return sconv_scaled<F>(p, c);
+  }
+  double Y = __dadd_rn(0.0, __dmul_rn((double)car[0], B::bin6(X)));
+#pragma unroll
+  for (int i = 1; i < F; i++) {
+    Y = __dadd_rn(Y, __dmul_rn((double)car[i * inc], B::bin6(X + i)));
+    Y = __dadd_rn(Y, (double)__fsub_rn(pri[(i - 1) * inc], B::bin(X + i - 1)));
+  }
+  Y = __dadd_rn(Y, (double)__fsub_rn(pri[(F - 1) * inc], B::bin(X + F - 1)));
+  return __double2float_rn(Y);
 }
 
 }  // namespace rb

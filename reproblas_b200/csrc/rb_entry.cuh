@@ -147,19 +147,17 @@ __device__ __forceinline__ void put_rec(const Acc<E, F>& a, E* rec, long long st
   }
   rec[2 * F * stride] = flags_to<E>(a.flags);
 }
-// GLOBAL: the record was written by another CTA (read through L2); else shared memory.
-template <typename E, int F, bool GLOBAL>
-__device__ __forceinline__ void merge_rec(Acc<E, F>& a, const E* rec, long long stride) {
-  Acc<E, F> o;
+// Read a record another CTA wrote (through L2).
+template <typename E, int F>
+__device__ __forceinline__ void read_rec(Acc<E, F>& o, const E* rec, long long stride) {
   o.zero();
 #pragma unroll
   for (int i = 0; i < F; i++) {
-    o.pri[i] = GLOBAL ? __ldcg(rec + i * stride) : rec[i * stride];
-    o.car[i] = GLOBAL ? __ldcg(rec + (F + i) * stride) : rec[(F + i) * stride];
+    o.pri[i] = __ldcg(rec + i * stride);
+    o.car[i] = __ldcg(rec + (F + i) * stride);
   }
-  o.flags = flags_from<E>(GLOBAL ? __ldcg(rec + 2 * F * stride) : rec[2 * F * stride]);
+  o.flags = flags_from<E>(__ldcg(rec + 2 * F * stride));
   o.set_idx_from_pri();
-  a.merge(o);
 }
 
 // 16-byte read-only load of 16 / sizeof(E) reals (the address is 16-byte aligned).

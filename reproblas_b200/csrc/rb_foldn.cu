@@ -20,7 +20,7 @@
 
 #include "rb_blas1_impl.cuh"
 #include "rb_host.h"
-#include "rb_xblas23_impl.cuh"
+#include "rb_entry.cuh"
 #include "../../include/reproblas_b200.h"
 
 namespace rb {

@@ -507,8 +507,8 @@ struct Tile {
     }
   }
 
-  // Finish the entries of the whole tile at (m0, n0). With others > 0 the tile was cut: the
-  // partial states of `others` other CTAs (their records, PART reals apart) are merged first.
+  // Finish the entries of the whole tile at (m0, n0). With first < last the tile was cut: the
+  // partial states of the other CTAs of [first, last] (in slot(v) of the scratch) are merged first.
   template <class Slot>
   __device__ __forceinline__ void finish(const XGemmArgs<E>& g, long long m0, long long n0,
                                          const E* scratch, long long first, long long last,
@@ -523,14 +523,22 @@ struct Tile {
           Acc<E, F> a[NC];
 #pragma unroll
           for (int c = 0; c < NC; c++) get((i * TN + j) * NC + c, a[c]);
-#pragma unroll 1
-          for (long long v = first; v <= last; v++) {
-            if (v == self) continue;
-            const E* rec = scratch + slot(v) * (long long)G::PART + threadIdx.x;
+          if (first < last) {
 #pragma unroll
-            for (int c = 0; c < NC; c++)
-              xb::merge_rec<E, F, true>(a[c], rec + (size_t)((i * TN + j) * NC + c) * G::REC * kThreads,
-                                        kThreads);
+            for (int c = 0; c < NC; c++) {
+              SumAcc<E, F> sum;
+              sum.zero();
+              sum.add(a[c]);
+#pragma unroll 2
+              for (long long v = first; v <= last; v++) {
+                if (v == self) continue;
+                const E* rec = scratch + slot(v) * (long long)G::PART + threadIdx.x;
+                Acc<E, F> o;
+                xb::read_rec<E, F>(o, rec + (size_t)((i * TN + j) * NC + c) * G::REC * kThreads, kThreads);
+                sum.add(o);
+              }
+              sum.get(a[c]);
+            }
           }
           const long long off = gi * g.sci + gj * g.scj;
           xb::finish<E, CX, F>(a, g.mode, g.C + off * NC, g.br, g.bi, g.Cbin + off * 2 * F * NC);

@@ -1,100 +1,92 @@
-// rb_gemv_stream.cuh -- binned dgemv kernels fed by TMA: A streams through a ring of
-// shared-memory stages filled by one producer thread, so the bytes in flight per SM are set
-// by the ring's size rather than by the consumers' registers.
+// rb_gemv_stream.cuh -- binned gemv of every element type (FP64 / FP32, real and complex): A
+// streams through a ring of shared-memory stages filled by bulk copies, so the bytes in
+// flight per SM are set by the ring's size rather than by the consumers' registers.
 //
-// Both kernels compute the same entries as the register-streaming kernels in
-// rb_blas23_impl.cuh (the state of an entry depends only on the multiset of its products),
-//   y_i <- conv( binned(beta*y_i) + sum_j fl(A_ij * bx_j) ),  bx_j = fl(alpha*x_j)
-// (src/reproBLAS/rdgemv.c:35-87, src/binnedBLAS/dbdgemv.ccog:57-162), with A row-major
-// R x C (leading dimension lda, lda*8 a multiple of 16, A 16-byte aligned) described by a
-// 2-D tensor map and x by a 1-D one: either x itself (unit stride, 16-byte aligned; the
-// kernel forms fl(alpha*x_j)) or bx formed by the host's scaling kernel. Boxes that reach
-// past the matrix or the vector are zero-filled by the TMA; zero products deposit nothing.
+//   y_i <- conv( binned(beta*y_i) + sum_j products of op(A)_ij and bx_j ),  bx_j = fl(alpha*x_j)
+// (src/reproBLAS/r[dszc]gemv.c, src/binnedBLAS/[dszc]b[dszc]gemv.ccog; the deposited values are
+// listed in rb_entry.cuh). A is row-major R x C (leading dimension lda); the rows kernel
+// reduces along rows (R outputs), the columns kernel along columns (C outputs).
 //
-// CTA = 8 consumer warps + 1 producer warp, one CTA per resident slot, each streaming an
-// equal share of A's stages. Every consumer thread owns whole outputs (a row of a band, or a
-// column of a block), so no states cross threads while streaming. The producer's lane 0
-// walks the same stage sequence as the consumers and keeps up to kStages stages in flight
-// (full/empty mbarrier pair per stage). Every wait is bounded: a wait that gives up sets
-// the CTA's abort flag, the affected entries come out NaN (their states get the NaN class),
-// *status is set to 2, and the producer lets its copies in flight land (bounded) before the
-// CTA exits.
+// What bounds it: HBM (A is read once), as long as the deposits keep up. One SM receives a
+// 64 KB stage in ~1.5 us = 2900 cycles, in which each of its four sub-partitions has 128 rows
+// of 128 bytes to deposit; a fold-3 FP64 element costs ~25 issue cycles, an FP32 one ~14, so
+// real types need 50-60 % of the stage's time and complex types, with four deposits per
+// element, about all of it. Per-element checks are therefore left out as in the gemm tile
+// (rb_gemm_tile.cuh): per stage a thread bounds its products by max|A| * max|bx| and deposits
+// them unchecked when the bound stays below its accumulator's cap.
 //
-// Instantiated for folds 2 and 3: with 17 warps on an SM a thread has 96 registers, which
-// larger folds would spill; they use the register-streaming kernels.
-//
-// Included by rb_blas23_impl.cuh after finish_entry, which it uses.
+// CTA = 16 consumer warps, a copy warp and an x warp, one CTA per SM, each streaming an equal
+// share of A's stages. Every consumer thread owns whole outputs (a row of a band, or a column
+// of a block). A stage is brought in by TMA box loads. TMA wants 16-byte aligned rows, which
+// an odd leading dimension does not give, so the rows are taken in NPH phases (1, 2 or 4):
+// phase h holds rows h, h + NPH, ..., whose pitch NPH*lda is a multiple of 16 bytes, behind a
+// tensor map of its own that starts at the 16-byte boundary at or before row h. A row then
+// lands `shift` bytes (0 to 15, its phase's distance from that boundary) into its slot; slots
+// are 16 bytes longer than a row's elements, which also keeps a thread-per-row access free of
+// bank conflicts. Any leading dimension and alignment streams at the same rate (row-by-row
+// cp.async.bulk copies did not: ~80 issue cycles each, 82 us against 40 at 4096^2). The x
+// warp reads x at any stride, forms fl(alpha*x) and the stage's largest key. Every wait is
+// bounded: a wait that gives up sets the CTA's abort flag, the affected entries come out NaN
+// (their states get the NaN class), *status is set to 2, and the copy warp lets its copies
+// in flight land (bounded) before the CTA exits.
 #pragma once
-#include <cuda.h>
-
-#include "rb_binned.cuh"
-#include "rb_kernels.cuh"
+#include "rb_entry.cuh"
+#include "rb_gemm_tile.cuh"
 #include "rb_ptx.cuh"
 
 namespace rb {
 namespace gs {
 
+using xb::Val;
+
 constexpr int kConsumers = 512;                 // 16 consumer warps
-constexpr int kThreads = kConsumers + 32;       // + the producer warp
+constexpr int kThreads = kConsumers + 64;       // + the copy warp and the x warp
+constexpr int kStages = 3;
+constexpr uint32_t kThreadBytes = 128;          // of A per consumer thread and stage
 
-// Both kernels split the 512 consumer threads into G groups of P = 512/G (G = g.groups in
-// {2, 4, 8}, chosen by the host). Group q's thread p owns output p of the current unit
-// for the part of the stage that belongs to group q; at the end of a unit's run the G
-// partial states of an output meet in shared memory (log2 G levels). A larger G makes
-// units narrower, hence more of them, and fewer CTAs share a unit, which shortens the
-// merge of the cut units' parts in the last CTA.
-//
-// Row reduction (out_r = sum_c A_rc bx_c): units are bands of P rows. A stage holds G TMA
-// boxes of P rows x 16 columns (128 B per row, 128-byte swizzle: 16-byte chunk c of box row
-// r sits at chunk position c ^ (r & 7)), i.e. 16G columns of the band, then their 16G x;
-// group q deposits box q. A warp's 16-byte reads cover 4 full 128-byte wavefronts. One CTA
-// of 17 warps per SM, whose ring takes most of the shared memory.
-constexpr int kRowBoxC = 16;
-constexpr uint32_t kRowStageA = kConsumers * 128;        // G boxes of P x 16 doubles (64 KB)
-constexpr uint32_t kRowStageBytes = kRowStageA + 1024;  // + up to 128 x, 1 KB aligned
-template <int F> __host__ __device__ constexpr int row_stages() { return 3; }
-// Column reduction (out_c = sum_r A_rc bx_r): units are blocks of P columns. A stage is one
-// box of 16G rows x P columns (64 KB, no swizzle) and the 16G matching x; group q takes rows
-// q, q+G, ..., q+15G of it (even and odd ones into two accumulators), 16 elements per thread
-// per stage like the row reduction.
-constexpr int kColRowsPerGroup = 16;
-constexpr uint32_t kColStageA = kConsumers * 128;        // 64 KB
-constexpr uint32_t kColStageBytes = kColStageA + 1024;  // + up to 128 x
-template <int F> __host__ __device__ constexpr int col_stages() { return 3; }
-
-template <int F>
-__host__ __device__ constexpr size_t tree_bytes() { return (size_t)(2 * F + 1) * kConsumers * 8; }
-template <int F>
-__host__ __device__ constexpr size_t row_smem_bytes() {
-  return (size_t)row_stages<F>() * kRowStageBytes + tree_bytes<F>() + 1024;
+// The 512 consumer threads own P = 512/G outputs (G = g.groups in {2, 4, 8}, chosen by the
+// host), G threads each: lane l of a warp is group l / (32/G) of the warp's output l mod
+// (32/G). Units are bands of P rows (rows kernel) or blocks of P columns (columns kernel); a
+// stage covers SC = PE*G elements of the reduction, PE = 128 bytes / element. Rows kernel:
+// group q deposits columns q*PE .. q*PE + PE - 1 of the stage; columns kernel: rows q, q + G,
+// q + 2G, ... (so that a thread's rows belong to one phase). At the end of a unit's run the G partial states of an output
+// meet by shuffles within their warp: no warp waits for another from the first stage to the
+// finished entries. A larger G makes units narrower, hence more of them, and fewer CTAs share
+// a unit, which shortens the merge of the cut units' parts.
+// Bytes per row slot of a stage in phases (shifted rows): 16 more than the row's elements. A stage
+// of unshifted rows (one phase) has no slack -- boxes wider than their rows cost bandwidth (2 %
+// per 16 bytes at 528, 11 % for 64 bytes at 1088): the rows kernel takes G boxes of 128 bytes x P
+// rows with the 128-byte swizzle (16-byte chunk c of box row r sits at c ^ (r & 7), so lanes on
+// neighbouring rows read different banks), the columns kernel one box, whose groups' reads
+// conflict on banks (2-way for 8-byte elements, 4-way for 4-byte ones) within what the
+// shared memory has to spare.
+template <bool ROWS>
+__host__ __device__ constexpr uint32_t slot_bytes(int G, int es, int phases) {
+  return (ROWS ? kThreadBytes * (uint32_t)G : (uint32_t)(kConsumers / G) * (uint32_t)es) + (phases > 1 ? 16u : 0u);
 }
-template <int F>
-__host__ __device__ constexpr size_t col_smem_bytes() {
-  return (size_t)col_stages<F>() * kColStageBytes + tree_bytes<F>() + 128;
-}
-
-using StreamArgs = GemvStreamArgs;
-
-__device__ __forceinline__ void consumer_sync() { named_sync(1, kConsumers); }
-
-__device__ __forceinline__ unsigned nan_class() { return kNaN; }
+constexpr uint32_t kStageA = kConsumers * kThreadBytes + 4096;   // rows in slots (at most 256 rows)
+constexpr uint32_t kStageX = 1024;                               // PE*G elements of bx
+constexpr uint32_t kStageBytes = kStageA + kStageX;              // a multiple of 1024
+constexpr size_t kSmemBytes = (size_t)kStages * kStageBytes + 1024;
+static_assert(kSmemBytes + 256 <= 227 * 1024, "shared memory of the gemv kernel");
 
 // Work split. The stages are numbered unit-major, x = u * nb + j (unit u = band of rows or
-// block of columns; j = its j-th stage), T = nunits * nb in all, and CTA i streams the
-// contiguous range [i*T/grid, (i+1)*T/grid): every CTA gets the same number of stages (+-1),
-// whatever the shape. A unit whose boxes all fall in one CTA is finished there; a unit cut
-// between CTAs leaves one partial state per CTA in slot k = i - owner(first box of u), and the
-// last of those CTAs to finish (ticket) merges them.
+// block of columns; j = its j-th stage), and every CTA streams a contiguous range of q or q + 1
+// of them, whatever the shape. A unit whose stages all fall in one CTA is finished there; a
+// unit cut between CTAs leaves one partial state per CTA in slot k = i - owner(first stage of
+// u), and the last of those CTAs to finish (ticket) merges them.
 struct Split {
-  long long T, x0, x1;
-  __device__ __forceinline__ Split(long long nunits, long long nb) {
-    T = nunits * nb;
-    x0 = (long long)blockIdx.x * T / gridDim.x;
-    x1 = ((long long)blockIdx.x + 1) * T / gridDim.x;
+  int q, rem, x0, x1;
+  template <typename E>
+  __device__ __forceinline__ explicit Split(const XGemvArgs<E>& g) : q(g.q), rem(g.rem) {
+    const int b = (int)blockIdx.x;
+    x0 = b * q + (b < rem ? b : rem);
+    x1 = x0 + q + (b < rem ? 1 : 0);
   }
-  // CTA whose range holds box x
-  __device__ __forceinline__ long long owner(long long x) const {
-    return ((x + 1) * (long long)gridDim.x - 1) / T;
+  // CTA whose range holds stage x
+  __device__ __forceinline__ int owner(int x) const {
+    const int big = rem * (q + 1);
+    return x < big ? x / (q + 1) : rem + (x - big) / q;
   }
 };
 
@@ -102,430 +94,514 @@ struct Split {
 struct Ring {
   int st = 0;
   unsigned ph = 0;
-  __device__ __forceinline__ void next(int nst) {
-    if (++st == nst) { st = 0; ph ^= 1u; }
+  __device__ __forceinline__ void next() {
+    if (++st == kStages) { st = 0; ph ^= 1u; }
   }
 };
 
-// Producer (lane 0 of warp 8): per stage, `issue(u, j, dst, fb)` starts the copies of
-// stage j of unit u into shared address dst, all completing on mbarrier fb with TX bytes in
-// total. Before returning it waits (bounded) until every copy it issued has landed, so that
-// none is still writing shared memory when the CTA exits, whichever side gave up.
-template <int NST, uint32_t STAGE, class Issue>
-__device__ __forceinline__ void produce(unsigned char* ring, unsigned long long* full,
-                                        unsigned long long* empty, int* abort_flag,
-                                        const Split& sp, long long nb, uint32_t TX,
-                                        long long stop_after, Issue issue) {
+// Geometry of a launch, the same for every role.
+template <typename E, bool CX, bool ROWS>
+struct Geom {
+  static constexpr int NC = CX ? 2 : 1;
+  static constexpr int ES = NC * (int)sizeof(E);          // bytes per element
+  static constexpr int PE = (int)kThreadBytes / ES;       // elements per thread and stage
+  int G, lgG, P, lgP, SC; // SC = PE*G elements of the reduction per stage
+  int lgN;                // log2 of the phases
+  uint32_t pitch;         // bytes per row slot
+  uint32_t phase_bytes;   // of one phase's slots in a stage
+  long long nout, nred;
+  __device__ __forceinline__ explicit Geom(const XGemvArgs<E>& g) {
+    G = g.groups;
+    lgG = __ffs(G) - 1;
+    P = kConsumers >> lgG;
+    lgP = __ffs(kConsumers) - 1 - lgG;
+    SC = PE << lgG;
+    lgN = __ffs(g.phases) - 1;
+    pitch = slot_bytes<ROWS>(G, ES, g.phases);
+    phase_bytes = ((uint32_t)(ROWS ? P : SC) >> lgN) * pitch;
+    nout = ROWS ? g.R : g.C;
+    nred = ROWS ? g.C : g.R;
+  }
+};
+
+// mbarriers and small words shared by the roles
+struct Sync {
+  unsigned long long full[kStages];     // A of the stage has landed
+  unsigned long long xfull[kStages];    // bx of the stage is written
+  unsigned long long empty[kStages];    // the consumers are done with the stage
+  unsigned xkey[kStages];
+  int abort_flag;
+};
+
+// Copy warp (its lane 0): the boxes of each stage, all completing on the stage's `full` mbarrier.
+// Rows and columns outside A are zero-filled. Before returning it waits (bounded) until every
+// copy it issued has landed, so that none is still writing shared memory when the CTA exits.
+template <typename E, bool CX, bool ROWS>
+__device__ __forceinline__ void copy_stages(const XGemvArgs<E>& g, const Geom<E, CX, ROWS>& m,
+                                            const GemvMaps& maps, const Split& sp, unsigned char* ring,
+                                            Sync& sy) {
+  using Gm = Geom<E, CX, ROWS>;
+  const int nph = m.nred > 0 ? 1 << m.lgN : 0;   // no reduction: nothing to copy
+  const int boxes = ROWS && nph == 1 ? m.G : nph;
+  const uint32_t box_bytes = ROWS && nph == 1 ? (uint32_t)m.P * kThreadBytes : m.phase_bytes;
   Ring r;
-  long long u = sp.x0 / nb, j = sp.x0 % nb, issued = 0;
-  for (long long x = sp.x0; x < sp.x1; x++, issued++) {
-    if (stop_after >= 0 && issued >= stop_after) break;   // test hook: stop feeding the ring
-    if (issued >= NST && !mbar_wait_bounded(smem_u32(&empty[r.st]), r.ph ^ 1u)) {
-      atomicExch(abort_flag, 1);
+  int u = sp.x0 / g.nb, j = sp.x0 - u * g.nb;
+  long long issued = 0;
+  for (int x = sp.x0; x < sp.x1; x++, issued++) {
+    if (g.stop_after >= 0 && issued >= g.stop_after) break;   // test hook: stop feeding the ring
+    if (issued >= kStages && !mbar_wait_bounded(smem_u32(&sy.empty[r.st]), r.ph ^ 1u)) {
+      atomicExch(&sy.abort_flag, 1);
       break;
     }
-    if (*(volatile int*)abort_flag) break;
-    const uint32_t fb = smem_u32(&full[r.st]);
-    mbar_expect_tx(fb, TX);
-    issue(u, j, smem_u32(ring + (size_t)r.st * STAGE), fb);
-    r.next(NST);
-    if (++j == nb) { j = 0; u++; }
+    if (*(volatile int*)&sy.abort_flag) break;
+    const uint32_t fb = smem_u32(&sy.full[r.st]);
+    mbar_expect_tx(fb, (uint32_t)boxes * box_bytes);
+    const uint32_t dst = smem_u32(ring + (size_t)r.st * kStageBytes);
+    // coordinates in 8-byte words (a multiple of 16 bytes) and rows of the phase
+    const int c = (int)((ROWS ? (long long)j * m.SC : (long long)u * m.P) * Gm::ES / 8);
+    const int row = (int)((ROWS ? (long long)u * m.P : (long long)j * m.SC) >> m.lgN);
+    for (int h = 0; h < boxes; h++)
+      tma_load_2d(dst + (uint32_t)h * box_bytes, &maps.m[nph == 1 ? 0 : h],
+                  ROWS && nph == 1 ? c + h * (int)(kThreadBytes / 8) : c, row, fb);
+    r.next();
+    if (++j == g.nb) { j = 0; u++; }
   }
-  // the last phase of each slot it used belongs to one of the last NST stages it issued
-  const long long first = issued > NST ? issued - NST : 0;
+  // the last phase of each slot it used belongs to one of the last kStages stages it issued
+  const long long first = issued > kStages ? issued - kStages : 0;
   for (long long k = first; k < issued; k++)
-    mbar_wait_bounded(smem_u32(&full[k % NST]), (unsigned)((k / NST) & 1));
+    mbar_wait_bounded(smem_u32(&sy.full[k % kStages]), (unsigned)((k / kStages) & 1));
 }
 
-// Consumer side of one stage: wait for it (unless aborted); false when the data is not
-// there (abort), in which case the caller skips its deposits.
-__device__ __forceinline__ bool stage_ready(unsigned long long* full, const Ring& r,
-                                            int* abort_flag, long long polls) {
-  if (*(volatile int*)abort_flag) return false;
-  if (!mbar_wait_bounded(smem_u32(&full[r.st]), r.ph, polls)) {
-    atomicExch(abort_flag, 1);
+// x warp: bx = fl(alpha*x) of each stage and its largest key, into the stage's x area; one
+// arrival on the stage's `xfull` mbarrier.
+template <typename E, bool CX, bool ROWS>
+__device__ __forceinline__ void scale_stages(const XGemvArgs<E>& g, const Geom<E, CX, ROWS>& m,
+                                             const Split& sp, unsigned char* ring, Sync& sy) {
+  constexpr int NC = Geom<E, CX, ROWS>::NC;
+  const int lane = threadIdx.x & 31;
+  Ring r;
+  int j = sp.x0 % g.nb;
+  for (int x = sp.x0; x < sp.x1; x++) {
+    bool go = x - sp.x0 < kStages || mbar_wait_bounded(smem_u32(&sy.empty[r.st]), r.ph ^ 1u);
+    if (!go) atomicExch(&sy.abort_flag, 1);
+    go = go && *(volatile int*)&sy.abort_flag == 0;
+    if (!__all_sync(0xffffffffu, go)) break;
+    E* xs = (E*)(ring + (size_t)r.st * kStageBytes + kStageA);
+    unsigned key = 0;
+    for (int i = lane; i < m.SC; i += 32) {
+      const long long e = (long long)j * m.SC + i;
+      Val<E, CX> v{E(0), E(0)};
+      if (e < m.nred) {
+        v = xb::ldv<E, CX>(g.x, e * g.incx);
+        if (!g.alpha_one) v = xb::scale<E, CX>(v, g.ar, g.ai);
+      }
+      // in the order the groups read it (columns kernel: element e of group q is row e*G + q)
+      const int pos = ROWS ? i : (i & (m.G - 1)) * Geom<E, CX, ROWS>::PE + (i >> m.lgG);
+      xs[pos * NC] = v.r;
+      unsigned k = BT<E>::key(v.r);
+      if constexpr (CX) {
+        xs[pos * NC + 1] = v.i;
+        const unsigned ki = BT<E>::key(v.i);
+        k = ki > k ? ki : k;
+      }
+      key = k > key ? k : key;
+    }
+    key = __reduce_max_sync(0xffffffffu, key);
+    if (lane == 0) sy.xkey[r.st] = key;
+    __syncwarp();
+    if (lane == 0) mbar_arrive(smem_u32(&sy.xfull[r.st]));
+    r.next();
+    if (++j == g.nb) j = 0;
+  }
+}
+
+// Consumer side of one stage: wait for its A and x (unless aborted); false when the data is
+// not there (abort), in which case the caller skips its deposits.
+__device__ __forceinline__ bool stage_ready(Sync& sy, const Ring& r, long long polls) {
+  if (*(volatile int*)&sy.abort_flag) return false;
+  if (!mbar_wait_bounded(smem_u32(&sy.full[r.st]), r.ph, polls) ||
+      !mbar_wait_bounded(smem_u32(&sy.xfull[r.st]), r.ph, polls)) {
+    atomicExch(&sy.abort_flag, 1);
     return false;
   }
   return true;
 }
 
-// Partial states of units cut between CTAs, structure of arrays over the outputs:
-// field i (< 2F+1: pri, car, flags) of slot k for output o at scratch[(i*kslots + k)*nout + o].
-template <int F>
-__device__ __forceinline__ void save_partial(const GemvStreamArgs& g, long long nout, long long k,
-                                             long long o, const Acc<double, F>& a) {
-  const long long fs = g.kslots * nout;
-  double* p = g.scratch + k * nout + o;
+// Largest key of |a|, |b| and the running maximum m (a float that holds a key's bits): FP64
+// values contribute their high word, whose bits order magnitudes as a float's do; NaN (and
+// the FP64 magnitudes whose high word is a float NaN) propagate as a key above every bound.
+__device__ __forceinline__ float max_abs3(float m, float a, float b) {
+  float d;
+  asm("max.NaN.abs.f32 %0, %1, %2, %3;" : "=f"(d) : "f"(m), "f"(a), "f"(b));
+  return d;
+}
+__device__ __forceinline__ float key_word(double x) { return __int_as_float(__double2hiint(x)); }
+__device__ __forceinline__ float key_word(float x) { return x; }
+
+// The PE elements of this thread in one stage, and their deposit into its accumulators.
+template <typename E, bool CX, int F, bool ROWS>
+struct Consumer {
+  using Gm = Geom<E, CX, ROWS>;
+  using B = BT<E>;
+  static constexpr int NC = Gm::NC, PE = Gm::PE, ES = Gm::ES, D = CX ? 2 : 1, ND = PE * D;
+  static constexpr int NR = PE * NC;   // reals per thread and stage
+
+  Acc<E, F> a[NC];
+  __device__ __forceinline__ void zero() {
 #pragma unroll
-  for (int i = 0; i < F; i++) {
-    p[i * fs] = a.pri[i];
-    p[(F + i) * fs] = a.car[i];
+    for (int c = 0; c < NC; c++) a[c].zero();
   }
-  p[2 * F * fs] = __longlong_as_double((long long)a.flags);
-}
 
-template <int F>
-__device__ __forceinline__ void load_partial(const GemvStreamArgs& g, long long nout, long long k,
-                                             long long o, Acc<double, F>& a) {
-  const long long fs = g.kslots * nout;
-  const double* p = g.scratch + k * nout + o;
-  a.zero();
+  // Where this thread's elements are in a stage: element e at base + e*stride + shift; or, rows
+  // kernel with unshifted rows (vec), in 16-byte chunks c at base + ((c ^ swz) << 4).
+  struct Place {
+    uint32_t stride, shift, swz;
+    bool vec;
+  };
+
+  __device__ __forceinline__ void load(const unsigned char* base, const Place& pl, E (&v)[NR]) const {
+    if (pl.vec) {
+      if constexpr (ROWS) {
+        constexpr int PER = 16 / (int)sizeof(E);
 #pragma unroll
-  for (int i = 0; i < F; i++) {
-    a.pri[i] = __ldcg(p + i * fs);
-    a.car[i] = __ldcg(p + (F + i) * fs);
+        for (int c = 0; c < (int)kThreadBytes / 16; c++) {
+          E t[PER];
+          gt::lds_vec<E, PER>((const E*)(base + (((uint32_t)c ^ pl.swz) << 4)), t);
+#pragma unroll
+          for (int i = 0; i < PER; i++) v[c * PER + i] = t[i];
+        }
+      } else {
+#pragma unroll
+        for (int e = 0; e < PE; e++) {
+          E t[NC];
+          gt::lds_vec<E, NC>((const E*)(base + (uint32_t)e * pl.stride), t);
+#pragma unroll
+          for (int c = 0; c < NC; c++) v[e * NC + c] = t[c];
+        }
+      }
+    } else {
+      const unsigned char* p = base + pl.shift;
+#pragma unroll
+      for (int e = 0; e < PE; e++)
+#pragma unroll
+        for (int c = 0; c < NC; c++)
+          v[e * NC + c] = ((const E*)(p + (uint32_t)e * (ROWS ? (uint32_t)ES : pl.stride)))[c];
+    }
   }
-  a.flags = (unsigned)__double_as_longlong(__ldcg(p + 2 * F * fs));
-  a.set_idx_from_pri();
-}
+  // real i of element e, the same way
+  __device__ __forceinline__ static const E* at(const unsigned char* base, const Place& pl, int e) {
+    const uint32_t o = (uint32_t)e * pl.stride;
+    return (const E*)(base + (ROWS && pl.vec ? o ^ (pl.swz << 4) : o + pl.shift));
+  }
 
-// Ticket of a cut unit: an acquire-release atomic (release: this CTA's saved parts, made
-// visible CTA-wide by the named barrier before it; acquire: the parts of the CTAs that
-// arrived earlier).
-__device__ __forceinline__ unsigned ticket_acq_rel(unsigned* t) {
-  unsigned old;
-  asm volatile("atom.acq_rel.gpu.global.add.u32 %0, [%1], 1;" : "=r"(old) : "l"(t) : "memory");
-  return old;
-}
+  // the D products of component c of (ar, ai) * (xr, xi)
+  static __device__ __forceinline__ void prods(const E* av, const E* xv, int c, E (&p)[D]) {
+    if constexpr (CX) {
+      p[0] = c == 0 ? B::mul(av[0], xv[0]) : B::mul(av[0], xv[1]);
+      p[1] = c == 0 ? -B::mul(av[1], xv[1]) : B::mul(av[1], xv[0]);
+    } else {
+      p[0] = B::mul(av[0], xv[0]);
+    }
+  }
 
-// Tree merge of the G groups' states through shared memory (sm[i * 512 + thread], i <
-// 2F+1): group 0 ends with the merged state of its output. All consumer threads call it.
-template <int F>
-__device__ __forceinline__ void merge_groups(Acc<double, F>& a, double* sm, int grp, int P, int G) {
-  const int tid = threadIdx.x;
+  // one by one: nval elements, with every check (Acc::tile)
+  __device__ __forceinline__ void deposit_careful(const unsigned char* base, const Place& pl,
+                                                  const E* xs, int nval, bool conj) {
 #pragma unroll 1
-  for (int s = 1; s < G; s <<= 1) {
-    const int m = grp & (2 * s - 1);
-    if (m == s) {
+    for (int e = 0; e < nval; e++) {
+      const E* p = at(base, pl, e);
+      E av[NC], xv[NC];
 #pragma unroll
-      for (int i = 0; i < F; i++) { sm[i * kConsumers + tid] = a.pri[i]; sm[(F + i) * kConsumers + tid] = a.car[i]; }
-      sm[2 * F * kConsumers + tid] = __longlong_as_double((long long)a.flags);
-    }
-    consumer_sync();
-    if (m == 0) {
-      const int src = tid + s * P;
-      Acc<double, F> o;
-      o.zero();
+      for (int c = 0; c < NC; c++) {
+        av[c] = p[c];
+        xv[c] = xs[e * NC + c];
+      }
+      if (CX && conj) av[NC - 1] = -av[NC - 1];
 #pragma unroll
-      for (int i = 0; i < F; i++) { o.pri[i] = sm[i * kConsumers + src]; o.car[i] = sm[(F + i) * kConsumers + src]; }
-      o.flags = (unsigned)__double_as_longlong(sm[2 * F * kConsumers + src]);
-      o.set_idx_from_pri();
-      a.merge(o);
+      for (int c = 0; c < NC; c++) {
+        E v[D];
+        prods(av, xv, c, v);
+        a[c].template tile<D>(v, D);
+      }
     }
-    consumer_sync();
   }
-}
 
-// A CTA's range of stages holds whole units in its middle and possibly cut units at its two
-// ends. close_run() ends the run of unit u in this CTA for output `o` (valid when o < nout),
-// held by thread (grp, p) in a0: the groups merge; a whole unit's entry is finished at once,
-// a cut unit's part is saved and the unit is recorded as pending (at most two per CTA).
-// settle() then, after the CTA's last stage, takes the tickets of the pending units (one
-// thread, back to back); in the last CTA of a unit the parts are merged (group q takes parts
-// q, q+G, ...) and the entry finished. Deferring the tickets keeps their atomics out of the
-// stream. All consumer threads call both.
-struct Pending {
-  long long u[2], count[2];
-  int n = 0;
+  __device__ __forceinline__ void stage(const unsigned char* base, const Place& pl, const E* xs,
+                                        unsigned xkey, int nval, bool conj) {
+    if (nval <= 0) return;
+    bool careful = nval < PE;
+    E v[NR];
+    if (!careful) {
+      load(base, pl, v);
+      float m = 0.0f;
+#pragma unroll
+      for (int i = 0; i < NR; i += 2) m = max_abs3(m, key_word(v[i]), key_word(v[i + 1]));
+      const unsigned bound =
+          B::key(B::mul(gt::key_ceiling<E>(__float_as_uint(m)), gt::key_ceiling<E>(xkey)));
+      bool fast = true;
+#pragma unroll
+      for (int c = 0; c < NC; c++) fast = fast && a[c].fast(bound, ND);
+      if (CX && conj) {
+#pragma unroll
+        for (int e = 0; e < PE; e++) v[e * NC + NC - 1] = -v[e * NC + NC - 1];
+      }
+      if (fast) {
+#pragma unroll
+        for (int c = 0; c < NC; c++) a[c].deposits += ND;
+      } else if (bound >= B::kInfKey) {
+        careful = true;
+      } else {
+        // the exact largest key of each component's products, then the index that needs
+        unsigned mk[NC];
+#pragma unroll
+        for (int c = 0; c < NC; c++) mk[c] = 0u;
+#pragma unroll
+        for (int e = 0; e < PE; e++)
+#pragma unroll
+          for (int c = 0; c < NC; c++) {
+            E p[D], xv[NC];
+#pragma unroll
+            for (int q = 0; q < NC; q++) xv[q] = xs[e * NC + q];
+            prods(v + e * NC, xv, c, p);
+#pragma unroll
+            for (int d = 0; d < D; d++) {
+              const unsigned kk = B::key(p[d]);
+              mk[c] = kk > mk[c] ? kk : mk[c];
+            }
+          }
+#pragma unroll
+        for (int c = 0; c < NC; c++) {
+          a[c].prepare(mk[c], ND);
+          if (a[c].idx == 0) careful = true;
+        }
+      }
+    }
+    if (careful) {
+      deposit_careful(base, pl, xs, nval, conj);
+      return;
+    }
+#pragma unroll
+    for (int e = 0; e < PE; e += 16 / ES) {
+      constexpr int XR = 16 / (int)sizeof(E);   // reals of one 16-byte vector of bx
+      E xv[XR];
+      gt::lds_vec<E, XR>(xs + e * NC, xv);
+#pragma unroll
+      for (int q = 0; q < 16 / ES; q++)
+#pragma unroll
+        for (int c = 0; c < NC; c++) {
+          E p[D];
+          prods(v + (e + q) * NC, xv + q * NC, c, p);
+#pragma unroll
+          for (int d = 0; d < D; d++) a[c].deposit(p[d]);
+        }
+    }
+  }
 };
 
-template <int F>
-__device__ __forceinline__ void close_run(const GemvStreamArgs& g, const Split& sp, long long nb,
-                                          long long u, long long o, long long nout, int grp, int P,
-                                          int G, Acc<double, F>& a0, double* tsm, Pending& pend) {
-  const bool valid = o < nout;
-  const long long first = sp.owner(u * nb), count = sp.owner(u * nb + nb - 1) - first + 1;
-  // the entry's current value, loaded early so that its latency overlaps the group merge
-  const double yv = (count == 1 && grp == 0 && valid && g.mode == kOutValue) ? g.y[o * g.incy] : 0.0;
-  merge_groups<F>(a0, tsm, grp, P, G);
-  if (count == 1) {
-    if (grp == 0 && valid)
-      finish_entry_pre<F>(a0, g.mode, yv, g.y + o * g.incy, g.beta, g.ybin + o * g.incy * 2 * F);
-    return;
-  }
-  if (grp == 0 && valid) save_partial<F>(g, nout, (long long)blockIdx.x - first, o, a0);
-  pend.u[pend.n] = u;
-  pend.count[pend.n] = count;
-  pend.n++;
-}
+// Partial states of units cut between CTAs, structure of arrays over the outputs: field i
+// (< NC*(2F+1): pri, car, flags per component) of slot k for output o at
+// scratch[(i*kslots + k)*nout + o].
+//
+// A CTA's range of stages holds whole units in its middle and possibly cut units at its two
+// ends. Ends::close() ends the run of unit u in this CTA for the warp's outputs: the groups
+// merge; a whole unit's entry is finished at once, a cut unit's part is saved and the unit is
+// recorded as pending (at most two per CTA). Ends::settle() then, after the CTA's last stage,
+// takes the tickets of the pending units (one per unit and warp: warps settle by themselves);
+// the warp of the last CTA to arrive merges the parts (group q takes parts q, q+G, ...) and
+// finishes its entries. Deferring the tickets keeps their atomics out of the stream.
+template <typename E, bool CX, int F>
+struct Ends {
+  static constexpr int NC = CX ? 2 : 1, REC = 2 * F + 1;
+  const XGemvArgs<E>& g;
+  int P, lgG, grp, pp, out;   // group of this lane, its output's offset in a unit, lanes per group
+  long long nout, fs;
+  int n, u0, u1, c0, c1;      // pending units and the CTAs they meet
 
-template <int F>
-__device__ __forceinline__ void settle(const GemvStreamArgs& g, long long nout, int grp, int P,
-                                       int G, const Pending& pend, double* tsm, unsigned* s_last) {
-  if (pend.n == 0) return;
-  const long long o0 = pend.u[0] * P + (threadIdx.x & (P - 1));
-  const long long o1 = pend.n > 1 ? pend.u[1] * P + (threadIdx.x & (P - 1)) : 0;
-  const bool y0 = grp == 0 && o0 < nout && g.mode == kOutValue;
-  const bool y1 = grp == 0 && pend.n > 1 && o1 < nout && g.mode == kOutValue;
-  // the entries' current values, loaded early so that their latency overlaps the tickets
-  const double yv[2] = {y0 ? g.y[o0 * g.incy] : 0.0, y1 ? g.y[o1 * g.incy] : 0.0};
-  // all of this CTA's tickets at once
-  consumer_sync();
-  if (threadIdx.x == 0) {
-    unsigned mask = 0;
-    for (int k = 0; k < pend.n; k++) {
-      if (ticket_acq_rel(g.tickets + pend.u[k]) == (unsigned)pend.count[k] - 1) {
-        mask |= 1u << k;
-        g.tickets[pend.u[k]] = 0u;
-      }
-    }
-    *s_last = mask;
+  __device__ __forceinline__ void finish(long long o, Acc<E, F> (&a)[NC], const E (&y)[NC]) const {
+    xb::finish_from<E, CX, F>(a, g.mode, y, g.y + o * g.incy * NC, g.br, g.bi,
+                              g.ybin + o * g.incy * 2 * F * NC);
   }
-  consumer_sync();
-  const unsigned mask = *s_last;
-  for (int k = 0; k < pend.n; k++) {
-    if (!(mask & (1u << k))) continue;
-    const long long count = pend.count[k];
-    const long long o = k ? o1 : o0;
-    const bool valid = o < nout;
-    Acc<double, F> a0;
-    a0.zero();
-    if (valid) {
-      // two parts in flight at a time
-      for (long long q = grp; q < count; q += 2 * G) {
-        Acc<double, F> t0;
-        load_partial<F>(g, nout, q, o, t0);
-        if (q + G < count) {
-          Acc<double, F> t1;
-          load_partial<F>(g, nout, q + G, o, t1);
-          a0.merge(t1);
+  __device__ __forceinline__ void read_y(long long o, bool want, E (&y)[NC]) const {
+#pragma unroll
+    for (int c = 0; c < NC; c++) y[c] = want && g.mode == kOutValue ? g.y[o * g.incy * NC + c] : E(0);
+  }
+  __device__ __forceinline__ void close(const Split& sp, int u, Acc<E, F> (&a)[NC]) {
+    const long long o = (long long)u * P + pp;
+    const bool mine = grp == 0 && o < nout;
+    const int first = sp.owner(u * g.nb), count = sp.owner(u * g.nb + g.nb - 1) - first + 1;
+    E y[NC];   // the entry's current value, loaded early
+    read_y(o, mine && count == 1, y);
+    lanes_merge<E, F, NC>(a, out);
+    if (count == 1) {
+      if (mine) finish(o, a, y);
+      return;
+    }
+    if (mine) {
+      E* rec = g.scratch + (long long)((int)blockIdx.x - first) * nout + o;
+#pragma unroll
+      for (int c = 0; c < NC; c++) xb::put_rec<E, F>(a[c], rec + c * REC * fs, fs);
+    }
+    if (n == 0) { u0 = u; c0 = count; }
+    else { u1 = u; c1 = count; }
+    n++;
+  }
+  __device__ __forceinline__ void settle() {
+    if (n == 0) return;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    // release this warp's parts, then take its tickets (lanes 0 and 1, one each)
+    __threadfence();
+    __syncwarp();
+    bool last = false;
+    if (lane < n) {
+      unsigned* t = g.tickets + (size_t)(lane == 0 ? u0 : u1) * (kConsumers / 32) + warp;
+      last = atomicAdd(t, 1u) == (unsigned)(lane == 0 ? c0 : c1) - 1;
+      if (last) *t = 0u;
+    }
+    const unsigned mask = __ballot_sync(0xffffffffu, last);
+    if (mask == 0) return;
+    __threadfence();
+#pragma unroll 1
+    for (int k = 0; k < n; k++) {
+      if (!(mask & (1u << k))) continue;
+      const long long o = (long long)(k == 0 ? u0 : u1) * P + pp;
+      const int count = k == 0 ? c0 : c1;
+      E y[NC];
+      read_y(o, grp == 0 && o < nout, y);
+      Acc<E, F> a[NC];
+#pragma unroll
+      for (int c = 0; c < NC; c++) {
+        SumAcc<E, F> sum;
+        sum.zero();
+        if (o < nout) {
+#pragma unroll 2
+          for (int q = grp; q < count; q += 1 << lgG) {
+            Acc<E, F> part;
+            xb::read_rec<E, F>(part, g.scratch + q * nout + o + c * REC * fs, fs);
+            sum.add(part);
+          }
         }
-        a0.merge(t0);
+        sum.get(a[c]);
       }
+      lanes_merge<E, F, NC>(a, out);
+      if (grp == 0 && o < nout) finish(o, a, y);
     }
-    merge_groups<F>(a0, tsm, grp, P, G);
-    if (grp == 0 && valid)
-      finish_entry_pre<F>(a0, g.mode, yv[k], g.y + o * g.incy, g.beta, g.ybin + o * g.incy * 2 * F);
   }
-}
+};
 
-// ---------------------------------------------------------------------------------------
-// Row reduction: units are bands of P = 512/G rows, nb = ceil(C / 16G) stages each.
-// ---------------------------------------------------------------------------------------
-template <int F>
+template <typename E, bool CX, int F, bool ROWS>
 __global__ void __launch_bounds__(kThreads, 1)
-gemv_rows_stream_kernel(StreamArgs g, const __grid_constant__ CUtensorMap tm,
-                        const __grid_constant__ CUtensorMap tmx) {
-  constexpr int NST = row_stages<F>();
+gemv_stream_kernel(const __grid_constant__ XGemvArgs<E> g, const __grid_constant__ GemvMaps maps) {
+  using Gm = Geom<E, CX, ROWS>;
+  constexpr int NC = Gm::NC, PE = Gm::PE, ES = Gm::ES;
   extern __shared__ unsigned char smem_raw[];
-  __shared__ __align__(8) unsigned long long full[NST];
-  __shared__ __align__(8) unsigned long long empty[NST];
-  __shared__ int abort_flag;
-  __shared__ unsigned s_last;
+  __shared__ Sync sy;
   unsigned char* ring = (unsigned char*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
-  double* tsm = (double*)(ring + (size_t)NST * kRowStageBytes);
   const int tid = threadIdx.x, lane = tid & 31;
-  const int G = g.groups, P = kConsumers / G, lgP = __ffs(P) - 1;
-  const int SC = kRowBoxC * G;                           // columns per stage
-  const int grp = tid >> lgP, p = tid & (P - 1);
-  const long long nb = (g.C + SC - 1) / SC;
-  const Split sp((g.R + P - 1) / P, nb);
+  const Gm m(g);
+  const Split sp(g);
 
-  if (tid == 0) {
-    for (int i = 0; i < NST; i++) {
-      mbar_init(smem_u32(&full[i]), 1);
-      mbar_init(smem_u32(&empty[i]), kConsumers / 32);
+  if (tid == kConsumers) {
+    for (int h = 0; h < g.phases; h++)
+      asm volatile("prefetch.tensormap [%0];" ::"l"(&maps.m[h]) : "memory");
+    for (int i = 0; i < kStages; i++) {
+      mbar_init(smem_u32(&sy.full[i]), 1);
+      mbar_init(smem_u32(&sy.xfull[i]), 1);
+      mbar_init(smem_u32(&sy.empty[i]), kConsumers / 32);
     }
-    abort_flag = 0;
+    sy.abort_flag = 0;
     fence_barrier_init();
   }
   __syncthreads();
 
-  if (tid >= kConsumers) {
-    if (tid == kConsumers) {
-      const CUtensorMap* tmp = &tm;
-      const CUtensorMap* tmxp = &tmx;
-      auto issue = [tmp, tmxp, G, P, SC](long long u, long long j, uint32_t dst, uint32_t fb) {
-        const int c = (int)(j * SC), rr = (int)(u * P);
-        for (int q = 0; q < G; q++)
-          tma_load_2d(dst + (uint32_t)q * (kRowStageA / G), tmp, c + kRowBoxC * q, rr, fb);
-        tma_load_1d(dst + kRowStageA, tmxp, c, fb);
-      };
-      produce<NST, kRowStageBytes>(ring, full, empty, &abort_flag, sp, nb,
-                                   kRowStageA + (uint32_t)SC * 8, g.stop_after, issue);
-    }
+  if (tid >= kConsumers + 32) {
+    scale_stages<E, CX, ROWS>(g, m, sp, ring, sy);
+  } else if (tid >= kConsumers) {
+    if (lane == 0) copy_stages<E, CX, ROWS>(g, m, maps, sp, ring, sy);
   } else {
-    Ring r;
-    Pending pend;
     const long long polls = g.wait_polls > 0 ? g.wait_polls : kWaitPolls;
-    long long u = sp.x0 / nb, j = sp.x0 % nb;
-    Acc<double, F> a0, a1;
-    a0.zero();
-    a1.zero();
+    const bool conj = CX && g.conj;
+    const int lgN = m.lgN, nph = 1 << lgN;
+    Ends<E, CX, F> ends{g, m.P, m.lgG, 0, 0, 32 >> m.lgG, m.nout, g.kslots * m.nout, 0, 0, 0, 0, 0};
+    const int grp = lane >> (5 - m.lgG);
+    // rows kernel: thread p takes slot p, i.e. row (p mod P/NPH)*NPH + p / (P/NPH) of the band,
+    // so that neighbouring lanes read neighbouring slots; columns kernel: column p
+    const int p = (tid >> 5) * ends.out + (lane & (ends.out - 1));
+    const int pp = ROWS ? ((p & ((m.P >> lgN) - 1)) << lgN) + (p >> (m.lgP - lgN)) : p;
+    ends.grp = grp;
+    ends.pp = pp;
+    // phase of its row(s): columns kernel rows grp, grp + G, ... with G a multiple of NPH
+    const int ph = (ROWS ? pp : grp) & (nph - 1);
+    typename Consumer<E, CX, F, ROWS>::Place pl;
+    pl.vec = lgN == 0;
+    pl.stride = ROWS ? (uint32_t)ES : (uint32_t)(m.G >> lgN) * m.pitch;
+    pl.shift = (uint32_t)((uintptr_t)g.A + (unsigned long long)ph * g.lda * ES) & 15u;
+    pl.swz = (uint32_t)p & 7u;
+    const uint32_t off =
+        ROWS ? (pl.vec ? (uint32_t)(grp * m.P + p) * kThreadBytes : (uint32_t)p * m.pitch + (uint32_t)grp * kThreadBytes)
+             : (uint32_t)ph * m.phase_bytes + (uint32_t)(grp >> lgN) * m.pitch + (uint32_t)p * ES;
+    Ring r;
+    int u = sp.x0 / g.nb, j = sp.x0 - u * g.nb;
+    Consumer<E, CX, F, ROWS> con;
+    con.zero();
     bool lost = false;
-    const uint32_t rowoff = (uint32_t)grp * (kRowStageA / G) + (uint32_t)p * 128;
-    const int sw = p & 7;
-    for (long long x = sp.x0; x < sp.x1; x++) {
-      if (stage_ready(full, r, &abort_flag, polls)) {
-        const unsigned char* st = ring + (size_t)r.st * kRowStageBytes;
-        const double* xs = (const double*)(st + kRowStageA) + grp * kRowBoxC;
-#pragma unroll
-        for (int h = 0; h < 2; h++) {
-          double ve[4], vo[4];
-#pragma unroll
-          for (int c = 0; c < 4; c++) {
-            const int cc = 4 * h + c;
-            const double2 av = *(const double2*)(st + rowoff + ((cc ^ sw) << 4));
-            double2 xv = *(const double2*)(xs + 2 * cc);
-            if (g.scale_x) {
-              xv.x = __dmul_rn(xv.x, g.alpha);
-              xv.y = __dmul_rn(xv.y, g.alpha);
-            }
-            ve[c] = __dmul_rn(av.x, xv.x);
-            vo[c] = __dmul_rn(av.y, xv.y);
-          }
-          tile2<double, F, 4>(a0, ve, a1, vo);
-        }
+#pragma unroll 1
+    for (int x = sp.x0; x < sp.x1; x++) {
+      if (stage_ready(sy, r, polls)) {
+        const unsigned char* st = ring + (size_t)r.st * kStageBytes;
+        // elements of this thread that exist; the columns kernel takes a partial last stage
+        // whole (rows outside A arrive as zeros, and so do their x) unless A has fewer rows
+        // than phases
+        const long long k0 = (long long)j * m.SC;
+        const long long rem = ROWS ? m.nred - k0 - grp * PE : (m.nred - k0 - grp + m.G - 1) >> m.lgG;
+        const bool whole = rem >= PE || (!ROWS && m.nred >= 4);
+        const int nval = (long long)u * m.P + pp >= m.nout || rem <= 0 ? 0 : whole ? PE : (int)rem;
+        con.stage(st + off, pl, (const E*)(st + kStageA) + grp * PE * NC, sy.xkey[r.st], nval, conj);
       } else {
         lost = true;
       }
       __syncwarp();
-      if (lane == 0) mbar_arrive(smem_u32(&empty[r.st]));
-      r.next(NST);
-      if (++j < nb && x + 1 < sp.x1) continue;
-      // ---- the run of band u in this CTA ends here ----
-      a0.renorm();
-      a1.renorm();
-      a0.merge(a1);
-      if (lost) a0.flags |= nan_class();
-      close_run<F>(g, sp, nb, u, u * P + p, g.R, grp, P, G, a0, tsm, pend);
-      a0.zero();
-      a1.zero();
-      lost = false;
-      j = 0;
-      u++;
-    }
-    settle<F>(g, g.R, grp, P, G, pend, tsm, &s_last);
-  }
-  __syncthreads();
-  if (tid == 0 && abort_flag) atomicExch(g.status, 2);
-}
-
-// ---------------------------------------------------------------------------------------
-// Column reduction: units are blocks of P = 512/G columns, nb = ceil(R / 16G) stages each.
-// ---------------------------------------------------------------------------------------
-template <int F>
-__global__ void __launch_bounds__(kThreads, 1)
-gemv_cols_stream_kernel(StreamArgs g, const __grid_constant__ CUtensorMap tm,
-                        const __grid_constant__ CUtensorMap tmx) {
-  constexpr int NST = col_stages<F>();
-  extern __shared__ unsigned char smem_raw[];
-  __shared__ __align__(8) unsigned long long full[NST];
-  __shared__ __align__(8) unsigned long long empty[NST];
-  __shared__ int abort_flag;
-  __shared__ unsigned s_last;
-  unsigned char* ring = (unsigned char*)(((uintptr_t)smem_raw + 127) & ~(uintptr_t)127);
-  double* tsm = (double*)(ring + (size_t)NST * kColStageBytes);
-  const int tid = threadIdx.x, lane = tid & 31;
-  const int G = g.groups, P = kConsumers / G, lgP = __ffs(P) - 1;
-  const int RS = kColRowsPerGroup * G;                   // rows per stage
-  const int grp = tid >> lgP, p = tid & (P - 1);
-  const long long nb = (g.R + RS - 1) / RS;
-  const Split sp((g.C + P - 1) / P, nb);
-
-  if (tid == 0) {
-    for (int i = 0; i < NST; i++) {
-      mbar_init(smem_u32(&full[i]), 1);
-      mbar_init(smem_u32(&empty[i]), kConsumers / 32);
-    }
-    abort_flag = 0;
-    fence_barrier_init();
-  }
-  __syncthreads();
-
-  if (tid >= kConsumers) {
-    if (tid == kConsumers) {
-      const CUtensorMap* tmp = &tm;
-      const CUtensorMap* tmxp = &tmx;
-      auto issue = [tmp, tmxp, P, RS](long long u, long long j, uint32_t dst, uint32_t fb) {
-        tma_load_2d(dst, tmp, (int)(u * P), (int)(j * RS), fb);
-        tma_load_1d(dst + kColStageA, tmxp, (int)(j * RS), fb);
-      };
-      produce<NST, kColStageBytes>(ring, full, empty, &abort_flag, sp, nb,
-                                   kColStageA + (uint32_t)RS * 8, g.stop_after, issue);
-    }
-  } else {
-    Ring r;
-    Pending pend;
-    const long long polls = g.wait_polls > 0 ? g.wait_polls : kWaitPolls;
-    long long u = sp.x0 / nb, j = sp.x0 % nb;
-    Acc<double, F> a0, a1;
-    a0.zero();
-    a1.zero();
-    bool lost = false;
-    for (long long x = sp.x0; x < sp.x1; x++) {
-      if (stage_ready(full, r, &abort_flag, polls)) {
-        const double* As = (const double*)(ring + (size_t)r.st * kColStageBytes);
-        const double* xs = (const double*)((const unsigned char*)As + kColStageA);
+      if (lane == 0) mbar_arrive(smem_u32(&sy.empty[r.st]));
+      r.next();
+      if (++j < g.nb && x + 1 < sp.x1) continue;
+      // ---- the run of unit u in this CTA ends here ----
 #pragma unroll
-        for (int h = 0; h < 2; h++) {
-          double ve[4], vo[4];
-#pragma unroll
-          for (int k = 0; k < 4; k++) {
-            const int r0 = grp + G * (8 * h + 2 * k), r1 = r0 + G;
-            double x0 = xs[r0], x1 = xs[r1];
-            if (g.scale_x) {
-              x0 = __dmul_rn(x0, g.alpha);
-              x1 = __dmul_rn(x1, g.alpha);
-            }
-            ve[k] = __dmul_rn(As[r0 * P + p], x0);
-            vo[k] = __dmul_rn(As[r1 * P + p], x1);
-          }
-          tile2<double, F, 4>(a0, ve, a1, vo);
-        }
-      } else {
-        lost = true;
+      for (int c = 0; c < NC; c++) {
+        con.a[c].renorm();
+        if (lost) con.a[c].flags |= kNaN;
       }
-      __syncwarp();
-      if (lane == 0) mbar_arrive(smem_u32(&empty[r.st]));
-      r.next(NST);
-      if (++j < nb && x + 1 < sp.x1) continue;
-      // ---- the run of column block u in this CTA ends here ----
-      a0.renorm();
-      a1.renorm();
-      a0.merge(a1);
-      if (lost) a0.flags |= nan_class();
-      close_run<F>(g, sp, nb, u, u * P + p, g.C, grp, P, G, a0, tsm, pend);
-      a0.zero();
-      a1.zero();
+      ends.close(sp, u, con.a);
+      con.zero();
       lost = false;
       j = 0;
       u++;
     }
-    settle<F>(g, g.C, grp, P, G, pend, tsm, &s_last);
+    ends.settle();
   }
   __syncthreads();
-  if (tid == 0 && abort_flag) atomicExch(g.status, 2);
+  if (tid == 0 && sy.abort_flag) atomicExch(g.status, 2);
 }
 
-template <int F>
-cudaError_t launch_gemv_stream(const StreamArgs& g, const CUtensorMap& tm, const CUtensorMap& tmx,
-                               bool rows, int grid, cudaStream_t s) {
-  if (rows) {
-    gemv_rows_stream_kernel<F><<<grid, kThreads, row_smem_bytes<F>(), s>>>(g, tm, tmx);
-  } else {
-    gemv_cols_stream_kernel<F><<<grid, kThreads, col_smem_bytes<F>(), s>>>(g, tm, tmx);
+template <typename E, bool CX, int F>
+cudaError_t launch_gemv(const XGemvArgs<E>& g, const GemvMaps& maps, bool rows, int grid, cudaStream_t s) {
+  constexpr size_t smem = kSmemBytes;
+  // opt in to the shared memory, once per device (the call is idempotent)
+  constexpr int kMaxDevices = 64;
+  static std::atomic<int> ready[kMaxDevices];
+  int dev = 0;
+  cudaError_t e = cudaGetDevice(&dev);
+  if (e != cudaSuccess) return e;
+  if (dev >= kMaxDevices || !ready[dev].load(std::memory_order_relaxed)) {
+    e = cudaFuncSetAttribute(gemv_stream_kernel<E, CX, F, true>,
+                             cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e == cudaSuccess)
+      e = cudaFuncSetAttribute(gemv_stream_kernel<E, CX, F, false>,
+                               cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e != cudaSuccess) return e;
+    if (dev < kMaxDevices) ready[dev].store(1, std::memory_order_relaxed);
   }
+  if (rows) gemv_stream_kernel<E, CX, F, true><<<grid, kThreads, smem, s>>>(g, maps);
+  else gemv_stream_kernel<E, CX, F, false><<<grid, kThreads, smem, s>>>(g, maps);
   return cudaGetLastError();
-}
-
-// Opt in to the kernels' dynamic shared memory (once per process and device is enough; the
-// call is cheap and idempotent) and report how many CTAs of each fit on one SM.
-template <int F>
-cudaError_t prepare_gemv_stream(int* rows_per_sm, int* cols_per_sm) {
-  cudaError_t e = cudaFuncSetAttribute(gemv_rows_stream_kernel<F>,
-                                       cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                       (int)row_smem_bytes<F>());
-  if (e == cudaSuccess)
-    e = cudaFuncSetAttribute(gemv_cols_stream_kernel<F>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (int)col_smem_bytes<F>());
-  if (e == cudaSuccess)
-    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(rows_per_sm, gemv_rows_stream_kernel<F>,
-                                                      kThreads, row_smem_bytes<F>());
-  if (e == cudaSuccess)
-    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(cols_per_sm, gemv_cols_stream_kernel<F>,
-                                                      kThreads, col_smem_bytes<F>());
-  return e;
 }
 
 }  // namespace gs

@@ -92,45 +92,6 @@ enum OutMode : int {
   kOutBinned = 1,   // binnedBLAS_dbd*: merge into the caller's binned states
 };
 
-struct GemvArgs {
-  long long R, C;             // rows kernel: R outputs x C reduction; cols kernel: C outputs x R
-  const double* A;
-  long long lda;
-  const double* x;
-  long long incx;
-  double alpha, beta;
-  int mode;
-  double* y;                  // kOutValue: values (stride incy)
-  double* ybin;               // kOutBinned: binned states (stride incy states)
-  long long incy;
-  int split;                  // rows kernel: warps per row; cols kernel: row groups (1, 2, 4, 8)
-  int vec;                    // 16-byte loads (alignment checked by the host)
-  double* scratch;            // cols kernel: partial states
-  unsigned* tickets;          // cols kernel: one per column block, zero on entry
-};
-
-// TMA-fed dgemv (rb_gemv_stream.cuh): A is R x C row-major behind a 2-D tensor map.
-struct GemvStreamArgs {
-  long long R, C;        // A is R x C (row-major view)
-  double alpha;          // multiplies the x the kernel reads when scale_x is set
-  int scale_x;           // 0: the x tensor holds fl(alpha*x) already
-  double beta;
-  int mode;              // kOutValue / kOutBinned
-  double* y;             // kOutValue: values (stride incy)
-  double* ybin;          // kOutBinned: binned states (stride incy states)
-  long long incy;
-  double* scratch;       // partial states
-  unsigned* tickets;     // one per band (rows) / column block (cols), zero on entry
-  int* status;           // set to 2 when a pipeline wait gives up
-  long long kslots;      // partial-state slots per output of a unit cut between CTAs
-  int groups;            // thread groups per output (power of two, 1..8)
-  // failure-path test hook (rb_debug_pipeline_fault): each CTA's producer issues at most
-  // `stop_after` stages (< 0: all), and consumers give up waiting for a stage's data after
-  // `wait_polls` polls (0: the default ~2 s)
-  long long stop_after;
-  long long wait_polls;
-};
-
 // Failure-path test hook (rb_runtime.cu): stop_after / wait_polls for the next TMA-fed
 // kernels (stop_after < 0 and wait_polls 0 when unset).
 void pipeline_fault(long long* stop_after, long long* wait_polls);
@@ -170,27 +131,10 @@ struct GemmPlan {
   unsigned* tickets;
 };
 
-struct Blas23FoldOps {
-  cudaError_t (*gemv)(const GemvArgs& g, bool rows, dim3 grid, cudaStream_t s);
-  // decomposition of an M x N x K product (whole_tiles: no tile is cut between CTAs)
-  cudaError_t (*gemm_plan)(long long M, long long N, long long K, int sms, bool whole_tiles,
-                           GemmPlan* p);
-  cudaError_t (*gemm)(const XGemmArgs<double>& g, const GemmPlan& p, cudaStream_t s);
-  // TMA-fed dgemv (nullptr for folds it does not cover)
-  cudaError_t (*gemv_stream)(const GemvStreamArgs& g, const CUtensorMap& tm, const CUtensorMap& tmx,
-                             bool rows, int grid, cudaStream_t s);
-  // opt in to the stream kernels' shared memory; CTAs per SM of each
-  cudaError_t (*gemv_stream_prepare)(int* rows_per_sm, int* cols_per_sm);
-};
-extern const Blas23FoldOps blas23_fold2, blas23_fold3, blas23_fold4, blas23_fold5,
-    blas23_fold6, blas23_fold7, blas23_fold8;
-
-// ---- gemv / gemm for FP32 real, FP64 complex and FP32 complex elements (rb_xblas23_*.cu).
-// E is the real element type; complex operands are interleaved (re, im) pairs and every
-// stride / leading dimension counts whole (complex) elements.
+// One gemv of any element type (rb_gemv_stream.cuh): A is the stored matrix seen row-major.
 template <typename E>
 struct XGemvArgs {
-  long long R, C;             // rows kernel: R outputs x C reduction; cols kernel: C outputs x R
+  long long R, C;             // A is R x C; the rows kernel has R outputs, the columns kernel C
   const E* A;
   long long lda;
   const E* x;
@@ -199,32 +143,43 @@ struct XGemvArgs {
   int alpha_one;              // skip the alpha multiply
   int conj;                   // conjugate A's elements (complex ConjTrans)
   int mode;                   // kOutValue / kOutBinned
-  int split;                  // cols kernel: row groups per CTA (1, 2, 4, 8)
-  int vec;                    // rows kernel: 16-byte loads (rows and x aligned, incx 1, x
-                              // already multiplied by alpha)
+  int phases;                 // phases the rows of A are taken in (1, 2, 4; rb_gemv_stream.cuh)
   E* y;                       // kOutValue: values (stride incy)
   E* ybin;                    // kOutBinned: binned states (stride incy states)
   long long incy;
-  E* scratch;                 // partial states: rows kernel 2 per warp, cols kernel per chunk
-  unsigned* tickets;          // rows kernel: one per row; cols kernel: one per column block;
-                              // zero on entry, zero again on exit
+  // decomposition into stages (rb_gemv_stream.cuh)
+  int nb;                     // stages per unit
+  int q, rem;                 // stages per CTA: q, and one more in the first `rem` CTAs
+  E* scratch;                 // partial states of units cut between CTAs
+  long long kslots;           // partial-state slots per output of a cut unit
+  unsigned* tickets;          // one per unit and consumer warp, zero on entry and on exit
+  int* status;                // set to 2 when a pipeline wait gives up
+  int groups;                 // thread groups per output (2, 4, 8)
+  // failure-path test hook (rb_debug_pipeline_fault): each CTA's copy warp issues at most
+  // `stop_after` stages (< 0: all), and consumers give up waiting for a stage's data after
+  // `wait_polls` polls (0: the default ~2 s)
+  long long stop_after;
+  long long wait_polls;
+};
+
+// One tensor map of A per phase.
+struct GemvMaps {
+  CUtensorMap m[4];
 };
 
 template <typename E>
 struct XOps {
-  cudaError_t (*gemv)(const XGemvArgs<E>& g, bool rows, dim3 grid, cudaStream_t s);
+  cudaError_t (*gemv)(const XGemvArgs<E>& g, const GemvMaps& maps, bool rows, int grid, cudaStream_t s);
   // decomposition of an M x N x K product (whole_tiles: no tile is cut between CTAs)
   cudaError_t (*gemm_plan)(long long M, long long N, long long K, int sms, bool whole_tiles,
                            GemmPlan* p);
   cudaError_t (*gemm)(const XGemmArgs<E>& g, const GemmPlan& p, cudaStream_t s);
-  // bx_i = fl(alpha * x_i) for i < n, contiguous (the rows kernel's vector input)
-  cudaError_t (*scale_x)(const E* x, long long n, long long incx, E ar, E ai, int alpha_one,
-                         E* bx, int grid, cudaStream_t s);
 };
-// indexed by fold - 2 (folds 2..8)
-extern const XOps<float> xops_s[7];    // rb_xblas23_s.cu
-extern const XOps<double> xops_z[7];   // rb_xblas23_z.cu
-extern const XOps<float> xops_c[7];    // rb_xblas23_c.cu
+// Kernels of folds 2..8, per element type (rb_blas23_[dszc]{2_4,5_8}.cu).
+extern const XOps<double> xops_d_f2, xops_d_f3, xops_d_f4, xops_d_f5, xops_d_f6, xops_d_f7, xops_d_f8;
+extern const XOps<float> xops_s_f2, xops_s_f3, xops_s_f4, xops_s_f5, xops_s_f6, xops_s_f7, xops_s_f8;
+extern const XOps<double> xops_z_f2, xops_z_f3, xops_z_f4, xops_z_f5, xops_z_f6, xops_z_f7, xops_z_f8;
+extern const XOps<float> xops_c_f2, xops_c_f3, xops_c_f4, xops_c_f5, xops_c_f6, xops_c_f7, xops_c_f8;
 
 bool fold_supported(int fold);
 // Folds of the register-resident kernels (2..kMaxFold, a template parameter) and the largest

@@ -173,6 +173,12 @@ bool Workspace::ensure_tickets(size_t n) {
   return true;
 }
 
+bool Workspace::reset_after_abort() {
+  return cuda_ok(cudaMemsetAsync(dstatus(), 0, 4, stream), "cudaMemsetAsync") &&
+         (!tickets || cuda_ok(cudaMemsetAsync(tickets, 0, ntickets * sizeof(unsigned), stream), "cudaMemsetAsync")) &&
+         cuda_ok(cudaStreamSynchronize(stream), "cudaStreamSynchronize");
+}
+
 bool gemm_decompose(cudaError_t (*plan)(long long, long long, long long, int, bool, GemmPlan*),
                     Workspace* w, long long M, long long N, long long K, GemmPlan* p) {
   DeviceInfo di;
@@ -328,9 +334,7 @@ int rb_synchronize(void) {
       !rb::cuda_ok(cudaStreamSynchronize(s), "cudaStreamSynchronize"))
     return RB_ERR_CUDA;
   if (*hs != 0) {
-    if (!rb::cuda_ok(cudaMemsetAsync(w->dstatus(), 0, 4, s), "cudaMemsetAsync") ||
-        !rb::cuda_ok(cudaStreamSynchronize(s), "cudaStreamSynchronize"))
-      return RB_ERR_CUDA;
+    if (!w->reset_after_abort()) return RB_ERR_CUDA;
     rb::set_error(RB_ERR_CUDA, "a pipeline wait timed out in an earlier call on this stream "
                                "(its affected outputs are NaN)");
     return RB_ERR_CUDA;
