@@ -119,6 +119,118 @@ bool gemv_maps(GemvMaps* maps, const void* A, size_t es, long long Rs, long long
   return true;
 }
 
+// Decomposition of the streaming gemv (rb_gemv_stream.cuh): G thread groups per output, units of P
+// = 512/G outputs, stages of 128/es*G elements of the reduction, and the split of the stages
+// over at most one CTA per SM.
+struct GemvShape {
+  int G, grid, q, rem, parts;
+  long long nunits, nb, kslots;
+};
+GemvShape gemv_shape(bool rows, long long nout, long long nred, int es, bool cx, int fold, int phases,
+                     int sms) {
+  // Cost in us, from a sweep over G and the grid on the shapes of 128 MiB and below. A stage takes
+  // its CTA 1.45 us (64 KB at the SM's share of HBM) or the deposits' issue time: measured 3.1 at
+  // fold 3 for complex elements. Behind the last stage: 5 us when no unit is cut, 8 when
+  // every CTA has one part of one unit, 10 when the ranges cut anywhere (two runs per CTA), and
+  // about 0.4 per part a lane merges.
+  const double work = (es == 8 && !cx) || es == 16 ? (3 * fold - 1) * 2 + 2 * fold : (3 * fold - 1) + fold;
+  const double dep = cx ? 4.0 * (128 / es) : 128 / es;
+  double stage = dep * work * 4 / 1900 * (cx ? 2.0 : 1.15);
+  if (stage < 1.45) stage = 1.45;
+  GemvShape best{};
+  double best_cost = 0;
+  for (int G = 2; G <= 8; G *= 2) {
+    // columns: a box is at most 256 words of 8 bytes wide, and a thread's rows are of one phase
+    if (!rows && (gemv_slot(false, G, es, phases) > 2048 || G < phases)) continue;
+    // bank conflicts between a warp's groups
+    const double m = G == 8 ? (rows ? (phases > 1 ? 1.2 : 1.0) : es == 16 ? 0.98 : es == 4 ? 1.4 : cx ? 1.04 : 1.13)
+                            : (G == 2 ? 1.05 : 1.0);
+    GemvShape s{};
+    s.G = G;
+    const long long P = 512 / G, SC = (long long)(128 / es) * G;
+    s.nunits = (nout + P - 1) / P;
+    s.nb = nred > 0 ? (nred + SC - 1) / SC : 1;
+    const long long T = s.nunits * s.nb;
+    for (int way = 0; way < 2; way++) {
+      double ends;
+      long long per;   // stages of the busiest CTA
+      if (way == 0) {
+        s.parts = 0;
+        s.grid = (int)(T < sms ? T : sms);
+        s.q = (int)(T / s.grid);
+        s.rem = (int)(T % s.grid);
+        per = (T + s.grid - 1) / s.grid;
+        // a unit meets at most ceil((nb-1) / q) + 1 ranges
+        s.kslots = s.nb / s.q + 2;
+        ends = s.grid == s.nunits && s.rem == 0 ? 5 : 10 + 0.4 * (double)(s.kslots / G);
+      } else if (s.nunits <= sms) {
+        long long p = sms / s.nunits;
+        if (p > s.nb) p = s.nb;
+        s.parts = (int)p;
+        s.grid = (int)(s.nunits * p);
+        s.q = 1;
+        s.rem = (int)s.nunits;
+        per = (s.nb + p - 1) / p;
+        s.kslots = p;
+        ends = p == 1 ? 5 : 8 + 0.4 * (double)((p + G - 1) / G);
+      } else {
+        const long long wu = (s.nunits + sms - 1) / sms;
+        s.parts = 1;
+        s.q = (int)wu;
+        s.rem = (int)s.nunits;
+        s.grid = (int)((s.nunits + wu - 1) / wu);
+        per = wu * s.nb;
+        s.kslots = 1;
+        ends = 5;
+      }
+      const double cost = (double)per * stage * m + ends;
+      if (best.G == 0 || cost < best_cost) {
+        best = s;
+        best_cost = cost;
+      }
+    }
+  }
+  return best;
+}
+
+// Shape of the direct columns kernel: G row groups per CTA and `parts` row chunks. Cost model in
+// units of one row per thread: the streaming part (waves of CTAs, two per SM, times rows per
+// thread, plus the groups' merge) and the sum of the chunks' partial states.
+GemvShape gemv_direct_shape(long long nout, long long nred, int sms) {
+  GemvShape best{};
+  long long best_cost = -1;
+  const long long slots = (long long)sms * 2;
+  for (int G = 1, lg = 0; G <= 8; G *= 2, lg++) {
+    const long long cb = (nout + 256 / G - 1) / (256 / G);
+    const long long most = (nred + 8 * G - 1) / (8 * G);   // at least 8 rows per group
+    for (long long ch : {slots / cb, (slots + cb - 1) / cb}) {
+      if (ch > most) ch = most;
+      if (ch > 1024) ch = 1024;
+      if (ch < 1) ch = 1;
+      const long long rpt = ((nred + ch - 1) / ch + G - 1) / G;
+      const long long waves = (cb * ch + slots - 1) / slots;
+      const long long cost = waves * (rpt + 8 * lg) + 4 * ((ch + G - 1) / G + 2 * lg);
+      if (best_cost < 0 || cost < best_cost) {
+        best_cost = cost;
+        best.G = G;
+        best.grid = (int)cb;
+        best.parts = (int)ch;
+        best.nunits = cb;
+        best.kslots = ch;
+      }
+    }
+  }
+  return best;
+}
+
+// Matrices whose rows the direct kernel reduces sooner than the streaming one (us a call, direct /
+// streaming): FP64 1000x500 10.3 / 12.8, 2048x1024 10.5 / 14.5, 64x20000 14.5 / 27.3, FP32
+// 2000x2001 14.5 / 18.6, FP64 complex 1024^2 16.5 / 22.0, fold 8 2048^2 24.7 / 28.9; about even at
+// 32 MB (FP64 2000x2001 17.2 / 18.7). Many short rows stream: 20000x64 20.6 / 11.4.
+bool gemv_small(long long nout, long long nred, int es) {
+  return nout * nred * es <= (24ll << 20) && nout <= 8192;
+}
+
 template <typename E, bool CX>
 bool run_xgemv(const XGemvReq<E, CX>& q) {
   constexpr int NC = CX ? 2 : 1;
@@ -171,21 +283,6 @@ bool run_xgemv(const XGemvReq<E, CX>& q) {
   const size_t x_bytes = span(nred_eff, q.incX, es);
   const size_t y_bytes = q.mode == kOutValue ? span(nout, q.incY, es)
                                              : ((size_t)(nout - 1) * q.incY + 1) * per_state;
-  // Decomposition (rb_gemv_stream.cuh): G thread groups per output; units are bands or blocks
-  // of P = 512/G outputs, stages cover 128/es*G elements of the reduction, and the stages of
-  // all units are split evenly over one CTA per SM (every CTA gets at least one). Take the
-  // smallest G for which the last CTA of a cut unit merges at most about 4 parts per thread.
-  const long long pe = 128 / (long long)es;
-  long long nunits = 0, nb = 0, T = 0, grid = 0, parts = 0;
-  auto shape = [&](int G) {
-    const long long P = 512 / G;
-    nunits = (nout + P - 1) / P;
-    nb = nred_eff > 0 ? (nred_eff + pe * G - 1) / (pe * G) : 1;
-    T = nunits * nb;
-    grid = T < di.sms ? T : di.sms;
-    // a unit meets at most ceil((nb-1) / min_range) + 1 CTA ranges, min_range = floor(T/grid)
-    parts = nb / (T / grid) + 2;
-  };
   // phases the rows are taken in: the fewest whose pitch is a multiple of 16 bytes, at least
   // two when A itself is misaligned (host operands are copied to aligned device memory)
   const bool a_dev = a_bytes && on_device(q.A);
@@ -193,31 +290,15 @@ bool run_xgemv(const XGemvReq<E, CX>& q) {
   int phases = 1;
   while (((size_t)phases * q.lda * es) % 16 != 0) phases *= 2;
   if (phases == 1 && a_mis != 0) phases = 2;
-  // columns: a box is at most 256 words of 8 bytes wide, and a thread's rows are of one phase
-  int G = 2;
-  if (!nt)
-    while (gemv_slot(false, G, (int)es, phases) > 2048 || G < phases) G *= 2;
-  for (;;) {
-    shape(G);
-    if ((parts + G - 1) / G <= 4 || G == 8) break;
-    G *= 2;
-  }
-  // rows: G = 4 measured as fast or faster than the rule above on every band shape tried
-  // (2048^2 to 16384^2, 1024 x 16384 to 32768 x 4096), as long as its final merge stays within
-  // about 8 parts per thread
-  if (nt && G != 4) {
-    const int g0 = G;
-    shape(4);
-    if ((parts + 3) / 4 <= 8) {
-      G = 4;
-    } else {
-      G = g0;
-      shape(G);
-    }
-  }
-  const long long kslots = nb / (T / grid) + 2;
-  const size_t part_bytes = (size_t)nout * kslots * NC * (2 * q.fold + 1) * sizeof(E);
-  if (!w->ensure_tickets((size_t)nunits * 16)) return false;   // one per unit and consumer warp
+  const bool small = nt && gemv_small(nout, nred_eff, (int)es);
+  // (bounds: see gemv_cols_direct_kernel)
+  const bool direct = !nt && (gs::direct_cols<E, CX>() ||
+                              (nred_eff >= 256 && nout * nred_eff * (long long)es <= (16ll << 20)));
+  GemvShape sh{};
+  if (direct) sh = gemv_direct_shape(nout, nred_eff, di.sms);
+  else if (!small) sh = gemv_shape(nt, nout, nred_eff, (int)es, CX, q.fold, phases, di.sms);
+  const size_t part_bytes = (size_t)nout * sh.kslots * NC * (2 * q.fold + 1) * sizeof(E);
+  if (!small && !w->ensure_tickets((size_t)sh.nunits * 16)) return false;   // per unit and consumer warp
   const bool a_host = a_bytes && !a_dev, x_host = x_bytes && !on_device(q.X);
   const bool y_host = !on_device(q.Y);
   const size_t need = part_bytes + (a_host ? a_bytes : 0) + (x_host ? x_bytes : 0) +
@@ -248,20 +329,30 @@ bool run_xgemv(const XGemvReq<E, CX>& q) {
   g.y = q.mode == kOutValue ? dY : nullptr;
   g.ybin = q.mode == kOutBinned ? dY : nullptr;
   g.incy = q.incY;
-  g.nb = (int)nb;
-  g.q = (int)(T / grid);
-  g.rem = (int)(T % grid);
+  g.nb = (int)sh.nb;
+  g.q = sh.q;
+  g.rem = sh.rem;
+  g.parts = sh.parts;
   g.scratch = part;
-  g.kslots = kslots;
+  g.kslots = sh.kslots;
   g.tickets = w->tickets;
   g.status = w->dstatus();
-  g.groups = G;
+  g.groups = sh.G;
   g.phases = phases;
   pipeline_fault(&g.stop_after, &g.wait_polls);
   GemvMaps maps{};
-  if (nred_eff > 0 && !gemv_maps(&maps, dA, (size_t)es, Rs, Cs, q.lda, phases, nt, G)) return false;
+  int grid = sh.grid;
+  if (small) {
+    // enough warps to fill the device, at least 64 elements to each
+    int S = 1;
+    while (S < 8 && nout * S < (long long)di.sms * 16 && nred_eff >= 128 * S) S *= 2;
+    g.groups = S;
+    grid = (int)((nout + 8 / S - 1) / (8 / S));
+  } else if (!direct && nred_eff > 0 && !gemv_maps(&maps, dA, (size_t)es, Rs, Cs, q.lda, phases, nt, sh.G)) {
+    return false;
+  }
   count_launch();
-  if (!cuda_ok(o->gemv(g, maps, nt, (int)grid, s), "gemv launch")) return false;
+  if (!cuda_ok(o->gemv(g, small || direct ? nullptr : &maps, nt, grid, s), "gemv launch")) return false;
   if (y_host) {
     int* hs = w->hstatus();
     if (!cuda_ok(cudaMemcpyAsync(q.Y, dY, y_bytes, cudaMemcpyDeviceToHost, s), "copy y") ||

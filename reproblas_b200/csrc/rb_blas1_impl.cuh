@@ -476,9 +476,9 @@ __device__ __forceinline__ void cprod(T xr, T xi, T yr, T yi, T& r0, T& r1, T& i
   i0 = B::mul(xr, yi);
   if (OP == kOpCDotc) {
     r1 = B::mul(xi, yi);
-    i1 = -B::mul(xi, yr);
+    i1 = B::mul(-xi, yr);
   } else {
-    r1 = -B::mul(xi, yi);
+    r1 = B::mul(-xi, yi);
     i1 = B::mul(xi, yr);
   }
 }

@@ -47,7 +47,7 @@ __device__ __forceinline__ void products(Val<E, CX> a, Val<E, CX> b, E (&v)[CX ?
   using B = BT<E>;
   if constexpr (CX) {
     v[0][2 * q] = B::mul(a.r, b.r);
-    v[0][2 * q + 1] = -B::mul(a.i, b.i);
+    v[0][2 * q + 1] = B::mul(-a.i, b.i);
     v[1][2 * q] = B::mul(a.r, b.i);
     v[1][2 * q + 1] = B::mul(a.i, b.r);
   } else {

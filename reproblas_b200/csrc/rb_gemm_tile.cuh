@@ -196,7 +196,7 @@ struct Tile {
     if constexpr (CX) {
       const E ar = a[2 * i], ai = a[2 * i + 1], br = b[2 * j], bi = b[2 * j + 1];
       p[0] = c == 0 ? B::mul(ar, br) : B::mul(ar, bi);
-      p[1] = c == 0 ? -B::mul(ai, bi) : B::mul(ai, br);
+      p[1] = c == 0 ? B::mul(-ai, bi) : B::mul(ai, br);
     } else {
       p[0] = B::mul(a[i], b[j]);
     }
@@ -323,7 +323,7 @@ struct Tile {
   // CTA call it together.
   __device__ __forceinline__ void reduce(const XGemmArgs<E>& g, long long m0, long long n0,
                                          long long kb0, long long kb1) {
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int tid = threadIdx.x, lane = tid & 31;
     const int ra = (tid >> 4) * TM, cb = (tid & 15) * TN;
     // element copies of a stage: thread t copies AEL elements of op(A) and BEL of op(B), at a
     // fixed distance, along the operand's unit stride

@@ -71,22 +71,34 @@ constexpr size_t kSmemBytes = (size_t)kStages * kStageBytes + 1024;
 static_assert(kSmemBytes + 256 <= 227 * 1024, "shared memory of the gemv kernel");
 
 // Work split. The stages are numbered unit-major, x = u * nb + j (unit u = band of rows or
-// block of columns; j = its j-th stage), and every CTA streams a contiguous range of q or q + 1
-// of them, whatever the shape. A unit whose stages all fall in one CTA is finished there; a
-// unit cut between CTAs leaves one partial state per CTA in slot k = i - owner(first stage of
-// u), and the last of those CTAs to finish (ticket) merges them.
+// block of columns; j = its j-th stage), and every CTA streams a contiguous range of them: with
+// `parts` = 0, q or q + 1 stages each, whatever the shape; with parts = p > 0, the p-th part of a
+// unit (p > 1) or q whole units (p = 1), so that a CTA has one run, or no unit is cut. A unit
+// whose stages all fall in one CTA is finished there; a unit cut between CTAs leaves one
+// partial state per CTA in slot k = i - owner(first stage of u), and the last of those CTAs to
+// finish (ticket) merges them.
 struct Split {
-  int q, rem, x0, x1;
+  int q, rem, parts, nb, x0, x1;
   template <typename E>
-  __device__ __forceinline__ explicit Split(const XGemvArgs<E>& g) : q(g.q), rem(g.rem) {
-    const int b = (int)blockIdx.x;
-    x0 = b * q + (b < rem ? b : rem);
-    x1 = x0 + q + (b < rem ? 1 : 0);
+  __device__ __forceinline__ explicit Split(const XGemvArgs<E>& g)
+      : q(g.q), rem(g.rem), parts(g.parts), nb(g.nb) {
+    x0 = start((int)blockIdx.x);
+    x1 = start((int)blockIdx.x + 1);
+  }
+  __device__ __forceinline__ int start(int b) const {
+    if (parts == 0) return b * q + (b < rem ? b : rem);
+    if (parts == 1) return (b * q < rem ? b * q : rem) * nb;   // rem: units in all
+    return b / parts * nb + (int)((long long)(b % parts) * nb / parts);
   }
   // CTA whose range holds stage x
   __device__ __forceinline__ int owner(int x) const {
-    const int big = rem * (q + 1);
-    return x < big ? x / (q + 1) : rem + (x - big) / q;
+    if (parts == 0) {
+      const int big = rem * (q + 1);
+      return x < big ? x / (q + 1) : rem + (x - big) / q;
+    }
+    const int u = x / nb;
+    if (parts == 1) return u / q;
+    return u * parts + (int)(((long long)(x - u * nb + 1) * parts - 1) / nb);
   }
 };
 
@@ -243,8 +255,12 @@ template <typename E, bool CX, int F, bool ROWS>
 struct Consumer {
   using Gm = Geom<E, CX, ROWS>;
   using B = BT<E>;
-  static constexpr int NC = Gm::NC, PE = Gm::PE, ES = Gm::ES, D = CX ? 2 : 1, ND = PE * D;
-  static constexpr int NR = PE * NC;   // reals per thread and stage
+  static constexpr int NC = Gm::NC, PE = Gm::PE, ES = Gm::ES, D = CX ? 2 : 1;
+  // a stage's elements are taken in STEPS steps of PS: FP64 complex would spill with all 128
+  // bytes in registers
+  static constexpr int STEPS = (CX && sizeof(E) == 8) ? 2 : 1;
+  static constexpr int PS = PE / STEPS, ND = PS * D;
+  static constexpr int NR = PS * NC;   // reals per thread and step
 
   Acc<E, F> a[NC];
   __device__ __forceinline__ void zero() {
@@ -259,33 +275,35 @@ struct Consumer {
     bool vec;
   };
 
-  __device__ __forceinline__ void load(const unsigned char* base, const Place& pl, E (&v)[NR]) const {
+  // the elements of step h
+  __device__ __forceinline__ void load(const unsigned char* base, const Place& pl, int h, E (&v)[NR]) const {
     if (pl.vec) {
       if constexpr (ROWS) {
-        constexpr int PER = 16 / (int)sizeof(E);
+        constexpr int PER = 16 / (int)sizeof(E), CH = NR / PER;
 #pragma unroll
-        for (int c = 0; c < (int)kThreadBytes / 16; c++) {
+        for (int c = 0; c < CH; c++) {
           E t[PER];
-          gt::lds_vec<E, PER>((const E*)(base + (((uint32_t)c ^ pl.swz) << 4)), t);
+          gt::lds_vec<E, PER>((const E*)(base + (((uint32_t)(h * CH + c) ^ pl.swz) << 4)), t);
 #pragma unroll
           for (int i = 0; i < PER; i++) v[c * PER + i] = t[i];
         }
       } else {
+        const unsigned char* p = base + (uint32_t)(h * PS) * pl.stride;
 #pragma unroll
-        for (int e = 0; e < PE; e++) {
+        for (int e = 0; e < PS; e++) {
           E t[NC];
-          gt::lds_vec<E, NC>((const E*)(base + (uint32_t)e * pl.stride), t);
+          gt::lds_vec<E, NC>((const E*)(p + (uint32_t)e * pl.stride), t);
 #pragma unroll
           for (int c = 0; c < NC; c++) v[e * NC + c] = t[c];
         }
       }
     } else {
-      const unsigned char* p = base + pl.shift;
+      const uint32_t stride = ROWS ? (uint32_t)ES : pl.stride;
+      const unsigned char* p = base + pl.shift + (uint32_t)(h * PS) * stride;
 #pragma unroll
-      for (int e = 0; e < PE; e++)
+      for (int e = 0; e < PS; e++)
 #pragma unroll
-        for (int c = 0; c < NC; c++)
-          v[e * NC + c] = ((const E*)(p + (uint32_t)e * (ROWS ? (uint32_t)ES : pl.stride)))[c];
+        for (int c = 0; c < NC; c++) v[e * NC + c] = ((const E*)(p + (uint32_t)e * stride))[c];
     }
   }
   // real i of element e, the same way
@@ -298,17 +316,17 @@ struct Consumer {
   static __device__ __forceinline__ void prods(const E* av, const E* xv, int c, E (&p)[D]) {
     if constexpr (CX) {
       p[0] = c == 0 ? B::mul(av[0], xv[0]) : B::mul(av[0], xv[1]);
-      p[1] = c == 0 ? -B::mul(av[1], xv[1]) : B::mul(av[1], xv[0]);
+      p[1] = c == 0 ? B::mul(-av[1], xv[1]) : B::mul(av[1], xv[0]);
     } else {
       p[0] = B::mul(av[0], xv[0]);
     }
   }
 
-  // one by one: nval elements, with every check (Acc::tile)
-  __device__ __forceinline__ void deposit_careful(const unsigned char* base, const Place& pl,
-                                                  const E* xs, int nval, bool conj) {
+  // one by one: elements [e0, e1), with every check (Acc::tile)
+  __device__ __forceinline__ void deposit_careful(const unsigned char* base, const Place& pl, const E* xs,
+                                                  int e0, int e1, bool conj) {
 #pragma unroll 1
-    for (int e = 0; e < nval; e++) {
+    for (int e = e0; e < e1; e++) {
       const E* p = at(base, pl, e);
       E av[NC], xv[NC];
 #pragma unroll
@@ -328,11 +346,20 @@ struct Consumer {
 
   __device__ __forceinline__ void stage(const unsigned char* base, const Place& pl, const E* xs,
                                         unsigned xkey, int nval, bool conj) {
+    if constexpr (STEPS > 1) {
+      if (nval < PE) {
+        if (nval > 0) deposit_careful(base, pl, xs, 0, nval, conj);
+        return;
+      }
+#pragma unroll 1
+      for (int h = 0; h < STEPS; h++) step(base, pl, h, xs + h * NR, xs, xkey, conj);
+      return;
+    }
     if (nval <= 0) return;
     bool careful = nval < PE;
     E v[NR];
     if (!careful) {
-      load(base, pl, v);
+      load(base, pl, 0, v);
       float m = 0.0f;
 #pragma unroll
       for (int i = 0; i < NR; i += 2) m = max_abs3(m, key_word(v[i]), key_word(v[i + 1]));
@@ -377,7 +404,7 @@ struct Consumer {
       }
     }
     if (careful) {
-      deposit_careful(base, pl, xs, nval, conj);
+      deposit_careful(base, pl, xs, 0, nval, conj);
       return;
     }
 #pragma unroll
@@ -387,6 +414,73 @@ struct Consumer {
       gt::lds_vec<E, XR>(xs + e * NC, xv);
 #pragma unroll
       for (int q = 0; q < 16 / ES; q++)
+#pragma unroll
+        for (int c = 0; c < NC; c++) {
+          E p[D];
+          prods(v + (e + q) * NC, xv + q * NC, c, p);
+#pragma unroll
+          for (int d = 0; d < D; d++) a[c].deposit(p[d]);
+        }
+    }
+  }
+  // step h of a whole stage (xh: its bx)
+  __device__ __forceinline__ void step(const unsigned char* base, const Place& pl, int h, const E* xh,
+                                       const E* xs, unsigned xkey, bool conj) {
+    E v[NR];
+    load(base, pl, h, v);
+    float m = 0.0f;
+#pragma unroll
+    for (int i = 0; i < NR; i += 2) m = max_abs3(m, key_word(v[i]), key_word(v[i + 1]));
+    const unsigned bound = B::key(B::mul(gt::key_ceiling<E>(__float_as_uint(m)), gt::key_ceiling<E>(xkey)));
+    bool fast = true;
+#pragma unroll
+    for (int c = 0; c < NC; c++) fast = fast && a[c].fast(bound, ND);
+    if (CX && conj) {
+#pragma unroll
+      for (int e = 0; e < PS; e++) v[e * NC + NC - 1] = -v[e * NC + NC - 1];
+    }
+    if (fast) {
+#pragma unroll
+      for (int c = 0; c < NC; c++) a[c].deposits += ND;
+    } else {
+      bool careful = bound >= B::kInfKey;
+      if (!careful) {
+        // the exact largest key of each component's products, then the index that needs
+        unsigned mk[NC];
+#pragma unroll
+        for (int c = 0; c < NC; c++) mk[c] = 0u;
+#pragma unroll
+        for (int e = 0; e < PS; e++)
+#pragma unroll
+          for (int c = 0; c < NC; c++) {
+            E p[D], xv[NC];
+#pragma unroll
+            for (int q = 0; q < NC; q++) xv[q] = xh[e * NC + q];
+            prods(v + e * NC, xv, c, p);
+#pragma unroll
+            for (int d = 0; d < D; d++) {
+              const unsigned kk = B::key(p[d]);
+              mk[c] = kk > mk[c] ? kk : mk[c];
+            }
+          }
+#pragma unroll
+        for (int c = 0; c < NC; c++) {
+          a[c].prepare(mk[c], ND);
+          if (a[c].idx == 0) careful = true;
+        }
+      }
+      if (careful) {
+        deposit_careful(base, pl, xs, h * PS, (h + 1) * PS, conj);
+        return;
+      }
+    }
+    constexpr int XR = 16 / (int)sizeof(E);   // reals of one 16-byte vector of bx
+#pragma unroll
+    for (int e = 0; e < PS; e += XR / NC) {
+      E xv[XR];
+      gt::lds_vec<E, XR>(xh + e * NC, xv);
+#pragma unroll
+      for (int q = 0; q < XR / NC; q++)
 #pragma unroll
         for (int c = 0; c < NC; c++) {
           E p[D];
@@ -581,8 +675,232 @@ gemv_stream_kernel(const __grid_constant__ XGemvArgs<E> g, const __grid_constant
   if (tid == 0 && sy.abort_flag) atomicExch(g.status, 2);
 }
 
+// ---------------------------------------------------------------------------------------
+// Rows kernel for small matrices: a CTA of 8 warps takes 8/S rows, S = g.groups warps to a row
+// (S = 1, 2, 4, 8), and reads A and x straight from global memory. No pipeline to fill and no
+// unit to merge across CTAs: 7-8 us a call where the streaming kernel takes 10-12.
+// ---------------------------------------------------------------------------------------
 template <typename E, bool CX, int F>
-cudaError_t launch_gemv(const XGemvArgs<E>& g, const GemvMaps& maps, bool rows, int grid, cudaStream_t s) {
+__global__ void __launch_bounds__(256) gemv_rows_small_kernel(const __grid_constant__ XGemvArgs<E> g) {
+  constexpr int NC = CX ? 2 : 1, D = CX ? 2 : 1, REC = 2 * F + 1;
+  constexpr int K = CX ? 4 : 8;   // elements per lane and step
+  __shared__ E sm[8][NC * REC];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, S = g.groups;
+  const int part = warp & (S - 1), rows = 8 / S;
+  const long long r = (long long)blockIdx.x * rows + warp / S;
+  Acc<E, F> a[NC];
+#pragma unroll
+  for (int c = 0; c < NC; c++) a[c].zero();
+  if (r < g.R) {
+    const E* row = g.A + r * g.lda * NC;
+#pragma unroll 1
+    for (long long b = part * 32 + lane; b < g.C; b += (long long)K * 32 * S) {
+      Val<E, CX> av[K], xv[K];
+      int n = 0;   // elements that exist; all loads before the math
+#pragma unroll
+      for (int k = 0; k < K; k++) {
+        const long long e = b + (long long)k * 32 * S;
+        av[k] = Val<E, CX>{E(0), E(0)};
+        xv[k] = Val<E, CX>{E(0), E(0)};
+        if (e < g.C) {
+          av[k] = xb::ldv<E, CX>(row, e);
+          xv[k] = xb::ldv<E, CX>(g.x, e * g.incx);
+          n = k + 1;
+        }
+      }
+      E v[NC][K * D];
+#pragma unroll
+      for (int k = 0; k < K; k++) {
+        if (!g.alpha_one && k < n) xv[k] = xb::scale<E, CX>(xv[k], g.ar, g.ai);
+        if (CX && g.conj) av[k].i = -av[k].i;
+        xb::products<E, CX, K * D>(av[k], xv[k], v, k);
+      }
+#pragma unroll
+      for (int c = 0; c < NC; c++) a[c].template tile<K * D>(v[c], n * D);
+    }
+  }
+#pragma unroll
+  for (int c = 0; c < NC; c++) a[c].renorm();
+  warp_merge_all<E, F, NC>(a);
+  if (S > 1) {
+    if (lane == 0) {
+#pragma unroll
+      for (int c = 0; c < NC; c++) xb::put_rec<E, F>(a[c], &sm[warp][c * REC], 1);
+    }
+    __syncthreads();
+    if (part == 0 && lane == 0) {
+#pragma unroll
+      for (int c = 0; c < NC; c++) {
+        SumAcc<E, F> sum;
+        sum.zero();
+        sum.add(a[c]);
+#pragma unroll 1
+        for (int q = 1; q < S; q++) {
+          Acc<E, F> o;
+          o.zero();
+#pragma unroll
+          for (int i = 0; i < F; i++) {
+            o.pri[i] = sm[warp + q][c * REC + i];
+            o.car[i] = sm[warp + q][c * REC + F + i];
+          }
+          o.flags = xb::flags_from<E>(sm[warp + q][c * REC + 2 * F]);
+          o.set_idx_from_pri();
+          sum.add(o);
+        }
+        sum.get(a[c]);
+      }
+    }
+  }
+  if (part == 0 && lane == 0 && r < g.R)
+    xb::finish<E, CX, F>(a, g.mode, g.y + r * g.incy * NC, g.br, g.bi, g.ybin + r * g.incy * 2 * F * NC);
+}
+
+// ---------------------------------------------------------------------------------------
+// Columns kernel straight from global memory. For FP64 complex, whose two accumulators and
+// operands do not fit the streaming kernel's 96 registers (us a call at 2048^2, this kernel /
+// the streaming one: fold 3 33 / 39, fold 4 37 / 45, fold 6 48 / 68, fold 8 60 / 113), and for
+// small matrices of the other types, which pay for filling the streaming kernel's pipeline
+// and for its ends (FP64 500x2000 10.7 / 13.5, 2048x1024 14.5 / 16.6, FP32 1000x500 10.4 /
+// 13.7; even at 32 MB, and slower for short reductions: FP32 100x5000 10.4 / 8.3).
+// A CTA of 256 threads is G = g.groups row groups of 256/G threads, one column each; grid =
+// (column blocks, row chunks), inside a chunk group q takes rows q, q + G, ..., four per step.
+// fl(alpha*x) of 256 rows at a time is formed in shared memory. The groups' states merge
+// through shared memory; with several chunks each leaves a partial state (structure of
+// arrays), and the last CTA of a column block to arrive sums them and finishes.
+// ---------------------------------------------------------------------------------------
+template <typename E, bool CX>
+constexpr bool direct_cols() { return CX && sizeof(E) == 8; }
+
+// Sum of the G row groups' states (renormalised) through sm[i * 256 + thread]: group 0 ends with
+// the merged state. All 256 threads call it.
+template <typename E, int F>
+__device__ __forceinline__ void sum_groups(Acc<E, F>& a, E* sm, int grp, int t, int G, int T) {
+  __syncthreads();
+  if (grp > 0) xb::put_rec<E, F>(a, sm + threadIdx.x, 256);
+  __syncthreads();
+  if (grp == 0 && G > 1) {
+    SumAcc<E, F> sum;
+    sum.zero();
+    sum.add(a);
+#pragma unroll 1
+    for (int q = 1; q < G; q++) {
+      const E* rec = sm + q * T + t;
+      Acc<E, F> o;
+      o.zero();
+#pragma unroll
+      for (int i = 0; i < F; i++) {
+        o.pri[i] = rec[i * 256];
+        o.car[i] = rec[(F + i) * 256];
+      }
+      o.flags = xb::flags_from<E>(rec[2 * F * 256]);
+      o.set_idx_from_pri();
+      sum.add(o);
+    }
+    sum.get(a);
+  }
+}
+
+template <typename E, bool CX, int F>
+__global__ void __launch_bounds__(256, 2) gemv_cols_direct_kernel(const __grid_constant__ XGemvArgs<E> g) {
+  constexpr int NC = CX ? 2 : 1, D = CX ? 2 : 1, K = 4, REC = 2 * F + 1;
+  __shared__ E sm[REC * 256];
+  __shared__ E xs[256 * NC];
+  __shared__ unsigned s_last;
+  const int G = g.groups, T = 256 / G;
+  const int grp = threadIdx.x / T, t = threadIdx.x % T;
+  const long long col = (long long)blockIdx.x * T + t;
+  const int chunk = blockIdx.y, nchunks = gridDim.y;
+  const long long per = (g.R + nchunks - 1) / nchunks;
+  const long long r0 = (long long)chunk * per < g.R ? (long long)chunk * per : g.R;
+  const long long r1 = r0 + per < g.R ? r0 + per : g.R;
+  Acc<E, F> a[NC];
+#pragma unroll
+  for (int c = 0; c < NC; c++) a[c].zero();
+  const E* A = g.A + col * NC;
+#pragma unroll 1
+  for (long long base = r0; base < r1; base += 256) {
+    const int n = r1 - base < 256 ? (int)(r1 - base) : 256;
+    __syncthreads();
+    if ((int)threadIdx.x < n) {
+      Val<E, CX> v = xb::ldv<E, CX>(g.x, (base + threadIdx.x) * g.incx);
+      if (!g.alpha_one) v = xb::scale<E, CX>(v, g.ar, g.ai);
+      xs[threadIdx.x * NC] = v.r;
+      if constexpr (CX) xs[threadIdx.x * NC + 1] = v.i;
+    }
+    __syncthreads();
+    if (col >= g.C) continue;
+#pragma unroll 1
+    for (int b = grp; b < n; b += K * G) {
+      Val<E, CX> av[K];
+      int m = 0;   // rows that exist; all loads before the math
+#pragma unroll
+      for (int k = 0; k < K; k++) {
+        av[k] = Val<E, CX>{E(0), E(0)};
+        if (b + k * G < n) {
+          av[k] = xb::ldv<E, CX>(A + (base + b + k * G) * g.lda * NC, 0);
+          m = k + 1;
+        }
+      }
+      E v[NC][K * D];
+#pragma unroll
+      for (int k = 0; k < K; k++) {
+        const int i = b + k * G < n ? b + k * G : b;   // absent rows multiply zeros
+        Val<E, CX> xv{xs[i * NC], CX ? xs[i * NC + NC - 1] : E(0)};
+        if (CX && g.conj) av[k].i = -av[k].i;
+        if (k >= m) xv = Val<E, CX>{E(0), E(0)};
+        xb::products<E, CX, K * D>(av[k], xv, v, k);
+      }
+      if constexpr (CX) tile2<E, F, K * D>(a[0], v[0], a[1], v[1]);
+      else a[0].template tile<K * D>(v[0], m * D);
+    }
+  }
+  E* part = g.scratch + (long long)chunk * NC * REC * g.C + col;   // field i at part[i * C]
+#pragma unroll
+  for (int c = 0; c < NC; c++) {
+    a[c].renorm();
+    sum_groups<E, F>(a[c], sm, grp, t, G, T);
+    if (nchunks > 1 && grp == 0 && col < g.C) xb::put_rec<E, F>(a[c], part + c * REC * g.C, g.C);
+  }
+  if (nchunks > 1) {
+    __threadfence();
+    __syncthreads();
+    if (threadIdx.x == 0) {
+      s_last = atomicAdd(g.tickets + blockIdx.x, 1u) == (unsigned)nchunks - 1 ? 1u : 0u;
+      if (s_last) g.tickets[blockIdx.x] = 0u;
+    }
+    __syncthreads();
+    if (!s_last) return;
+    __threadfence();
+#pragma unroll
+    for (int c = 0; c < NC; c++) {
+      SumAcc<E, F> sum;
+      sum.zero();
+      if (col < g.C) {
+#pragma unroll 2
+        for (int ch = grp; ch < nchunks; ch += G) {
+          Acc<E, F> o;
+          xb::read_rec<E, F>(o, g.scratch + ((long long)ch * NC + c) * REC * g.C + col, g.C);
+          sum.add(o);
+        }
+      }
+      sum.get(a[c]);
+      sum_groups<E, F>(a[c], sm, grp, t, G, T);
+    }
+  }
+  if (grp == 0 && col < g.C)
+    xb::finish<E, CX, F>(a, g.mode, g.y + col * g.incy * NC, g.br, g.bi, g.ybin + col * g.incy * 2 * F * NC);
+}
+
+template <typename E, bool CX, int F>
+cudaError_t launch_gemv(const XGemvArgs<E>& g, const GemvMaps* maps, bool rows, int grid, cudaStream_t s) {
+  if (!maps) {
+    if (rows) {
+      gemv_rows_small_kernel<E, CX, F><<<grid, 256, 0, s>>>(g);
+    } else {
+      gemv_cols_direct_kernel<E, CX, F><<<dim3(grid, g.parts), 256, 0, s>>>(g);
+    }
+    return cudaGetLastError();
+  }
   constexpr size_t smem = kSmemBytes;
   // opt in to the shared memory, once per device (the call is idempotent)
   constexpr int kMaxDevices = 64;
@@ -593,14 +911,16 @@ cudaError_t launch_gemv(const XGemvArgs<E>& g, const GemvMaps& maps, bool rows, 
   if (dev >= kMaxDevices || !ready[dev].load(std::memory_order_relaxed)) {
     e = cudaFuncSetAttribute(gemv_stream_kernel<E, CX, F, true>,
                              cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e == cudaSuccess)
-      e = cudaFuncSetAttribute(gemv_stream_kernel<E, CX, F, false>,
-                               cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if constexpr (!direct_cols<E, CX>()) {
+      if (e == cudaSuccess)
+        e = cudaFuncSetAttribute(gemv_stream_kernel<E, CX, F, false>,
+                                 cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    }
     if (e != cudaSuccess) return e;
     if (dev < kMaxDevices) ready[dev].store(1, std::memory_order_relaxed);
   }
-  if (rows) gemv_stream_kernel<E, CX, F, true><<<grid, kThreads, smem, s>>>(g, maps);
-  else gemv_stream_kernel<E, CX, F, false><<<grid, kThreads, smem, s>>>(g, maps);
+  if (rows) gemv_stream_kernel<E, CX, F, true><<<grid, kThreads, smem, s>>>(g, *maps);
+  else if constexpr (!direct_cols<E, CX>()) gemv_stream_kernel<E, CX, F, false><<<grid, kThreads, smem, s>>>(g, *maps);
   return cudaGetLastError();
 }
 

@@ -149,7 +149,7 @@ struct XGemvArgs {
   long long incy;
   // decomposition into stages (rb_gemv_stream.cuh)
   int nb;                     // stages per unit
-  int q, rem;                 // stages per CTA: q, and one more in the first `rem` CTAs
+  int q, rem, parts;          // split over the CTAs (Split)
   E* scratch;                 // partial states of units cut between CTAs
   long long kslots;           // partial-state slots per output of a cut unit
   unsigned* tickets;          // one per unit and consumer warp, zero on entry and on exit
@@ -169,7 +169,8 @@ struct GemvMaps {
 
 template <typename E>
 struct XOps {
-  cudaError_t (*gemv)(const XGemvArgs<E>& g, const GemvMaps& maps, bool rows, int grid, cudaStream_t s);
+  // maps == nullptr: the rows kernel for small matrices (g.groups warps to a row)
+  cudaError_t (*gemv)(const XGemvArgs<E>& g, const GemvMaps* maps, bool rows, int grid, cudaStream_t s);
   // decomposition of an M x N x K product (whole_tiles: no tile is cut between CTAs)
   cudaError_t (*gemm_plan)(long long M, long long N, long long K, int sms, bool whole_tiles,
                            GemmPlan* p);
