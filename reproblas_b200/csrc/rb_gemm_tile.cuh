@@ -264,21 +264,48 @@ struct Tile {
           }
     }
   }
-  __device__ __forceinline__ bool prepare(const E* sa, const E* sb, int kend, bool finite) {
+  __device__ __forceinline__ bool prepare(const E* sa, const E* sb, int kend, bool finite,
+                                          const unsigned* kra, const unsigned* kcb) {
     unsigned mk[NA];
-    if (finite) max_keys<true>(sa, sb, kend, mk);
-    else max_keys<false>(sa, sb, kend, mk);
     bool careful = !finite;
+    bool exact = false;
+    if (finite) {
+      // The index wanted is that of the largest product. Where that of the bound and that of the
+      // largest of the first four products agree, as they nearly always do (an index spans 40
+      // binades, 13 in FP32), it lies between the two and is known.
+      max_keys<true>(sa, sb, 4, mk);
+      exact = true;
+#pragma unroll
+      for (int i = 0; i < TM; i++)
+#pragma unroll
+        for (int j = 0; j < TN; j++) {
+          const int ib = B::index_of_key(B::key(B::mul(key_ceiling<E>(kra[i]), key_ceiling<E>(kcb[j]))));
+#pragma unroll
+          for (int c = 0; c < NC; c++) exact = exact && B::index_of_key(mk[(i * TN + j) * NC + c]) == ib;
+        }
+      if (!exact) max_keys<true>(sa, sb, kend, mk);
+    } else {
+      max_keys<false>(sa, sb, kend, mk);
+    }
     cap = 0xffffffffu;
 #pragma unroll
     for (int e = 0; e < NA; e++) {
-      // through a copy: the call takes an address, and pri must stay in registers
-      E t[F];
+      unsigned c;
+      if (pri[e][0] == E(0)) {
+        // empty: straight to the index (its carries are zero)
+        const int ni = B::index_of_key(mk[e]);
 #pragma unroll
-      for (int i = 0; i < F; i++) t[i] = pri[e][i];
-      const unsigned c = raise_entry(t, car + e * F * kThreads, mk[e]);
+        for (int i = 0; i < F; i++) pri[e][i] = B::bin(ni + i);
+        c = B::cap_of(ni) | (ni == 0 ? 1u : 0u);
+      } else {
+        // through a copy: the call takes an address, and pri must stay in registers
+        E t[F];
 #pragma unroll
-      for (int i = 0; i < F; i++) pri[e][i] = t[i];
+        for (int i = 0; i < F; i++) t[i] = pri[e][i];
+        c = raise_entry(t, car + e * F * kThreads, mk[e]);
+#pragma unroll
+        for (int i = 0; i < F; i++) pri[e][i] = t[i];
+      }
       careful = careful || (c & 1u);
       cap = (c & ~1u) < cap ? (c & ~1u) : cap;
     }
@@ -479,7 +506,7 @@ struct Tile {
           }
       }
       bool careful = false;
-      if (!ok) careful = prepare(ta, tb, kend, all < B::kInfKey);
+      if (!ok) careful = prepare(ta, tb, kend, all < B::kInfKey, kcur + ra, kcur + BM + cb);
       dep += kend * D;
       if (careful) {
         deposit_careful(ta, tb, kend);
@@ -633,20 +660,19 @@ cudaError_t resident_ctas(int sms, int* out) {
   return cudaSuccess;
 }
 
-// Tile shapes per element type and fold: the most accumulators a thread's 128 registers hold
-// beside the operands (up to 64 registers of primaries). Issue cycles per fold-3 product at
-// 1536^3 (real) / 768^3 (complex): FP64 4x2 24.2, 2x2 25.5, 2x1 28.8; FP32 4x4 14.7, 4x2 15.5,
-// 2x2 17.1; FP64 complex 2x2 23.5, 1x2 23.9, 1x1 25.2; FP32 complex 2x2 14.6, 2x4 14.4 (and
-// slower with the longer loop body). Three CTAs per SM (80 registers) spill: FP64 2x2 29.7.
-// The small shape serves sizes that fill the large tile badly; `ratio` is its cost per
-// product against the large one's.
+// Tile shapes per element type and fold: as many accumulators as 128 registers hold beside the
+// operands without spilling. Issue cycles per fold-3 product at 2048^3 (real) / 1024^3
+// (complex): FP64 2x2 24.3, 4x2 24.8 (spills); FP32 2x4 14.8, 4x2 15.2, 4x4 15.3 (spills), 2x2
+// 16.5; FP64 complex 1x2 22.7, 1x1 24.2, 2x2 24.5 (spills); FP32 complex 2x2 13.9, 2x4 14.3. Three
+// CTAs per SM (80 registers) spill: FP64 2x2 29.7. The small shape serves sizes that fill the
+// large tile badly; `ratio` is its cost per product against the large one's.
 template <typename E, bool CX, int F>
 struct Shapes {
   static constexpr bool f32 = sizeof(E) == 4;
-  static constexpr int TM = CX ? (f32 || F <= 3 ? 2 : 1) : f32 ? 4 : (F <= 3 ? 4 : F <= 6 ? 2 : 1);
-  static constexpr int TN = CX ? (f32 || F <= 5 ? 2 : 1) : f32 ? (F <= 4 ? 4 : 2) : 2;
-  static constexpr int SM = TM > 1 ? TM / 2 : 1, SN = TN > 2 ? TN / 2 : (TM > 1 ? TN : 1);
-  static constexpr double ratio = f32 ? 1.16 : 1.05;
+  static constexpr int TM = CX ? (f32 ? 2 : 1) : f32 ? 2 : (F <= 6 ? 2 : 1);
+  static constexpr int TN = CX ? (f32 || F <= 5 ? 2 : 1) : f32 ? 4 : 2;
+  static constexpr int SM = TM > 1 && TN <= 2 ? TM / 2 : TM, SN = TM > 1 && TN <= 2 ? TN : TN > 1 ? TN / 2 : 1;
+  static constexpr double ratio = 1.12;
 };
 
 // Decomposition for one tile shape; returns its cost estimate in K-block units of the large
@@ -664,7 +690,9 @@ cudaError_t plan_shape(long long M, long long N, long long K, int sms, bool whol
   p->nkb = K > 0 ? (K + G::BK - 1) / G::BK : 1;
   p->units = p->tiles * p->nkb;
   // Whole tiles: waves of CTAs. Cut tiles: an even share of the units, plus (in units) one for
-  // the partial states and the tickets and about a quarter per state merged.
+  // the partial states and the tickets -- more where whole tiles would not even take one CTA per
+  // SM, whose units are short -- and about a quarter per state merged.
+  const double over = p->tiles <= sms ? 2.5 : 1.0;
   double best = (double)((p->tiles + slots - 1) / slots) * p->nkb;
   long long grid = p->tiles;
   if (!whole) {
@@ -672,7 +700,7 @@ cudaError_t plan_shape(long long M, long long N, long long K, int sms, bool whol
       if (gr <= 0 || gr > slots || gr >= p->units) return;
       if (p->units % gr == 0 && (p->units / gr) % p->nkb == 0) return;   // whole tiles
       const double share = (double)((p->units + gr - 1) / gr);
-      const double c = share + 1.0 + 0.25 * (p->nkb / share + 1.0);
+      const double c = share + over + 0.25 * (p->nkb / share + 1.0);
       if (c < 0.97 * best) {
         best = c;
         grid = gr;
