@@ -112,7 +112,7 @@ int run_int8(const Int8Req& q) {
   if (!w) return rb_get_last_error();
   cudaStream_t s = w->stream;
   const size_t slice_bytes = (size_t)q.S * (sa.Mp + sa.Np) * Kp;
-  const size_t exp_bytes = ((size_t)q.M + q.N) * 4 + 512;
+  const size_t exp_bytes = ((size_t)q.M + q.N) * 12 + 1024;   // exponents, and words for the maxima
   const size_t cbin_bytes = nchunks > 1 ? (size_t)q.M * q.N * 2 * q.fold * 8 : 0;
   if (!w->ensure_big(slice_bytes + exp_bytes + cbin_bytes + 1024)) return rb_get_last_error();
   unsigned char* p = w->big;
@@ -122,16 +122,16 @@ int run_int8(const Int8Req& q) {
   sa.fb = (int*)p; p += (size_t)q.N * 4;
   p = (unsigned char*)(((uintptr_t)p + 255) / 256 * 256);
   sa.status = (int*)p; p += 256;
+  unsigned long long* top = (unsigned long long*)p; p += ((size_t)q.M + q.N) * 8;
   double* cbin = (double*)p;
   if (!cuda_ok(cudaMemsetAsync(sa.status, 0, 4, s), "cudaMemsetAsync")) return RB_ERR_CUDA;
 
   // exponents over the whole K (every chunk uses the same scales); then check that the
   // operands are finite before C is touched
   count_launch(2);
-  i8::exponent_kernel<true><<<(unsigned)((sa.M * 32 + 255) / 256), 256, 0, s>>>(sa);
-  i8::exponent_kernel<false><<<(unsigned)((sa.N * 32 + 255) / 256), 256, 0, s>>>(sa);
   int* hs = (int*)w->hresult();
-  if (!cuda_ok(cudaGetLastError(), "exponent launch") ||
+  if (!cuda_ok(i8::launch_exponents<true>(sa, top, s), "exponent launch") ||
+      !cuda_ok(i8::launch_exponents<false>(sa, top + q.M, s), "exponent launch") ||
       !cuda_ok(cudaMemcpyAsync(hs, sa.status, 4, cudaMemcpyDeviceToHost, s), "copy status") ||
       !cuda_ok(cudaStreamSynchronize(s), "cudaStreamSynchronize"))
     return RB_ERR_CUDA;
@@ -150,10 +150,9 @@ int run_int8(const Int8Req& q) {
     c.A = q.A + k0 * sa.sak;
     c.B = q.B + k0 * sa.sbk;
     count_launch(2);
-    const long long na = sa.Mp * (Kp / 16), nb = sa.Np * (Kp / 16);
-    i8::slice_kernel<true><<<(unsigned)((na + 255) / 256), 256, 0, s>>>(c);
-    i8::slice_kernel<false><<<(unsigned)((nb + 255) / 256), 256, 0, s>>>(c);
-    if (!cuda_ok(cudaGetLastError(), "slice launch")) return RB_ERR_CUDA;
+    if (!cuda_ok(i8::launch_slice<true>(c, s), "slice launch") ||
+        !cuda_ok(i8::launch_slice<false>(c, s), "slice launch"))
+      return RB_ERR_CUDA;
     if (ch == 0 && q.as_out)
       cudaMemcpyAsync(q.as_out, sa.As, (size_t)q.S * sa.Mp * Kp, cudaMemcpyDeviceToDevice, s);
     if (ch == 0 && q.bs_out)

@@ -173,54 +173,156 @@ __global__ void __launch_bounds__(256) exponent_kernel(SliceArgs g) {
   }
 }
 
-// Slices of op(A): thread per (row, 16-byte K chunk); writes S chunks of 16 digits.
-// Slices of op(B) are written transposed (row j of Bs = column j of op(B)).
+// The same for an operand whose rows (columns) lie side by side in memory (unit stride across
+// them): a CTA takes 64 of them and kMaxK elements of the reduction, reading 512 contiguous
+// bytes at a time, and the CTAs of one row meet in an atomic maximum of the bit pattern
+// (`top`, zero on entry). finish_exponents turns the maxima into exponents. 4096^2: 73 -> 27 us
+// against a warp per column reading with the leading dimension as its stride.
+constexpr int kMaxK = 256;
 template <bool IS_A>
-__global__ void __launch_bounds__(256) slice_kernel(SliceArgs g) {
-  const long long R = IS_A ? g.Mp : g.Np;
-  const long long nchunk = g.Kp / 16;
-  const long long id = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (id >= R * nchunk) return;
-  const long long r = id / nchunk, kc = id % nchunk;
-  const long long Rv = IS_A ? g.M : g.N;
-  int8_t dig[kMaxSlices][16];
-#pragma unroll
-  for (int p = 0; p < kMaxSlices; p++)
-#pragma unroll
-    for (int c = 0; c < 16; c++) dig[p][c] = 0;
-  if (r < Rv) {
-    const int e = (IS_A ? g.ea : g.fb)[r];
-#pragma unroll
-    for (int c = 0; c < 16; c++) {
-      const long long k = kc * 16 + c;
-      if (k < g.K) {
-        double x = IS_A ? a_elem(g, r, k) : b_elem(g, k, r);
-        double v = scalbn(x, -e);   // |v| < 1, exact for normal operands
-#pragma unroll
-        for (int p = 0; p < kMaxSlices; p++) {
-          if (p < g.S) {
-            v = __dmul_rn(v, 128.0);
-            double d = trunc(v);
-            v = __dsub_rn(v, d);
-            dig[p][c] = (int8_t)(int)d;
-          }
-        }
-      }
+__global__ void __launch_bounds__(256) exponent_across_kernel(SliceArgs g, unsigned long long* top) {
+  __shared__ unsigned long long sm[4][64];
+  const long long R = IS_A ? g.M : g.N;
+  const int c = threadIdx.x & 63, kg = threadIdx.x >> 6;
+  const long long r = (long long)blockIdx.x * 64 + c;
+  unsigned long long m = 0;
+#pragma unroll 1
+  for (long long k0 = (long long)blockIdx.y * kMaxK; r < R && k0 < g.K; k0 += (long long)gridDim.y * kMaxK) {
+    const long long k1 = k0 + kMaxK < g.K ? k0 + kMaxK : g.K;
+#pragma unroll 8
+    for (long long k = k0 + kg; k < k1; k += 4) {
+      const double x = IS_A ? a_elem(g, r, k) : b_elem(g, k, r);
+      const unsigned long long b = (unsigned long long)__double_as_longlong(x) & 0x7fffffffffffffffull;
+      m = b > m ? b : m;
     }
   }
-  // Pre-tiled layout [K column kc][slice p][row group r/8][8 rows][16 B]: every 16-byte K
-  // column of an 8-row group (a core matrix of the MMA operand) is 128 contiguous bytes, and
-  // for one K column all slices' row groups follow each other, so one TMA box with a
-  // 128-byte inner dimension moves a whole pipeline stage.
-  int8_t* base = IS_A ? g.As : g.Bs;
-  for (int p = 0; p < g.S; p++) {
-    int4 out;
-    memcpy(&out, dig[p], 16);
-    const long long off = (((long long)kc * g.S + p) * (R / 8) + r / 8) * 128 + (r % 8) * 16;
-    *(int4*)(base + off) = out;
+  sm[kg][c] = m;
+  __syncthreads();
+  if (kg == 0 && r < R) {
+#pragma unroll
+    for (int q = 1; q < 4; q++) m = sm[q][c] > m ? sm[q][c] : m;
+    if (m != 0) atomicMax(top + r, m);
   }
 }
+template <bool IS_A>
+__global__ void __launch_bounds__(256) finish_exponents(SliceArgs g, const unsigned long long* top) {
+  const long long r = (long long)blockIdx.x * 256 + threadIdx.x;
+  if (r >= (IS_A ? g.M : g.N)) return;
+  const unsigned long long m = top[r];
+  if (m >= 0x7ff0000000000000ull) atomicExch(g.status, 1);
+  int e = 0;
+  if (m != 0) frexp(__longlong_as_double((long long)m), &e);
+  (IS_A ? g.ea : g.fb)[r] = e;
+}
 
+// Slices of op(A) (columns of op(B) as rows of Bs): a CTA takes 64 rows x 64 K, reads them along
+// the operand's unit stride (512 contiguous bytes per row either way) into shared memory, and
+// thread (row r, 16-byte K column kc) cuts its 16 elements into the digits of all S slices.
+// Digits: |x| * 2^-e is a fraction below 1, so the 7-bit groups of its fixed-point expansion are
+// the digits of r <- 128 r, d <- trunc(r), r <- r - d, and each takes x's sign. They are read
+// off a 128-bit shift of the mantissa: conversions and roundings of FP64 values run at a small
+// fraction of the integer rate. Pre-tiled layout [K column kc][slice p][row group r/8][8 rows]
+// [16 B]: every 16-byte K column of an 8-row group (a core matrix of the MMA operand) is 128
+// contiguous bytes, and for one K column all slices' row groups follow each other, so one TMA
+// box with a 128-byte inner dimension moves a whole pipeline stage; the 32 lanes of a warp
+// (rows) write 512 contiguous bytes per slice. 4096^2, 8 slices: 215 us per operand with a
+// thread per K column of a row reading and writing on its own (16-byte pieces on distant
+// lines), against 2 x 134 MB = 41 us of memory traffic.
+template <bool IS_A, int S>
+__global__ void __launch_bounds__(256) slice_kernel(SliceArgs g) {
+  __shared__ double sm[64][65];   // [row][k]
+  const long long R = IS_A ? g.Mp : g.Np, Rv = IS_A ? g.M : g.N;
+  const long long r0 = (long long)blockIdx.x * 64, k0 = (long long)blockIdx.y * 64;
+  const bool along_k = (IS_A ? g.sak : g.sbk) == 1;
+  const int lo = threadIdx.x & 63, hi = threadIdx.x >> 6;
+#pragma unroll 4
+  for (int i = hi; i < 64; i += 4) {
+    const int rr = along_k ? i : lo, kk = along_k ? lo : i;
+    const long long r = r0 + rr, k = k0 + kk;
+    double x = 0.0;
+    if (r < Rv && k < g.K) x = IS_A ? a_elem(g, r, k) : b_elem(g, k, r);
+    sm[rr][kk] = x;
+  }
+  __syncthreads();
+  const int rr = lo;
+  const long long r = r0 + rr, kc = k0 / 16 + hi;
+  if (r >= R || kc >= g.Kp / 16) return;
+  const int e = r < Rv ? (IS_A ? g.ea : g.fb)[r] : 0;
+  uint32_t out[S][4];
+#pragma unroll
+  for (int p = 0; p < S; p++)
+#pragma unroll
+    for (int w = 0; w < 4; w++) out[p][w] = 0u;
+#pragma unroll
+  for (int c = 0; c < 16; c++) {
+    const unsigned long long u = (unsigned long long)__double_as_longlong(sm[rr][hi * 16 + c]);
+    const int ef = (int)(u >> 52) & 0x7ff;
+    const unsigned long long mant = (u & 0xfffffffffffffull) | (ef ? 1ull << 52 : 0ull);
+    // |x| * 2^-e = mant * 2^(q - e) with q = max(ef, 1) - 1075; as a 128-bit fraction that is
+    // mant * 2^(128 + q - e), at most 75 to the left (the fraction is below 1)
+    const int sh = 128 + (ef ? ef : 1) - 1075 - e;
+    unsigned long long fh, fl;
+    if (sh >= 64) {
+      fh = mant << (sh - 64);
+      fl = 0;
+    } else if (sh > 0) {
+      fh = mant >> (64 - sh);
+      fl = mant << sh;
+    } else {
+      fh = 0;
+      fl = sh > -64 ? mant >> -sh : 0;
+    }
+    const int neg = (int)(u >> 63);
+#pragma unroll
+    for (int p = 0; p < S; p++) {
+      // digit p: bits 127 - 7p .. 121 - 7p of (fh, fl)
+      constexpr int top = 128;
+      const int s = top - 7 * (p + 1);
+      unsigned d;
+      if (s >= 64) d = (unsigned)(fh >> (s - 64));
+      else if (s + 7 <= 64) d = (unsigned)(fl >> s);
+      else d = (unsigned)((fl >> s) | (fh << (64 - s)));
+      d &= 127u;
+      d = neg ? (0u - d) & 0xffu : d;
+      out[p][c / 4] |= d << (8 * (c % 4));
+    }
+  }
+  int8_t* base = (IS_A ? g.As : g.Bs) + (r / 8) * 128 + (r % 8) * 16;
+#pragma unroll
+  for (int p = 0; p < S; p++)
+    *(uint4*)(base + (kc * S + p) * (R / 8) * 128) = make_uint4(out[p][0], out[p][1], out[p][2], out[p][3]);
+}
+
+template <bool IS_A>
+cudaError_t launch_slice(const SliceArgs& g, cudaStream_t s) {
+  const long long R = IS_A ? g.Mp : g.Np;
+  const dim3 grid((unsigned)((R + 63) / 64), (unsigned)((g.Kp + 63) / 64));
+  switch (g.S) {
+#define RB_SLICE(S_) case S_: slice_kernel<IS_A, S_><<<grid, 256, 0, s>>>(g); break;
+    RB_SLICE(2) RB_SLICE(3) RB_SLICE(4) RB_SLICE(5) RB_SLICE(6) RB_SLICE(7) RB_SLICE(8) RB_SLICE(9)
+    RB_SLICE(10) RB_SLICE(11) RB_SLICE(12)
+#undef RB_SLICE
+    default: return cudaErrorInvalidValue;
+  }
+  return cudaGetLastError();
+}
+
+// Exponents of op(A)'s rows (op(B)'s columns); `top`: one word per row for the side-by-side form.
+template <bool IS_A>
+cudaError_t launch_exponents(const SliceArgs& g, unsigned long long* top, cudaStream_t s) {
+  const long long R = IS_A ? g.M : g.N;
+  if ((IS_A ? g.sak : g.sbk) == 1 || g.K == 0) {
+    exponent_kernel<IS_A><<<(unsigned)((R * 32 + 255) / 256), 256, 0, s>>>(g);
+    return cudaGetLastError();
+  }
+  cudaError_t e = cudaMemsetAsync(top, 0, (size_t)R * 8, s);
+  if (e != cudaSuccess) return e;
+  exponent_across_kernel<IS_A>
+      <<<dim3((unsigned)((R + 63) / 64), (unsigned)(g.K < 4096ll * kMaxK ? (g.K + kMaxK - 1) / kMaxK : 4096)), 256, 0,
+         s>>>(g, top);
+  finish_exponents<IS_A><<<(unsigned)((R + 255) / 256), 256, 0, s>>>(g, top);
+  return cudaGetLastError();
+}
 
 // ---- kernel: tcgen05 GEMM with binned epilogue ----------------------------------------------
 
