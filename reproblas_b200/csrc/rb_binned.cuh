@@ -394,6 +394,26 @@ template <typename T, int F> struct Acc {
   }
 };
 
+// Largest key of |a|, |b| and the running maximum m (a float that holds a key's bits): FP64
+// values contribute their high word, whose bits order magnitudes as a float's do; NaN (and
+// the FP64 magnitudes whose high word is a float NaN) propagate as a key above every bound.
+__device__ __forceinline__ float max_abs3(float m, float a, float b) {
+  float d;
+  asm("max.NaN.abs.f32 %0, %1, %2, %3;" : "=f"(d) : "f"(m), "f"(a), "f"(b));
+  return d;
+}
+__device__ __forceinline__ float key_word(double x) { return __int_as_float(__double2hiint(x)); }
+__device__ __forceinline__ float key_word(float x) { return x; }
+// Upper bound of every magnitude whose key (BT::key) is at most k: FP64 keys are the high word,
+// so the largest double with that high word; FP32 keys are the whole value.
+template <typename E>
+__device__ __forceinline__ E key_ceiling(unsigned k) {
+  if constexpr (sizeof(E) == 8)
+    return __longlong_as_double((long long)(((unsigned long long)k << 32) | 0xffffffffull));
+  else
+    return __uint_as_float(k);
+}
+
 // Deposit K values into each of two accumulators (all K counted as elements; zeros deposit
 // nothing). Same result as a.tile<K>(va, K); b.tile<K>(vb, K), but in the common case (both
 // tiles on their fast path) the two deposit chains sit in one straight-line block, so their

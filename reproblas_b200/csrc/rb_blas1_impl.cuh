@@ -142,10 +142,10 @@ template <typename T, int F, int OP>
 struct Red1 {
   Acc<T, F> a;
   double scl;   // sum of squares: current power-of-two scale (0 = none yet)
-  T inv;        // sum of squares: 1/scl, valid while inv_of == scl
-  double inv_of;
+  T inv;        // sum of squares: 1/scl, while lim is not 0
+  unsigned lim; // sum of squares: keys below need no larger scale (0: scl or inv not set)
 
-  __device__ __forceinline__ void init() { a.zero(); scl = 0.0; inv_of = -1.0; }
+  __device__ __forceinline__ void init() { a.zero(); scl = 0.0; lim = 0u; }
 
   // Deposit K elements (x[k], y[k]) of which the first nv are real.
   template <int K>
@@ -168,43 +168,75 @@ struct Red1 {
     }
   }
 
-  // dmdssq.ccog:70-101 for one tile
+  // dmdssq.ccog:70-101 for one tile. The largest |x| settles everything the tile's checks need:
+  // whether the scale grows (lim) and, squaring being monotone, the largest square.
   template <int K>
   __device__ __forceinline__ void ssq_tile(const T (&x)[K], int nv) {
+    using B = BT<T>;
     if (nv <= 0) return;
+    float mf = 0.0f;   // elements past nv are zeros
+#pragma unroll
+    for (int k = 0; k < K; k += 2) mf = max_abs3(mf, key_word(x[k]), key_word(x[k + 1 < K ? k + 1 : k]));
+    const unsigned m = __float_as_uint(mf);
+    if (m >= lim) {
+      if (m >= B::kInfKey || (sizeof(T) == 8 && m >= 0x7f800000u)) {
+        if (nonfinite<K>(x, nv)) return;
+      }
+      grow<K>(x);
+    }
+    T v[K];
+#pragma unroll
+    for (int k = 0; k < K; k++) {
+      const T t = B::mul(x[k], inv);
+      v[k] = B::mul(t, t);
+    }
+    // x * (1/scale), squared (depositSSq.py:17-26); 1/scale is an exact power of two
+    const T b = B::mul(key_ceiling<T>(m), inv);
+    if (a.fast(B::key(B::mul(b, b)), nv)) {
+      a.deposits += nv;
+#pragma unroll
+      for (int k = 0; k < K; k++) a.deposit(v[k]);
+      return;
+    }
+    a.template tile<K>(v, nv);
+  }
+  // the classes of a tile's non-finite values, if it has any: the reference adds |x| naively,
+  // so NaN stays NaN and any infinity becomes +Inf
+  template <int K>
+  __device__ __forceinline__ bool nonfinite(const T (&x)[K], int nv) {
+    bool any = false;
+#pragma unroll
+    for (int k = 0; k < K; k++)
+      if (k < nv && BT<T>::key(x[k]) >= BT<T>::kInfKey) {
+        a.flags |= (x[k] != x[k]) ? kNaN : kPosInf;
+        any = true;
+      }
+    return any;
+  }
+  // the scale of the tile's largest magnitude, if larger than the current one, and its reciprocal
+  template <int K>
+  __device__ __forceinline__ void grow(const T (&x)[K]) {
+    using B = BT<T>;
     unsigned m = 0;
 #pragma unroll
     for (int k = 0; k < K; k++) {
-      unsigned kk = BT<T>::key(x[k]);
-      m = (k < nv && kk > m) ? kk : m;
-    }
-    if (m >= BT<T>::kInfKey) {
-      // the reference adds |x| naively: NaN stays NaN, any infinity becomes +Inf
-#pragma unroll
-      for (int k = 0; k < K; k++)
-        if (k < nv && BT<T>::key(x[k]) >= BT<T>::kInfKey)
-          a.flags |= (x[k] != x[k]) ? kNaN : kPosInf;
-      return;
+      const unsigned kk = B::key(x[k]);
+      m = kk > m ? kk : m;
     }
     const T nscl = scale_of_key<T>(m);
     if ((double)nscl > scl) {
       if (scl > 0.0) rescale(a, nscl, (T)scl);
       scl = (double)nscl;
     }
-    // x * (1/scale), squared (depositSSq.py:17-26); 1/scale is an exact power of two
-    // FP32: 1/scl kept between tiles (the division dominated the FP32 tile); FP64 recomputes
-    // it, which keeps the FP64 kernel's registers within its 4-CTA budget
-    if (sizeof(T) == 8 || inv_of != scl) {
-      inv = recip_scale((T)scl);
-      inv_of = scl;
-    }
-    T v[K];
-#pragma unroll
-    for (int k = 0; k < K; k++) {
-      const T t = BT<T>::mul(x[k], inv);
-      v[k] = BT<T>::mul(t, t);
-    }
-    a.template tile<K>(v, nv);
+    inv = recip_scale((T)scl);
+    // scale_of_key rises by steps of W binades: from 1 up at W, 2W, ... above it, below 1 just
+    // above each scale
+    constexpr int W = sizeof(T) == 8 ? 40 : 13, ONE = sizeof(T) == 8 ? 1023 : 127;
+    constexpr int SH = sizeof(T) == 8 ? 20 : 23;
+    const int e = (int)((B::bits((T)scl) >> B::kExpShift) & B::kExpMask);
+    const int next = e >= ONE ? e + W : e + 1;
+    lim = next < (int)B::kExpMask ? (unsigned)next << SH : B::kInfKey;
+    if (sizeof(T) == 8 && lim > 0x7f800000u) lim = 0x7f800000u;   // where key words turn NaN
   }
 
   __device__ __forceinline__ void merge(const Red1& o) {
@@ -219,8 +251,26 @@ struct Red1 {
     Red1 o;
     o.a = a.shfl_xor(mask);
     o.scl = __shfl_xor_sync(0xffffffffu, scl, mask);
-    o.inv_of = -1.0;
+    o.lim = 0u;
     return o;
+  }
+
+  // Merge the (renormalised) states of the warp's lanes; every lane ends with the merged one.
+  __device__ __forceinline__ void warp_merge() {
+    if constexpr (OP == kOpSsq) {
+      // one scale in the warp, as nearly always (a lane without a scale holds nothing): the
+      // states add as they are; else pair by pair, rescaling
+      const unsigned h = (unsigned)__double2hiint(scl);
+      const unsigned top = __reduce_max_sync(0xffffffffu, h);
+      lim = 0u;
+      if (!__all_sync(0xffffffffu, h == top || h == 0u)) {
+#pragma unroll 1
+        for (int m = 16; m; m >>= 1) merge(shfl_xor(m));
+        return;
+      }
+      scl = __hiloint2double((int)top, 0);
+    }
+    warp_merge_all(a);
   }
 
   // Scratch / shared-memory record: [pri F][car F][flags][scale]
@@ -236,7 +286,7 @@ struct Red1 {
     for (int i = 0; i < F; i++) { a.pri[i] = ldrec<G>(r + i); a.car[i] = ldrec<G>(r + F + i); }
     a.flags = (unsigned)BT<T>::bits(ldrec<G>(r + 2 * F));
     scl = (double)ldrec<G>(r + 2 * F + 1);
-    inv_of = -1.0;
+    lim = 0u;
     a.set_idx_from_pri();
     a.deposits = 0;
   }
@@ -246,18 +296,27 @@ struct Red1 {
 // Block-level merge: warp butterflies, then the warps through shared memory. On return
 // thread 0 holds the merge of every thread's state.
 // ---------------------------------------------------------------------------------------
-template <typename S, typename T, int REC>
+template <typename S, bool ANY>
+__device__ __forceinline__ void warp_step(S& st) {
+  if constexpr (ANY) {
+#pragma unroll 1
+    for (int m = 16; m; m >>= 1) st.merge(st.shfl_xor(m));
+  } else {
+    st.warp_merge();
+  }
+}
+// ANY: the states come from the caller, so their carries may be of any size (pairwise FP64
+// merges); else they are states of this kernel (integer merges, see warp_merge_all).
+template <typename S, typename T, int REC, bool ANY = false>
 __device__ __forceinline__ void block_merge(S& st, T* smem) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
-#pragma unroll 1
-  for (int m = 16; m; m >>= 1) st.merge(st.shfl_xor(m));
+  warp_step<S, ANY>(st);
   if (lane == 0) st.save(smem + warp * REC);
   __syncthreads();
   if (warp == 0) {
     if (lane < nwarps) st.restore(smem + lane * REC);
     else st.init();
-#pragma unroll 1
-    for (int m = 16; m; m >>= 1) st.merge(st.shfl_xor(m));
+    warp_step<S, ANY>(st);
   }
   __syncthreads();
 }
@@ -425,6 +484,10 @@ struct RedC {
   Acc<T, F> re, im;
   __device__ __forceinline__ void init() { re.zero(); im.zero(); }
   __device__ __forceinline__ void merge(const RedC& o) { re.merge(o.re); im.merge(o.im); }
+  __device__ __forceinline__ void warp_merge() {
+    warp_merge_all(re);
+    warp_merge_all(im);
+  }
   __device__ __forceinline__ RedC shfl_xor(int m) const {
     RedC o;
     o.re = re.shfl_xor(m);
@@ -658,7 +721,7 @@ __global__ void __launch_bounds__(256) merge_states_kernel(int count, const doub
     o.a.renorm();
     st.merge(o);
   }
-  block_merge<Red1<double, F, kOpSum>, double, REC>(st, smem);
+  block_merge<Red1<double, F, kOpSum>, double, REC, true>(st, smem);
   if (threadIdx.x == 0) {
     Red1<double, F, kOpSum> o;
     o.init();

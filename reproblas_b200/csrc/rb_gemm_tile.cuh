@@ -36,16 +36,6 @@ namespace gt {
 
 using xb::Val;
 
-// Upper bound of every magnitude whose key (BT<E>::key) is at most k: FP64 keys are the high
-// word, so the largest double with that high word; FP32 keys are the whole value.
-template <typename E>
-__device__ __forceinline__ E key_ceiling(unsigned k) {
-  if constexpr (sizeof(E) == 8)
-    return __longlong_as_double((long long)(((unsigned long long)k << 32) | 0xffffffffull));
-  else
-    return __uint_as_float(k);
-}
-
 // N adjacent reals of shared memory, as the widest vectors their total size allows.
 template <typename E, int N>
 __device__ __forceinline__ void lds_vec(const E* p, E (&v)[N]) {

@@ -239,17 +239,6 @@ __device__ __forceinline__ bool stage_ready(Sync& sy, const Ring& r, long long p
   return true;
 }
 
-// Largest key of |a|, |b| and the running maximum m (a float that holds a key's bits): FP64
-// values contribute their high word, whose bits order magnitudes as a float's do; NaN (and
-// the FP64 magnitudes whose high word is a float NaN) propagate as a key above every bound.
-__device__ __forceinline__ float max_abs3(float m, float a, float b) {
-  float d;
-  asm("max.NaN.abs.f32 %0, %1, %2, %3;" : "=f"(d) : "f"(m), "f"(a), "f"(b));
-  return d;
-}
-__device__ __forceinline__ float key_word(double x) { return __int_as_float(__double2hiint(x)); }
-__device__ __forceinline__ float key_word(float x) { return x; }
-
 // The PE elements of this thread in one stage, and their deposit into its accumulators.
 template <typename E, bool CX, int F, bool ROWS>
 struct Consumer {
@@ -364,7 +353,7 @@ struct Consumer {
 #pragma unroll
       for (int i = 0; i < NR; i += 2) m = max_abs3(m, key_word(v[i]), key_word(v[i + 1]));
       const unsigned bound =
-          B::key(B::mul(gt::key_ceiling<E>(__float_as_uint(m)), gt::key_ceiling<E>(xkey)));
+          B::key(B::mul(key_ceiling<E>(__float_as_uint(m)), key_ceiling<E>(xkey)));
       bool fast = true;
 #pragma unroll
       for (int c = 0; c < NC; c++) fast = fast && a[c].fast(bound, ND);
@@ -431,7 +420,7 @@ struct Consumer {
     float m = 0.0f;
 #pragma unroll
     for (int i = 0; i < NR; i += 2) m = max_abs3(m, key_word(v[i]), key_word(v[i + 1]));
-    const unsigned bound = B::key(B::mul(gt::key_ceiling<E>(__float_as_uint(m)), gt::key_ceiling<E>(xkey)));
+    const unsigned bound = B::key(B::mul(key_ceiling<E>(__float_as_uint(m)), key_ceiling<E>(xkey)));
     bool fast = true;
 #pragma unroll
     for (int c = 0; c < NC; c++) fast = fast && a[c].fast(bound, ND);
