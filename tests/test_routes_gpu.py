@@ -1,0 +1,266 @@
+"""The routes a gemv / gemm / sum-of-squares call takes by its sizes, alignment and type, each at
+the sizes where it can go wrong, bit for bit against the oracle: gemm tiles cut between CTAs (and
+the whole-tile fallback when their scratch cannot be had), K blocks that leave the unchecked
+path (non-finite products, the top bin, zero rows, raises in a late block), gemv rows that
+start at every 4-byte alignment, matrices with fewer rows than alignment phases, both sides
+of the direct kernels' size limits, scales that grow inside and between warps, and the int8
+digits of magnitudes far below their row's largest."""
+import numpy as np
+import pytest
+
+from _cmp import same_bits, same_state, same_value
+from _data import gen, gen_complex
+from _ffi import binned_zeros, ptr
+from _xblas import lib_gemm, lib_gemv, rb_gemm, rb_gemv
+
+pytestmark = pytest.mark.gpu
+
+REAL = {"d": np.float64, "s": np.float32, "z": np.float64, "c": np.float32}
+FULL = {"d": np.float64, "s": np.float32, "z": np.complex128, "c": np.complex64}
+
+
+def ops(t, n, seed, dist="uniform"):
+    return gen(dist, n, seed, REAL[t]) if t in "ds" else gen_complex(dist, n, seed, FULL[t])
+
+
+def dev(cuda, a):
+    return cuda.from_numpy(np.ascontiguousarray(a).view(a.real.dtype)).cuda()
+
+
+def scalars(t):
+    return (1.5, 0.5) if t in "ds" else (1.5 - 0.25j, 0.5 + 0.125j)
+
+
+def oracle_gemm(port, t, fold, ta, tb, M, N, K, A, lda, B, ldb, C, ldc):
+    al, be = scalars(t)
+    if t == "d":
+        port.rdgemm(fold, b"r", ta.encode(), tb.encode(), M, N, K, al, ptr(A), lda, ptr(B), ldb, be,
+                    ptr(C), ldc)
+    else:
+        lib_gemm(port, t, fold, "r", ta, tb, M, N, K, al, A, lda, B, ldb, be, C, ldc)
+
+
+def gpu_gemm(rb, t, fold, ta, tb, M, N, K, A, lda, B, ldb, C, ldc):
+    al, be = scalars(t)
+    if t == "d":
+        rb.call("reproBLAS_rdgemm", fold, "r", ta, tb, M, N, K, al, A, lda, B, ldb, be, C, ldc)
+    else:
+        rb_gemm(rb, t, fold, "r", ta, tb, M, N, K, al, A, lda, B, ldb, be, C, ldc)
+
+
+def check_gemm(cuda, rb, port, t, fold, ta, tb, M, N, K, A, B, seed):
+    C = ops(t, M * N, seed + 2)
+    want = C.copy()
+    lda, ldb = (K if ta == "n" else M), (N if tb == "n" else K)
+    oracle_gemm(port, t, fold, ta, tb, M, N, K, A, lda, B, ldb, want, N)
+    Cd = dev(cuda, C)
+    gpu_gemm(rb, t, fold, ta, tb, M, N, K, dev(cuda, A), lda, dev(cuda, B), ldb, Cd, N)
+    got = Cd.cpu().numpy().view(FULL[t])
+    assert same_value(got.view(REAL[t]), want.view(REAL[t])), (t, fold, ta, tb, M, N, K)
+
+
+@pytest.mark.parametrize("t", list("dszc"))
+@pytest.mark.parametrize("fold", [2, 3, 5, 8])
+def test_gemm_cut_tiles(cuda, rb, port, t, fold):
+    # few tiles and a long sum: every tile is cut into many parts; then K one beyond, at and
+    # before the end of a K block, and sizes one off the tiles
+    for i, (M, N, K, ta, tb) in enumerate([(33, 17, 4001, "t", "n"), (1, 1, 3000, "n", "t"), (16, 31, 2047, "n", "n"),
+                                           (65, 33, 32, "t", "t"), (32, 64, 33, "n", "n"), (31, 63, 31, "n", "t")]):
+        check_gemm(cuda, rb, port, t, fold, ta, tb, M, N, K, ops(t, M * K, i), ops(t, K * N, i + 50), i)
+
+
+@pytest.mark.parametrize("t", list("dszc"))
+def test_gemm_without_scratch(cuda, rb, port, t):
+    M, N, K = 33, 17, 4001
+    A, B, C = ops(t, M * K, 1), ops(t, K * N, 2), ops(t, M * N, 3)
+    want = C.copy()
+    oracle_gemm(port, t, 3, "n", "n", M, N, K, A, K, B, N, want, N)
+    stream = cuda.cuda.Stream()
+    rb.lib.rb_set_stream(stream.cuda_stream)
+    try:
+        x = cuda.ones(16, dtype=cuda.float64, device="cuda")
+        cuda.cuda.synchronize()
+        rb.call("reproBLAS_rdsum", 3, 16, x, 1)       # makes the stream's workspace
+        rb.lib.rb_debug_fail_allocations(8)           # neither scratch nor tickets can be had
+        Ad, Bd, Cd = dev(cuda, A), dev(cuda, B), dev(cuda, C)
+        cuda.cuda.synchronize()
+        gpu_gemm(rb, t, 3, "n", "n", M, N, K, Ad, K, Bd, N, Cd, N)
+        stream.synchronize()
+        assert same_bits(Cd.cpu().numpy(), want.view(REAL[t]))
+    finally:
+        rb.lib.rb_debug_fail_allocations(0)
+        rb.lib.rb_set_stream(None)
+
+
+@pytest.mark.parametrize("t", list("dszc"))
+def test_gemm_captured(cuda, rb, port, t):
+    # a graph must not hold scratch that a later, larger call replaces: capture, grow, replay
+    M, N, K = 33, 17, 2000
+    A, B, C = ops(t, M * K, 4), ops(t, K * N, 5), ops(t, M * N, 6)
+    want = C.copy()
+    oracle_gemm(port, t, 3, "n", "n", M, N, K, A, K, B, N, want, N)
+    Ad, Bd, Cd = dev(cuda, A), dev(cuda, B), dev(cuda, C)
+    big = 400
+    Ab, Bb, Cb = dev(cuda, ops(t, big * 5000, 7)), dev(cuda, ops(t, 5000 * big, 8)), dev(cuda, ops(t, big * big, 9))
+    graph, stream = cuda.cuda.CUDAGraph(), cuda.cuda.Stream()
+    rb.lib.rb_set_stream(stream.cuda_stream)
+    try:
+        stream.wait_stream(cuda.cuda.current_stream())
+        keep = Cd.clone()
+        gpu_gemm(rb, t, 3, "n", "n", M, N, K, Ad, K, Bd, N, keep, N)
+        stream.synchronize()
+        with cuda.cuda.graph(graph, stream=stream):
+            gpu_gemm(rb, t, 3, "n", "n", M, N, K, Ad, K, Bd, N, Cd, N)
+        gpu_gemm(rb, t, 3, "n", "n", big, big, 5000, Ab, 5000, Bb, big, Cb, big)
+        stream.synchronize()
+        graph.replay()
+        cuda.cuda.synchronize()
+        assert same_bits(Cd.cpu().numpy(), want.view(REAL[t]))
+    finally:
+        rb.lib.rb_set_stream(None)
+
+
+@pytest.mark.parametrize("t", list("dszc"))
+@pytest.mark.parametrize("fold", [2, 3, 4])
+def test_gemm_blocks_off_the_unchecked_path(cuda, rb, port, t, fold):
+    M, N, K = 40, 35, 100
+    A, B = ops(t, M * K, 11).reshape(M, K), ops(t, K * N, 12).reshape(K, N)
+    hi, lo = (2.0 ** 500, 2.0 ** -500) if t in "dz" else (2.0 ** 60, 2.0 ** -60)
+    A[0] = 0                        # a zero row
+    A[1] *= lo                      # the finest bins (products down to the subnormals)
+    B[:, 2] *= lo
+    A[2, 70] *= hi                  # a raise in the third K block
+    A[3] *= hi                      # products near the top: the compressed first bin
+    B[:, 3] *= hi
+    check_gemm(cuda, rb, port, t, fold, "n", "n", M, N, K, A.ravel(), B.ravel(), 13)
+    A[4, 5], A[5, 90], A[6, 0] = np.inf, -np.inf, np.nan
+    A[7, 1], A[7, 2] = np.inf, -np.inf
+    C = ops(t, M * N, 15)
+    want = C.copy()
+    oracle_gemm(port, t, fold, "n", "n", M, N, K, A.ravel(), K, B.ravel(), N, want, N)
+    Cd = dev(cuda, C)
+    gpu_gemm(rb, t, fold, "n", "n", M, N, K, dev(cuda, A.ravel()), K, dev(cuda, B.ravel()), N, Cd, N)
+    assert same_value(Cd.cpu().numpy(), want.view(REAL[t]))
+
+
+def gemv_both(cuda, rb, port, t, fold, ta, M, N, lda, off, incx, seed, dist="normal"):
+    """A starting `off` reals into its buffer, against the oracle"""
+    al, be = scalars(t)
+    per = 1 if t in "ds" else 2
+    buf = gen(dist, off + M * lda * per, seed, REAL[t])
+    A = np.ascontiguousarray(buf[off:]).view(FULL[t])
+    nx, ny = (N, M) if ta == "n" else (M, N)
+    x, y = ops(t, nx * incx, seed + 1, dist), ops(t, ny, seed + 2, dist)
+    want = y.copy()
+    Ad = cuda.from_numpy(buf).cuda()[off:]
+    yd = dev(cuda, y)
+    if t == "d":
+        port.rdgemv(fold, b"r", ta.encode(), M, N, al, ptr(A), lda, ptr(x), incx, be, ptr(want), 1)
+        rb.call("reproBLAS_rdgemv", fold, "r", ta, M, N, al, Ad, lda, dev(cuda, x), incx, be, yd, 1)
+    else:
+        lib_gemv(port, t, fold, "r", ta, M, N, al, A, lda, x, incx, be, want, 1)
+        rb_gemv(rb, t, fold, "r", ta, M, N, al, Ad, lda, dev(cuda, x), incx, be, yd, 1)
+    assert rb.lib.rb_synchronize() == 0
+    assert same_bits(yd.cpu().numpy(), want.view(REAL[t])), (t, fold, ta, M, N, lda, off, incx)
+
+
+@pytest.mark.parametrize("t", list("dszc"))
+@pytest.mark.parametrize("ta", ["n", "t"])
+def test_gemv_alignments(cuda, rb, port, t, ta):
+    # above the direct kernels' limits, so that the streaming kernel takes the rows in 1, 2 and 4
+    # phases: every distance of A from a 16-byte boundary, leading dimensions of all residues
+    M, N = (8200, 130) if ta == "n" else (3000, 1500)
+    for off in range(4):
+        for pad in range(4):
+            gemv_both(cuda, rb, port, t, 3, ta, M, N, N + pad, off, 1 + (off & 1), 31 * off + pad)
+
+
+@pytest.mark.parametrize("t", list("dszc"))
+@pytest.mark.parametrize("fold", [2, 4, 6, 8])
+def test_gemv_stream_folds(cuda, rb, port, t, fold):
+    for ta, M, N, pad in [("n", 8193, 257, 1), ("t", 255, 9000, 1), ("t", 2049, 2050, 0), ("n", 8200, 64, 0)]:
+        gemv_both(cuda, rb, port, t, fold, ta, M, N, N + pad, 0, 1, fold)
+
+
+@pytest.mark.parametrize("t", list("dszc"))
+@pytest.mark.parametrize("ta", ["n", "t"])
+def test_gemv_few_rows_and_limits(cuda, rb, port, t, ta):
+    es = {"d": 8, "s": 4, "z": 16, "c": 8}[t]
+    rows = 300
+    limit = (24 if ta == "n" else 16) << 20
+    n = limit // (rows * es)
+    shapes = [(1, 70001), (2, 9001), (3, 4097), (rows, n), (rows, n + 1), (255, 300), (256, 300), (8192, 5), (8193, 5)]
+    for i, (M, N) in enumerate(shapes):
+        gemv_both(cuda, rb, port, t, 3, ta, M, N, N + (i & 1), 0, 1, i)
+    # infinities, NaN and the top bin through the streaming kernel
+    M, N = (8200, 64) if ta == "n" else (200, 8200)
+    al, be = scalars(t)
+    A = ops(t, M * N, 5).reshape(M, N)
+    A[5, 3], A[6, 4], A[7, 5] = np.inf, np.nan, -np.inf
+    A[9] *= 2.0 ** (1000 if t in "dz" else 120)
+    x, y = ops(t, N if ta == "n" else M, 6), ops(t, M if ta == "n" else N, 7)
+    want = y.copy()
+    yd = dev(cuda, y)
+    if t == "d":
+        port.rdgemv(3, b"r", ta.encode(), M, N, al, ptr(A), N, ptr(x), 1, be, ptr(want), 1)
+        rb.call("reproBLAS_rdgemv", 3, "r", ta, M, N, al, dev(cuda, A.ravel()), N, dev(cuda, x), 1, be, yd, 1)
+    else:
+        lib_gemv(port, t, 3, "r", ta, M, N, al, A, N, x, 1, be, want, 1)
+        rb_gemv(rb, t, 3, "r", ta, M, N, al, dev(cuda, A.ravel()), N, dev(cuda, x), 1, be, yd, 1)
+    assert same_value(yd.cpu().numpy(), want.view(REAL[t]))
+
+
+@pytest.mark.parametrize("fold", [2, 3, 4])
+def test_sums_of_squares_scales(cuda, rb, port, fold):
+    # the scale grows element by element, lane by lane and warp by warp, across the steps of the
+    # scale (40 binades, 13 in FP32) and around 1; non-finite values at a tile's ends
+    for dt, names, lo, hi in [(np.float64, ("dbdssq", "rdnrm2"), -120, 120), (np.float32, ("sbsssq", "rsnrm2"), -50, 50)]:
+        for n in (1, 15, 512, 4099, 70001):
+            e = np.linspace(lo, hi, n)
+            for k, ex in enumerate((e, e[::-1], np.round(e / 13) * 13, np.where(np.arange(n) % 64 < 32, lo, hi))):
+                x = np.exp2(np.asarray(ex, dtype=np.float64)).astype(dt)
+                x[1::2] *= dt(-1.25)
+                X = cuda.from_numpy(x).cuda()
+                want = binned_zeros(fold, "d" if dt is np.float64 else "s")
+                ws = getattr(port, names[0])(fold, n, ptr(x), 1, 0.0, ptr(want))
+                Z = cuda.zeros(2 * fold, dtype=X.dtype, device="cuda")
+                gs = rb.call("binnedBLAS_" + names[0], fold, n, X, 1, 0.0, Z)
+                assert gs == ws, (dt, n, k)
+                assert same_state(Z.cpu().numpy(), want, fold, 1), (dt, n, k)
+                assert rb.call("reproBLAS_" + names[1], fold, n, X, 1) == getattr(port, names[1])(fold, n, ptr(x), 1)
+            for bad in (np.inf, -np.inf, np.nan):
+                y = x.copy()
+                y[-1] = bad
+                a = rb.call("reproBLAS_" + names[1], fold, n, cuda.from_numpy(y).cuda(), 1)
+                b = getattr(port, names[1])(fold, n, ptr(y), 1)
+                assert a == b or (a != a and b != b)
+
+
+@pytest.mark.parametrize("S", [2, 5, 8, 12])
+def test_int8_digits_of_small_magnitudes(cuda, rb, S):
+    # elements up to 2^200 below their row's largest (their digits lie behind the last slice),
+    # subnormals, zero rows and columns: the digits of r <- 128 r, d <- trunc(r), r <- r - d
+    rng = np.random.default_rng(S)
+    M, N, K = 70, 65, 90
+    A = np.ldexp(rng.uniform(1, 2, (M, K)), rng.integers(-200, 1, (M, K))) * rng.choice([-1.0, 1.0], (M, K))
+    B = np.ldexp(rng.uniform(1, 2, (K, N)), rng.integers(-90, 1, (K, N))) * rng.choice([-1.0, 1.0], (K, N))
+    A[3] = 0
+    B[:, 4] = 0
+    A[5] = 5e-324 * rng.integers(-9, 10, K)
+    Mp, Np, Kp = -(-M // 128) * 128, -(-N // (64 if S <= 4 else 32)) * (64 if S <= 4 else 32), -(-K // 32) * 32
+    z = lambda n, t: cuda.zeros(n, dtype=t, device="cuda")
+    raw, As, Bs = z(S * Mp * Np, cuda.int32), z(S * Mp * Kp, cuda.int8), z(S * Np * Kp, cuda.int8)
+    ea, fb = z(M, cuda.int32), z(N, cuda.int32)
+    assert rb.call("rb_dgemm_int8_inspect", M, N, K, cuda.from_numpy(A).cuda(), cuda.from_numpy(B).cuda(), S, raw,
+                   As, Bs, ea, fb) == 0
+    for X, dig, ex, R, Rp in [(A, As, ea, M, Mp), (B.T, Bs, fb, N, Np)]:
+        e = np.frexp(np.abs(X).max(axis=1))[1]
+        assert np.array_equal(ex.cpu().numpy(), e)
+        d = dig.cpu().numpy().reshape(Kp // 16, S, Rp // 8, 8, 16).transpose(1, 2, 3, 0, 4).reshape(S, Rp, Kp)
+        r = np.ldexp(X, -e[:, None])
+        for p in range(S):
+            r = r * 128
+            t = np.trunc(r)
+            r = r - t
+            assert np.array_equal(d[p, :R, :K], t.astype(np.int8)), p
+        assert not d[:, R:].any() and not d[:, :, K:].any()
