@@ -126,8 +126,9 @@ struct GemvShape {
   int G, grid, q, rem, parts;
   long long nunits, nb, kslots;
 };
+// `uncut`: no unit is cut between CTAs (no scratch).
 GemvShape gemv_shape(bool rows, long long nout, long long nred, int es, bool cx, int fold, int phases,
-                     int sms) {
+                     int sms, bool uncut) {
   // Cost in us, from a sweep over G and the grid on the shapes of 128 MiB and below. A stage takes
   // its CTA 1.45 us (64 KB at the SM's share of HBM) or the deposits' issue time: measured 3.1 at
   // fold 3 for complex elements. Behind the last stage: 5 us when no unit is cut, 8 when
@@ -151,7 +152,7 @@ GemvShape gemv_shape(bool rows, long long nout, long long nred, int es, bool cx,
     s.nunits = (nout + P - 1) / P;
     s.nb = nred > 0 ? (nred + SC - 1) / SC : 1;
     const long long T = s.nunits * s.nb;
-    for (int way = 0; way < 2; way++) {
+    for (int way = uncut ? 1 : 0; way < 2; way++) {
       double ends;
       long long per;   // stages of the busiest CTA
       if (way == 0) {
@@ -163,7 +164,7 @@ GemvShape gemv_shape(bool rows, long long nout, long long nred, int es, bool cx,
         // a unit meets at most ceil((nb-1) / q) + 1 ranges
         s.kslots = s.nb / s.q + 2;
         ends = s.grid == s.nunits && s.rem == 0 ? 5 : 10 + 0.4 * (double)(s.kslots / G);
-      } else if (s.nunits <= sms) {
+      } else if (s.nunits <= sms && !uncut) {
         long long p = sms / s.nunits;
         if (p > s.nb) p = s.nb;
         s.parts = (int)p;
@@ -196,7 +197,8 @@ GemvShape gemv_shape(bool rows, long long nout, long long nred, int es, bool cx,
 // Shape of the direct columns kernel: G row groups per CTA and `parts` row chunks. Cost model in
 // units of one row per thread: the streaming part (waves of CTAs, two per SM, times rows per
 // thread, plus the groups' merge) and the sum of the chunks' partial states.
-GemvShape gemv_direct_shape(long long nout, long long nred, int sms) {
+// `uncut`: one chunk (no scratch).
+GemvShape gemv_direct_shape(long long nout, long long nred, int sms, bool uncut) {
   GemvShape best{};
   long long best_cost = -1;
   const long long slots = (long long)sms * 2;
@@ -206,7 +208,7 @@ GemvShape gemv_direct_shape(long long nout, long long nred, int sms) {
     for (long long ch : {slots / cb, (slots + cb - 1) / cb}) {
       if (ch > most) ch = most;
       if (ch > 1024) ch = 1024;
-      if (ch < 1) ch = 1;
+      if (ch < 1 || uncut) ch = 1;
       const long long rpt = ((nred + ch - 1) / ch + G - 1) / G;
       const long long waves = (cb * ch + slots - 1) / slots;
       const long long cost = waves * (rpt + 8 * lg) + 4 * ((ch + G - 1) / G + 2 * lg);
@@ -295,10 +297,11 @@ bool run_xgemv(const XGemvReq<E, CX>& q) {
   const bool direct = !nt && (gs::direct_cols<E, CX>() ||
                               (nred_eff >= 256 && nout * nred_eff * (long long)es <= (16ll << 20)));
   GemvShape sh{};
-  if (direct) sh = gemv_direct_shape(nout, nred_eff, di.sms);
-  else if (!small) sh = gemv_shape(nt, nout, nred_eff, (int)es, CX, q.fold, phases, di.sms);
-  const size_t part_bytes = (size_t)nout * sh.kslots * NC * (2 * q.fold + 1) * sizeof(E);
-  if (!small && !w->ensure_tickets((size_t)sh.nunits * 16)) return false;   // per unit and consumer warp
+  const bool uncut = stream_capturing(s);
+  if (direct) sh = gemv_direct_shape(nout, nred_eff, di.sms, uncut);
+  else if (!small) sh = gemv_shape(nt, nout, nred_eff, (int)es, CX, q.fold, phases, di.sms, uncut);
+  const size_t part_bytes = uncut ? 0 : (size_t)nout * sh.kslots * NC * (2 * q.fold + 1) * sizeof(E);
+  if (!small && !uncut && !w->ensure_tickets((size_t)sh.nunits * 16)) return false;   // per unit and consumer warp
   const bool a_host = a_bytes && !a_dev, x_host = x_bytes && !on_device(q.X);
   const bool y_host = !on_device(q.Y);
   const size_t need = part_bytes + (a_host ? a_bytes : 0) + (x_host ? x_bytes : 0) +

@@ -96,6 +96,10 @@ struct Workspace {
 // set); with create = false, nullptr when no call has made one yet.
 Workspace* acquire_workspace(std::unique_lock<std::mutex>* lock, bool create = true);
 
+// Whether stream s is being captured into a graph (or cannot tell): kernels then take forms without
+// scratch where they have one, since a later call may replace the scratch a graph would hold.
+bool stream_capturing(cudaStream_t s);
+
 // Decomposition of an M x N x K gemm on workspace w's stream through a fold's planner: cut tiles
 // when that pays and the scratch for their partial states can be had, else whole tiles (no
 // scratch). A captured launch keeps to whole tiles, so that a graph never holds the address

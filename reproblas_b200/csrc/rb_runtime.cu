@@ -173,6 +173,13 @@ bool Workspace::ensure_tickets(size_t n) {
   return true;
 }
 
+bool stream_capturing(cudaStream_t s) {
+  cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing(s, &st) == cudaSuccess) return st != cudaStreamCaptureStatusNone;
+  cudaGetLastError();
+  return true;
+}
+
 bool Workspace::reset_after_abort() {
   return cuda_ok(cudaMemsetAsync(dstatus(), 0, 4, stream), "cudaMemsetAsync") &&
          (!tickets || cuda_ok(cudaMemsetAsync(tickets, 0, ntickets * sizeof(unsigned), stream), "cudaMemsetAsync")) &&
@@ -185,9 +192,7 @@ bool gemm_decompose(cudaError_t (*plan)(long long, long long, long long, int, bo
   if (!device_info(&di)) return false;
   if (!cuda_ok(plan(M, N, K, di.sms, false, p), "gemm kernel attributes")) return false;
   if (!p->cut) return true;
-  cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
-  bool have = cudaStreamIsCapturing(w->stream, &st) == cudaSuccess && st == cudaStreamCaptureStatusNone;
-  if (!have) cudaGetLastError();
+  bool have = !stream_capturing(w->stream);
   if (have && p->scratch_bytes > w->parts_bytes) {
     // drain the stream first: kernels in flight may still use the old buffer
     if (!cuda_ok(cudaStreamSynchronize(w->stream), "cudaStreamSynchronize")) return false;

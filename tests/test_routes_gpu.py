@@ -121,6 +121,44 @@ def test_gemm_captured(cuda, rb, port, t):
 
 
 @pytest.mark.parametrize("t", list("dszc"))
+@pytest.mark.parametrize("ta", ["n", "t"])
+def test_gemv_captured(cuda, rb, port, t, ta):
+    # the same for gemv, through the streaming and the direct kernels
+    M, N, al, be = 3000, 1500, *scalars(t)
+    A, x, y = ops(t, M * N, 4), ops(t, max(M, N), 5), ops(t, max(M, N), 6)
+    want = y.copy()
+    if t == "d":
+        port.rdgemv(3, b"r", ta.encode(), M, N, al, ptr(A), N, ptr(x), 1, be, ptr(want), 1)
+    else:
+        lib_gemv(port, t, 3, "r", ta, M, N, al, A, N, x, 1, be, want, 1)
+    Ad, xd, yd, keep = dev(cuda, A), dev(cuda, x), dev(cuda, y), dev(cuda, y)
+    rows = 9000
+    Ab, xb, yb = dev(cuda, ops(t, rows * N, 7)), dev(cuda, ops(t, rows, 8)), dev(cuda, ops(t, rows, 9))
+
+    def call(m, a, v, out):
+        if t == "d":
+            rb.call("reproBLAS_rdgemv", 3, "r", ta, m, N, al, a, N, v, 1, be, out, 1)
+        else:
+            rb_gemv(rb, t, 3, "r", ta, m, N, al, a, N, v, 1, be, out, 1)
+
+    graph, stream = cuda.cuda.CUDAGraph(), cuda.cuda.Stream()
+    rb.lib.rb_set_stream(stream.cuda_stream)
+    try:
+        stream.wait_stream(cuda.cuda.current_stream())
+        call(M, Ad, xd, keep)
+        stream.synchronize()
+        with cuda.cuda.graph(graph, stream=stream):
+            call(M, Ad, xd, yd)
+        call(rows, Ab, xb, yb)
+        stream.synchronize()
+        graph.replay()
+        cuda.cuda.synchronize()
+        assert same_bits(yd.cpu().numpy(), want.view(REAL[t]))
+    finally:
+        rb.lib.rb_set_stream(None)
+
+
+@pytest.mark.parametrize("t", list("dszc"))
 @pytest.mark.parametrize("fold", [2, 3, 4])
 def test_gemm_blocks_off_the_unchecked_path(cuda, rb, port, t, fold):
     M, N, K = 40, 35, 100
