@@ -294,8 +294,7 @@ bool run_xgemv(const XGemvReq<E, CX>& q) {
   if (phases == 1 && a_mis != 0) phases = 2;
   const bool small = nt && gemv_small(nout, nred_eff, (int)es);
   // (bounds: see gemv_cols_direct_kernel)
-  const bool direct = !nt && (gs::direct_cols<E, CX>() ||
-                              (nred_eff >= 256 && nout * nred_eff * (long long)es <= (16ll << 20)));
+  const bool direct = !nt && gs::direct_cols<E, CX>(nred_eff, nout * nred_eff * (long long)es, q.fold);
   GemvShape sh{};
   const bool uncut = stream_capturing(s);
   if (direct) sh = gemv_direct_shape(nout, nred_eff, di.sms, uncut);

@@ -40,8 +40,19 @@ namespace gs {
 using xb::Val;
 
 constexpr int kConsumers = 512;                 // 16 consumer warps
-constexpr int kThreads = kConsumers + 64;       // + the copy warp and the x warp
 constexpr int kStages = 3;
+// FP64 complex consumers need 97-104 registers (without them fold 3 spilled: 297 us at 8192^2,
+// 266 with, rows kernel); 18 warps leave each thread 96. Their CTA therefore
+// has a whole warpgroup of producers (two warps of it idle), launches at 96 registers a thread
+// and moves 32 from each producer to the four consumer warpgroups: 512 * 104 + 128 * 64 =
+// 640 * 96, all that the launch owns (launch_gemv checks that it was built so).
+template <typename E, bool CX>
+__host__ __device__ constexpr bool moves_regs() { return CX && sizeof(E) == 8; }
+template <typename E, bool CX>
+__host__ __device__ constexpr int threads() { return kConsumers + (moves_regs<E, CX>() ? 128 : 64); }
+constexpr int kMoveLaunch = 96, kMoveConsumer = 104, kMoveProducer = 64;
+static_assert(kConsumers * kMoveConsumer + 128 * kMoveProducer <= (kConsumers + 128) * kMoveLaunch,
+              "registers moved must be registers launched with");
 constexpr uint32_t kThreadBytes = 128;          // of A per consumer thread and stage
 
 // The 512 consumer threads own P = 512/G outputs (G = g.groups in {2, 4, 8}, chosen by the
@@ -572,7 +583,7 @@ struct Ends {
 };
 
 template <typename E, bool CX, int F, bool ROWS>
-__global__ void __launch_bounds__(kThreads, 1)
+__global__ void __launch_bounds__((threads<E, CX>()), 1)
 gemv_stream_kernel(const __grid_constant__ XGemvArgs<E> g, const __grid_constant__ GemvMaps maps) {
   using Gm = Geom<E, CX, ROWS>;
   constexpr int NC = Gm::NC, PE = Gm::PE, ES = Gm::ES;
@@ -596,11 +607,13 @@ gemv_stream_kernel(const __grid_constant__ XGemvArgs<E> g, const __grid_constant
   }
   __syncthreads();
 
-  if (tid >= kConsumers + 32) {
-    scale_stages<E, CX, ROWS>(g, m, sp, ring, sy);
-  } else if (tid >= kConsumers) {
-    if (lane == 0) copy_stages<E, CX, ROWS>(g, m, maps, sp, ring, sy);
+  if (tid >= kConsumers) {
+    if constexpr (moves_regs<E, CX>()) asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kMoveProducer));
+    const int w = tid >> 5;
+    if (w == kConsumers / 32 + 1) scale_stages<E, CX, ROWS>(g, m, sp, ring, sy);
+    else if (w == kConsumers / 32 && lane == 0) copy_stages<E, CX, ROWS>(g, m, maps, sp, ring, sy);
   } else {
+    if constexpr (moves_regs<E, CX>()) asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(kMoveConsumer));
     const long long polls = g.wait_polls > 0 ? g.wait_polls : kWaitPolls;
     const bool conj = CX && g.conj;
     const int lgN = m.lgN, nph = 1 << lgN;
@@ -745,12 +758,14 @@ __global__ void __launch_bounds__(256) gemv_rows_small_kernel(const __grid_const
 }
 
 // ---------------------------------------------------------------------------------------
-// Columns kernel straight from global memory. For FP64 complex, whose two accumulators and
-// operands do not fit the streaming kernel's 96 registers (us a call at 2048^2, this kernel /
-// the streaming one: fold 3 33 / 39, fold 4 37 / 45, fold 6 48 / 68, fold 8 60 / 113), and for
-// small matrices of the other types, which pay for filling the streaming kernel's pipeline
-// and for its ends (FP64 500x2000 10.7 / 13.5, 2048x1024 14.5 / 16.6, FP32 1000x500 10.4 /
-// 13.7; even at 32 MB, and slower for short reductions: FP32 100x5000 10.4 / 8.3).
+// Columns kernel straight from global memory, for small matrices, which pay for filling the
+// streaming kernel's pipeline and for its ends (us a call, this kernel / the streaming one:
+// FP64 500x2000 10.7 / 13.5, 2048x1024 14.5 / 16.6, FP32 1000x500 10.4 / 13.7; even at
+// 32 MB, and slower for short reductions: FP32 100x5000 10.4 / 8.3), and for FP64 complex up to
+// 192 MB, where four deposits per element leave the stream little to hide (fold 3: 2048^2
+// 35.0 / 37.7, 20000x500 66.0 / 68.9, but 4096^2 91.0 / 85.0 and 8192^2 307 / 270; fold 6: 2048^2
+// 48.6 / 58.4, 5000^2 210 / 202), or of any size from fold 7, whose two accumulators spill in
+// the streaming kernel (fold 8, 5000^2: 254 / 329).
 // A CTA of 256 threads is G = g.groups row groups of 256/G threads, one column each; grid =
 // (column blocks, row chunks), inside a chunk group q takes rows q, q + G, ..., four per step.
 // fl(alpha*x) of 256 rows at a time is formed in shared memory. The groups' states merge
@@ -758,7 +773,12 @@ __global__ void __launch_bounds__(256) gemv_rows_small_kernel(const __grid_const
 // arrays), and the last CTA of a column block to arrive sums them and finishes.
 // ---------------------------------------------------------------------------------------
 template <typename E, bool CX>
-constexpr bool direct_cols() { return CX && sizeof(E) == 8; }
+__host__ __device__ constexpr bool stream_cols(int fold) { return !(CX && sizeof(E) == 8 && fold > 6); }
+template <typename E, bool CX>
+constexpr bool direct_cols(long long nred, long long bytes, int fold) {
+  if (!stream_cols<E, CX>(fold)) return true;
+  return CX && sizeof(E) == 8 ? bytes <= (192ll << 20) : nred >= 256 && bytes <= (16ll << 20);
+}
 
 // Sum of the G row groups' states (renormalised) through sm[i * 256 + thread]: group 0 ends with
 // the merged state. All 256 threads call it.
@@ -898,18 +918,20 @@ cudaError_t launch_gemv(const XGemvArgs<E>& g, const GemvMaps* maps, bool rows, 
   cudaError_t e = cudaGetDevice(&dev);
   if (e != cudaSuccess) return e;
   if (dev >= kMaxDevices || !ready[dev].load(std::memory_order_relaxed)) {
-    e = cudaFuncSetAttribute(gemv_stream_kernel<E, CX, F, true>,
-                             cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if constexpr (!direct_cols<E, CX>()) {
-      if (e == cudaSuccess)
-        e = cudaFuncSetAttribute(gemv_stream_kernel<E, CX, F, false>,
-                                 cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    for (auto k : {gemv_stream_kernel<E, CX, F, true>, gemv_stream_kernel<E, CX, F, !stream_cols<E, CX>(F)>}) {
+      e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+      if (e != cudaSuccess) return e;
+      if constexpr (moves_regs<E, CX>()) {
+        cudaFuncAttributes at;
+        e = cudaFuncGetAttributes(&at, k);
+        if (e != cudaSuccess) return e;
+        if (at.numRegs != kMoveLaunch) return cudaErrorLaunchOutOfResources;
+      }
     }
-    if (e != cudaSuccess) return e;
     if (dev < kMaxDevices) ready[dev].store(1, std::memory_order_relaxed);
   }
-  if (rows) gemv_stream_kernel<E, CX, F, true><<<grid, kThreads, smem, s>>>(g, *maps);
-  else if constexpr (!direct_cols<E, CX>()) gemv_stream_kernel<E, CX, F, false><<<grid, kThreads, smem, s>>>(g, *maps);
+  if (rows) gemv_stream_kernel<E, CX, F, true><<<grid, threads<E, CX>(), smem, s>>>(g, *maps);
+  else if constexpr (stream_cols<E, CX>(F)) gemv_stream_kernel<E, CX, F, false><<<grid, threads<E, CX>(), smem, s>>>(g, *maps);
   return cudaGetLastError();
 }
 

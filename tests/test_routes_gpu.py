@@ -220,6 +220,13 @@ def test_gemv_stream_folds(cuda, rb, port, t, fold):
         gemv_both(cuda, rb, port, t, fold, ta, M, N, N + pad, 0, 1, fold)
 
 
+@pytest.mark.parametrize("fold, ta", [(2, "t"), (3, "c"), (4, "t"), (6, "c"), (7, "t")])
+def test_gemv_large_complex_columns(cuda, rb, port, fold, ta):
+    # FP64 complex columns above 192 MB: the streaming kernel up to fold 6
+    for M, N in [(41003, 307), (307, 41003)]:
+        gemv_both(cuda, rb, port, "z", fold, ta, M, N, N + 1, 0, 1, fold)
+
+
 @pytest.mark.parametrize("t", list("dszc"))
 @pytest.mark.parametrize("ta", ["n", "t"])
 def test_gemv_few_rows_and_limits(cuda, rb, port, t, ta):
