@@ -233,6 +233,15 @@ bool gemv_small(long long nout, long long nred, int es) {
   return nout * nred * es <= (24ll << 20) && nout <= 8192;
 }
 
+// Whether TMA can address every stage of the matrix: a box's coordinates are ints, in 8-byte words
+// along a row (two per FP64 complex element) and in rows of a phase. A box is at most 130 words wide
+// and 256 rows high, and its end is kept within int as well. Longer rows (16 GiB and more) and
+// taller matrices take the direct kernels, whose addresses are 64-bit.
+bool gemv_in_reach(long long Rs, long long Cs, int es, int phases) {
+  constexpr long long most = (1ll << 31) - 512;
+  return Cs * es / 8 + 2 <= most && Rs / phases <= most;
+}
+
 template <typename E, bool CX>
 bool run_xgemv(const XGemvReq<E, CX>& q) {
   constexpr int NC = CX ? 2 : 1;
@@ -292,15 +301,18 @@ bool run_xgemv(const XGemvReq<E, CX>& q) {
   int phases = 1;
   while (((size_t)phases * q.lda * es) % 16 != 0) phases *= 2;
   if (phases == 1 && a_mis != 0) phases = 2;
-  const bool small = nt && gemv_small(nout, nred_eff, (int)es);
+  const bool reach = gemv_in_reach(Rs, Cs, (int)es, phases);
+  const bool small = nt && (!reach || gemv_small(nout, nred_eff, (int)es));
   // (bounds: see gemv_cols_direct_kernel)
-  const bool direct = !nt && gs::direct_cols<E, CX>(nred_eff, nout * nred_eff * (long long)es, q.fold);
+  const bool direct =
+      !nt && (!reach || gs::direct_cols<E, CX>(nred_eff, nout * nred_eff * (long long)es, q.fold));
   GemvShape sh{};
   const bool uncut = stream_capturing(s);
   if (direct) sh = gemv_direct_shape(nout, nred_eff, di.sms, uncut);
   else if (!small) sh = gemv_shape(nt, nout, nred_eff, (int)es, CX, q.fold, phases, di.sms, uncut);
-  const size_t part_bytes = uncut ? 0 : (size_t)nout * sh.kslots * NC * (2 * q.fold + 1) * sizeof(E);
-  if (!small && !uncut && !w->ensure_tickets((size_t)sh.nunits * 16)) return false;   // per unit and consumer warp
+  const bool whole = uncut || (direct && sh.parts == 1);   // no output's reduction is cut: no scratch
+  const size_t part_bytes = whole ? 0 : (size_t)nout * sh.kslots * NC * (2 * q.fold + 1) * sizeof(E);
+  if (!small && !whole && !w->ensure_tickets((size_t)sh.nunits * 16)) return false;   // per unit and consumer warp
   const bool a_host = a_bytes && !a_dev, x_host = x_bytes && !on_device(q.X);
   const bool y_host = !on_device(q.Y);
   const size_t need = part_bytes + (a_host ? a_bytes : 0) + (x_host ? x_bytes : 0) +

@@ -309,3 +309,33 @@ def test_int8_digits_of_small_magnitudes(cuda, rb, S):
             r = r - t
             assert np.array_equal(d[p, :R, :K], t.astype(np.int8)), p
         assert not d[:, R:].any() and not d[:, :, K:].any()
+
+
+@pytest.mark.parametrize("ta", ["n", "t", "c"])
+def test_gemv_rows_of_more_than_16_gib(cuda, rb, port, ta):
+    # FP64 complex rows of more than 2^30 elements (2^31 words of 8 bytes): products on both sides
+    # of element 2^30 count. The matrix is zero but for a few elements and x has stride 0 (one
+    # element), so the oracle's sum is that of the few
+    n = 2 ** 30 + 300
+    at = [0, 5, 2 ** 30 - 1, 2 ** 30, 2 ** 30 + 1, n - 1]
+    vals, x = ops("z", len(at), 3), ops("z", 1, 4)
+    al, be = 1.5 - 0.25j, 0.0
+    A = cuda.zeros((n, 2), dtype=cuda.float64, device="cuda")
+    A[cuda.tensor(at, device="cuda")] = cuda.from_numpy(vals.view(np.float64).reshape(-1, 2)).cuda()
+    if ta == "n":
+        # row-major, one row; column-major, the transpose of one column
+        want = np.zeros(1, np.complex128)
+        lib_gemv(port, "z", 3, "r", "n", 1, len(at), al, vals, len(at), x, 0, be, want, 1)
+        for order, t, M, N, lda in [("r", "n", 1, n, n), ("c", "t", n, 1, n)]:
+            y = dev(cuda, np.zeros(1, np.complex128))
+            rb_gemv(rb, "z", 3, order, t, M, N, al, A, lda, dev(cuda, x), 0, be, y, 1)
+            assert same_bits(y.cpu().numpy(), want.view(np.float64)), order
+        return
+    # one row, transposed: n outputs of one product each
+    want = np.zeros(len(at), np.complex128)
+    lib_gemv(port, "z", 3, "r", ta, 1, len(at), al, vals, len(at), x, 0, be, want, 1)
+    y = cuda.full((n, 2), 7.0, dtype=cuda.float64, device="cuda")
+    rb_gemv(rb, "z", 3, "r", ta, 1, n, al, A, n, dev(cuda, x), 0, be, y, 1)
+    got = y[cuda.tensor(at, device="cuda")].cpu().numpy()
+    assert same_bits(got.ravel(), want.view(np.float64))
+    assert int(cuda.count_nonzero(y)) == np.count_nonzero(want.view(np.float64))
