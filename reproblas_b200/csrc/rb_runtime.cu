@@ -157,6 +157,13 @@ bool Workspace::ensure_big(size_t bytes) {
   return true;
 }
 
+// Not cudaMemset: that runs on the legacy default stream, behind whatever is queued there, and a
+// non-blocking stream does not wait for it.
+bool Workspace::zero_now(void* p, size_t bytes) {
+  return cuda_ok(cudaMemsetAsync(p, 0, bytes, copy_stream), "cudaMemsetAsync") &&
+         cuda_ok(cudaStreamSynchronize(copy_stream), "cudaStreamSynchronize");
+}
+
 bool Workspace::ensure_tickets(size_t n) {
   if (n <= ntickets) return true;
   // drain the stream first: kernels in flight may still use the old ticket array
@@ -168,7 +175,11 @@ bool Workspace::ensure_tickets(size_t n) {
     set_error(RB_ERR_ALLOC, "ticket allocation failed");
     return false;
   }
-  if (!cuda_ok(cudaMemset(tickets, 0, want * sizeof(unsigned)), "cudaMemset")) return false;
+  if (!zero_now(tickets, want * sizeof(unsigned))) {
+    cudaFree(tickets);
+    tickets = nullptr;
+    return false;
+  }
   ntickets = want;
   return true;
 }
@@ -245,8 +256,9 @@ static bool init_workspace(Workspace* w, int dev, cudaStream_t s, int sms) {
     set_error(RB_ERR_ALLOC, "workspace allocation failed");
     return false;
   }
-  if (!cuda_ok(cudaMemset(w->scratch.ticket, 0, 256), "cudaMemset") ||
-      !cuda_ok(cudaMemset(w->dsmall, 0, Workspace::kSmallBytes), "cudaMemset"))
+  if (!cuda_ok(cudaStreamCreateWithFlags(&w->copy_stream, cudaStreamNonBlocking),
+               "cudaStreamCreate") ||
+      !w->zero_now(w->scratch.ticket, 256) || !w->zero_now(w->dsmall, Workspace::kSmallBytes))
     return false;
   if (host_malloc((void**)&w->hsmall, Workspace::kSmallBytes) != cudaSuccess) {
     w->hsmall = nullptr;
@@ -255,9 +267,6 @@ static bool init_workspace(Workspace* w, int dev, cudaStream_t s, int sms) {
   }
   // the device's address of the pinned slots (kernels store value results straight there)
   if (!cuda_ok(cudaHostGetDevicePointer((void**)&w->hsmall_dev, w->hsmall, 0), "cudaHostGetDevicePointer"))
-    return false;
-  if (!cuda_ok(cudaStreamCreateWithFlags(&w->copy_stream, cudaStreamNonBlocking),
-               "cudaStreamCreate"))
     return false;
   return true;
 }

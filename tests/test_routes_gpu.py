@@ -120,6 +120,39 @@ def test_gemm_captured(cuda, rb, port, t):
         rb.lib.rb_set_stream(None)
 
 
+def test_first_calls_on_a_stream_while_the_default_stream_is_busy(cuda, rb, port):
+    # a new workspace's tickets and status word must be zero before its non-blocking stream uses
+    # them, whatever is queued on the legacy default stream: products cut between CTAs are the
+    # stream's first calls here, behind no work of their own
+    M, N, K = 33, 17, 4001
+    A, B, C = ops("d", M * K, 1), ops("d", K * N, 2), ops("d", M * N, 3)
+    want = C.copy()
+    oracle_gemm(port, "d", 3, "n", "n", M, N, K, A, K, B, N, want, N)
+    m, n = 9000, 700
+    G, x, y = ops("d", m * n, 4), ops("d", n, 5), ops("d", m, 6)
+    wy = y.copy()
+    port.rdgemv(3, b"r", b"n", m, n, 1.5, ptr(G), n, ptr(x), 1, 0.5, ptr(wy), 1)
+    Ad, Bd, Cd, Gd, xd, yd = (dev(cuda, v) for v in (A, B, C, G, x, y))
+    big = cuda.rand(8192, 8192, device="cuda")
+    for first in ("gemm", "gemv"):
+        stream = cuda.cuda.Stream(priority=-1)   # a pool of its own: no call has used its streams
+        cuda.cuda.synchronize()
+        for _ in range(20):
+            big @ big
+        rb.lib.rb_set_stream(stream.cuda_stream)
+        try:
+            if first == "gemm":
+                gpu_gemm(rb, "d", 3, "n", "n", M, N, K, Ad, K, Bd, N, Cd, N)
+            else:
+                rb.call("reproBLAS_rdgemv", 3, "r", "n", m, n, 1.5, Gd, n, xd, 1, 0.5, yd, 1)
+            assert rb.lib.rb_synchronize() == 0
+        finally:
+            rb.lib.rb_set_stream(None)
+        cuda.cuda.synchronize()
+    assert same_bits(Cd.cpu().numpy(), want)
+    assert same_bits(yd.cpu().numpy(), wy)
+
+
 @pytest.mark.parametrize("t", list("dszc"))
 @pytest.mark.parametrize("ta", ["n", "t"])
 def test_gemv_captured(cuda, rb, port, t, ta):
