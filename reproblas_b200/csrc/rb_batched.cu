@@ -450,6 +450,9 @@ bool build_config(rb_batch_plan* p) {
   }
   int per_sm = p->ctas_per_sm > 0 ? std::min(p->ctas_per_sm, std::max(occ, 1)) : std::max(occ, 1);
   p->grid = std::max(1, std::min(di.sms * per_sm, p->nitems));
+  // the plan's arrays were copied and cleared on the legacy default stream, which a run's
+  // non-blocking stream does not wait for
+  if (!cuda_ok(cudaStreamSynchronize(cudaStreamLegacy), "cudaStreamSynchronize")) return false;
   p->built = true;
   return true;
 }

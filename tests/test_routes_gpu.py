@@ -153,6 +153,25 @@ def test_first_calls_on_a_stream_while_the_default_stream_is_busy(cuda, rb, port
     assert same_bits(yd.cpu().numpy(), wy)
 
 
+def test_batch_plan_made_while_the_default_stream_is_busy(cuda, rb):
+    from test_batched_gpu import Problem
+    big, stream = cuda.rand(8192, 8192, device="cuda"), cuda.cuda.Stream(priority=-1)
+    P = Problem(cuda, rb, nseg=200, max_log2=16, ngemm=8, seed=3)
+    try:
+        want, want_c = P.expected_segments()[0], P.expected_gemms()
+        cuda.cuda.synchronize()
+        for _ in range(20):
+            big @ big
+        assert rb.call("rb_batch_plan_set_config", P.plan, 1, 1 << 13, 512, 0) == 0
+        assert rb.call("rb_batch_plan_run", P.plan, stream.cuda_stream) == 0
+        cuda.cuda.synchronize()
+        assert same_bits(P.results.cpu().numpy(), want)
+        for got, w in zip(P.gemm_outputs(), want_c):
+            assert same_bits(got, w)
+    finally:
+        P.destroy()
+
+
 @pytest.mark.parametrize("t", list("dszc"))
 @pytest.mark.parametrize("ta", ["n", "t"])
 def test_gemv_captured(cuda, rb, port, t, ta):
