@@ -124,7 +124,8 @@ bool gemv_maps(GemvMaps* maps, const void* A, size_t es, long long Rs, long long
 // over at most one CTA per SM.
 struct GemvShape {
   int G, grid, q, rem, parts;
-  long long nunits, nb, kslots;
+  long long nunits, nb;
+  size_t records, tickets;   // partial states and tickets of what is cut between CTAs (0: nothing is)
 };
 // `uncut`: no unit is cut between CTAs (no scratch).
 GemvShape gemv_shape(bool rows, long long nout, long long nred, int es, bool cx, int fold, int phases,
@@ -155,15 +156,16 @@ GemvShape gemv_shape(bool rows, long long nout, long long nred, int es, bool cx,
     for (int way = uncut ? 1 : 0; way < 2; way++) {
       double ends;
       long long per;   // stages of the busiest CTA
+      bool cut;        // some unit is cut between CTAs
       if (way == 0) {
         s.parts = 0;
         s.grid = (int)(T < sms ? T : sms);
         s.q = (int)(T / s.grid);
         s.rem = (int)(T % s.grid);
         per = (T + s.grid - 1) / s.grid;
+        cut = s.rem != 0 || s.q % s.nb != 0;
         // a unit meets at most ceil((nb-1) / q) + 1 ranges
-        s.kslots = s.nb / s.q + 2;
-        ends = s.grid == s.nunits && s.rem == 0 ? 5 : 10 + 0.4 * (double)(s.kslots / G);
+        ends = s.grid == s.nunits && s.rem == 0 ? 5 : 10 + 0.4 * (double)((s.nb / s.q + 2) / G);
       } else if (s.nunits <= sms && !uncut) {
         long long p = sms / s.nunits;
         if (p > s.nb) p = s.nb;
@@ -172,7 +174,7 @@ GemvShape gemv_shape(bool rows, long long nout, long long nred, int es, bool cx,
         s.q = 1;
         s.rem = (int)s.nunits;
         per = (s.nb + p - 1) / p;
-        s.kslots = p;
+        cut = p > 1;
         ends = p == 1 ? 5 : 8 + 0.4 * (double)((p + G - 1) / G);
       } else {
         const long long wu = (s.nunits + sms - 1) / sms;
@@ -181,9 +183,11 @@ GemvShape gemv_shape(bool rows, long long nout, long long nred, int es, bool cx,
         s.rem = (int)s.nunits;
         s.grid = (int)((s.nunits + wu - 1) / wu);
         per = wu * s.nb;
-        s.kslots = 1;
+        cut = false;
         ends = 5;
       }
+      s.records = cut ? (size_t)2 * s.grid * P : 0;           // see Ends
+      s.tickets = cut ? (size_t)s.grid * (gs::kConsumers / 32) : 0;
       const double cost = (double)per * stage * m + ends;
       if (best.G == 0 || cost < best_cost) {
         best = s;
@@ -218,7 +222,8 @@ GemvShape gemv_direct_shape(long long nout, long long nred, int sms, bool uncut)
         best.grid = (int)cb;
         best.parts = (int)ch;
         best.nunits = cb;
-        best.kslots = ch;
+        best.records = ch > 1 ? (size_t)ch * nout : 0;
+        best.tickets = ch > 1 ? (size_t)cb : 0;
       }
     }
   }
@@ -307,23 +312,22 @@ bool run_xgemv(const XGemvReq<E, CX>& q) {
   const bool direct =
       !nt && (!reach || gs::direct_cols<E, CX>(nred_eff, nout * nred_eff * (long long)es, q.fold));
   GemvShape sh{};
+  const auto shape = [&](bool uncut) {
+    if (direct) sh = gemv_direct_shape(nout, nred_eff, di.sms, uncut);
+    else if (!small) sh = gemv_shape(nt, nout, nred_eff, (int)es, CX, q.fold, phases, di.sms, uncut);
+  };
   const bool uncut = stream_capturing(s);
-  if (direct) sh = gemv_direct_shape(nout, nred_eff, di.sms, uncut);
-  else if (!small) sh = gemv_shape(nt, nout, nred_eff, (int)es, CX, q.fold, phases, di.sms, uncut);
-  const bool whole = uncut || (direct && sh.parts == 1);   // no output's reduction is cut: no scratch
-  const size_t part_bytes = whole ? 0 : (size_t)nout * sh.kslots * NC * (2 * q.fold + 1) * sizeof(E);
-  if (!small && !whole && !w->ensure_tickets((size_t)sh.nunits * 16)) return false;   // per unit and consumer warp
+  shape(uncut);
+  if (sh.records && !cut_scratch(w, sh.records * NC * (2 * q.fold + 1) * sizeof(E), sh.tickets)) shape(true);
   const bool a_host = a_bytes && !a_dev, x_host = x_bytes && !on_device(q.X);
   const bool y_host = !on_device(q.Y);
-  const size_t need = part_bytes + (a_host ? a_bytes : 0) + (x_host ? x_bytes : 0) +
-                      (y_host ? y_bytes : 0) + 4 * 256;
-  if (!w->ensure_big(need)) return false;
+  const size_t need = (a_host ? a_bytes : 0) + (x_host ? x_bytes : 0) + (y_host ? y_bytes : 0) + 3 * 256;
+  if (need > 3 * 256 && !w->ensure_big(need)) return false;
   Bump b{w->big};
   bool ok = true;
   const E* dA = (const E*)to_device(q.A, a_bytes, &b, s, &ok);
   const E* dX = (const E*)to_device(q.X, x_bytes, &b, s, &ok);
   E* dY = (E*)to_device(q.Y, y_bytes, &b, s, &ok);
-  E* part = (E*)b.take(part_bytes);
   if (!ok) return false;
 
   XGemvArgs<E> g{};
@@ -347,8 +351,7 @@ bool run_xgemv(const XGemvReq<E, CX>& q) {
   g.q = sh.q;
   g.rem = sh.rem;
   g.parts = sh.parts;
-  g.scratch = part;
-  g.kslots = sh.kslots;
+  g.scratch = (E*)w->parts;
   g.tickets = w->tickets;
   g.status = w->dstatus();
   g.groups = sh.G;

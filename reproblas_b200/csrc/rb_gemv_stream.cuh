@@ -86,8 +86,7 @@ static_assert(kSmemBytes + 256 <= 227 * 1024, "shared memory of the gemv kernel"
 // `parts` = 0, q or q + 1 stages each, whatever the shape; with parts = p > 0, the p-th part of a
 // unit (p > 1) or q whole units (p = 1), so that a CTA has one run, or no unit is cut. A unit
 // whose stages all fall in one CTA is finished there; a unit cut between CTAs leaves one
-// partial state per CTA in slot k = i - owner(first stage of u), and the last of those CTAs to
-// finish (ticket) merges them.
+// partial state per CTA, and the last of those CTAs to finish (ticket) merges them.
 struct Split {
   int q, rem, parts, nb, x0, x1;
   template <typename E>
@@ -492,9 +491,12 @@ struct Consumer {
   }
 };
 
-// Partial states of units cut between CTAs, structure of arrays over the outputs: field i
-// (< NC*(2F+1): pri, car, flags per component) of slot k for output o at
-// scratch[(i*kslots + k)*nout + o].
+// Partial states of units cut between CTAs: a CTA holds at most two, that of the unit its range
+// begins inside (slot 2*cta) and that of the unit that begins in its range and goes on in the next
+// CTA's (slot 2*cta + 1), whatever the number of outputs. Structure of arrays: field i
+// (< NC*(2F+1): pri, car, flags per component) of slot s for the unit's output pp at
+// scratch[(i*2*grid + s)*P + pp]. A cut unit's tickets, one per warp, are those of the CTA it
+// begins in.
 //
 // A CTA's range of stages holds whole units in its middle and possibly cut units at its two
 // ends. Ends::close() ends the run of unit u in this CTA for the warp's outputs: the groups
@@ -508,8 +510,9 @@ struct Ends {
   static constexpr int NC = CX ? 2 : 1, REC = 2 * F + 1;
   const XGemvArgs<E>& g;
   int P, lgG, grp, pp, out;   // group of this lane, its output's offset in a unit, lanes per group
-  long long nout, fs;
-  int n, u0, u1, c0, c1;      // pending units and the CTAs they meet
+  long long nout;
+  int fs;                     // distance of a record's fields
+  int n, u0, u1;              // pending units
 
   __device__ __forceinline__ void finish(long long o, Acc<E, F> (&a)[NC], const E (&y)[NC]) const {
     xb::finish_from<E, CX, F>(a, g.mode, y, g.y + o * g.incy * NC, g.br, g.bi,
@@ -519,27 +522,29 @@ struct Ends {
 #pragma unroll
     for (int c = 0; c < NC; c++) y[c] = want && g.mode == kOutValue ? g.y[o * g.incy * NC + c] : E(0);
   }
+  // this lane's output in the partial state of CTA i; begins: of the unit that begins in its range
+  __device__ __forceinline__ int slot(int i, bool begins) const { return (2 * i + (begins ? 1 : 0)) * P + pp; }
   __device__ __forceinline__ void close(const Split& sp, int u, Acc<E, F> (&a)[NC]) {
     const long long o = (long long)u * P + pp;
     const bool mine = grp == 0 && o < nout;
-    const int first = sp.owner(u * g.nb), count = sp.owner(u * g.nb + g.nb - 1) - first + 1;
+    const bool begins = u * g.nb >= sp.x0, whole = begins && u * g.nb + g.nb <= sp.x1;
     E y[NC];   // the entry's current value, loaded early
-    read_y(o, mine && count == 1, y);
+    read_y(o, mine && whole, y);
     lanes_merge<E, F, NC>(a, out);
-    if (count == 1) {
+    if (whole) {
       if (mine) finish(o, a, y);
       return;
     }
     if (mine) {
-      E* rec = g.scratch + (long long)((int)blockIdx.x - first) * nout + o;
+      E* rec = g.scratch + slot((int)blockIdx.x, begins);
 #pragma unroll
       for (int c = 0; c < NC; c++) xb::put_rec<E, F>(a[c], rec + c * REC * fs, fs);
     }
-    if (n == 0) { u0 = u; c0 = count; }
-    else { u1 = u; c1 = count; }
+    if (n == 0) u0 = u;
+    else u1 = u;
     n++;
   }
-  __device__ __forceinline__ void settle() {
+  __device__ __forceinline__ void settle(const Split& sp) {
     if (n == 0) return;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     // release this warp's parts, then take its tickets (lanes 0 and 1, one each)
@@ -547,8 +552,9 @@ struct Ends {
     __syncwarp();
     bool last = false;
     if (lane < n) {
-      unsigned* t = g.tickets + (size_t)(lane == 0 ? u0 : u1) * (kConsumers / 32) + warp;
-      last = atomicAdd(t, 1u) == (unsigned)(lane == 0 ? c0 : c1) - 1;
+      const int b = (lane == 0 ? u0 : u1) * g.nb, first = sp.owner(b);
+      unsigned* t = g.tickets + first * (kConsumers / 32) + warp;
+      last = atomicAdd(t, 1u) == (unsigned)(sp.owner(b + g.nb - 1) - first);
       if (last) *t = 0u;
     }
     const unsigned mask = __ballot_sync(0xffffffffu, last);
@@ -557,8 +563,9 @@ struct Ends {
 #pragma unroll 1
     for (int k = 0; k < n; k++) {
       if (!(mask & (1u << k))) continue;
-      const long long o = (long long)(k == 0 ? u0 : u1) * P + pp;
-      const int count = k == 0 ? c0 : c1;
+      const int u = k == 0 ? u0 : u1, first = sp.owner(u * g.nb);
+      const int count = sp.owner(u * g.nb + g.nb - 1) - first + 1;
+      const long long o = (long long)u * P + pp;
       E y[NC];
       read_y(o, grp == 0 && o < nout, y);
       Acc<E, F> a[NC];
@@ -570,7 +577,7 @@ struct Ends {
 #pragma unroll 2
           for (int q = grp; q < count; q += 1 << lgG) {
             Acc<E, F> part;
-            xb::read_rec<E, F>(part, g.scratch + q * nout + o + c * REC * fs, fs);
+            xb::read_rec<E, F>(part, g.scratch + slot(first + q, q == 0) + c * REC * fs, fs);
             sum.add(part);
           }
         }
@@ -617,7 +624,7 @@ gemv_stream_kernel(const __grid_constant__ XGemvArgs<E> g, const __grid_constant
     const long long polls = g.wait_polls > 0 ? g.wait_polls : kWaitPolls;
     const bool conj = CX && g.conj;
     const int lgN = m.lgN, nph = 1 << lgN;
-    Ends<E, CX, F> ends{g, m.P, m.lgG, 0, 0, 32 >> m.lgG, m.nout, g.kslots * m.nout, 0, 0, 0, 0, 0};
+    Ends<E, CX, F> ends{g, m.P, m.lgG, 0, 0, 32 >> m.lgG, m.nout, 2 * (int)gridDim.x * m.P, 0, 0, 0};
     const int grp = lane >> (5 - m.lgG);
     // rows kernel: thread p takes slot p, i.e. row (p mod P/NPH)*NPH + p / (P/NPH) of the band,
     // so that neighbouring lanes read neighbouring slots; columns kernel: column p
@@ -671,7 +678,7 @@ gemv_stream_kernel(const __grid_constant__ XGemvArgs<E> g, const __grid_constant
       j = 0;
       u++;
     }
-    ends.settle();
+    ends.settle(sp);
   }
   __syncthreads();
   if (tid == 0 && sy.abort_flag) atomicExch(g.status, 2);

@@ -80,7 +80,7 @@ struct Workspace {
   void* hresult() { return (void*)(hsmall + 2112); }
   void* hresult_dev() { return (void*)(hsmall_dev + 2112); }   // hresult() as kernels address it
 
-  // partial states of gemm tiles cut between CTAs (grow on demand; see gemm_decompose)
+  // partial states of gemm tiles and gemv units cut between CTAs (grows on demand; see cut_scratch)
   unsigned char* parts = nullptr;
   size_t parts_bytes = 0;
 
@@ -100,6 +100,10 @@ Workspace* acquire_workspace(std::unique_lock<std::mutex>* lock, bool create = t
 // Whether stream s is being captured into a graph (or cannot tell): kernels then take forms without
 // scratch where they have one, since a later call may replace the scratch a graph would hold.
 bool stream_capturing(cudaStream_t s);
+
+// Room in w->parts and w->tickets for the partial states and tickets of what a launch cuts between
+// CTAs; false (no error set) when it cannot be had: the caller takes a form that cuts nothing.
+bool cut_scratch(Workspace* w, size_t bytes, size_t tickets);
 
 // Decomposition of an M x N x K gemm on workspace w's stream through a fold's planner: cut tiles
 // when that pays and the scratch for their partial states can be had, else whole tiles (no

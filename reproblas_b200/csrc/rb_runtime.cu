@@ -197,33 +197,33 @@ bool Workspace::reset_after_abort() {
          cuda_ok(cudaStreamSynchronize(stream), "cudaStreamSynchronize");
 }
 
+bool cut_scratch(Workspace* w, size_t bytes, size_t tickets) {
+  if (bytes > w->parts_bytes) {
+    // drain the stream first: kernels in flight may still use the old buffer
+    if (cudaStreamSynchronize(w->stream) != cudaSuccess) return false;
+    if (w->parts) { cudaFree(w->parts); w->parts = nullptr; w->parts_bytes = 0; }
+    if (dev_malloc((void**)&w->parts, bytes) != cudaSuccess) {
+      cudaGetLastError();
+      w->parts = nullptr;
+      return false;
+    }
+    w->parts_bytes = bytes;
+  }
+  if (tickets > w->ntickets && !w->ensure_tickets(tickets)) {
+    cudaGetLastError();
+    rb_clear_error();   // uncut forms need none
+    return false;
+  }
+  return true;
+}
+
 bool gemm_decompose(cudaError_t (*plan)(long long, long long, long long, int, bool, GemmPlan*),
                     Workspace* w, long long M, long long N, long long K, GemmPlan* p) {
   DeviceInfo di;
   if (!device_info(&di)) return false;
   if (!cuda_ok(plan(M, N, K, di.sms, false, p), "gemm kernel attributes")) return false;
   if (!p->cut) return true;
-  bool have = !stream_capturing(w->stream);
-  if (have && p->scratch_bytes > w->parts_bytes) {
-    // drain the stream first: kernels in flight may still use the old buffer
-    if (!cuda_ok(cudaStreamSynchronize(w->stream), "cudaStreamSynchronize")) return false;
-    if (w->parts) { cudaFree(w->parts); w->parts = nullptr; w->parts_bytes = 0; }
-    if (dev_malloc((void**)&w->parts, p->scratch_bytes) == cudaSuccess) {
-      w->parts_bytes = p->scratch_bytes;
-    } else {
-      cudaGetLastError();
-      w->parts = nullptr;
-      have = false;
-    }
-  }
-  if (have && (size_t)p->tiles > w->ntickets) {
-    // a failed ticket allocation is no error here: whole tiles need none
-    have = w->ensure_tickets((size_t)p->tiles);
-    if (!have) {
-      cudaGetLastError();
-      rb_clear_error();
-    }
-  }
+  const bool have = !stream_capturing(w->stream) && cut_scratch(w, p->scratch_bytes, (size_t)p->tiles);
   if (!have) return cuda_ok(plan(M, N, K, di.sms, true, p), "gemm kernel attributes");
   p->scratch = w->parts;
   p->tickets = w->tickets;

@@ -93,6 +93,58 @@ def test_gemm_without_scratch(cuda, rb, port, t):
 
 
 @pytest.mark.parametrize("t", list("dszc"))
+@pytest.mark.parametrize("ta", ["n", "t"])
+def test_gemv_without_scratch(cuda, rb, port, t, ta):
+    # units that would be cut between CTAs stay whole when their scratch cannot be had
+    M, N, al, be = (9000, 700, *scalars(t)) if ta == "n" else (3000, 1500, *scalars(t))
+    A, x, y = ops(t, M * N, 1), ops(t, max(M, N), 2), ops(t, M if ta == "n" else N, 3)
+    want = y.copy()
+    Ad, xd, yd = dev(cuda, A), dev(cuda, x), dev(cuda, y)
+    stream = cuda.cuda.Stream()
+    rb.lib.rb_set_stream(stream.cuda_stream)
+    try:
+        one = cuda.ones(16, dtype=cuda.float64, device="cuda")
+        cuda.cuda.synchronize()
+        rb.call("reproBLAS_rdsum", 3, 16, one, 1)     # makes the stream's workspace
+        rb.lib.rb_debug_fail_allocations(8)
+        if t == "d":
+            port.rdgemv(3, b"r", ta.encode(), M, N, al, ptr(A), N, ptr(x), 1, be, ptr(want), 1)
+            rb.call("reproBLAS_rdgemv", 3, "r", ta, M, N, al, Ad, N, xd, 1, be, yd, 1)
+        else:
+            lib_gemv(port, t, 3, "r", ta, M, N, al, A, N, x, 1, be, want, 1)
+            rb_gemv(rb, t, 3, "r", ta, M, N, al, Ad, N, xd, 1, be, yd, 1)
+        stream.synchronize()
+        assert same_bits(yd.cpu().numpy(), want.view(REAL[t]))
+    finally:
+        rb.lib.rb_debug_fail_allocations(0)
+        rb.lib.rb_set_stream(None)
+
+
+@pytest.mark.parametrize("t, ta, M, N", [("d", "n", 20_000_000, 4), ("z", "n", 4_000_000, 8), ("s", "t", 16, 8_000_000),
+                                         ("c", "n", 400_003, 100), ("z", "t", 300, 200_000)])
+def test_gemv_scratch_does_not_grow_with_the_outputs(cuda, rb, t, ta, M, N):
+    # at most two units per CTA are cut: the device memory a call takes stays below 64 MB
+    A = cuda.zeros(M * N * (2 if t in "zc" else 1), dtype={"d": cuda.float64, "z": cuda.float64}.get(t, cuda.float32),
+                   device="cuda")
+    x, y = cuda.zeros_like(A[:2 * max(M, N)]), cuda.ones_like(A[:2 * max(M, N)])
+    stream = cuda.cuda.Stream(priority=-1)
+    cuda.cuda.synchronize()
+    rb.lib.rb_set_stream(stream.cuda_stream)
+    try:
+        free = cuda.cuda.mem_get_info()[0]
+        if t == "d":
+            rb.call("reproBLAS_rdgemv", 3, "r", ta, M, N, 1.5, A, N, x, 1, 0.0, y, 1)
+        else:
+            rb_gemv(rb, t, 3, "r", ta, M, N, 1.5, A, N, x, 1, 0.0, y, 1)
+        assert rb.lib.rb_synchronize() == 0
+        assert free - cuda.cuda.mem_get_info()[0] < 64 << 20
+        n = (M if ta == "n" else N) * (2 if t in "zc" else 1)
+        assert int(cuda.count_nonzero(y[:n])) == 0
+    finally:
+        rb.lib.rb_set_stream(None)
+
+
+@pytest.mark.parametrize("t", list("dszc"))
 def test_gemm_captured(cuda, rb, port, t):
     # a graph must not hold scratch that a later, larger call replaces: capture, grow, replay
     M, N, K = 33, 17, 2000
