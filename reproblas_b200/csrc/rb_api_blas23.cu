@@ -316,9 +316,9 @@ bool run_xgemv(const XGemvReq<E, CX>& q) {
     if (direct) sh = gemv_direct_shape(nout, nred_eff, di.sms, uncut);
     else if (!small) sh = gemv_shape(nt, nout, nred_eff, (int)es, CX, q.fold, phases, di.sms, uncut);
   };
-  const bool uncut = stream_capturing(s);
-  shape(uncut);
-  if (sh.records && !cut_scratch(w, sh.records * NC * (2 * q.fold + 1) * sizeof(E), sh.tickets)) shape(true);
+  shape(false);
+  CutScratch cs{};
+  if (sh.records && !cut_scratch(w, sh.records * NC * (2 * q.fold + 1) * sizeof(E), sh.tickets, &cs)) shape(true);
   const bool a_host = a_bytes && !a_dev, x_host = x_bytes && !on_device(q.X);
   const bool y_host = !on_device(q.Y);
   const size_t need = (a_host ? a_bytes : 0) + (x_host ? x_bytes : 0) + (y_host ? y_bytes : 0) + 3 * 256;
@@ -351,8 +351,8 @@ bool run_xgemv(const XGemvReq<E, CX>& q) {
   g.q = sh.q;
   g.rem = sh.rem;
   g.parts = sh.parts;
-  g.scratch = (E*)w->parts;
-  g.tickets = w->tickets;
+  g.scratch = (E*)cs.parts;
+  g.tickets = cs.tickets;
   g.status = w->dstatus();
   g.groups = sh.G;
   g.phases = phases;

@@ -97,18 +97,21 @@ struct Workspace {
 // set); with create = false, nullptr when no call has made one yet.
 Workspace* acquire_workspace(std::unique_lock<std::mutex>* lock, bool create = true);
 
-// Whether stream s is being captured into a graph (or cannot tell): kernels then take forms without
-// scratch where they have one, since a later call may replace the scratch a graph would hold.
+// Whether stream s is being captured into a graph (or cannot tell).
 bool stream_capturing(cudaStream_t s);
 
-// Room in w->parts and w->tickets for the partial states and tickets of what a launch cuts between
-// CTAs; false (no error set) when it cannot be had: the caller takes a form that cuts nothing.
-bool cut_scratch(Workspace* w, size_t bytes, size_t tickets);
+// Room for the partial states and tickets of what a launch on workspace w's stream cuts between CTAs:
+// the workspace's own or, while the stream is captured, a block that belongs to the graph. False
+// (no error set) when it cannot be had: the caller takes a form that cuts nothing.
+struct CutScratch {
+  void* parts;
+  unsigned* tickets;   // zero
+};
+bool cut_scratch(Workspace* w, size_t bytes, size_t tickets, CutScratch* out);
 
 // Decomposition of an M x N x K gemm on workspace w's stream through a fold's planner: cut tiles
 // when that pays and the scratch for their partial states can be had, else whole tiles (no
-// scratch). A captured launch keeps to whole tiles, so that a graph never holds the address
-// of scratch that a later call may replace.
+// scratch). A captured launch keeps to whole tiles.
 bool gemm_decompose(cudaError_t (*plan)(long long, long long, long long, int, bool, GemmPlan*),
                     Workspace* w, long long M, long long N, long long K, GemmPlan* p);
 

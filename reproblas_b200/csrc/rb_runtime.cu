@@ -197,7 +197,121 @@ bool Workspace::reset_after_abort() {
          cuda_ok(cudaStreamSynchronize(stream), "cudaStreamSynchronize");
 }
 
-bool cut_scratch(Workspace* w, size_t bytes, size_t tickets) {
+// ---- scratch of captured launches -------------------------------------------------------------
+// A graph may be replayed on any stream, at any time, so a captured launch must not hold the
+// workspace's scratch, which later calls use and replace. It gets a block of its own, which the
+// graph (and every executable made of it) owns as a user object; with the last of them gone it
+// waits in `idle` for the next capture. Idle blocks above kIdleMost bytes are freed by the next
+// call that is not captured.
+namespace {
+struct GraphScratch {
+  void* mem;
+  size_t bytes;
+  int device;
+  GraphScratch* next;
+};
+constexpr size_t kIdleMost = 64u << 20;
+std::mutex g_idle_mu;
+GraphScratch* g_idle = nullptr;
+std::atomic<size_t> g_idle_bytes{0};
+
+// Destructor of the user object. It runs on a thread of the CUDA runtime, where no CUDA call is
+// allowed.
+void CUDART_CB graph_scratch_idle(void* p) {
+  GraphScratch* b = (GraphScratch*)p;
+  std::lock_guard<std::mutex> g(g_idle_mu);
+  b->next = g_idle;
+  g_idle = b;
+  g_idle_bytes += b->bytes;
+}
+
+// allocation and freeing are allowed in this thread during a capture (any thread's) meanwhile
+struct RelaxedCapture {
+  cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+  RelaxedCapture() { cudaThreadExchangeStreamCaptureMode(&mode); }
+  ~RelaxedCapture() { cudaThreadExchangeStreamCaptureMode(&mode); }
+};
+
+void trim_idle() {
+  if (g_idle_bytes.load() <= kIdleMost) return;
+  GraphScratch* b;
+  {
+    std::lock_guard<std::mutex> g(g_idle_mu);
+    b = g_idle;
+    g_idle = nullptr;
+    g_idle_bytes = 0;
+  }
+  RelaxedCapture relaxed;
+  while (b) {
+    GraphScratch* next = b->next;
+    cudaFree(b->mem);
+    delete b;
+    b = next;
+  }
+}
+
+// a block of at least `bytes` whose first `zeroed` are zero
+GraphScratch* take_block(Workspace* w, size_t bytes, size_t zeroed) {
+  GraphScratch* b = nullptr;
+  {
+    std::lock_guard<std::mutex> g(g_idle_mu);
+    for (GraphScratch** p = &g_idle; *p; p = &(*p)->next)
+      if ((*p)->device == w->device && (*p)->bytes >= bytes && (*p)->bytes / 4 <= bytes) {
+        b = *p;
+        *p = b->next;
+        g_idle_bytes -= b->bytes;
+        break;
+      }
+  }
+  RelaxedCapture relaxed;
+  if (!b) {
+    void* mem = nullptr;
+    if (dev_malloc(&mem, bytes) != cudaSuccess) {
+      cudaGetLastError();
+      return nullptr;
+    }
+    b = new GraphScratch{mem, bytes, w->device, nullptr};
+  }
+  if (cudaMemsetAsync(b->mem, 0, zeroed, w->copy_stream) != cudaSuccess ||
+      cudaStreamSynchronize(w->copy_stream) != cudaSuccess) {
+    cudaGetLastError();
+    graph_scratch_idle(b);
+    return nullptr;
+  }
+  return b;
+}
+
+bool graph_scratch(Workspace* w, size_t bytes, size_t tickets, CutScratch* out) {
+  cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
+  cudaGraph_t graph = nullptr;
+  if (cudaStreamGetCaptureInfo(w->stream, &st, nullptr, &graph) != cudaSuccess ||
+      st != cudaStreamCaptureStatusActive) {
+    cudaGetLastError();
+    return false;
+  }
+  const size_t ticket_bytes = (tickets * sizeof(unsigned) + 255) / 256 * 256;
+  GraphScratch* b = take_block(w, ticket_bytes + bytes, ticket_bytes);
+  if (!b) return false;
+  cudaUserObject_t obj;
+  if (cudaUserObjectCreate(&obj, b, graph_scratch_idle, 1, cudaUserObjectNoDestructorSync) != cudaSuccess) {
+    cudaGetLastError();
+    graph_scratch_idle(b);
+    return false;
+  }
+  if (cudaGraphRetainUserObject(graph, obj, 1, cudaGraphUserObjectMove) != cudaSuccess) {
+    cudaGetLastError();
+    cudaUserObjectRelease(obj, 1);
+    return false;
+  }
+  out->tickets = (unsigned*)b->mem;
+  out->parts = (char*)b->mem + ticket_bytes;
+  return true;
+}
+}  // namespace
+
+bool cut_scratch(Workspace* w, size_t bytes, size_t tickets, CutScratch* out) {
+  if (stream_capturing(w->stream)) return graph_scratch(w, bytes, tickets, out);
+  trim_idle();
   if (bytes > w->parts_bytes) {
     // drain the stream first: kernels in flight may still use the old buffer
     if (cudaStreamSynchronize(w->stream) != cudaSuccess) return false;
@@ -214,6 +328,8 @@ bool cut_scratch(Workspace* w, size_t bytes, size_t tickets) {
     rb_clear_error();   // uncut forms need none
     return false;
   }
+  out->parts = w->parts;
+  out->tickets = w->tickets;
   return true;
 }
 
@@ -223,10 +339,11 @@ bool gemm_decompose(cudaError_t (*plan)(long long, long long, long long, int, bo
   if (!device_info(&di)) return false;
   if (!cuda_ok(plan(M, N, K, di.sms, false, p), "gemm kernel attributes")) return false;
   if (!p->cut) return true;
-  const bool have = !stream_capturing(w->stream) && cut_scratch(w, p->scratch_bytes, (size_t)p->tiles);
-  if (!have) return cuda_ok(plan(M, N, K, di.sms, true, p), "gemm kernel attributes");
-  p->scratch = w->parts;
-  p->tickets = w->tickets;
+  CutScratch cs{};
+  if (stream_capturing(w->stream) || !cut_scratch(w, p->scratch_bytes, (size_t)p->tiles, &cs))
+    return cuda_ok(plan(M, N, K, di.sms, true, p), "gemm kernel attributes");
+  p->scratch = cs.parts;
+  p->tickets = cs.tickets;
   return true;
 }
 

@@ -262,6 +262,58 @@ def test_gemv_captured(cuda, rb, port, t, ta):
         rb.lib.rb_set_stream(None)
 
 
+@pytest.mark.parametrize("t, ta, M, N", [("d", "n", 100, 60000), ("d", "t", 3000, 1500), ("s", "t", 40000, 100),
+                                         ("z", "n", 3000, 1500), ("z", "t", 2000, 500), ("c", "n", 9000, 300)])
+def test_gemv_replays_beside_other_calls(cuda, rb, port, t, ta, M, N):
+    # a captured call whose units are cut has scratch of its own: captured with the workspace warmed by
+    # a reduction alone, replayed on one stream while the stream it was captured on runs other
+    # calls; a second graph of the same call at the same time; and after the graphs are gone
+    al, be = scalars(t)
+    A, x, y = ops(t, M * N, 4), ops(t, max(M, N), 5), ops(t, M if ta == "n" else N, 6)
+    want = y.copy()
+    if t == "d":
+        port.rdgemv(3, b"r", ta.encode(), M, N, al, ptr(A), N, ptr(x), 1, be, ptr(want), 1)
+    else:
+        lib_gemv(port, t, 3, "r", ta, M, N, al, A, N, x, 1, be, want, 1)
+    Ad, xd, y0 = dev(cuda, A), dev(cuda, x), dev(cuda, y)
+
+    def call(out):
+        if t == "d":
+            rb.call("reproBLAS_rdgemv", 3, "r", ta, M, N, al, Ad, N, xd, 1, be, out, 1)
+        else:
+            rb_gemv(rb, t, 3, "r", ta, M, N, al, Ad, N, xd, 1, be, out, 1)
+
+    stream, others = cuda.cuda.Stream(priority=-1), [cuda.cuda.Stream(), cuda.cuda.Stream()]
+    rb.lib.rb_set_stream(stream.cuda_stream)
+    try:
+        one = cuda.ones(16, dtype=cuda.float64, device="cuda")
+        cuda.cuda.synchronize()
+        rb.call("reproBLAS_rdsum", 3, 16, one, 1)
+        for again in range(2):
+            outs = [y0.clone() for _ in range(3)]
+            cuda.cuda.synchronize()
+            graphs = []
+            for k in range(2):
+                g = cuda.cuda.CUDAGraph()
+                with cuda.cuda.graph(g, stream=stream):
+                    outs[k].copy_(y0)
+                    call(outs[k])
+                graphs.append(g)
+            for rep in range(20):
+                for k in range(2):
+                    with cuda.cuda.stream(others[k]):
+                        graphs[k].replay()
+                with cuda.cuda.stream(stream):
+                    outs[2].copy_(y0)
+                call(outs[2])
+            cuda.cuda.synchronize()
+            for out in outs:
+                assert same_bits(out.cpu().numpy(), want.view(REAL[t])), again
+            del graphs, g
+    finally:
+        rb.lib.rb_set_stream(None)
+
+
 @pytest.mark.parametrize("t", list("dszc"))
 @pytest.mark.parametrize("fold", [2, 3, 4])
 def test_gemm_blocks_off_the_unchecked_path(cuda, rb, port, t, fold):
