@@ -15,6 +15,7 @@
 // cbcgemv cut each column's dot into blocks of MIN(X_BLOCK, N - j) elements while j runs
 // over the M rows (zbzgemv.ccog:214-218, cbcgemv.ccog:214-218), which equals the mathematical
 // A^H x only when M == N. Here every entry is the full A^H x.
+#include <algorithm>
 #include <cstring>
 #include <string>
 
@@ -187,7 +188,7 @@ GemvShape gemv_shape(bool rows, long long nout, long long nred, int es, bool cx,
         ends = 5;
       }
       s.records = cut ? (size_t)2 * s.grid * P : 0;           // see Ends
-      s.tickets = cut ? (size_t)s.grid * (gs::kConsumers / 32) : 0;
+      s.tickets = cut ? (size_t)s.grid * 3 * (gs::kConsumers / 32) : 0;
       const double cost = (double)per * stage * m + ends;
       if (best.G == 0 || cost < best_cost) {
         best = s;
@@ -202,7 +203,7 @@ GemvShape gemv_shape(bool rows, long long nout, long long nred, int es, bool cx,
 // units of one row per thread: the streaming part (waves of CTAs, two per SM, times rows per
 // thread, plus the groups' merge) and the sum of the chunks' partial states.
 // `uncut`: one chunk (no scratch).
-GemvShape gemv_direct_shape(long long nout, long long nred, int sms, bool uncut) {
+GemvShape gemv_cols_direct_shape(long long nout, long long nred, int sms, bool uncut) {
   GemvShape best{};
   long long best_cost = -1;
   const long long slots = (long long)sms * 2;
@@ -231,11 +232,45 @@ GemvShape gemv_direct_shape(long long nout, long long nred, int sms, bool uncut)
 }
 
 // Matrices whose rows the direct kernel reduces sooner than the streaming one (us a call, direct /
-// streaming): FP64 1000x500 10.3 / 12.8, 2048x1024 10.5 / 14.5, 64x20000 14.5 / 27.3, FP32
-// 2000x2001 14.5 / 18.6, FP64 complex 1024^2 16.5 / 22.0, fold 8 2048^2 24.7 / 28.9; about even at
-// 32 MB (FP64 2000x2001 17.2 / 18.7). Many short rows stream: 20000x64 20.6 / 11.4.
-bool gemv_small(long long nout, long long nred, int es) {
-  return nout * nred * es <= (24ll << 20) && nout <= 8192;
+// streaming). Small ones, up to 48 MB of FP64: 1000x4195 16.1 / 20.1, 4000x1573 20.1 / 22.7, 200x20971
+// 22.7 / 28.6; up to 32 MB of the others: FP32 4000x2097 21.6 / 24.6, but 4000x3145 28.2 / 26.8; FP64
+// complex 4000x525 26.1 / 30.7, 4000x787 32.7 / 34.7; FP32 complex 1000x4195 26.7 / 27.7, 1000x6291
+// 34.8 / 37.0. Many rows fill the streaming kernel's units: FP64 20000x64 20.6 / 11.4, FP32
+// 8192x1000 23.0 / 16.5, FP64 complex 8000x131 22.6 / 14.4, but 5000x209 18.5 / 24.7. And few rows of any length, which fill
+// a band of the streaming kernel (64 rows or more) badly: FP64 1x3000000 18.5 / 156, 8x8000000 121 / 391,
+// 48x400000 47.5 / 51.8, FP32 16x500000 26.7 / 28.8 but 32x500000 39.0 / 35.4, FP64 complex 16x500000
+// 58.7 / 94.8 but 32x500000 111 / 107, FP32 complex 48x400000 79.8 / 89.2.
+bool gemv_rows_direct(long long nout, long long nred, int es, bool cx) {
+  const long long bytes = nout * nred * es;
+  if (nout > 6144) return nout <= 8192 && bytes <= 8ll << 20;
+  return nout <= (es == 8 ? 48 : 24) || bytes <= (es == 8 && !cx ? 48ll << 20 : 32ll << 20);
+}
+
+// Shape of the direct rows kernel: S warps to a row, enough to fill the device with at least 64
+// elements to each, and `parts` CTAs to a row where rows alone leave it idle: 8 CTAs per SM in
+// all (4 of FP64 complex, of which 2 are resident), each with four steps of its 8 warps or more, two
+// while there are two CTAs per SM. us a call with 4 / 8 / 16 / 32 CTAs per SM (an earlier form of the
+// kernel): FP64 8x8000000 164 / 153 / 162 / 172, FP32 32x500000 43.4 / 41.0 / 43.4 / 53.4, FP64 complex
+// 16x500000 61.5 / 71.1 / 84.0 / 118.
+// `uncut`: one part (no scratch).
+GemvShape gemv_rows_direct_shape(long long nout, long long nred, int es, int sms, bool uncut) {
+  GemvShape s{};
+  int S = 1;
+  while (S < 8 && nout * S < (long long)sms * 16 && nred >= 128 * S) S *= 2;
+  s.G = S;
+  s.grid = (int)((nout + 8 / S - 1) / (8 / S));
+  s.parts = 1;
+  if (S == 8 && !uncut) {
+    const long long steps = nred / 1024;   // of a whole CTA: 4 elements a lane
+    const long long most = ((long long)sms * (es == 16 ? 4 : 8) + nout - 1) / nout, once = (long long)sms * 2 / nout;
+    const long long p = std::min(most, std::max(steps / 4, std::min(steps / 2, once)));
+    if (p > 1 && steps - steps / p >= 6) {   // the sum of the parts takes as long as about five steps
+      s.parts = (int)p;
+      s.records = (size_t)nout * p;
+      s.tickets = (size_t)nout;
+    }
+  }
+  return s;
 }
 
 // Whether TMA can address every stage of the matrix: a box's coordinates are ints, in 8-byte words
@@ -307,14 +342,15 @@ bool run_xgemv(const XGemvReq<E, CX>& q) {
   while (((size_t)phases * q.lda * es) % 16 != 0) phases *= 2;
   if (phases == 1 && a_mis != 0) phases = 2;
   const bool reach = gemv_in_reach(Rs, Cs, (int)es, phases);
-  const bool small = nt && (!reach || gemv_small(nout, nred_eff, (int)es));
+  const bool rows_direct = nt && (!reach || gemv_rows_direct(nout, nred_eff, (int)es, CX));
   // (bounds: see gemv_cols_direct_kernel)
-  const bool direct =
+  const bool cols_direct =
       !nt && (!reach || gs::direct_cols<E, CX>(nred_eff, nout * nred_eff * (long long)es, q.fold));
   GemvShape sh{};
   const auto shape = [&](bool uncut) {
-    if (direct) sh = gemv_direct_shape(nout, nred_eff, di.sms, uncut);
-    else if (!small) sh = gemv_shape(nt, nout, nred_eff, (int)es, CX, q.fold, phases, di.sms, uncut);
+    if (cols_direct) sh = gemv_cols_direct_shape(nout, nred_eff, di.sms, uncut);
+    else if (rows_direct) sh = gemv_rows_direct_shape(nout, nred_eff, (int)es, di.sms, uncut);
+    else sh = gemv_shape(nt, nout, nred_eff, (int)es, CX, q.fold, phases, di.sms, uncut);
   };
   shape(false);
   CutScratch cs{};
@@ -358,18 +394,11 @@ bool run_xgemv(const XGemvReq<E, CX>& q) {
   g.phases = phases;
   pipeline_fault(&g.stop_after, &g.wait_polls);
   GemvMaps maps{};
-  int grid = sh.grid;
-  if (small) {
-    // enough warps to fill the device, at least 64 elements to each
-    int S = 1;
-    while (S < 8 && nout * S < (long long)di.sms * 16 && nred_eff >= 128 * S) S *= 2;
-    g.groups = S;
-    grid = (int)((nout + 8 / S - 1) / (8 / S));
-  } else if (!direct && nred_eff > 0 && !gemv_maps(&maps, dA, (size_t)es, Rs, Cs, q.lda, phases, nt, sh.G)) {
+  const bool direct = rows_direct || cols_direct;
+  if (!direct && nred_eff > 0 && !gemv_maps(&maps, dA, (size_t)es, Rs, Cs, q.lda, phases, nt, sh.G))
     return false;
-  }
   count_launch();
-  if (!cuda_ok(o->gemv(g, small || direct ? nullptr : &maps, nt, grid, s), "gemv launch")) return false;
+  if (!cuda_ok(o->gemv(g, direct ? nullptr : &maps, nt, sh.grid, s), "gemv launch")) return false;
   if (y_host) {
     int* hs = w->hstatus();
     if (!cuda_ok(cudaMemcpyAsync(q.Y, dY, y_bytes, cudaMemcpyDeviceToHost, s), "copy y") ||

@@ -10,11 +10,20 @@ namespace xb {
 
 template <typename E, bool CX> struct Val { E r, i; };
 
-// Element `idx` of a real or complex (interleaved pair) array.
-template <typename E, bool CX>
+// Element `idx` of a real or complex (interleaved pair) array; PAIR: as one load, p being aligned to
+// pairs.
+template <typename E, bool CX, bool PAIR = false>
 __device__ __forceinline__ Val<E, CX> ldv(const E* p, long long idx) {
   Val<E, CX> v;
-  if constexpr (CX) {
+  if constexpr (CX && PAIR && sizeof(E) == 8) {
+    const double2 t = __ldg((const double2*)p + idx);
+    v.r = t.x;
+    v.i = t.y;
+  } else if constexpr (CX && PAIR) {
+    const float2 t = __ldg((const float2*)p + idx);
+    v.r = t.x;
+    v.i = t.y;
+  } else if constexpr (CX) {
     v.r = __ldg(p + 2 * idx);
     v.i = __ldg(p + 2 * idx + 1);
   } else {

@@ -495,8 +495,11 @@ struct Consumer {
 // begins inside (slot 2*cta) and that of the unit that begins in its range and goes on in the next
 // CTA's (slot 2*cta + 1), whatever the number of outputs. Structure of arrays: field i
 // (< NC*(2F+1): pri, car, flags per component) of slot s for the unit's output pp at
-// scratch[(i*2*grid + s)*P + pp]. A cut unit's tickets, one per warp, are those of the CTA it
-// begins in.
+// scratch[(i*2*grid + s)*P + pp]. A unit's parts are summed in groups of kGroup CTAs by the last of
+// each group to arrive, and the groups' sums, left in the records of their first CTAs, by the last of
+// those: with 64 rows of 400,000, which all 148 CTAs share, one CTA would read 148 parts (z: 1 MB).
+// Tickets, one per warp and kind: of the group that begins in a CTA (0, or 1 if the unit begins there
+// too) and of the groups of the unit that begins in it (2).
 //
 // A CTA's range of stages holds whole units in its middle and possibly cut units at its two
 // ends. Ends::close() ends the run of unit u in this CTA for the warp's outputs: the groups
@@ -508,6 +511,7 @@ struct Consumer {
 template <typename E, bool CX, int F>
 struct Ends {
   static constexpr int NC = CX ? 2 : 1, REC = 2 * F + 1;
+  static constexpr int kGroup = 12;
   const XGemvArgs<E>& g;
   int P, lgG, grp, pp, out;   // group of this lane, its output's offset in a unit, lanes per group
   long long nout;
@@ -553,9 +557,8 @@ struct Ends {
     bool last = false;
     if (lane < n) {
       const int b = (lane == 0 ? u0 : u1) * g.nb, first = sp.owner(b);
-      unsigned* t = g.tickets + first * (kConsumers / 32) + warp;
-      last = atomicAdd(t, 1u) == (unsigned)(sp.owner(b + g.nb - 1) - first);
-      if (last) *t = 0u;
+      const int j = ((int)blockIdx.x - first) / kGroup * kGroup, count = sp.owner(b + g.nb - 1) - first + 1;
+      last = take(first + j, j == 0 ? 1 : 0, warp, count - j < kGroup ? count - j : kGroup);
     }
     const unsigned mask = __ballot_sync(0xffffffffu, last);
     if (mask == 0) return;
@@ -565,27 +568,58 @@ struct Ends {
       if (!(mask & (1u << k))) continue;
       const int u = k == 0 ? u0 : u1, first = sp.owner(u * g.nb);
       const int count = sp.owner(u * g.nb + g.nb - 1) - first + 1;
+      const int j = ((int)blockIdx.x - first) / kGroup * kGroup;
       const long long o = (long long)u * P + pp;
-      E y[NC];
-      read_y(o, grp == 0 && o < nout, y);
-      Acc<E, F> a[NC];
+      // first the group's parts (CTAs i, i + 1, ...), then the groups' sums (i, i + kGroup, ...)
+      int i = first + j, parts = count - j < kGroup ? count - j : kGroup, step = 1;
+#pragma unroll 1
+      for (;;) {
+        Acc<E, F> a[NC];
 #pragma unroll
-      for (int c = 0; c < NC; c++) {
-        SumAcc<E, F> sum;
-        sum.zero();
-        if (o < nout) {
+        for (int c = 0; c < NC; c++) {
+          SumAcc<E, F> sum;
+          sum.zero();
+          if (o < nout) {
 #pragma unroll 2
-          for (int q = grp; q < count; q += 1 << lgG) {
-            Acc<E, F> part;
-            xb::read_rec<E, F>(part, g.scratch + slot(first + q, q == 0) + c * REC * fs, fs);
-            sum.add(part);
+            for (int q = grp; q < parts; q += 1 << lgG) {
+              Acc<E, F> part;
+              xb::read_rec<E, F>(part, g.scratch + slot(i + q * step, i + q == first) + c * REC * fs, fs);
+              sum.add(part);
+            }
           }
+          sum.get(a[c]);
         }
-        sum.get(a[c]);
+        lanes_merge<E, F, NC>(a, out);
+        const bool mine = grp == 0 && o < nout;
+        if (step > 1 || count <= kGroup) {
+          E y[NC];
+          read_y(o, mine, y);
+          if (mine) finish(o, a, y);
+          break;
+        }
+        if (mine) {
+          E* rec = g.scratch + slot(i, i == first);
+#pragma unroll
+          for (int c = 0; c < NC; c++) xb::put_rec<E, F>(a[c], rec + c * REC * fs, fs);
+        }
+        __threadfence();
+        __syncwarp();
+        i = first;
+        parts = (count + kGroup - 1) / kGroup;
+        step = kGroup;
+        bool all = false;
+        if (lane == 0) all = take(first, 2, warp, parts);
+        if (!__ballot_sync(0xffffffffu, all)) break;
+        __threadfence();
       }
-      lanes_merge<E, F, NC>(a, out);
-      if (grp == 0 && o < nout) finish(o, a, y);
     }
+  }
+  // ticket `kind` of CTA i: true for the last of n to arrive, which leaves it zero
+  __device__ __forceinline__ bool take(int i, int kind, int warp, int n) const {
+    unsigned* t = g.tickets + (3 * i + kind) * (kConsumers / 32) + warp;
+    const bool last = atomicAdd(t, 1u) == (unsigned)n - 1;
+    if (last) *t = 0u;
+    return last;
   }
 };
 
@@ -685,82 +719,147 @@ gemv_stream_kernel(const __grid_constant__ XGemvArgs<E> g, const __grid_constant
 }
 
 // ---------------------------------------------------------------------------------------
-// Rows kernel for small matrices: a CTA of 8 warps takes 8/S rows, S = g.groups warps to a row
-// (S = 1, 2, 4, 8), and reads A and x straight from global memory. No pipeline to fill and no
-// unit to merge across CTAs: 7-8 us a call where the streaming kernel takes 10-12.
+// Rows kernel straight from global memory, for small matrices and for few rows. A CTA of 8 warps
+// takes 8/S rows, S = g.groups warps to a row (S = 1, 2, 4, 8). No pipeline to fill and no unit to
+// merge across CTAs: 7-8 us a call where the streaming kernel takes 10-12. Few long rows are cut
+// between gridDim.y CTAs each (S = 8): every CTA leaves a partial state, record `part` of the row,
+// and the last one to arrive (ticket) sums them. Field i of the record is at
+// scratch[(i*R + row)*parts + part].
 // ---------------------------------------------------------------------------------------
+// Sum of the states of the S warps of a row (each the same in all its lanes), into the first of
+// them. All threads of the CTA call it.
+template <typename E, int F, int NC>
+__device__ __forceinline__ void sum_warps(Acc<E, F> (&a)[NC], E (*sm)[NC * (2 * F + 1)], int S) {
+  constexpr int REC = 2 * F + 1;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  if (lane == 0) {
+#pragma unroll
+    for (int c = 0; c < NC; c++) xb::put_rec<E, F>(a[c], &sm[warp][c * REC], 1);
+  }
+  __syncthreads();
+  if ((warp & (S - 1)) == 0 && lane == 0) {
+#pragma unroll
+    for (int c = 0; c < NC; c++) {
+      SumAcc<E, F> sum;
+      sum.zero();
+      sum.add(a[c]);
+#pragma unroll 1
+      for (int q = 1; q < S; q++) {
+        Acc<E, F> o;
+        o.zero();
+#pragma unroll
+        for (int i = 0; i < F; i++) {
+          o.pri[i] = sm[warp + q][c * REC + i];
+          o.car[i] = sm[warp + q][c * REC + F + i];
+        }
+        o.flags = xb::flags_from<E>(sm[warp + q][c * REC + 2 * F]);
+        o.set_idx_from_pri();
+        sum.add(o);
+      }
+      sum.get(a[c]);
+    }
+  }
+}
+
+// CTAs per SM it is built for: as many as hold its accumulators without spilling much (FP64 500x6291:
+// 14.4 us with four against 18.5 with three).
+template <typename E, bool CX>
+constexpr int rows_direct_ctas(int fold) {
+  if (sizeof(E) == 8) return CX ? (fold <= 2 ? 3 : 2) : fold <= 4 ? 4 : fold <= 6 ? 3 : 2;
+  return CX ? (fold <= 3 ? 4 : fold <= 5 ? 3 : 2) : 4;
+}
+
 template <typename E, bool CX, int F>
-__global__ void __launch_bounds__(256) gemv_rows_small_kernel(const __grid_constant__ XGemvArgs<E> g) {
+__global__ void __launch_bounds__(256, (rows_direct_ctas<E, CX>(F))) gemv_rows_direct_kernel(const __grid_constant__ XGemvArgs<E> g) {
   constexpr int NC = CX ? 2 : 1, D = CX ? 2 : 1, REC = 2 * F + 1;
-  constexpr int K = CX ? 4 : 8;   // elements per lane and step
+  constexpr int K = 4;   // elements per lane and step
   __shared__ E sm[8][NC * REC];
+  __shared__ unsigned s_last;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, S = g.groups;
-  const int part = warp & (S - 1), rows = 8 / S;
+  const int rows = 8 / S, parts = gridDim.y;
   const long long r = (long long)blockIdx.x * rows + warp / S;
+  // this CTA's columns of the row: whole steps of the S warps
+  const long long stride = (long long)K * 32 * S;
+  const long long per = ((g.C + parts - 1) / parts + stride - 1) / stride * stride;
+  const long long c0 = blockIdx.y * per, c1 = c0 + per < g.C ? c0 + per : g.C;
   Acc<E, F> a[NC];
 #pragma unroll
   for (int c = 0; c < NC; c++) a[c].zero();
   if (r < g.R) {
     const E* row = g.A + r * g.lda * NC;
-#pragma unroll 1
-    for (long long b = part * 32 + lane; b < g.C; b += (long long)K * 32 * S) {
+    // K elements from b (which exists) on, 32*S apart; WHOLE: all of them exist; PAIR: whole pairs are
+    // loaded. All loads before the math and without branches: an absent element loads element b
+    auto step = [&](long long b, auto whole, auto pair) {
+      constexpr bool WHOLE = decltype(whole)::value != 0, PAIR = decltype(pair)::value != 0;
       Val<E, CX> av[K], xv[K];
-      int n = 0;   // elements that exist; all loads before the math
 #pragma unroll
       for (int k = 0; k < K; k++) {
-        const long long e = b + (long long)k * 32 * S;
-        av[k] = Val<E, CX>{E(0), E(0)};
-        xv[k] = Val<E, CX>{E(0), E(0)};
-        if (e < g.C) {
-          av[k] = xb::ldv<E, CX>(row, e);
-          xv[k] = xb::ldv<E, CX>(g.x, e * g.incx);
-          n = k + 1;
-        }
+        long long e = b + (long long)k * 32 * S;
+        if (!WHOLE) e = e < c1 ? e : b;
+        av[k] = xb::ldv<E, CX, PAIR>(row, e);
+        xv[k] = xb::ldv<E, CX, PAIR>(g.x, e * g.incx);
+      }
+      int n = K;   // elements that exist
+      if (!WHOLE) {
+#pragma unroll
+        for (int k = 1; k < K; k++)
+          if (b + (long long)k * 32 * S >= c1) {
+            av[k] = xv[k] = Val<E, CX>{E(0), E(0)};
+            n = n < k ? n : k;
+          }
       }
       E v[NC][K * D];
 #pragma unroll
       for (int k = 0; k < K; k++) {
-        if (!g.alpha_one && k < n) xv[k] = xb::scale<E, CX>(xv[k], g.ar, g.ai);
+        if (!g.alpha_one && (WHOLE || k < n)) xv[k] = xb::scale<E, CX>(xv[k], g.ar, g.ai);
         if (CX && g.conj) av[k].i = -av[k].i;
         xb::products<E, CX, K * D>(av[k], xv[k], v, k);
       }
 #pragma unroll
       for (int c = 0; c < NC; c++) a[c].template tile<K * D>(v[c], n * D);
-    }
+    };
+    auto steps = [&](auto pair) {
+      long long w = c0 + (warp & (S - 1)) * 32;   // the warp's first element: it takes one of the two together
+#pragma unroll 1
+      for (; w + (long long)(K - 1) * 32 * S + 31 < c1; w += stride) step(w + lane, gt::Const<1>{}, pair);
+      if (w + lane < c1) step(w + lane, gt::Const<0>{}, pair);
+    };
+    if (CX && ((uintptr_t)g.A | (uintptr_t)g.x) % (2 * sizeof(E)) == 0) steps(gt::Const<1>{});
+    else steps(gt::Const<0>{});
   }
 #pragma unroll
   for (int c = 0; c < NC; c++) a[c].renorm();
   warp_merge_all<E, F, NC>(a);
-  if (S > 1) {
-    if (lane == 0) {
+  if (S > 1) sum_warps<E, F, NC>(a, sm, S);
+  if (parts > 1) {   // S = 8: one row per CTA
+    const long long fs = g.R * parts;
+    if (threadIdx.x == 0) {
+      E* rec = g.scratch + r * parts + blockIdx.y;
 #pragma unroll
-      for (int c = 0; c < NC; c++) xb::put_rec<E, F>(a[c], &sm[warp][c * REC], 1);
+      for (int c = 0; c < NC; c++) xb::put_rec<E, F>(a[c], rec + c * REC * fs, fs);
+      __threadfence();
+      s_last = atomicAdd(g.tickets + blockIdx.x, 1u) == (unsigned)parts - 1 ? 1u : 0u;
+      if (s_last) g.tickets[blockIdx.x] = 0u;
     }
     __syncthreads();
-    if (part == 0 && lane == 0) {
+    if (!s_last) return;
+    __threadfence();
 #pragma unroll
-      for (int c = 0; c < NC; c++) {
-        SumAcc<E, F> sum;
-        sum.zero();
-        sum.add(a[c]);
+    for (int c = 0; c < NC; c++) {
+      SumAcc<E, F> sum;
+      sum.zero();
 #pragma unroll 1
-        for (int q = 1; q < S; q++) {
-          Acc<E, F> o;
-          o.zero();
-#pragma unroll
-          for (int i = 0; i < F; i++) {
-            o.pri[i] = sm[warp + q][c * REC + i];
-            o.car[i] = sm[warp + q][c * REC + F + i];
-          }
-          o.flags = xb::flags_from<E>(sm[warp + q][c * REC + 2 * F]);
-          o.set_idx_from_pri();
-          sum.add(o);
-        }
-        sum.get(a[c]);
+      for (int q = threadIdx.x; q < parts; q += 256) {
+        Acc<E, F> o;
+        xb::read_rec<E, F>(o, g.scratch + r * parts + q + c * REC * fs, fs);
+        sum.add(o);
       }
+      sum.get(a[c]);
     }
+    warp_merge_all<E, F, NC>(a);
+    sum_warps<E, F, NC>(a, sm, S);
   }
-  if (part == 0 && lane == 0 && r < g.R)
+  if ((warp & (S - 1)) == 0 && lane == 0 && r < g.R)
     xb::finish<E, CX, F>(a, g.mode, g.y + r * g.incy * NC, g.br, g.bi, g.ybin + r * g.incy * 2 * F * NC);
 }
 
@@ -911,7 +1010,7 @@ template <typename E, bool CX, int F>
 cudaError_t launch_gemv(const XGemvArgs<E>& g, const GemvMaps* maps, bool rows, int grid, cudaStream_t s) {
   if (!maps) {
     if (rows) {
-      gemv_rows_small_kernel<E, CX, F><<<grid, 256, 0, s>>>(g);
+      gemv_rows_direct_kernel<E, CX, F><<<dim3(grid, g.parts), 256, 0, s>>>(g);
     } else {
       gemv_cols_direct_kernel<E, CX, F><<<dim3(grid, g.parts), 256, 0, s>>>(g);
     }

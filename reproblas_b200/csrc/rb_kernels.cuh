@@ -168,7 +168,7 @@ struct GemvMaps {
 
 template <typename E>
 struct XOps {
-  // maps == nullptr: the rows kernel for small matrices (g.groups warps to a row)
+  // maps == nullptr: the direct kernels (g.groups, g.parts: their split of a reduction)
   cudaError_t (*gemv)(const XGemvArgs<E>& g, const GemvMaps* maps, bool rows, int grid, cudaStream_t s);
   // decomposition of an M x N x K product (whole_tiles: no tile is cut between CTAs)
   cudaError_t (*gemm_plan)(long long M, long long N, long long K, int sms, bool whole_tiles,

@@ -384,6 +384,33 @@ def test_gemv_large_complex_columns(cuda, rb, port, fold, ta):
 
 
 @pytest.mark.parametrize("t", list("dszc"))
+@pytest.mark.parametrize("fold", [2, 3, 8])
+def test_gemv_few_long_rows(cuda, rb, port, t, fold):
+    # rows cut between CTAs: around the first cut (seven steps of 8 warps), ragged last parts, both
+    # sides of the limits of 24 and 48 rows, every alignment, strided x, units that all CTAs share
+    # (their parts summed in two stages), and raises and non-finite values in a late part
+    step = 1024
+    for i, (M, N) in enumerate([(1, 7 * step - 1), (1, 7 * step), (2, 8 * step + 1), (3, 100003), (24, 9001), (25, 9003),
+                                (48, 70001), (49, 70003), (64, 90001), (1, 600011)]):
+        gemv_both(cuda, rb, port, t, fold, "n", M, N, N + (i & 3), i & 3, 1 + (i & 1), i)
+    M, N = 2, 200000
+    al, be = scalars(t)
+    A = ops(t, M * N, 5).reshape(M, N)
+    A[0, N - 5] = 2.0 ** (600 if t in "dz" else 90)
+    A[1, 150000], A[1, 7] = np.inf, 2.0 ** (1000 if t in "dz" else 120)
+    x, y = ops(t, N, 6), ops(t, M, 7)
+    want = y.copy()
+    yd = dev(cuda, y)
+    if t == "d":
+        port.rdgemv(fold, b"r", b"n", M, N, al, ptr(A), N, ptr(x), 1, be, ptr(want), 1)
+        rb.call("reproBLAS_rdgemv", fold, "r", "n", M, N, al, dev(cuda, A.ravel()), N, dev(cuda, x), 1, be, yd, 1)
+    else:
+        lib_gemv(port, t, fold, "r", "n", M, N, al, A, N, x, 1, be, want, 1)
+        rb_gemv(rb, t, fold, "r", "n", M, N, al, dev(cuda, A.ravel()), N, dev(cuda, x), 1, be, yd, 1)
+    assert same_value(yd.cpu().numpy(), want.view(REAL[t]))
+
+
+@pytest.mark.parametrize("t", list("dszc"))
 @pytest.mark.parametrize("ta", ["n", "t"])
 def test_gemv_few_rows_and_limits(cuda, rb, port, t, ta):
     es = {"d": 8, "s": 4, "z": 16, "c": 8}[t]
