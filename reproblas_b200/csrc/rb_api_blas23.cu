@@ -239,8 +239,11 @@ GemvShape gemv_cols_direct_shape(long long nout, long long nred, int sms, bool u
 // 8192x1000 23.0 / 16.5, FP64 complex 8000x131 22.6 / 14.4, but 5000x209 18.5 / 24.7. And few rows of any length, which fill
 // a band of the streaming kernel (64 rows or more) badly: FP64 1x3000000 18.5 / 156, 8x8000000 121 / 391,
 // 48x400000 47.5 / 51.8, FP32 16x500000 26.7 / 28.8 but 32x500000 39.0 / 35.4, FP64 complex 16x500000
-// 58.7 / 94.8 but 32x500000 111 / 107, FP32 complex 48x400000 79.8 / 89.2.
-bool gemv_rows_direct(long long nout, long long nred, int es, bool cx) {
+// 58.7 / 94.8 but 32x500000 111 / 107, FP32 complex 48x400000 79.8 / 89.2. And FP64 complex rows from fold 7
+// on, whose accumulators spill in the streaming kernel: fold 7 8192^2 528 / 707, 20000x500 140 / 141, fold
+// 8 8192^2 591 / 768, 300x100000 363 / 403, but fold 8 100000x100 467 / 191.
+bool gemv_rows_direct(long long nout, long long nred, int es, bool cx, int fold) {
+  if (es == 16 && fold > 6 && nred >= 500) return true;
   const long long bytes = nout * nred * es;
   if (nout > 6144) return nout <= 8192 && bytes <= 8ll << 20;
   return nout <= (es == 8 ? 48 : 24) || bytes <= (es == 8 && !cx ? 48ll << 20 : 32ll << 20);
@@ -342,7 +345,7 @@ bool run_xgemv(const XGemvReq<E, CX>& q) {
   while (((size_t)phases * q.lda * es) % 16 != 0) phases *= 2;
   if (phases == 1 && a_mis != 0) phases = 2;
   const bool reach = gemv_in_reach(Rs, Cs, (int)es, phases);
-  const bool rows_direct = nt && (!reach || gemv_rows_direct(nout, nred_eff, (int)es, CX));
+  const bool rows_direct = nt && (!reach || gemv_rows_direct(nout, nred_eff, (int)es, CX, q.fold));
   // (bounds: see gemv_cols_direct_kernel)
   const bool cols_direct =
       !nt && (!reach || gs::direct_cols<E, CX>(nred_eff, nout * nred_eff * (long long)es, q.fold));

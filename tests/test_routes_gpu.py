@@ -410,6 +410,13 @@ def test_gemv_few_long_rows(cuda, rb, port, t, fold):
     assert same_value(yd.cpu().numpy(), want.view(REAL[t]))
 
 
+@pytest.mark.parametrize("fold", [6, 7, 8])
+def test_gemv_complex_rows_of_high_folds(cuda, rb, port, fold):
+    # FP64 complex rows from fold 7 on take the direct kernel from 500 elements a row
+    for i, (M, N) in enumerate([(6200, 499), (6200, 500), (700, 5003)]):
+        gemv_both(cuda, rb, port, "z", fold, "n", M, N, N + i, i & 1, 1, fold)
+
+
 @pytest.mark.parametrize("t", list("dszc"))
 @pytest.mark.parametrize("ta", ["n", "t"])
 def test_gemv_few_rows_and_limits(cuda, rb, port, t, ta):
