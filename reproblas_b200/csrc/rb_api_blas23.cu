@@ -348,7 +348,7 @@ bool run_xgemv(const XGemvReq<E, CX>& q) {
   const bool rows_direct = nt && (!reach || gemv_rows_direct(nout, nred_eff, (int)es, CX, q.fold));
   // (bounds: see gemv_cols_direct_kernel)
   const bool cols_direct =
-      !nt && (!reach || gs::direct_cols<E, CX>(nred_eff, nout * nred_eff * (long long)es, q.fold));
+      !nt && (!reach || gs::direct_cols<E, CX>(nout, nred_eff, q.fold));
   GemvShape sh{};
   const auto shape = [&](bool uncut) {
     if (cols_direct) sh = gemv_cols_direct_shape(nout, nred_eff, di.sms, uncut);

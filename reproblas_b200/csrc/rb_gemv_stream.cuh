@@ -872,6 +872,11 @@ __global__ void __launch_bounds__(256, (rows_direct_ctas<E, CX>(F))) gemv_rows_d
 // 35.0 / 37.7, 20000x500 66.0 / 68.9, but 4096^2 91.0 / 85.0 and 8192^2 307 / 270; fold 6: 2048^2
 // 48.6 / 58.4, 5000^2 210 / 202), or of any size from fold 7, whose two accumulators spill in
 // the streaming kernel (fold 8, 5000^2: 254 / 329).
+// Short reductions of many columns come here too: a unit of the streaming kernel is 128/es*G rows deep,
+// whatever the number of rows, and its ends cost as much as a stage (FP64 8x4000000 109 / 270, 100x500000
+// 96 / 115, but 160x200000 72 / 55; FP32 8x4000000 106 / 304, 40x2000000 141 / 156, but 64x1000000 106 / 84;
+// FP64 complex 8x4000000 273 / 1004, 300x100000 148 / 168, but 500x40000 117 / 105; FP32 complex 8x4000000
+// 189 / 488, 128x300000 115 / 125, but 160x200000 107 / 95; and fewer columns: FP64 100x50000 24.6 / 20.6).
 // A CTA of 256 threads is G = g.groups row groups of 256/G threads, one column each; grid =
 // (column blocks, row chunks), inside a chunk group q takes rows q, q + G, ..., four per step.
 // fl(alpha*x) of 256 rows at a time is formed in shared memory. The groups' states merge
@@ -881,19 +886,22 @@ __global__ void __launch_bounds__(256, (rows_direct_ctas<E, CX>(F))) gemv_rows_d
 template <typename E, bool CX>
 __host__ __device__ constexpr bool stream_cols(int fold) { return !(CX && sizeof(E) == 8 && fold > 6); }
 template <typename E, bool CX>
-constexpr bool direct_cols(long long nred, long long bytes, int fold) {
+constexpr bool direct_cols(long long nout, long long nred, int fold) {
+  constexpr int es = (CX ? 2 : 1) * (int)sizeof(E);
   if (!stream_cols<E, CX>(fold)) return true;
-  return CX && sizeof(E) == 8 ? bytes <= (192ll << 20) : nred >= 256 && bytes <= (16ll << 20);
+  if (nout >= 80000 && nred <= (es == 16 ? 384 : es == 4 ? 48 : 128)) return true;
+  return es == 16 ? nout * nred * es <= (192ll << 20) : nred >= 256 && nout * nred * es <= (16ll << 20);
 }
 
 // Sum of the G row groups' states (renormalised) through sm[i * 256 + thread]: group 0 ends with
 // the merged state. All 256 threads call it.
 template <typename E, int F>
 __device__ __forceinline__ void sum_groups(Acc<E, F>& a, E* sm, int grp, int t, int G, int T) {
+  if (G == 1) return;
   __syncthreads();
   if (grp > 0) xb::put_rec<E, F>(a, sm + threadIdx.x, 256);
   __syncthreads();
-  if (grp == 0 && G > 1) {
+  if (grp == 0) {
     SumAcc<E, F> sum;
     sum.zero();
     sum.add(a);
@@ -915,8 +923,13 @@ __device__ __forceinline__ void sum_groups(Acc<E, F>& a, E* sm, int grp, int t, 
   }
 }
 
+template <typename E, bool CX>
+constexpr int cols_direct_ctas(int fold) {
+  return CX ? (sizeof(E) == 4 && fold <= 3 ? 3 : 2) : fold <= 4 ? 4 : fold <= 6 || sizeof(E) == 4 ? 3 : 2;
+}
+
 template <typename E, bool CX, int F>
-__global__ void __launch_bounds__(256, 2) gemv_cols_direct_kernel(const __grid_constant__ XGemvArgs<E> g) {
+__global__ void __launch_bounds__(256, (cols_direct_ctas<E, CX>(F))) gemv_cols_direct_kernel(const __grid_constant__ XGemvArgs<E> g) {
   constexpr int NC = CX ? 2 : 1, D = CX ? 2 : 1, K = 4, REC = 2 * F + 1;
   __shared__ E sm[REC * 256];
   __shared__ E xs[256 * NC];
@@ -944,30 +957,47 @@ __global__ void __launch_bounds__(256, 2) gemv_cols_direct_kernel(const __grid_c
     }
     __syncthreads();
     if (col >= g.C) continue;
-#pragma unroll 1
-    for (int b = grp; b < n; b += K * G) {
+    // K rows from b (which exists) on, G apart; WHOLE: all of them exist; PAIR: whole pairs are loaded.
+    // All loads before the math and without branches: an absent row loads row b
+    auto step = [&](int b, auto whole, auto pair) {
+      constexpr bool WHOLE = decltype(whole)::value != 0, PAIR = decltype(pair)::value != 0;
       Val<E, CX> av[K];
-      int m = 0;   // rows that exist; all loads before the math
 #pragma unroll
       for (int k = 0; k < K; k++) {
-        av[k] = Val<E, CX>{E(0), E(0)};
-        if (b + k * G < n) {
-          av[k] = xb::ldv<E, CX>(A + (base + b + k * G) * g.lda * NC, 0);
-          m = k + 1;
-        }
+        const int i = WHOLE || b + k * G < n ? b + k * G : b;
+        av[k] = xb::ldv<E, CX, PAIR>(A + (base + i) * g.lda * NC, 0);
       }
+      int m = K;   // rows that exist; the others multiply zeros
       E v[NC][K * D];
 #pragma unroll
       for (int k = 0; k < K; k++) {
-        const int i = b + k * G < n ? b + k * G : b;   // absent rows multiply zeros
-        Val<E, CX> xv{xs[i * NC], CX ? xs[i * NC + NC - 1] : E(0)};
+        Val<E, CX> xv{E(0), E(0)};
+        if (WHOLE || b + k * G < n) {
+          const int i = b + k * G;
+          xv = Val<E, CX>{xs[i * NC], CX ? xs[i * NC + NC - 1] : E(0)};
+        } else {
+          av[k] = Val<E, CX>{E(0), E(0)};
+          m = m < k ? m : k;
+        }
         if (CX && g.conj) av[k].i = -av[k].i;
-        if (k >= m) xv = Val<E, CX>{E(0), E(0)};
         xb::products<E, CX, K * D>(av[k], xv, v, k);
       }
       if constexpr (CX) tile2<E, F, K * D>(a[0], v[0], a[1], v[1]);
       else a[0].template tile<K * D>(v[0], m * D);
-    }
+    };
+    auto steps = [&](auto pair) {
+      int b = grp;
+      if constexpr (CX && sizeof(E) == 8 && F > 4) {   // whole steps of their own would spill
+#pragma unroll 1
+        for (; b < n; b += K * G) step(b, gt::Const<0>{}, pair);
+      } else {
+#pragma unroll 1
+        for (; b + (K - 1) * G < n; b += K * G) step(b, gt::Const<1>{}, pair);
+        if (b < n) step(b, gt::Const<0>{}, pair);
+      }
+    };
+    if (CX && (uintptr_t)g.A % (2 * sizeof(E)) == 0) steps(gt::Const<1>{});
+    else steps(gt::Const<0>{});
   }
   E* part = g.scratch + (long long)chunk * NC * REC * g.C + col;   // field i at part[i * C]
 #pragma unroll

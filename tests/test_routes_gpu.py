@@ -418,6 +418,15 @@ def test_gemv_complex_rows_of_high_folds(cuda, rb, port, fold):
 
 
 @pytest.mark.parametrize("t", list("dszc"))
+@pytest.mark.parametrize("fold", [2, 3, 6])
+def test_gemv_short_columns(cuda, rb, port, t, fold):
+    # many columns of few rows: both sides of the limits on each, whole and partial steps of four rows
+    most = {"d": 128, "s": 48, "z": 384, "c": 128}[t]
+    for i, (M, N) in enumerate([(1, 80001), (3, 80000), (5, 79999), (8, 100003), (most, 80000), (most + 1, 80001)]):
+        gemv_both(cuda, rb, port, t, fold, "t", M, N, N + (i & 3), i & 3, 1 + (i & 1), i)
+
+
+@pytest.mark.parametrize("t", list("dszc"))
 @pytest.mark.parametrize("ta", ["n", "t"])
 def test_gemv_few_rows_and_limits(cuda, rb, port, t, ta):
     es = {"d": 8, "s": 4, "z": 16, "c": 8}[t]
