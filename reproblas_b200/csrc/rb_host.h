@@ -87,7 +87,7 @@ struct Workspace {
   bool ensure_ring(size_t chunk);
   bool ensure_big(size_t bytes);
   bool ensure_tickets(size_t n);
-  bool zero_now(void* p, size_t bytes);   // device memory zeroed before it returns, whatever stream uses it
+  cudaError_t zero_now(void* p, size_t bytes);   // zeroed when it returns, whatever stream uses p
   // after a kernel gave up on a wait: status word, tickets and counters back to zero
   bool reset_after_abort();
   void release();   // frees everything held (a workspace whose set-up failed)

@@ -159,23 +159,24 @@ bool Workspace::ensure_big(size_t bytes) {
 
 // Not cudaMemset: that runs on the legacy default stream, behind whatever is queued there, and a
 // non-blocking stream does not wait for it.
-bool Workspace::zero_now(void* p, size_t bytes) {
-  return cuda_ok(cudaMemsetAsync(p, 0, bytes, copy_stream), "cudaMemsetAsync") &&
-         cuda_ok(cudaStreamSynchronize(copy_stream), "cudaStreamSynchronize");
+cudaError_t Workspace::zero_now(void* p, size_t bytes) {
+  const cudaError_t e = cudaMemsetAsync(p, 0, bytes, copy_stream);
+  return e == cudaSuccess ? cudaStreamSynchronize(copy_stream) : e;
 }
 
+// Leaves the thread's error as it is: the caller has a form that needs no tickets.
 bool Workspace::ensure_tickets(size_t n) {
   if (n <= ntickets) return true;
   // drain the stream first: kernels in flight may still use the old ticket array
-  if (!cuda_ok(cudaStreamSynchronize(stream), "cudaStreamSynchronize")) return false;
+  if (cudaStreamSynchronize(stream) != cudaSuccess) return false;
   if (tickets) { cudaFree(tickets); tickets = nullptr; ntickets = 0; }
   size_t want = n < 65536 ? 65536 : n;
   if (dev_malloc((void**)&tickets, want * sizeof(unsigned)) != cudaSuccess) {
+    cudaGetLastError();
     tickets = nullptr;
-    set_error(RB_ERR_ALLOC, "ticket allocation failed");
     return false;
   }
-  if (!zero_now(tickets, want * sizeof(unsigned))) {
+  if (zero_now(tickets, want * sizeof(unsigned)) != cudaSuccess) {
     cudaFree(tickets);
     tickets = nullptr;
     return false;
@@ -272,8 +273,7 @@ GraphScratch* take_block(Workspace* w, size_t bytes, size_t zeroed) {
     }
     b = new GraphScratch{mem, bytes, w->device, nullptr};
   }
-  if (cudaMemsetAsync(b->mem, 0, zeroed, w->copy_stream) != cudaSuccess ||
-      cudaStreamSynchronize(w->copy_stream) != cudaSuccess) {
+  if (w->zero_now(b->mem, zeroed) != cudaSuccess) {
     cudaGetLastError();
     graph_scratch_idle(b);
     return nullptr;
@@ -323,11 +323,7 @@ bool cut_scratch(Workspace* w, size_t bytes, size_t tickets, CutScratch* out) {
     }
     w->parts_bytes = bytes;
   }
-  if (tickets > w->ntickets && !w->ensure_tickets(tickets)) {
-    cudaGetLastError();
-    rb_clear_error();   // uncut forms need none
-    return false;
-  }
+  if (!w->ensure_tickets(tickets)) return false;
   out->parts = w->parts;
   out->tickets = w->tickets;
   return true;
@@ -375,7 +371,8 @@ static bool init_workspace(Workspace* w, int dev, cudaStream_t s, int sms) {
   }
   if (!cuda_ok(cudaStreamCreateWithFlags(&w->copy_stream, cudaStreamNonBlocking),
                "cudaStreamCreate") ||
-      !w->zero_now(w->scratch.ticket, 256) || !w->zero_now(w->dsmall, Workspace::kSmallBytes))
+      !cuda_ok(w->zero_now(w->scratch.ticket, 256), "clear workspace") ||
+      !cuda_ok(w->zero_now(w->dsmall, Workspace::kSmallBytes), "clear workspace"))
     return false;
   if (host_malloc((void**)&w->hsmall, Workspace::kSmallBytes) != cudaSuccess) {
     w->hsmall = nullptr;

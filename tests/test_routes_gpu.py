@@ -120,6 +120,33 @@ def test_gemv_without_scratch(cuda, rb, port, t, ta):
         rb.lib.rb_set_stream(None)
 
 
+def test_error_of_an_earlier_call_is_kept(cuda, rb):
+    # calls that do without scratch they could not have leave the thread's unread error alone
+    Ad, xd, yd = (cuda.ones(n, dtype=cuda.float64, device="cuda") for n in (3000 * 1500, 3000, 3000))
+    stream = cuda.cuda.Stream(priority=-1)
+    cuda.cuda.synchronize()
+    rb.lib.rb_set_stream(stream.cuda_stream)
+    try:
+        rb.call("reproBLAS_rdsum", 3, 16, Ad, 1)
+        rb.lib.reproBLAS_rdsum(1, 16, Ad.data_ptr(), 1)   # fold 1: refused
+        code, text = rb.lib.rb_get_last_error(), rb.lib.rb_get_last_error_message()
+        assert code != 0
+        for fails in (1, 2):
+            rb.lib.rb_debug_fail_allocations(fails)
+            rb.lib.reproBLAS_rdgemv(3, b"r", b"t", 3000, 1500, 1.5, Ad.data_ptr(), 1500, xd.data_ptr(), 1, 0.0,
+                                    yd.data_ptr(), 1)
+            rb.lib.rb_debug_fail_allocations(fails)
+            rb.lib.reproBLAS_rdgemm(3, b"r", b"n", b"n", 33, 17, 4001, 1.5, Ad.data_ptr(), 4001, Ad.data_ptr(), 17,
+                                    0.0, yd.data_ptr(), 17)
+            assert (rb.lib.rb_get_last_error(), rb.lib.rb_get_last_error_message()) == (code, text)
+        stream.synchronize()
+        assert bool((yd[:33 * 17] == 1.5 * 4001).all())
+    finally:
+        rb.lib.rb_debug_fail_allocations(0)
+        rb.lib.rb_clear_error()
+        rb.lib.rb_set_stream(None)
+
+
 @pytest.mark.parametrize("t, ta, M, N", [("d", "n", 20_000_000, 4), ("z", "n", 4_000_000, 8), ("s", "t", 16, 8_000_000),
                                          ("c", "n", 400_003, 100), ("z", "t", 300, 200_000)])
 def test_gemv_scratch_does_not_grow_with_the_outputs(cuda, rb, t, ta, M, N):
