@@ -152,7 +152,7 @@ GemvShape gemv_shape(bool rows, long long nout, long long nred, int es, bool cx,
     s.G = G;
     const long long P = 512 / G, SC = (long long)(128 / es) * G;
     s.nunits = (nout + P - 1) / P;
-    s.nb = nred > 0 ? (nred + SC - 1) / SC : 1;
+    s.nb = (nred + SC - 1) / SC;
     const long long T = s.nunits * s.nb;
     for (int way = uncut ? 1 : 0; way < 2; way++) {
       double ends;
@@ -344,7 +344,8 @@ bool run_xgemv(const XGemvReq<E, CX>& q) {
   int phases = 1;
   while (((size_t)phases * q.lda * es) % 16 != 0) phases *= 2;
   if (phases == 1 && a_mis != 0) phases = 2;
-  const bool reach = gemv_in_reach(Rs, Cs, (int)es, phases);
+  // the streaming kernels want a reduction, and tensor maps that hold it
+  const bool reach = nred_eff > 0 && gemv_in_reach(Rs, Cs, (int)es, phases);
   const bool rows_direct = nt && (!reach || gemv_rows_direct(nout, nred_eff, (int)es, CX, q.fold));
   // (bounds: see gemv_cols_direct_kernel)
   const bool cols_direct =
@@ -398,7 +399,7 @@ bool run_xgemv(const XGemvReq<E, CX>& q) {
   pipeline_fault(&g.stop_after, &g.wait_polls);
   GemvMaps maps{};
   const bool direct = rows_direct || cols_direct;
-  if (!direct && nred_eff > 0 && !gemv_maps(&maps, dA, (size_t)es, Rs, Cs, q.lda, phases, nt, sh.G))
+  if (!direct && !gemv_maps(&maps, dA, (size_t)es, Rs, Cs, q.lda, phases, nt, sh.G))
     return false;
   count_launch();
   if (!cuda_ok(o->gemv(g, direct ? nullptr : &maps, nt, sh.grid, s), "gemv launch")) return false;

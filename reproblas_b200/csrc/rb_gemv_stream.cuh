@@ -163,7 +163,7 @@ __device__ __forceinline__ void copy_stages(const XGemvArgs<E>& g, const Geom<E,
                                             const GemvMaps& maps, const Split& sp, unsigned char* ring,
                                             Sync& sy) {
   using Gm = Geom<E, CX, ROWS>;
-  const int nph = m.nred > 0 ? 1 << m.lgN : 0;   // no reduction: nothing to copy
+  const int nph = 1 << m.lgN;
   const int boxes = ROWS && nph == 1 ? m.G : nph;
   const uint32_t box_bytes = ROWS && nph == 1 ? (uint32_t)m.P * kThreadBytes : m.phase_bytes;
   Ring r;

@@ -445,6 +445,26 @@ def test_gemv_complex_rows_of_high_folds(cuda, rb, port, fold):
 
 
 @pytest.mark.parametrize("t", list("dszc"))
+@pytest.mark.parametrize("ta", ["n", "t"])
+def test_gemv_without_products(cuda, rb, port, t, ta):
+    # alpha 0 deposits nothing, whatever A and x hold: y is beta*y
+    for M, N in [(9001, 70), (70, 9001), (300, 300), (3000, 3001)]:
+        A, y = ops(t, M * N, 1), ops(t, M if ta == "n" else N, 2)
+        A[3] = np.nan
+        x = np.full(max(M, N), np.inf, FULL[t])
+        be, want = scalars(t)[1], y.copy()
+        al = 0.0 if t in "ds" else 0j
+        yd = dev(cuda, y)
+        if t == "d":
+            port.rdgemv(3, b"r", ta.encode(), M, N, al, ptr(A), N, ptr(x), 1, be, ptr(want), 1)
+            rb.call("reproBLAS_rdgemv", 3, "r", ta, M, N, al, dev(cuda, A), N, dev(cuda, x), 1, be, yd, 1)
+        else:
+            lib_gemv(port, t, 3, "r", ta, M, N, al, A, N, x, 1, be, want, 1)
+            rb_gemv(rb, t, 3, "r", ta, M, N, al, dev(cuda, A), N, dev(cuda, x), 1, be, yd, 1)
+        assert same_bits(yd.cpu().numpy(), want.view(REAL[t])), (M, N)
+
+
+@pytest.mark.parametrize("t", list("dszc"))
 @pytest.mark.parametrize("fold", [2, 3, 6])
 def test_gemv_short_columns(cuda, rb, port, t, fold):
     # many columns of few rows: both sides of the limits on each, whole and partial steps of four rows
