@@ -345,11 +345,13 @@ bool run_xgemv(const XGemvReq<E, CX>& q) {
   while (((size_t)phases * q.lda * es) % 16 != 0) phases *= 2;
   if (phases == 1 && a_mis != 0) phases = 2;
   // the streaming kernels want a reduction, and tensor maps that hold it
-  const bool reach = nred_eff > 0 && gemv_in_reach(Rs, Cs, (int)es, phases);
+  bool streams = false;
+  if (!cuda_ok(o->gemv_streams(nt, &streams), "gemv kernel attributes")) return false;
+  const bool reach = streams && nred_eff > 0 && gemv_in_reach(Rs, Cs, (int)es, phases);
   const bool rows_direct = nt && (!reach || gemv_rows_direct(nout, nred_eff, (int)es, CX, q.fold));
   // (bounds: see gemv_cols_direct_kernel)
   const bool cols_direct =
-      !nt && (!reach || gs::direct_cols<E, CX>(nout, nred_eff, q.fold));
+      !nt && (!reach || gs::direct_cols<E, CX>(nout, nred_eff));
   GemvShape sh{};
   const auto shape = [&](bool uncut) {
     if (cols_direct) sh = gemv_cols_direct_shape(nout, nred_eff, di.sms, uncut);

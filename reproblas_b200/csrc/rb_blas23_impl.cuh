@@ -8,7 +8,8 @@ namespace rb {
 
 template <typename E, bool CX, int F>
 constexpr XOps<E> make_xops() {
-  return XOps<E>{gs::launch_gemv<E, CX, F>, gt::plan_gemm<E, CX, F>, gt::launch_gemm<E, CX, F>};
+  return XOps<E>{gs::gemv_streams<E, CX, F>, gs::launch_gemv<E, CX, F>, gt::plan_gemm<E, CX, F>,
+                 gt::launch_gemm<E, CX, F>};
 }
 
 }  // namespace rb

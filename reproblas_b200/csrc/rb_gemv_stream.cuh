@@ -45,7 +45,7 @@ constexpr int kStages = 3;
 // 266 with, rows kernel); 18 warps leave each thread 96. Their CTA therefore
 // has a whole warpgroup of producers (two warps of it idle), launches at 96 registers a thread
 // and moves 32 from each producer to the four consumer warpgroups: 512 * 104 + 128 * 64 =
-// 640 * 96, all that the launch owns (launch_gemv checks that it was built so).
+// 640 * 96, all that the launch owns (gemv_streams checks that it was built so).
 template <typename E, bool CX>
 __host__ __device__ constexpr bool moves_regs() { return CX && sizeof(E) == 8; }
 template <typename E, bool CX>
@@ -886,9 +886,8 @@ __global__ void __launch_bounds__(256, (rows_direct_ctas<E, CX>(F))) gemv_rows_d
 template <typename E, bool CX>
 __host__ __device__ constexpr bool stream_cols(int fold) { return !(CX && sizeof(E) == 8 && fold > 6); }
 template <typename E, bool CX>
-constexpr bool direct_cols(long long nout, long long nred, int fold) {
+constexpr bool direct_cols(long long nout, long long nred) {
   constexpr int es = (CX ? 2 : 1) * (int)sizeof(E);
-  if (!stream_cols<E, CX>(fold)) return true;
   if (nout >= 80000 && nred <= (es == 16 ? 384 : es == 4 ? 48 : 128)) return true;
   return es == 16 ? nout * nred * es <= (192ll << 20) : nred >= 256 && nout * nred * es <= (16ll << 20);
 }
@@ -1036,6 +1035,38 @@ __global__ void __launch_bounds__(256, (cols_direct_ctas<E, CX>(F))) gemv_cols_d
     xb::finish<E, CX, F>(a, g.mode, g.y + col * g.incy * NC, g.br, g.bi, g.ybin + col * g.incy * 2 * F * NC);
 }
 
+// Whether the streaming kernel of rows (columns) can run on the current device; the first query
+// opts it in to its shared memory there. It cannot where the compiler built it with other than the
+// registers that moves_regs() deals out (its setmaxnreg would wait for ever): the direct kernel serves
+// then.
+template <typename E, bool CX, int F>
+cudaError_t gemv_streams(bool rows, bool* can) {
+  if (!rows && !stream_cols<E, CX>(F)) {
+    *can = false;
+    return cudaSuccess;
+  }
+  constexpr int kMaxDevices = 64;
+  static std::atomic<int> known[kMaxDevices][2];   // 0: not yet, 1: no, 2: yes
+  int dev = 0;
+  cudaError_t e = cudaGetDevice(&dev);
+  if (e != cudaSuccess) return e;
+  int k = dev < kMaxDevices ? known[dev][rows].load(std::memory_order_relaxed) : 0;
+  if (k == 0) {
+    const auto f = rows ? gemv_stream_kernel<E, CX, F, true> : gemv_stream_kernel<E, CX, F, !stream_cols<E, CX>(F)>;
+    k = 2;
+    if constexpr (moves_regs<E, CX>()) {
+      cudaFuncAttributes at;
+      if ((e = cudaFuncGetAttributes(&at, f)) != cudaSuccess) return e;
+      if (at.numRegs != kMoveLaunch) k = 1;
+    }
+    e = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemBytes);
+    if (e != cudaSuccess) return e;
+    if (dev < kMaxDevices) known[dev][rows].store(k, std::memory_order_relaxed);
+  }
+  *can = k == 2;
+  return cudaSuccess;
+}
+
 template <typename E, bool CX, int F>
 cudaError_t launch_gemv(const XGemvArgs<E>& g, const GemvMaps* maps, bool rows, int grid, cudaStream_t s) {
   if (!maps) {
@@ -1046,28 +1077,8 @@ cudaError_t launch_gemv(const XGemvArgs<E>& g, const GemvMaps* maps, bool rows, 
     }
     return cudaGetLastError();
   }
-  constexpr size_t smem = kSmemBytes;
-  // opt in to the shared memory, once per device (the call is idempotent)
-  constexpr int kMaxDevices = 64;
-  static std::atomic<int> ready[kMaxDevices];
-  int dev = 0;
-  cudaError_t e = cudaGetDevice(&dev);
-  if (e != cudaSuccess) return e;
-  if (dev >= kMaxDevices || !ready[dev].load(std::memory_order_relaxed)) {
-    for (auto k : {gemv_stream_kernel<E, CX, F, true>, gemv_stream_kernel<E, CX, F, !stream_cols<E, CX>(F)>}) {
-      e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-      if (e != cudaSuccess) return e;
-      if constexpr (moves_regs<E, CX>()) {
-        cudaFuncAttributes at;
-        e = cudaFuncGetAttributes(&at, k);
-        if (e != cudaSuccess) return e;
-        if (at.numRegs != kMoveLaunch) return cudaErrorLaunchOutOfResources;
-      }
-    }
-    if (dev < kMaxDevices) ready[dev].store(1, std::memory_order_relaxed);
-  }
-  if (rows) gemv_stream_kernel<E, CX, F, true><<<grid, threads<E, CX>(), smem, s>>>(g, *maps);
-  else if constexpr (stream_cols<E, CX>(F)) gemv_stream_kernel<E, CX, F, false><<<grid, threads<E, CX>(), smem, s>>>(g, *maps);
+  if (rows) gemv_stream_kernel<E, CX, F, true><<<grid, threads<E, CX>(), kSmemBytes, s>>>(g, *maps);
+  else if constexpr (stream_cols<E, CX>(F)) gemv_stream_kernel<E, CX, F, false><<<grid, threads<E, CX>(), kSmemBytes, s>>>(g, *maps);
   return cudaGetLastError();
 }
 

@@ -168,6 +168,8 @@ struct GemvMaps {
 
 template <typename E>
 struct XOps {
+  // whether gemv takes maps (the streaming kernel of rows or columns) on the current device
+  cudaError_t (*gemv_streams)(bool rows, bool* can);
   // maps == nullptr: the direct kernels (g.groups, g.parts: their split of a reduction)
   cudaError_t (*gemv)(const XGemvArgs<E>& g, const GemvMaps* maps, bool rows, int grid, cudaStream_t s);
   // decomposition of an M x N x K product (whole_tiles: no tile is cut between CTAs)

@@ -585,3 +585,27 @@ def test_gemv_rows_of_more_than_16_gib(cuda, rb, port, ta):
     got = y[cuda.tensor(at, device="cuda")].cpu().numpy()
     assert same_bits(got.ravel(), want.view(np.float64))
     assert int(cuda.count_nonzero(y)) == np.count_nonzero(want.view(np.float64))
+
+
+@pytest.mark.parametrize("t", list("dszc"))
+@pytest.mark.parametrize("fold", [2, 3, 6])
+def test_gemv_streams_as_built(cuda, rb, t, fold):
+    # the streaming kernels run, not the direct ones that stand in where the compiler gave FP64 complex
+    # other registers than the kernel deals out: only a pipeline can be told to stop feeding its ring
+    n = 4096
+    A, x, y = (cuda.ones(k * 2, dtype=cuda.float64 if t in "dz" else cuda.float32, device="cuda")
+               for k in (n * n, n, n))
+    lib = rb.lib
+    for ta in "nt":
+        try:
+            lib.rb_clear_error()
+            lib.rb_debug_pipeline_fault(2, 20000)
+            if t == "d":
+                rb.call("reproBLAS_rdgemv", fold, "r", ta, n, n, 1.5, A, n, x, 1, 0.0, y, 1)
+            else:
+                rb_gemv(rb, t, fold, "r", ta, n, n, 1.5, A, n, x, 1, 0.0, y, 1)
+            assert lib.rb_synchronize() == 2 and b"timed out" in lib.rb_get_last_error_message(), ta
+        finally:
+            lib.rb_debug_pipeline_fault(-1, 0)
+            lib.rb_clear_error()
+    assert lib.rb_synchronize() == 0
