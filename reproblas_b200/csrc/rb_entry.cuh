@@ -127,7 +127,7 @@ __device__ __forceinline__ void finish(Acc<E, F>* a, int mode, E* yv, E br, E bi
   E yin[NC];
 #pragma unroll
   for (int c = 0; c < NC; c++) yin[c] = E(0);
-  if (mode == kOutValue) {
+  if (mode == kOutValue && !(br == E(0) && (!CX || bi == E(0)))) {   // beta 0 reads nothing
 #pragma unroll
     for (int c = 0; c < NC; c++) yin[c] = yv[c];
   }

@@ -227,31 +227,50 @@ struct Tile {
     }
     return a.cap | (a.idx == 0 ? 1u : 0u);   // caps are multiples of 2^20 (2^23 in FP32)
   }
-  // largest key of each accumulator's products; FINITE: none of them is Inf or NaN, else
-  // only the finite ones count
+  // Largest key of each accumulator's products; FINITE: none of them is Inf or NaN (a float maximum
+  // then does: one three-input instruction for two products), else only the finite ones count.
   template <bool FINITE>
   __device__ __forceinline__ void max_keys(const E* sa, const E* sb, int kend, unsigned (&mk)[NA]) const {
+    // FP64 products of 2^1017 and more, whose high words are a float's NaN, give a key of index 0,
+    // which is theirs
+    float top[NA];
 #pragma unroll
-    for (int e = 0; e < NA; e++) mk[e] = 0u;
+    for (int e = 0; e < NA; e++) {
+      mk[e] = 0u;
+      top[e] = 0.0f;
+    }
 #pragma unroll 1
-    for (int k = 0; k < kend; k++) {
-      E a[TM * NC], b[TN * NC];
-      load_ab(sa, sb, k, a, b);
+    for (int k = 0; k < kend; k += 2) {   // kend is even
+      E a[2][TM * NC], b[2][TN * NC];
+#pragma unroll
+      for (int q = 0; q < 2; q++) load_ab(sa, sb, k + q, a[q], b[q]);
 #pragma unroll
       for (int i = 0; i < TM; i++)
 #pragma unroll
         for (int j = 0; j < TN; j++)
 #pragma unroll
           for (int c = 0; c < NC; c++) {
-            E p[D];
-            prods(a, b, i, j, c, p);
-            const int e = (i * TN + j) * NC + c;
+            E p[2][D];
 #pragma unroll
-            for (int d = 0; d < D; d++) {
-              const unsigned kk = B::key(p[d]);
-              mk[e] = kk > mk[e] && (FINITE || kk < B::kInfKey) ? kk : mk[e];
+            for (int q = 0; q < 2; q++) prods(a[q], b[q], i, j, c, p[q]);
+            const int e = (i * TN + j) * NC + c;
+            if constexpr (FINITE) {
+#pragma unroll
+              for (int d = 0; d < D; d++) top[e] = max_abs3(top[e], key_word(p[0][d]), key_word(p[1][d]));
+            } else {
+#pragma unroll
+              for (int q = 0; q < 2; q++)
+#pragma unroll
+                for (int d = 0; d < D; d++) {
+                  const unsigned kk = B::key(p[q][d]);
+                  mk[e] = kk > mk[e] && kk < B::kInfKey ? kk : mk[e];
+                }
             }
           }
+    }
+    if constexpr (FINITE) {
+#pragma unroll
+      for (int e = 0; e < NA; e++) mk[e] = __float_as_uint(top[e]);
     }
   }
   __device__ __forceinline__ bool prepare(const E* sa, const E* sb, int kend, bool finite,
@@ -261,18 +280,21 @@ struct Tile {
     bool exact = false;
     if (finite) {
       // The index wanted is that of the largest product. Where that of the bound and that of the
-      // largest of the first four products agree, as they nearly always do (an index spans 40
-      // binades, 13 in FP32), it lies between the two and is known.
-      max_keys<true>(sa, sb, 4, mk);
-      exact = true;
+      // largest of the first four products agree, as they nearly always do in FP64 (an index spans 40
+      // binades), it lies between the two and is known. In FP32 (13 binades) some entry of a warp
+      // nearly always needs the whole block.
+      if constexpr (sizeof(E) == 8) {
+        max_keys<true>(sa, sb, 4, mk);
+        exact = true;
 #pragma unroll
-      for (int i = 0; i < TM; i++)
+        for (int i = 0; i < TM; i++)
 #pragma unroll
-        for (int j = 0; j < TN; j++) {
-          const int ib = B::index_of_key(B::key(B::mul(key_ceiling<E>(kra[i]), key_ceiling<E>(kcb[j]))));
+          for (int j = 0; j < TN; j++) {
+            const int ib = B::index_of_key(B::key(B::mul(key_ceiling<E>(kra[i]), key_ceiling<E>(kcb[j]))));
 #pragma unroll
-          for (int c = 0; c < NC; c++) exact = exact && B::index_of_key(mk[(i * TN + j) * NC + c]) == ib;
-        }
+            for (int c = 0; c < NC; c++) exact = exact && B::index_of_key(mk[(i * TN + j) * NC + c]) == ib;
+          }
+      }
       if (!exact) max_keys<true>(sa, sb, kend, mk);
     } else {
       max_keys<false>(sa, sb, kend, mk);

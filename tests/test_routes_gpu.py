@@ -364,6 +364,31 @@ def test_gemm_blocks_off_the_unchecked_path(cuda, rb, port, t, fold):
     assert same_value(Cd.cpu().numpy(), want.view(REAL[t]))
 
 
+@pytest.mark.parametrize("t", list("dszc"))
+@pytest.mark.parametrize("fold", [2, 3, 7, 8])
+def test_gemm_short_sums(cuda, rb, port, t, fold):
+    # sums shorter than a K block, whose entries all take their index from the largest of few products:
+    # magnitudes around the borders between indices, and FP64 products of 2^1017 and more, whose high
+    # words are a float's NaN; beta 0 reads no C
+    for i, (M, N, K) in enumerate([(33, 65, 1), (70, 40, 2), (31, 33, 5), (64, 64, 8), (40, 70, 33)]):
+        A, B = ops(t, M * K, i).reshape(M, K), ops(t, K * N, i + 50).reshape(K, N)
+        e = (np.arange(M) - M // 2) * (24 if t in "dz" else 3)
+        A *= np.exp2(np.clip(e, -500, 510) if t in "dz" else np.clip(e, -60, 62)).astype(REAL[t])[:, None]
+        check_gemm(cuda, rb, port, t, fold, "n", "n", M, N, K, A.ravel(), B.ravel(), i)
+        B[:, 3:9] *= REAL[t](2.0 ** 511 if t in "dz" else 2.0 ** 62)
+        check_gemm(cuda, rb, port, t, fold, "n", "n", M, N, K, A.ravel(), B.ravel(), i)
+        al = scalars(t)[0]
+        want, C = np.zeros(M * N, FULL[t]), dev(cuda, np.full(M * N, np.nan, FULL[t]))
+        Ad, Bd = dev(cuda, A.ravel()), dev(cuda, B.ravel())
+        if t == "d":
+            port.rdgemm(fold, b"r", b"n", b"n", M, N, K, al, ptr(A), K, ptr(B), N, 0.0, ptr(want), N)
+            rb.call("reproBLAS_rdgemm", fold, "r", "n", "n", M, N, K, al, Ad, K, Bd, N, 0.0, C, N)
+        else:
+            lib_gemm(port, t, fold, "r", "n", "n", M, N, K, al, A, K, B, N, 0.0, want, N)
+            rb_gemm(rb, t, fold, "r", "n", "n", M, N, K, al, Ad, K, Bd, N, 0.0, C, N)
+        assert same_value(C.cpu().numpy(), want.view(REAL[t])), (t, fold, M, N, K)
+
+
 def gemv_both(cuda, rb, port, t, fold, ta, M, N, lda, off, incx, seed, dist="normal"):
     """A starting `off` reals into its buffer, against the oracle"""
     al, be = scalars(t)
