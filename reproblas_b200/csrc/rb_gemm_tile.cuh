@@ -673,15 +673,17 @@ cudaError_t resident_ctas(int sms, int* out) {
 }
 
 // Tile shapes per element type and fold: as many accumulators as 128 registers hold beside the
-// operands without spilling. Issue cycles per fold-3 product at 2048^3 (real) / 1024^3
+// operands, without spills at folds 2 and 3 (FP64 complex 1x2 spills 20 bytes at fold 4). Issue cycles
+// per fold-3 product at 2048^3 (real) / 1024^3
 // (complex): FP64 2x2 24.3, 4x2 24.8 (spills); FP32 2x4 14.8, 4x2 15.2, 4x4 15.3 (spills), 2x2
-// 16.5; FP64 complex 1x2 22.7, 1x1 24.2, 2x2 24.5 (spills); FP32 complex 2x2 13.9, 2x4 14.3. Three
+// 16.5; FP64 complex 1x2 22.7, 1x1 24.2, 2x2 24.5 (spills); FP32 complex 2x2 13.9, 2x4 14.3, and at
+// fold 8, 700^3, 2x2 2204 us (596 bytes spilled), 1x2 1481. Three
 // CTAs per SM (80 registers) spill: FP64 2x2 29.7. The small shape serves sizes that fill the
 // large tile badly; `ratio` is its cost per product against the large one's.
 template <typename E, bool CX, int F>
 struct Shapes {
   static constexpr bool f32 = sizeof(E) == 4;
-  static constexpr int TM = CX ? (f32 ? 2 : 1) : f32 ? 2 : (F <= 6 ? 2 : 1);
+  static constexpr int TM = CX ? (f32 && F <= 6 ? 2 : 1) : f32 ? 2 : (F <= 6 ? 2 : 1);
   static constexpr int TN = CX ? (f32 || F <= 5 ? 2 : 1) : f32 ? 4 : 2;
   static constexpr int SM = TM > 1 && TN <= 2 ? TM / 2 : TM, SN = TM > 1 && TN <= 2 ? TN : TN > 1 ? TN / 2 : 1;
   static constexpr double ratio = 1.12;
