@@ -158,6 +158,7 @@ GemvShape gemv_shape(bool rows, long long nout, long long nred, int es, bool cx,
       double ends;
       long long per;   // stages of the busiest CTA
       bool cut;        // some unit is cut between CTAs
+      long long share = 1;   // at most so many
       if (way == 0) {
         s.parts = 0;
         s.grid = (int)(T < sms ? T : sms);
@@ -165,8 +166,8 @@ GemvShape gemv_shape(bool rows, long long nout, long long nred, int es, bool cx,
         s.rem = (int)(T % s.grid);
         per = (T + s.grid - 1) / s.grid;
         cut = s.rem != 0 || s.q % s.nb != 0;
-        // a unit meets at most ceil((nb-1) / q) + 1 ranges
-        ends = s.grid == s.nunits && s.rem == 0 ? 5 : 10 + 0.4 * (double)((s.nb / s.q + 2) / G);
+        share = s.nb / s.q + 2;   // a unit meets at most ceil((nb-1) / q) + 1 ranges
+        ends = s.grid == s.nunits && s.rem == 0 ? 5 : 10 + 0.4 * (double)(share / G);
       } else if (s.nunits <= sms && !uncut) {
         long long p = sms / s.nunits;
         if (p > s.nb) p = s.nb;
@@ -176,6 +177,7 @@ GemvShape gemv_shape(bool rows, long long nout, long long nred, int es, bool cx,
         s.rem = (int)s.nunits;
         per = (s.nb + p - 1) / p;
         cut = p > 1;
+        share = p;
         ends = p == 1 ? 5 : 8 + 0.4 * (double)((p + G - 1) / G);
       } else {
         const long long wu = (s.nunits + sms - 1) / sms;
@@ -188,7 +190,7 @@ GemvShape gemv_shape(bool rows, long long nout, long long nred, int es, bool cx,
         ends = 5;
       }
       s.records = cut ? (size_t)2 * s.grid * P : 0;           // see Ends
-      s.tickets = cut ? (size_t)s.grid * 3 * (gs::kConsumers / 32) : 0;
+      s.tickets = cut && share <= gs::kWide ? (size_t)s.grid * (gs::kConsumers / 32) : 0;   // none: see gemv_sum_parts_kernel
       const double cost = (double)per * stage * m + ends;
       if (best.G == 0 || cost < best_cost) {
         best = s;
@@ -239,11 +241,11 @@ GemvShape gemv_cols_direct_shape(long long nout, long long nred, int sms, bool u
 // 8192x1000 23.0 / 16.5, FP64 complex 8000x131 22.6 / 14.4, but 5000x209 18.5 / 24.7. And few rows of any length, which fill
 // a band of the streaming kernel (64 rows or more) badly: FP64 1x3000000 18.5 / 156, 8x8000000 121 / 391,
 // 48x400000 47.5 / 51.8, FP32 16x500000 26.7 / 28.8 but 32x500000 39.0 / 35.4, FP64 complex 16x500000
-// 58.7 / 94.8 but 32x500000 111 / 107, FP32 complex 48x400000 79.8 / 89.2. And FP64 complex rows from fold 7
-// on, whose accumulators spill in the streaming kernel: fold 7 8192^2 528 / 707, 20000x500 140 / 141, fold
-// 8 8192^2 591 / 768, 300x100000 363 / 403, but fold 8 100000x100 467 / 191.
+// 58.7 / 94.8 but 32x500000 111 / 107, FP32 complex 48x400000 79.8 / 89.2. And FP64 complex rows from fold 6
+// on, whose accumulators spill in the streaming kernel: fold 6 8192^2 479 / 551, fold 7 8192^2 528 / 707,
+// 20000x500 121 / 141, fold 8 8192^2 591 / 768, 300x100000 363 / 403, but fold 8 100000x100 467 / 191.
 bool gemv_rows_direct(long long nout, long long nred, int es, bool cx, int fold) {
-  if (es == 16 && fold > 6 && nred >= 500) return true;
+  if (es == 16 && fold > 5 && nred >= 500) return true;
   const long long bytes = nout * nred * es;
   if (nout > 6144) return nout <= 8192 && bytes <= 8ll << 20;
   return nout <= (es == 8 ? 48 : 24) || bytes <= (es == 8 && !cx ? 48ll << 20 : 32ll << 20);
@@ -394,7 +396,7 @@ bool run_xgemv(const XGemvReq<E, CX>& q) {
   g.rem = sh.rem;
   g.parts = sh.parts;
   g.scratch = (E*)cs.parts;
-  g.tickets = cs.tickets;
+  g.tickets = sh.tickets ? cs.tickets : nullptr;
   g.status = w->dstatus();
   g.groups = sh.G;
   g.phases = phases;
@@ -403,7 +405,7 @@ bool run_xgemv(const XGemvReq<E, CX>& q) {
   const bool direct = rows_direct || cols_direct;
   if (!direct && !gemv_maps(&maps, dA, (size_t)es, Rs, Cs, q.lda, phases, nt, sh.G))
     return false;
-  count_launch();
+  count_launch(sh.records && !sh.tickets ? 2 : 1);
   if (!cuda_ok(o->gemv(g, direct ? nullptr : &maps, nt, sh.grid, s), "gemv launch")) return false;
   if (y_host) {
     int* hs = w->hstatus();

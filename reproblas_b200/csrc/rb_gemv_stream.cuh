@@ -495,11 +495,8 @@ struct Consumer {
 // begins inside (slot 2*cta) and that of the unit that begins in its range and goes on in the next
 // CTA's (slot 2*cta + 1), whatever the number of outputs. Structure of arrays: field i
 // (< NC*(2F+1): pri, car, flags per component) of slot s for the unit's output pp at
-// scratch[(i*2*grid + s)*P + pp]. A unit's parts are summed in groups of kGroup CTAs by the last of
-// each group to arrive, and the groups' sums, left in the records of their first CTAs, by the last of
-// those: with 64 rows of 400,000, which all 148 CTAs share, one CTA would read 148 parts (z: 1 MB).
-// Tickets, one per warp and kind: of the group that begins in a CTA (0, or 1 if the unit begins there
-// too) and of the groups of the unit that begins in it (2).
+// scratch[(i*2*grid + s)*P + pp]. A cut unit's tickets, one per warp, are those of the CTA it
+// begins in. Units that many CTAs share are summed by a kernel of their own (gemv_sum_parts_kernel).
 //
 // A CTA's range of stages holds whole units in its middle and possibly cut units at its two
 // ends. Ends::close() ends the run of unit u in this CTA for the warp's outputs: the groups
@@ -511,7 +508,6 @@ struct Consumer {
 template <typename E, bool CX, int F>
 struct Ends {
   static constexpr int NC = CX ? 2 : 1, REC = 2 * F + 1;
-  static constexpr int kGroup = 12;
   const XGemvArgs<E>& g;
   int P, lgG, grp, pp, out;   // group of this lane, its output's offset in a unit, lanes per group
   long long nout;
@@ -546,7 +542,7 @@ struct Ends {
     }
     if (n == 0) u0 = u;
     else u1 = u;
-    n++;
+    n += g.tickets != nullptr;   // without tickets gemv_sum_parts_kernel sums the parts
   }
   __device__ __forceinline__ void settle(const Split& sp) {
     if (n == 0) return;
@@ -557,8 +553,9 @@ struct Ends {
     bool last = false;
     if (lane < n) {
       const int b = (lane == 0 ? u0 : u1) * g.nb, first = sp.owner(b);
-      const int j = ((int)blockIdx.x - first) / kGroup * kGroup, count = sp.owner(b + g.nb - 1) - first + 1;
-      last = take(first + j, j == 0 ? 1 : 0, warp, count - j < kGroup ? count - j : kGroup);
+      unsigned* t = g.tickets + first * (kConsumers / 32) + warp;
+      last = atomicAdd(t, 1u) == (unsigned)(sp.owner(b + g.nb - 1) - first);
+      if (last) *t = 0u;
     }
     const unsigned mask = __ballot_sync(0xffffffffu, last);
     if (mask == 0) return;
@@ -568,58 +565,27 @@ struct Ends {
       if (!(mask & (1u << k))) continue;
       const int u = k == 0 ? u0 : u1, first = sp.owner(u * g.nb);
       const int count = sp.owner(u * g.nb + g.nb - 1) - first + 1;
-      const int j = ((int)blockIdx.x - first) / kGroup * kGroup;
       const long long o = (long long)u * P + pp;
-      // first the group's parts (CTAs i, i + 1, ...), then the groups' sums (i, i + kGroup, ...)
-      int i = first + j, parts = count - j < kGroup ? count - j : kGroup, step = 1;
-#pragma unroll 1
-      for (;;) {
-        Acc<E, F> a[NC];
+      E y[NC];
+      read_y(o, grp == 0 && o < nout, y);
+      Acc<E, F> a[NC];
 #pragma unroll
-        for (int c = 0; c < NC; c++) {
-          SumAcc<E, F> sum;
-          sum.zero();
-          if (o < nout) {
+      for (int c = 0; c < NC; c++) {
+        SumAcc<E, F> sum;
+        sum.zero();
+        if (o < nout) {
 #pragma unroll 2
-            for (int q = grp; q < parts; q += 1 << lgG) {
-              Acc<E, F> part;
-              xb::read_rec<E, F>(part, g.scratch + slot(i + q * step, i + q == first) + c * REC * fs, fs);
-              sum.add(part);
-            }
+          for (int q = grp; q < count; q += 1 << lgG) {
+            Acc<E, F> part;
+            xb::read_rec<E, F>(part, g.scratch + slot(first + q, q == 0) + c * REC * fs, fs);
+            sum.add(part);
           }
-          sum.get(a[c]);
         }
-        lanes_merge<E, F, NC>(a, out);
-        const bool mine = grp == 0 && o < nout;
-        if (step > 1 || count <= kGroup) {
-          E y[NC];
-          read_y(o, mine, y);
-          if (mine) finish(o, a, y);
-          break;
-        }
-        if (mine) {
-          E* rec = g.scratch + slot(i, i == first);
-#pragma unroll
-          for (int c = 0; c < NC; c++) xb::put_rec<E, F>(a[c], rec + c * REC * fs, fs);
-        }
-        __threadfence();
-        __syncwarp();
-        i = first;
-        parts = (count + kGroup - 1) / kGroup;
-        step = kGroup;
-        bool all = false;
-        if (lane == 0) all = take(first, 2, warp, parts);
-        if (!__ballot_sync(0xffffffffu, all)) break;
-        __threadfence();
+        sum.get(a[c]);
       }
+      lanes_merge<E, F, NC>(a, out);
+      if (grp == 0 && o < nout) finish(o, a, y);
     }
-  }
-  // ticket `kind` of CTA i: true for the last of n to arrive, which leaves it zero
-  __device__ __forceinline__ bool take(int i, int kind, int warp, int n) const {
-    unsigned* t = g.tickets + (3 * i + kind) * (kConsumers / 32) + warp;
-    const bool last = atomicAdd(t, 1u) == (unsigned)n - 1;
-    if (last) *t = 0u;
-    return last;
   }
 };
 
@@ -682,25 +648,30 @@ gemv_stream_kernel(const __grid_constant__ XGemvArgs<E> g, const __grid_constant
     con.zero();
     bool lost = false;
 #pragma unroll 1
-    for (int x = sp.x0; x < sp.x1; x++) {
-      if (stage_ready(sy, r, polls)) {
-        const unsigned char* st = ring + (size_t)r.st * kStageBytes;
-        // elements of this thread that exist; the columns kernel takes a partial last stage
-        // whole (rows outside A arrive as zeros, and so do their x) unless A has fewer rows
-        // than phases
-        const long long k0 = (long long)j * m.SC;
-        const long long rem = ROWS ? m.nred - k0 - grp * PE : (m.nred - k0 - grp + m.G - 1) >> m.lgG;
-        const bool whole = rem >= PE || (!ROWS && m.nred >= 4);
-        const int nval = (long long)u * m.P + pp >= m.nout || rem <= 0 ? 0 : whole ? PE : (int)rem;
-        con.stage(st + off, pl, (const E*)(st + kStageA) + grp * PE * NC, sy.xkey[r.st], nval, conj);
-      } else {
-        lost = true;
+    for (int x = sp.x0; x < sp.x1;) {
+      // the run of unit u in this CTA (a loop of its own: with the run's end inside the stage loop the
+      // compiler lengthens the stage; FP32 complex rows, 8192^2, 164 us against 152)
+      const int xe = sp.x1 - x < g.nb - j ? sp.x1 : x + (g.nb - j);
+#pragma unroll 1
+      for (; x < xe; x++) {
+        if (stage_ready(sy, r, polls)) {
+          const unsigned char* st = ring + (size_t)r.st * kStageBytes;
+          // elements of this thread that exist; the columns kernel takes a partial last stage
+          // whole (rows outside A arrive as zeros, and so do their x) unless A has fewer rows
+          // than phases
+          const long long k0 = (long long)j * m.SC;
+          const long long rem = ROWS ? m.nred - k0 - grp * PE : (m.nred - k0 - grp + m.G - 1) >> m.lgG;
+          const bool whole = rem >= PE || (!ROWS && m.nred >= 4);
+          const int nval = (long long)u * m.P + pp >= m.nout || rem <= 0 ? 0 : whole ? PE : (int)rem;
+          con.stage(st + off, pl, (const E*)(st + kStageA) + grp * PE * NC, sy.xkey[r.st], nval, conj);
+        } else {
+          lost = true;
+        }
+        __syncwarp();
+        if (lane == 0) mbar_arrive(smem_u32(&sy.empty[r.st]));
+        r.next();
+        j++;
       }
-      __syncwarp();
-      if (lane == 0) mbar_arrive(smem_u32(&sy.empty[r.st]));
-      r.next();
-      if (++j < g.nb && x + 1 < sp.x1) continue;
-      // ---- the run of unit u in this CTA ends here ----
 #pragma unroll
       for (int c = 0; c < NC; c++) {
         con.a[c].renorm();
@@ -716,6 +687,69 @@ gemv_stream_kernel(const __grid_constant__ XGemvArgs<E> g, const __grid_constant
   }
   __syncthreads();
   if (tid == 0 && sy.abort_flag) atomicExch(g.status, 2);
+}
+
+// Sum of the parts of cut units, after a streaming kernel that took no tickets: where units are shared
+// by more than kWide CTAs the last of them would sum all their parts alone (FP64 complex, 64 rows of
+// 400,000: 148 parts, 1 MB, 139 us a call against 121 with this launch behind the stream). A CTA takes
+// kSumOutputs outputs of a unit; thread (group, output) sums parts group, group + 32, ...; the groups
+// of a warp meet by shuffles, the warps in shared memory.
+constexpr int kWide = 12, kSumOutputs = 8;
+template <typename E, bool CX, int F, bool ROWS>
+__global__ void __launch_bounds__(256) gemv_sum_parts_kernel(const __grid_constant__ XGemvArgs<E> g, int grid) {
+  constexpr int NC = CX ? 2 : 1, REC = 2 * F + 1;
+  __shared__ E sm[8][kSumOutputs][NC * REC];
+  const Split sp(g);
+  const int P = kConsumers / g.groups, per = P / kSumOutputs;
+  const int u = (int)blockIdx.x / per, t = threadIdx.x % kSumOutputs, warp = threadIdx.x >> 5;
+  const int pp = (int)blockIdx.x % per * kSumOutputs + t, group = threadIdx.x / kSumOutputs;
+  const int first = sp.owner(u * g.nb), count = sp.owner(u * g.nb + g.nb - 1) - first + 1;
+  if (count == 1) return;   // finished by the streaming kernel
+  const long long o = (long long)u * P + pp;
+  const bool some = o < (ROWS ? g.R : g.C);
+  const int fs = 2 * grid * P;
+  Acc<E, F> a[NC];
+#pragma unroll
+  for (int c = 0; c < NC; c++) {
+    SumAcc<E, F> sum;
+    sum.zero();
+    if (some) {
+#pragma unroll 2
+      for (int q = group; q < count; q += 256 / kSumOutputs) {
+        Acc<E, F> part;
+        xb::read_rec<E, F>(part, g.scratch + (2 * (first + q) + (q == 0 ? 1 : 0)) * P + pp + c * REC * fs, fs);
+        sum.add(part);
+      }
+    }
+    sum.get(a[c]);
+  }
+  lanes_merge<E, F, NC>(a, kSumOutputs);
+  if ((threadIdx.x & 31) < kSumOutputs) {
+#pragma unroll
+    for (int c = 0; c < NC; c++) xb::put_rec<E, F>(a[c], &sm[warp][t][c * REC], 1);
+  }
+  __syncthreads();
+  if (threadIdx.x >= kSumOutputs || !some) return;
+#pragma unroll
+  for (int c = 0; c < NC; c++) {
+    SumAcc<E, F> sum;
+    sum.zero();
+#pragma unroll 1
+    for (int w = 0; w < 8; w++) {
+      Acc<E, F> part;
+      part.zero();
+#pragma unroll
+      for (int i = 0; i < F; i++) {
+        part.pri[i] = sm[w][t][c * REC + i];
+        part.car[i] = sm[w][t][c * REC + F + i];
+      }
+      part.flags = xb::flags_from<E>(sm[w][t][c * REC + 2 * F]);
+      part.set_idx_from_pri();
+      sum.add(part);
+    }
+    sum.get(a[c]);
+  }
+  xb::finish<E, CX, F>(a, g.mode, g.y + o * g.incy * NC, g.br, g.bi, g.ybin + o * g.incy * 2 * F * NC);
 }
 
 // ---------------------------------------------------------------------------------------
@@ -1077,8 +1111,16 @@ cudaError_t launch_gemv(const XGemvArgs<E>& g, const GemvMaps* maps, bool rows, 
     }
     return cudaGetLastError();
   }
-  if (rows) gemv_stream_kernel<E, CX, F, true><<<grid, threads<E, CX>(), kSmemBytes, s>>>(g, *maps);
-  else if constexpr (stream_cols<E, CX>(F)) gemv_stream_kernel<E, CX, F, false><<<grid, threads<E, CX>(), kSmemBytes, s>>>(g, *maps);
+  const auto f = rows ? gemv_stream_kernel<E, CX, F, true> : gemv_stream_kernel<E, CX, F, !stream_cols<E, CX>(F)>;
+  f<<<grid, threads<E, CX>(), kSmemBytes, s>>>(g, *maps);
+  cudaError_t e = cudaGetLastError();
+  if (e != cudaSuccess || !g.scratch || g.tickets) return e;
+  // parts without tickets: their sum
+  const long long nout = rows ? g.R : g.C;
+  const int P = kConsumers / g.groups;
+  const unsigned blocks = (unsigned)((nout + P - 1) / P * (P / kSumOutputs));
+  if (rows) gemv_sum_parts_kernel<E, CX, F, true><<<blocks, 256, 0, s>>>(g, grid);
+  else gemv_sum_parts_kernel<E, CX, F, false><<<blocks, 256, 0, s>>>(g, grid);
   return cudaGetLastError();
 }
 

@@ -151,7 +151,7 @@ struct XGemvArgs {
   int nb;                     // stages per unit
   int q, rem, parts;          // split over the CTAs (Split)
   E* scratch;                 // partial states of units cut between CTAs
-  unsigned* tickets;          // of cut units, zero on entry and on exit
+  unsigned* tickets;          // of cut units, zero on entry and on exit (null: a second kernel sums)
   int* status;                // set to 2 when a pipeline wait gives up
   int groups;                 // thread groups per output (2, 4, 8)
   // failure-path test hook (rb_debug_pipeline_fault): each CTA's copy warp issues at most
