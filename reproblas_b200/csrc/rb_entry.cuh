@@ -169,21 +169,5 @@ __device__ __forceinline__ void read_rec(Acc<E, F>& o, const E* rec, long long s
   o.set_idx_from_pri();
 }
 
-// 16-byte read-only load of 16 / sizeof(E) reals (the address is 16-byte aligned).
-template <typename E>
-__device__ __forceinline__ void ld16(const E* p, E (&v)[16 / sizeof(E)]) {
-  if constexpr (sizeof(E) == 8) {
-    const double2 t = __ldg((const double2*)p);
-    v[0] = t.x;
-    v[1] = t.y;
-  } else {
-    const float4 t = __ldg((const float4*)p);
-    v[0] = t.x;
-    v[1] = t.y;
-    v[2] = t.z;
-    v[3] = t.w;
-  }
-}
-
 }  // namespace xb
 }  // namespace rb

@@ -1,5 +1,5 @@
 // rb_ptx.cuh -- small inline-PTX helpers shared by the kernels that stream operands through
-// shared memory: 16-byte cp.async, mbarriers with bounded waits, and the bulk (TMA) copies
+// shared memory: cp.async groups, mbarriers with bounded waits, and the TMA copies
 // that complete on an mbarrier. No form here multicasts.
 #pragma once
 #include <cstdint>
@@ -10,9 +10,6 @@ __device__ __forceinline__ uint32_t smem_u32(const void* p) {
   return (uint32_t)__cvta_generic_to_shared(p);
 }
 
-__device__ __forceinline__ void cp_async16(uint32_t dst, const void* src) {
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
-}
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
 template <int N>
 __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
@@ -74,32 +71,6 @@ __device__ __forceinline__ void tma_load_2d(uint32_t dst, const void* tmap, int 
       :
       : "r"(dst), "l"(tmap), "r"(c0), "r"(c1), "r"(mbar)
       : "memory");
-}
-
-// TMA: 1-D tile load (elements outside the tensor are filled with zeros).
-__device__ __forceinline__ void tma_load_1d(uint32_t dst, const void* tmap, int c0, uint32_t mbar) {
-  asm volatile(
-      "cp.async.bulk.tensor.1d.shared::cluster.global.tile.mbarrier::complete_tx::bytes"
-      " [%0], [%1, {%2}], [%3];"
-      :
-      : "r"(dst), "l"(tmap), "r"(c0), "r"(mbar)
-      : "memory");
-}
-
-// Contiguous bulk copy global -> shared (both addresses 16-byte aligned, bytes a multiple
-// of 16), completion counted on an mbarrier.
-__device__ __forceinline__ void bulk_load(uint32_t dst, const void* src, uint32_t bytes,
-                                          uint32_t mbar) {
-  asm volatile(
-      "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
-      :
-      : "r"(dst), "l"(src), "r"(bytes), "r"(mbar)
-      : "memory");
-}
-
-// Barrier over the first `count` threads of the CTA (a multiple of 32), id 1..15.
-__device__ __forceinline__ void named_sync(int id, int count) {
-  asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(count) : "memory");
 }
 
 }  // namespace rb
