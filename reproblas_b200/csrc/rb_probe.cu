@@ -1,4 +1,4 @@
-// rb_probe.cu -- measurement kernels (no reference counterpart): the FP64 rates that bound the
+// rb_probe.cu -- measurement kernels (no reference counterpart): FP64 rates to set beside the
 // binned dgemm, timed by the caller around rb_probe_launch.
 //
 //   kind 0, FP64 add rate: every thread advances 8 independent chains x <- x + c, so the FP64
